@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(kBlock) apply_ptm_kernel(const __grid_constant
 #pragma unroll
             for (int l = 0; l < NL; ++l) {
               fb |= qsgb_df_suspect(s[l]);
-              acc[l] = df_to_double(s[l], c[l]);
+              acc[l] = qsgb_df_round(s[l], c[l]);
             }
             if (fb) {
               // outside the float-float range: the row again in native FP64

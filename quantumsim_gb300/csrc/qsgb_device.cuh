@@ -24,38 +24,31 @@ __device__ __forceinline__ qsgb_u64 qsgb_fdiv(qsgb_u64 n, qsgb_u64 m, int l) {
   return (t + ((n - t) >> 1)) >> (l - 1);
 }
 
-// Split an IEEE double into hi + lo floats with integer operations only (the
-// FP64<->FP32 converters run on the slow FP64 pipe on GB300).  hi keeps the
-// top 24 significant bits (truncated), lo the next 23 bits rounded to
-// nearest on the 24th, so hi + lo agrees with x to 2^-47 relative, with an
-// error of either sign: a truncated lo would shrink every input by 2^-48 on
-// average, and that bias accumulates linearly over a long circuit (1050
-// applications: ~1e-12 relative) where unbiased errors grow as a square
-// root.  Inputs the float pair cannot carry to that
-// precision set `bad`: a non-zero |x| < 2^-102 (|x| < 2^-126 flushes to 0,
-// [2^-126, 2^-102) keeps only hi) and |x| >= 2^128, inf and nan (which give
-// nan).  Callers recompute the affected results in native FP64.
+// Split an IEEE double into hi + lo floats with integer operations and one
+// I2F (the FP64<->FP32 converters run on the slow FP64 pipe on GB300, I2F at
+// 16 T/s).  hi is x rounded to 24 significant bits (ties away).  The 29 bits
+// below, read as a signed integer, are then exactly x - hi in units of
+// 2^(E-52): I2F rounds them to nearest even and a power of two scales them, so
+// hi + lo agrees with x to 2^-49 of its binade, without bias (a bias would
+// accumulate linearly over a long circuit where unbiased errors grow as a
+// square root), and |lo| <= 2^-24 |hi| keeps the cross terms and the dropped
+// lo * lo small.  Inputs the float pair cannot carry to that precision set
+// `bad`: a non-zero |x| < 2^-102 and |x| >= 2^127, inf and nan; hi and lo are
+// then meaningless, and callers recompute the affected results in native FP64.
 __device__ __forceinline__ void qsgb_split_f64(double x, float& hi, float& lo, unsigned& bad) {
   const unsigned h = (unsigned)__double2hiint(x);
   const unsigned l = (unsigned)__double2loint(x);
-  const unsigned e = (h >> 20) & 0x7ffu;
-  const unsigned sgn = h & 0x80000000u;
   // bits 30..23 <- e[7:0], 22..0 <- m[51:29]; rebias e-1023+127 = e-896,
   // which on the low 8 exponent bits is an xor with 0x80 (bit 30)
   const unsigned t = __funnelshift_l(l, h, 3);
-  const unsigned hb = ((t & 0x7fffffffu) ^ 0x40000000u) | sgn;
-  const unsigned base = (hb & 0xff800000u) - (23u << 23);  // weight of m[28] is 2^(E-24)
-  // m[28:6] rounded on m[5]: 0 .. 2^23, added (not or-ed) to base so that a
-  // carry out of the 23 bits lands in base's exponent (still exact)
-  const unsigned lb = base + ((l >> 6) & 0x7fffffu) + ((l >> 5) & 1u);
-  const float lo_full = __uint_as_float(lb) - __uint_as_float(base);
-  const bool in_range = (e - 897u) <= 253u;  // 897 <= e <= 1150
-  const bool has_lo = e >= 920u;
-  hi = in_range ? __uint_as_float(hb) : (e < 897u ? __uint_as_float(sgn) : __int_as_float(0x7fc00000));
-  lo = (in_range && has_lo) ? lo_full : 0.0f;
-  // e in [921, 1150] is 2^-102 <= |x| < 2^128; e == 0 with a zero
-  // mantissa is an exact zero, carried exactly
-  bad |= ((e - 921u) > 229u && ((h << 1) | l) != 0u) ? 1u : 0u;
+  const unsigned hb = ((t & 0x7fffffffu) | (h & 0x80000000u)) ^ 0x40000000u;
+  // x's sign and 2^(E-24); with the 2^-31 the scale of the integer l << 3
+  const float scale = __uint_as_float((hb & 0xff800000u) - (24u << 23));
+  lo = (__int2float_rn((int)(l << 3)) * 0x1p-31f) * scale;
+  // e in [921, 1149] is 2^-102 <= |x| < 2^127; zero is carried exactly
+  const bool out = h + h - (921u << 21) >= (229u << 21);
+  hi = out ? 0.0f : __uint_as_float(hb + ((l >> 28) & 1u));
+  if (out) bad |= (h + h) | l;
 }
 
 // A float-float row result whose leading float s is outside the range where
@@ -65,30 +58,62 @@ __device__ __forceinline__ void qsgb_split_f64(double x, float& hi, float& lo, u
 // (inputs below 2^-102 are flagged by qsgb_split_f64).  Callers recompute
 // such rows in native FP64.
 __device__ __forceinline__ unsigned qsgb_df_suspect(float s) {
-  const unsigned b = __float_as_uint(s) & 0x7fffffffu;
-  return ((b - 1u) < 0x1c7fffffu || b >= 0x7e800000u) ? 1u : 0u;
+  const float a = fabsf(s);
+  return (!(a < 0x1p126f) || (a < 0x1p-70f && s != 0.0f)) ? 1u : 0u;
 }
 
-// acc (s, c) += (ph + pl) * (xh + xl); pl*xl (2^-48 relative) is dropped.
+// acc (s, c) += (ph + pl) * (xh + xl); pl*xl (2^-49 relative) is dropped.
+// The two-sum of s and the rounded product p is Knuth's; its correction on
+// p's side and the product's rounding error are one fma, ph xh - bp, where bp
+// is what the sum took of p.  The small cross term is added first, so that
+// one rounding only is made at the size of the large one.  10 operations; the
+// product error and the correction apart took 12.  (Letting the fma add s to
+// the exact product as well, 9 operations, loses the low half whenever the
+// signs differ.)  With the split above and qsgb_df_round, on GB300: a fused
+// 13-qubit noisy circuit (44 passes of 3 to 8 terms per row, bound by
+// instruction issue) 10.86 -> 10.00 ms, one layer of a 14-qubit one (near the
+// HBM rate) 14.64 -> 14.40 ms; the RMS error of a row against long double
+// falls by 40 % at 2 and 3 terms, 30 % at 6, 10 to 16 % at 16.
 __device__ __forceinline__ void qsgb_df_fma(float& s, float& c, float ph, float pl, float xh, float xl) {
-  const float p = ph * xh;
-  float e = fmaf(ph, xh, -p);  // exact product error
-  e = fmaf(ph, xl, e);
-  e = fmaf(pl, xh, e);
-  const float s2 = s + p;  // two-sum (Knuth)
+  const float p = __fmul_rn(ph, xh);  // _rn: never contracted with the sum below
+  const float s2 = s + p;
   const float bp = s2 - s;
-  const float err = (s - (s2 - bp)) + (p - bp);
+  float e = fmaf(ph, xh, -bp);
+  e += s - (s2 - bp);
+  e = fmaf(pl, xh, e);
+  e = fmaf(ph, xl, e);
   s = s2;
-  c += err + e;
+  c += e;
 }
 
 // first term of a row: (s, c) = (ph + pl) * (xh + xl)
 __device__ __forceinline__ void qsgb_df_mul(float& s, float& c, float ph, float pl, float xh, float xl) {
-  const float p = ph * xh;
+  const float p = __fmul_rn(ph, xh);
   float e = fmaf(ph, xh, -p);
-  e = fmaf(ph, xl, e);
-  c = fmaf(pl, xh, e);
+  e = fmaf(pl, xh, e);
+  c = fmaf(ph, xl, e);
   s = p;
+}
+
+// Round s + t to the nearest double for a row that qsgb_df_suspect(s) does
+// not flag (a flagged row's value is discarded), with integer operations and
+// one float->int conversion: as qsgb_df_to_double below without its range
+// selects.  The sign of r goes into the scale, so that the correction T is in
+// the magnitude's direction.  Where r is below 2^-76 and unflagged, s is 0
+// and the two-sum is exact (u = 0): the wrapped scale is finite and T is 0.
+__device__ __forceinline__ double qsgb_df_round(float s, float t) {
+  const float r = s + t;  // two-sum: no ordering assumption on |s|, |t|
+  const float bt = r - s;
+  const float u = (s - (r - bt)) + (t - bt);
+  const unsigned rb = __float_as_uint(r);
+  unsigned sc = (306u << 23) - (rb & 0x7f800000u);
+  // a power of two with u toward zero: the next ulp is half as large
+  if ((rb & 0x7fffffu) == 0u && (int)(__float_as_uint(u) ^ rb) < 0) sc += 1u << 23;
+  const int T = __float2int_rn(u * __uint_as_float(sc ^ (rb & 0x80000000u)));  // in ulps of the result
+  unsigned h = ((unsigned)((int)rb >> 3) & 0x8fffffffu) + (896u << 20);
+  if (r == 0.0f) h = 0u;
+  const qsgb_u64 bits = (((qsgb_u64)h << 32) | (qsgb_u64)(rb << 29)) + (qsgb_u64)(qsgb_i64)T;
+  return __longlong_as_double((long long)bits);
 }
 
 // Round s + t (any magnitudes) to the nearest double, with integer

@@ -510,7 +510,7 @@ std::string gen_source(const Spec& s) {
         }
         std::snprintf(buf, sizeof buf, "      fb |= qsgb_df_suspect(s%d);\n", l);
         src += buf;
-        vals[l] = "qsgb_df_to_double(s" + std::to_string(l) + ", c" + std::to_string(l) + ")";
+        vals[l] = "qsgb_df_round(s" + std::to_string(l) + ", c" + std::to_string(l) + ")";
       }
     }
     if (s.pair) {

@@ -86,11 +86,6 @@ struct Hdr {
 };
 static_assert(sizeof(Hdr) == 18 * 8, "header layout");
 constexpr int kMaxCoef = (32764 - (int)sizeof(Hdr)) / 8;
-// Patterns with more terms are left to the generic kernel: they are
-// arithmetic-bound whatever the code, and NVRTC needs 12-65 s for a 2000-term
-// 81x81 pattern (255 registers plus spills), against ~1 s for the sparse
-// PTMs of physical gates (<= 256 terms).
-constexpr int kMaxJitTerms = 1024;
 
 const char* kHdrSrc =
     "struct H { const void* in; void* out; unsigned* status; qsgb_u64 n_items;\n"

@@ -13,6 +13,12 @@ namespace jit {
 
 enum { kModeZero = 0, kModeDP = 1, kModeDF = 2, kModeF32 = 3 };
 
+// Patterns with more terms are left to other kernels (the tensor cores of
+// qsgb_tcw.cu): they are arithmetic-bound whatever the code, and NVRTC needs
+// 12-65 s for a 2000-term 81x81 pattern (255 registers plus spills), against
+// ~1 s for the sparse PTMs of physical gates (<= 256 terms).
+constexpr int kMaxJitTerms = 1024;
+
 // Everything that determines the generated code.
 struct Spec {
   int kin, kout;

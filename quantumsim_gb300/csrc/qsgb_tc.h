@@ -98,5 +98,11 @@ int launch(const double* op, const void* in, void* out, uint64_t X, uint64_t Y, 
 int launch_device(const double* dptm, int layout, const void* in, void* out, uint64_t X, uint64_t Y, uint64_t Z,
                   unsigned* status, cudaStream_t stream);
 
+// Larger dense PTMs (Kin, Kout <= kWideMax) in device memory, FP64 or FP32
+// vectors (qsgb_tcw.cu); dimensions and strides as for launch_device.
+constexpr int kWideMax = 96;
+int launch_wide(const double* dptm, int layout, const void* in, void* out, int dtype, int da_out, int db_out,
+                int da_in, int db_in, uint64_t X, uint64_t Y, uint64_t Z, unsigned* status, cudaStream_t stream);
+
 }  // namespace tc
 }  // namespace qsgb

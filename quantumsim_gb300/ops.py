@@ -222,10 +222,17 @@ def apply_ptm(pv: torch.Tensor, ptm: torch.Tensor, qudits: List[int],
     status = call(ptm, flags)
     if status == L.ERR_UNSUPPORTED and (flags & L.PTM_HOST):
         # no specialised kernel and too large to travel in the launch:
-        # the generic kernel reads it from device memory
-        # (stream-ordered allocator: freeing dev_ptm after the enqueue is
-        # safe for work on this stream)
-        dev_ptm = ptm.to(pv.device)
+        # the wide tensor-core kernel or the generic one reads it from
+        # device memory (stream-ordered allocator: freeing dev_ptm after the
+        # enqueue is safe for work on this stream).  The copy goes through a
+        # page-locked block of torch's host allocator, which keeps it until
+        # the copy is done, so the call does not wait for the stream; during
+        # a capture, whose replays would read that block later, it stays the
+        # synchronous copy that a capture refuses.
+        if torch.cuda.is_current_stream_capturing():
+            dev_ptm = ptm.to(pv.device)
+        else:
+            dev_ptm = ptm.pin_memory().to(pv.device, non_blocking=True)
         if max_terms < 1:
             max_terms = nnz_terms(ptm.numpy(), arith)
         status = call(dev_ptm, flags & ~L.PTM_HOST)

@@ -363,30 +363,35 @@ __global__ void __launch_bounds__(kStage2Entries* kStage2Slices)
 // groups, on mma.sync.m16n8k16 (FP16 operands, FP32 accumulators) with the
 // error-free digit split of the apply kernel (qsgb_tc.h): within a chunk,
 // row r of A = G^T is scaled by its largest exponent over the chunk's 16
-// groups and column k of B = X by its own, each value written as a 57-bit
-// fixed-point integer in six balanced base-1024 FP16 digits.  For every digit
-// pair (i, j) with i + j <= 5 two MMAs (k = 0..7, 8..15) add into level
-// i + j; levels 0..3 are exact FP32 integer sums (below 2^24).  The six levels
-// of each entry are combined in int64, scaled by 2^(E_r + E_k - 2098) and
-// added to FP64 accumulators in chunk order.  Error per chunk: about
-// 2^-47.7 max_g |g_out[g, r]| max_g |x_in[g, k]| over the chunk's groups.
-// A chunk holding inf or nan, or with a result outside the normal double
-// range, is recomputed in native FP64 from global memory.
+// groups and column k of B = X by its own, each value written as a 55-bit
+// fixed-point integer in seven balanced base-256 FP16 digits.  For every digit
+// pair (i, j) with i + j <= 7 two MMAs (n = 0..7, 8..15) add into level
+// i + j; all level sums are exact FP32 integers.  The eight levels of each
+// entry are combined in int64, scaled by 2^(E_r + E_k - kScale8) and added to
+// FP64 accumulators in chunk order.  Error per chunk: below
+// 2^-49 max_g |g_out[g, r]| max_g |x_in[g, k]| over the chunk's groups,
+// typically 2^-54.  A chunk holding inf or nan, values all below
+// 2^-959, or a result outside the normal double range, is recomputed in native
+// FP64 from global memory.
 //
 // A warp takes chunks; lane l = (h, i) = (l / 16, l % 16) loads group i of
 // the chunk, rows r = 8h .. 8h+7 of g_out and k = 8h .. 8h+7 of x_in, and
-// writes their digits into the warp's planes A[d][r][g] and B[d][k][g]
-// (FP16).  The fragments then follow the m16n8k16 layouts: lane
-// (gid, tig) = (l / 4, l % 4) reads A rows gid, gid + 8 at columns 2 tig and
-// 2 tig + 8, B rows (k) nt * 8 + gid, and ends with entries
-// (r, k) = (gid or gid + 8, nt * 8 + 2 tig + {0, 1}).
+// writes each digit of its 8 rows as one 16-byte half row into the warp's
+// planes A[d][g][r] and B[d][g][k] (the half rows of groups 4..7 and 12..15
+// exchanged, so that 8 groups' half rows fall into different banks).  The
+// fragments come back transposed (ldmatrix.trans): lane
+// (gid, tig) = (l / 4, l % 4) ends with entries
+// (r, k) = (gid or gid + 8, nt * 8 + 2 tig + {0, 1}).  Measured on GB300, a
+// gradient with its second stage, against base-1024 digits stored in two bytes
+// each and read by 4-byte loads: 10 qubits (4096 chunks) 21.8 -> 18.1 us, 12
+// qubits 173 -> 140 us.
 constexpr int kTcgBlock = 256;
 constexpr int kTcgWarps = kTcgBlock / 32;
-constexpr int kTcgPlane = 16 * 16;  // halves per digit plane
+constexpr int kTcgPlane = 16 * 16 * 2;  // bytes per digit plane
 
 struct TcgWarpSmem {
-  unsigned short a[tc::kDigits][kTcgPlane];  // digits of g_out: [r][g]
-  unsigned short b[tc::kDigits][kTcgPlane];  // digits of x_in: [k][g]
+  unsigned char a[tc::kPlanes * kTcgPlane];  // digits of g_out: [g][r]
+  unsigned char b[tc::kPlanes * kTcgPlane];  // digits of x_in: [g][k]
   int er[16], ek[16];                        // chunk exponents of rows, columns
 };
 struct TcgSmem {
@@ -394,8 +399,11 @@ struct TcgSmem {
   int64_t oin[16], oout[16];  // row offsets of x_in and g_out
 };
 
-__device__ __forceinline__ unsigned ld_pair(const unsigned short* plane, int row, int col) {
-  return *reinterpret_cast<const unsigned*>(plane + row * 16 + col);
+__device__ __forceinline__ void ldmatrix4_trans(unsigned (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
 }
 
 __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_constant__ GradParams p,
@@ -416,6 +424,13 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
     sm.oout[k] = ra * p.sao + rb * p.sbo;
   }
   __syncthreads();
+  // byte offset of half row c of group g in a plane
+  auto half_row = [](int g, int c) { return g * 32 + ((c ^ ((g >> 2) & 1)) << 4); };
+  // ldmatrix source rows: A tiles (g 0-7 | r 0-7), (0-7 | 8-15), (8-15 | 0-7), (8-15 | 8-15);
+  // B tiles (g 0-7 | k 0-7), (8-15 | 0-7), (0-7 | 8-15), (8-15 | 8-15)
+  const int lr = lane & 7, t1b = (lane >> 3) & 1, t2b = lane >> 4;
+  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(ws.a) + half_row(lr + 8 * t2b, t1b);
+  const uint32_t sb = (uint32_t)__cvta_generic_to_shared(ws.b) + half_row(lr + 8 * t1b, t2b);
   auto bases = [&](uint64_t g, int64_t& bi, int64_t& bo) {
     const uint64_t t1 = fdiv(g, p.div_z);
     const uint64_t z = g - t1 * p.div_z.d;
@@ -448,75 +463,76 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
 #pragma unroll
       for (int j = 0; j < 8; ++j) gv[j] = xv[j] = 0.0;
     }
-    // chunk exponents of rows 8h+j (g_out) and columns 8h+j (x_in): maxima
-    // over the 16 lanes of this half
-    unsigned eg[8], ex[8], nonfinite = 0;
+    // chunk exponents of rows 8h+j (g_out, low half word) and columns 8h+j
+    // (x_in, high half word): maxima over the 16 lanes of this half
+    unsigned e2[8], nonfinite = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const unsigned hg = (unsigned)__double2hiint(gv[j]), hx = (unsigned)__double2hiint(xv[j]);
-      nonfinite |= (((hg >> 20) & 0x7ffu) == 0x7ffu || ((hx >> 20) & 0x7ffu) == 0x7ffu) ? 1u : 0u;
-      eg[j] = tc::exp_eff(hg);
-      ex[j] = tc::exp_eff(hx);
+      e2[j] = ((hg >> 20) & 0x7ffu) | ((hx >> 4) & 0x7ff0000u);
+    }
 #pragma unroll
-      for (int o = 1; o < 16; o <<= 1) {
-        eg[j] = max(eg[j], __shfl_xor_sync(0xffffffffu, eg[j], o));
-        ex[j] = max(ex[j], __shfl_xor_sync(0xffffffffu, ex[j], o));
+    for (int o = 1; o < 16; o <<= 1)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) e2[j] = __vmaxu2(e2[j], __shfl_xor_sync(0xffffffffu, e2[j], o));
+    {
+      unsigned top = 0u, low = 0xffffffffu;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        top = __vmaxu2(top, e2[j]);
+        low = __vminu2(low, e2[j]);
+      }
+      nonfinite = ((top & 0xffffu) == 0x7ffu || (top >> 16) == 0x7ffu) ? 1u : 0u;
+      if ((low & 0xffffu) < tc::kMinExp || (low >> 16) < tc::kMinExp) {
+        // a row or column that is all zero (exact) or below the smallest scale
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if ((e2[j] & 0xffffu) < tc::kMinExp && gv[j] != 0.0) nonfinite = 1u;
+          if ((e2[j] >> 16) < tc::kMinExp && xv[j] != 0.0) nonfinite = 1u;
+          // any scale serves zeros
+          if ((e2[j] & 0xffffu) < tc::kMinExp) e2[j] = (e2[j] & 0xffff0000u) | 1023u;
+          if ((e2[j] >> 16) < tc::kMinExp) e2[j] = (e2[j] & 0xffffu) | (1023u << 16);
+        }
       }
     }
     if (i == 0) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        ws.er[8 * h + j] = (int)eg[j];
-        ws.ek[8 * h + j] = (int)ex[j];
+        ws.er[8 * h + j] = (int)(e2[j] & 0xffffu);
+        ws.ek[8 * h + j] = (int)(e2[j] >> 16);
       }
     }
-    // digits: low half of each pair the g_out digit, high half the x_in one
+    {
+      unsigned eh[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const unsigned long long ug =
-          tc::fixed_biased((unsigned)__double2hiint(gv[j]), (unsigned)__double2loint(gv[j]), eg[j]);
-      const unsigned long long ux =
-          tc::fixed_biased((unsigned)__double2hiint(xv[j]), (unsigned)__double2loint(xv[j]), ex[j]);
+      for (int j = 0; j < 8; ++j) eh[j] = (e2[j] & 0xffffu) << 20;
+      tc::split8<kTcgPlane>(ws.a + half_row(i, h), gv, eh);
 #pragma unroll
-      for (int d = 0; d < tc::kDigits; ++d) {
-        const unsigned pr = tc::digit_pair(ug, ux, 10 * (tc::kDigits - 1 - d));
-        ws.a[d][(8 * h + j) * 16 + i] = (unsigned short)(pr & 0xffffu);
-        ws.b[d][(8 * h + j) * 16 + i] = (unsigned short)(pr >> 16);
-      }
+      for (int j = 0; j < 8; ++j) eh[j] = (e2[j] & 0xffff0000u) << 4;
+      tc::split8<kTcgPlane>(ws.b + half_row(i, h), xv, eh);
     }
     const bool chunk_bad = __any_sync(0xffffffffu, nonfinite != 0u);
     __syncwarp();
-    long long v[2][4];
+    unsigned fa[tc::kPlanes][4], fb[tc::kPlanes][4];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[nt][q] = 0;
-#pragma unroll
-    for (int L = 0; L < tc::kDigits; ++L) {
-      float dl[2][4];
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dl[nt][q] = 0.f;
-#pragma unroll
-      for (int a = 0; a <= L; ++a) {
-        const unsigned fa[4] = {ld_pair(ws.a[a], gid, 2 * tig), ld_pair(ws.a[a], gid + 8, 2 * tig),
-                                ld_pair(ws.a[a], gid, 2 * tig + 8), ld_pair(ws.a[a], gid + 8, 2 * tig + 8)};
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          const unsigned fbv[2] = {ld_pair(ws.b[L - a], nt * 8 + gid, 2 * tig),
-                                   ld_pair(ws.b[L - a], nt * 8 + gid, 2 * tig + 8)};
-          tc::mma16816(dl[nt], fa, fbv);
-        }
-      }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const long long t = (long long)__float2int_rn(dl[nt][q]);
-          v[nt][q] += L < 5 ? (t << (10 * (4 - L))) : (t >> 10);
-        }
+    for (int d = 0; d < tc::kPlanes; ++d) {
+      ldmatrix4_trans(fa[d], sa + d * kTcgPlane);
+      ldmatrix4_trans(fb[d], sb + d * kTcgPlane);
     }
+    int pr[2][4][tc::kLevels / 2];  // two levels each
+#pragma unroll
+    for (int L = 0; L < tc::kLevels; L += 2)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int a = 0; a < tc::kPlanes; ++a) {
+          if (L - a >= 0 && L - a < tc::kPlanes) tc::mma16816(d[0], fa[a], fb[L - a] + 2 * nt);
+          if (L + 1 - a >= 0 && L + 1 - a < tc::kPlanes) tc::mma16816(d[1], fa[a], fb[L + 1 - a] + 2 * nt);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) pr[nt][q][L / 2] = tc::level_pair(d[0][q], d[1][q]);
+      }
     // scale and accumulate (in FP64 from global memory when the chunk or a
     // result is out of range)
     double y[2][4];
@@ -526,17 +542,10 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int r = gid + (q >= 2 ? 8 : 0), k = nt * 8 + 2 * tig + (q & 1);
-        const int sc = (ws.er[r] - 1022) + (ws.ek[k] - 1022) - 54;
-        const long long vv = v[nt][q];
-        double d = 0.0;
-        if (vv != 0) {
-          d = __ll2double_rn(vv);
-          const int hi = __double2hiint(d);
-          const int e = ((hi >> 20) & 0x7ff) + sc;
-          bad |= (e < 1 || e > 2046) ? 1u : 0u;
-          d = __hiloint2double(hi + (sc << 20), __double2loint(d));
-        }
-        y[nt][q] = d;
+        const int sc = ws.er[r] + ws.ek[k] - tc::kScale8;
+        bad |= tc::scale8_ok(sc) ? 0u : 1u;
+        y[nt][q] = tc::scale8(tc::combine8(pr[nt][q][0], pr[nt][q][1], pr[nt][q][2], pr[nt][q][3]),
+                              (unsigned)sc << 20);
       }
     if (chunk_bad || __any_sync(0xffffffffu, bad != 0u)) {
 #pragma unroll

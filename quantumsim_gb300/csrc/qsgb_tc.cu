@@ -3,47 +3,45 @@
 // A dense PTM row has 16 terms: in float-float on the FP32 pipes that is
 // ~12 instructions per term, and the kernel is bound by instruction issue at
 // a quarter of the HBM rate; in native FP64 it is bound by the FP64 pipe
-// (~0.6 T FMA/s on GB300).  This kernel computes the contraction exactly
+// (~0.6 T FMA/s on GB300).  These kernels compute the contraction exactly
 // enough for FP64 parity on the FP16 tensor cores instead, with an
 // error-free splitting in the spirit of the Ozaki scheme (Ozaki, Ogita,
 // Oishi and Rump, "Error-free transformations of matrix multiplication by
 // using fast routines of matrix multiplication and its applications",
 // Numer. Algorithms 59, 2012):
 //
-//  * Each group of 16 inputs (one bystander index) is scaled by its largest
-//    binary exponent and written as a signed fixed-point integer F of 57
-//    bits plus sign (|F| < 2^57), with integer operations on the double's
-//    bit pattern.  F + B, for B = 512 * sum_j 2^(10 j), is a non-negative
-//    60-bit integer whose six base-1024 digits v_j give F = sum_j (v_j - 512)
-//    2^(10 (5 - j)): six balanced digits d_j in [-512, 512), each exactly an
-//    FP16 number (|d_0| <= 128).
-//  * Each PTM row is split the same way on the host (per-row scale).
-//  * For every pair of digit planes (i, j) with i + j <= 5 one
-//    mma.sync.m16n8k16 (FP16 operands, FP32 accumulation) adds
-//    sum_k e_ik d_jk to the accumulator of level L = i + j.  A product of two
-//    digits is at most 2^18, a pair's K = 16 sum at most 2^22, and a level
-//    holds at most four such sums below 2^24, where FP32 sums of integers
-//    are exact; levels 4 and 5 may round their last bit, 2^-40 below level 0.
-//  * The six level sums are combined in 64-bit integer arithmetic,
-//    V = sum_L A_L 2^(10 (4 - L)), converted to double once and scaled by
-//    2^(Ex + Ep_r - 54) on the exponent field.
+//  * Each group of 16 inputs (one bystander index) and each PTM row is scaled
+//    by its largest binary exponent and written as fixed-point integers, with
+//    integer operations on the double's bit pattern, in balanced digits that
+//    are exact FP16 numbers.
+//  * For pairs of digit planes (i, j) up to a last level the tensor cores add
+//    sum_k e_ik d_jk to the FP32 accumulator of level L = i + j.
+//  * The level sums are combined in 64-bit integer arithmetic, converted to
+//    double once and scaled on the exponent field.
 //
-// The dropped levels (i + j >= 6) and the 57-bit truncation of inputs and
-// PTM entries bound the error by about 2^-47.7 * max_k |P_rk| * max_k |x_k|
-// of the row and group (4.4e-15 of that product), against 16 * 2^-53 *
-// sum_k |P_rk| |x_k| for an FP64 dot product.  Groups whose inputs hold inf,
-// nan, or whose results leave the normal double range are recomputed in
-// native FP64 by the same warp.
+// The tcgen05 kernel (the second half of this file, used by default) has
+// seven base-256 digits and levels 0 .. 7, all exact integer sums; the digits
+// and their error are described in qsgb_tc.h.  The warp-level kernel that
+// follows here (QSGB_TC_KERNEL=mma_sync) has six base-1024 digits of a 57-bit
+// F: with B = 512 * sum_j 2^(10 j), F + B is a non-negative 60-bit integer
+// whose digits v_j give d_j = v_j - 512; a product of two is at most 2^18, a
+// K = 16 sum at most 2^22, levels 0 .. 3 are exact and 4 and 5 may round their
+// last bit, 2^-40 below level 0.  Its error is about 2^-47.7 * max_k |P_rk| *
+// max_k |x_k| of the row and group, the tcgen05 kernel's below 2^-49 of it
+// (typically 2^-54), against 16 * 2^-53 * sum_k |P_rk| |x_k| for an FP64
+// dot product.  Groups whose inputs hold inf or nan, or whose results leave
+// the normal double range, are recomputed in native FP64.
 //
-// Work mapping: a warp takes tiles of 8 groups (the N of the MMA).  Lane
-// (g, c) = (lane / 4, lane % 4) loads inputs k in {2c, 2c+1, 2c+8, 2c+9} of
-// group g (the B fragment layout of m16n8k16), and ends with outputs rows
+// Warp-level work mapping: a warp takes tiles of 8 groups (the N of the MMA).
+// Lane (g, c) = (lane / 4, lane % 4) loads inputs k in {2c, 2c+1, 2c+8, 2c+9}
+// of group g (the B fragment layout of m16n8k16), and ends with outputs rows
 // {g, g+8} of groups {2c, 2c+1} (the accumulator layout).  The PTM digit
 // planes (the A fragments) are loaded into registers once per warp.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "qsgb_common.cuh"
 #include "qsgb_tc.h"
@@ -73,7 +71,7 @@ __device__ __forceinline__ double combine(const float (&acc)[kDigits][4], int s,
 }
 
 template <bool CONTIG>
-__global__ void __launch_bounds__(kBlock) apply16_tc_kernel(const __grid_constant__ TcParams p) {
+__global__ void __launch_bounds__(kBlock) apply16_tc_kernel(const __grid_constant__ TcWarpParams p) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, c = lane & 3;
   const int warps = kBlock / 32;
@@ -209,34 +207,46 @@ __global__ void __launch_bounds__(kBlock) apply16_tc_kernel(const __grid_constan
 
 // ---------------------------------------------------------------------------
 // tcgen05 form: one thread per group, 128 groups per tile (the M of one
-// tcgen05.mma), the six level accumulators in tensor memory.
+// tcgen05.mma), the eight level accumulators in tensor memory.
 //
-// Per tile, each thread loads its group's 16 inputs, splits them and writes
-// its row of the six input digit planes (the A operand, 128 x 16 FP16 each)
-// to shared memory; one thread issues the 21 tcgen05.mma.kind::f16 (A = input
-// plane j, B = PTM plane i, both K-major, D = level i + j: 16 FP32 columns of
-// tensor memory) and commits them to an mbarrier; after the barrier each warp
-// reads its 32 lanes (groups) of the accumulators with tcgen05.ld and
-// recombines its outputs.  Shared-memory operands use the canonical K-major
-// layout without swizzling: core matrices of 8 rows x 16 bytes (8 FP16 along
-// K) at (row / 8) * 256 + (k / 8) * 128, so the descriptors carry a leading
-// (K) byte offset of 128 and a stride (8-row) byte offset of 256.
+// Per tile, each thread splits its group's 16 inputs and writes its row of the
+// seven input digit planes (the A operand, 128 x 16 FP16 each) to shared
+// memory; then it loads its inputs of the next tile.  One thread issues seven
+// tcgen05.mma.kind::f16, one per input plane j: the B operand is PTM planes
+// 0 .. 7 - j stacked along N (plane 7 is zero), and since level i + j is
+// accumulator column block i + j, their levels are adjacent columns.  One MMA
+// per pair of planes (34 of N = 16) read the input planes five times as often
+// from shared memory.  After the commit's mbarrier each warp reads its 32
+// lanes (groups) of the accumulators with tcgen05.ld and recombines its
+// outputs.  Shared-memory operands use the canonical K-major layout without
+// swizzling: core matrices of 8 rows x 16 bytes (8 FP16 along K) at
+// (row / 8) * 256 + (k / 8) * 128, so the descriptors carry a leading (K) byte
+// offset of 128 and a stride (8-row) byte offset of 256.
+//
+// What bounds it: the serial chain of a tile (load, split, barrier, MMAs,
+// recombination, ~85 instructions per element) over the 4 blocks of an SM that
+// tensor memory allows; issue is about half busy, the FP64 pipe a third (one
+// conversion per output).  Measured on GB300, dense PTMs, us (start of this
+// design: base-1024 digits, 21 MMAs, two barriers a tile): 13 qubits 349 ->
+// 263 (3.07 -> 4.08 TB/s), 12 qubits 92.7 -> 71.4, 10 qubits 14.3 -> 10.2,
+// last two of 12 qubits 103.8 -> 75.1.  Of the 21 us at 12 qubits, byte digits
+// and fewer selects gave 11, the stacked MMAs 10.  Two threads a group (256
+// threads a block) measured 74.6 at 12 qubits.
 constexpr int kUBlock = 128;
 constexpr int kPlaneA = 128 * 16 * 2;  // one input digit plane: 128 rows x 16 FP16
 constexpr int kPlaneB = 16 * 16 * 2;   // one PTM digit plane: 16 rows x 16 FP16
-constexpr int kSmemB = kDigits * kPlaneA;             // 24576
-constexpr int kSmemBar = kSmemB + kDigits * kPlaneB;  // 27648
+constexpr int kSmemB = kPlanes * kPlaneA;             // 28672
+constexpr int kSmemBar = kSmemB + kLevels * kPlaneB;  // 32768: the PTM's planes and one of zeros
 constexpr int kSmemTmem = kSmemBar + 8;
-constexpr int kSmemFlag = kSmemTmem + 4;
 constexpr int kSmemRowExp = kSmemBar + 32;  // int[16] (device PTMs)
 static_assert(kSmemRowExp % 16 == 0 && kSmemRowExp + 64 <= 56 * 1024, "shared-memory layout");
 // the dynamic allocation is padded so that at most 4 blocks share an SM:
 // 4 x 128 tensor-memory columns fill its 512
 constexpr int kUmmaSmem = 56 * 1024;
-constexpr unsigned kTmemCols = 128;  // 6 levels x 16 columns, a power of two
+constexpr unsigned kTmemCols = 16 * kLevels;  // 128, a power of two
 // kind::f16 instruction descriptor: D F32 (bits 4-5 = 1), A and B F16 (0),
-// both K-major, N / 8 at bits 17-22, M / 16 at bits 24-28
-constexpr uint32_t kIdesc = (1u << 4) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
+// both K-major, M / 16 at bits 24-28; N / 8 (bits 17-22) is added
+constexpr uint32_t kIdesc0 = (1u << 4) | ((128u >> 4) << 24);
 constexpr long long kSpinLimit = 1ll << 26;
 
 __host__ __device__ constexpr int core_off(int row, int k) {
@@ -258,22 +268,6 @@ __device__ __forceinline__ uint32_t tmem_ld4(uint32_t addr, uint32_t (&r)[4]) {
   return 0;
 }
 
-// 2^sc * sum_L A_L 2^(10 (4 - L)) from the raw FP32 words of the six levels
-__device__ __forceinline__ double combine_words(const uint32_t (&w)[kDigits], int sc, unsigned& bad) {
-  long long v = (long long)__float2int_rn(__uint_as_float(w[0])) << 40;
-  v += (long long)__float2int_rn(__uint_as_float(w[1])) << 30;
-  v += (long long)__float2int_rn(__uint_as_float(w[2])) << 20;
-  v += (long long)__float2int_rn(__uint_as_float(w[3])) << 10;
-  v += (long long)__float2int_rn(__uint_as_float(w[4]));
-  v += (long long)(__float2int_rn(__uint_as_float(w[5])) >> 10);
-  if (v == 0) return 0.0;
-  const double d = __ll2double_rn(v);
-  const int hi = __double2hiint(d);
-  const int e = ((hi >> 20) & 0x7ff) + sc;
-  bad |= (e < 1 || e > 2046) ? 1u : 0u;
-  return __hiloint2double(hi + (sc << 20), __double2loint(d));
-}
-
 // Offset of op element (r, k) in a 16 x 16 two-qubit PTM stored in `layout`.
 __device__ __forceinline__ int dev_index(int layout, int r, int k) {
   const int ra = r >> 2, rb = r & 3, ka = k >> 2, kb = k & 3;
@@ -289,9 +283,11 @@ __device__ __forceinline__ int dev_index(int layout, int r, int k) {
   }
 }
 
-// DEVP: the PTM is in device memory (p.dptm); threads 0..15 split one row
-// each into the B operand planes (the fixed point and digits of the host
-// split) and the row scales, in shared memory.
+// DEVP: the PTM is in device memory (p.dptm), else in the parameters (p.ptm).
+// Every block splits it into the B operand planes and the row scales, in
+// shared memory: that costs less than carrying the planes in the parameters
+// (3.5 KB more a launch, read back with divergent constant loads: 11.9 against
+// 10.2 us on 10 qubits) and leaves the host nothing to split.
 template <bool CONTIG, bool DEVP>
 __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_constant__ TcParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -299,7 +295,6 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   const uint32_t sA = sbase, sB = sbase + kSmemB, bar = sbase + kSmemBar;
   volatile uint32_t* tslot = reinterpret_cast<volatile uint32_t*>(smem + kSmemTmem);
-  volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + kSmemFlag);
   const int64_t sai = p.sai, sbi = p.sbi;
 
   auto base = [&](uint64_t grp) -> int64_t {
@@ -311,7 +306,9 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
   };
 
   // a tile's inputs: this thread's group, 16 values; with unit stride along
-  // the last target (Z == 1, tensors 16-byte aligned) as 8 16-byte loads
+  // the last target (Z == 1, tensors 32-byte aligned) as 4 32-byte loads: lanes
+  // are 128 bytes apart there, and each access costs one sector a lane
+  // (last two of 12 qubits: 95.3 against 75.1 us with 16-byte accesses)
   auto load_tile = [&](uint64_t tile, double (&x)[16], int64_t& b, bool& live) {
     const uint64_t gi = tile * kUBlock + t;
     live = tile < p.n_tiles && gi < p.n_groups;
@@ -326,14 +323,10 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
       for (int k = 0; k < 16; ++k) x[k] = 0.0;
     } else if (p.vec_z1) {
 #pragma unroll
-      for (int ka = 0; ka < 4; ++ka) {
-        const double2 v0 = *reinterpret_cast<const double2*>(p.in + b + ka * sai);
-        const double2 v1 = *reinterpret_cast<const double2*>(p.in + b + ka * sai + 2);
-        x[4 * ka] = v0.x;
-        x[4 * ka + 1] = v0.y;
-        x[4 * ka + 2] = v1.x;
-        x[4 * ka + 3] = v1.y;
-      }
+      for (int ka = 0; ka < 4; ++ka)
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(x[4 * ka]), "=d"(x[4 * ka + 1]), "=d"(x[4 * ka + 2]), "=d"(x[4 * ka + 3])
+                     : "l"(p.in + b + ka * sai));
     } else {
 #pragma unroll
       for (int k = 0; k < 16; ++k) x[k] = p.in[b + (k >> 2) * sai + (k & 3) * sbi];
@@ -348,30 +341,34 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
   uint64_t tile = blockIdx.x;
   load_tile(tile, x, b, live);  // in flight during the set-up below
   int* srow = reinterpret_cast<int*>(smem + kSmemRowExp);
-  int ptm_bad = 0;  // device PTM with inf or nan entries (this thread's pair)
-  if (DEVP) {
+  int ptm_bad = 0;  // inf or nan entries, or a row too small to scale by (this thread's pair)
+  {
     // 8 threads per row (lanes 8r' .. 8r'+7 of a warp), two entries each
     const int r = t >> 3, k = 2 * (t & 7);
-    const double v0 = p.dptm[dev_index(p.dlayout, r, k)];
-    const double v1 = p.dptm[dev_index(p.dlayout, r, k + 1)];
+    const double v0 = DEVP ? p.dptm[dev_index(p.dlayout, r, k)] : p.ptm[r][k];
+    const double v1 = DEVP ? p.dptm[dev_index(p.dlayout, r, k + 1)] : p.ptm[r][k + 1];
     const unsigned h0 = (unsigned)__double2hiint(v0), h1 = (unsigned)__double2hiint(v1);
-    unsigned emax = max(exp_eff(h0), exp_eff(h1));
+    unsigned emax = max((h0 >> 20) & 0x7ffu, (h1 >> 20) & 0x7ffu);
     emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 1));
     emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 2));
     emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 4));
-    ptm_bad = (((h0 >> 20) & 0x7ffu) == 0x7ffu || ((h1 >> 20) & 0x7ffu) == 0x7ffu) ? 1 : 0;
-    const unsigned long long u0 = fixed_biased(h0, (unsigned)__double2loint(v0), emax);
-    const unsigned long long u1 = fixed_biased(h1, (unsigned)__double2loint(v1), emax);
-#pragma unroll
-    for (int j = 0; j < kDigits; ++j)
-      *reinterpret_cast<unsigned*>(smem + kSmemB + j * kPlaneB + core_off(r, k)) =
-          digit_pair(u0, u1, 10 * (kDigits - 1 - j));
-    if ((t & 7) == 0) srow[r] = (int)emax - 1022 - 54;
-  } else {  // PTM digit planes (the B operand), split on the host
-    const uint4* src = reinterpret_cast<const uint4*>(&p.bplanes[0][0]);
-    uint4* dst = reinterpret_cast<uint4*>(smem + kSmemB);
-    for (int i = t; i < kDigits * kPlaneB / 16; i += kUBlock) dst[i] = src[i];
+    // inf, nan, or a non-zero row below the smallest scale
+    ptm_bad = (emax == 0x7ffu || (emax < kMinExp && (v0 != 0.0 || v1 != 0.0))) ? 1 : 0;
+    if (emax < kMinExp) emax = 1023u;  // any scale serves a row of zeros
+    const unsigned long long u0 = fixed8(h0, (unsigned)__double2loint(v0), emax << 20);
+    const unsigned long long u1 = fixed8(h1, (unsigned)__double2loint(v1), emax << 20);
+    const Signs sg = signs_of(h0, h1);
+    unsigned char* dst = smem + kSmemB + core_off(r, k);
+    *reinterpret_cast<unsigned*>(dst + 0 * kPlaneB) = digit8_pair<0>(u0, u1, sg);
+    *reinterpret_cast<unsigned*>(dst + 1 * kPlaneB) = digit8_pair<1>(u0, u1, sg);
+    *reinterpret_cast<unsigned*>(dst + 2 * kPlaneB) = digit8_pair<2>(u0, u1, sg);
+    *reinterpret_cast<unsigned*>(dst + 3 * kPlaneB) = digit8_pair<3>(u0, u1, sg);
+    *reinterpret_cast<unsigned*>(dst + 4 * kPlaneB) = digit8_pair<4>(u0, u1, sg);
+    *reinterpret_cast<unsigned*>(dst + 5 * kPlaneB) = digit8_pair<5>(u0, u1, sg);
+    *reinterpret_cast<unsigned*>(dst + 6 * kPlaneB) = digit8_pair<6>(u0, u1, sg);
+    if ((t & 7) == 0) srow[r] = (int)emax - kScale8;
   }
+  if (t < kPlaneB / 16) *reinterpret_cast<uint4*>(smem + kSmemB + kPlanes * kPlaneB + 16 * t) = make_uint4(0, 0, 0, 0);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + kSmemTmem),
                  "r"(kTmemCols)
@@ -388,100 +385,98 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tslot;
   const uint32_t tlane = tmem + ((uint32_t)(32 * warp) << 16);
+  int rmin = srow[0], rmax = srow[0];  // row scales, least and greatest
+#pragma unroll
+  for (int r = 1; r < 16; ++r) {
+    rmin = min(rmin, srow[r]);
+    rmax = max(rmax, srow[r]);
+  }
+  bool done = true;  // this thread saw the last tile's MMAs complete
   for (; tile < p.n_tiles; tile += gridDim.x) {
-    unsigned emax = 1u, bad = ptm_bad ? 1u : 0u;
+    unsigned eh = 0u;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const unsigned h = (unsigned)__double2hiint(x[k]);
-      emax = max(emax, exp_eff(h));
-      bad |= ((h >> 20) & 0x7ffu) == 0x7ffu ? 1u : 0u;
+    for (int k = 0; k < 16; ++k) eh = max(eh, (unsigned)__double2hiint(x[k]) & 0x7ff00000u);
+    unsigned emax = eh >> 20;
+    unsigned bad = (ptm_bad || emax == 0x7ffu) ? 1u : 0u;  // inf, nan
+    if (emax < kMinExp) {  // all zero, or all below the smallest scale
+#pragma unroll
+      for (int k = 0; k < 16; ++k) bad |= x[k] != 0.0 ? 1u : 0u;
+      emax = 1023u;  // any scale serves zeros
     }
-    {
-      unsigned long long u[16];
+    bad |= (scale8_ok((int)emax + rmin) && scale8_ok((int)emax + rmax)) ? 0u : 1u;
+    eh = emax << 20;
+    // this thread's row of the seven input digit planes, 8 inputs at a time
 #pragma unroll
-      for (int k = 0; k < 16; ++k)
-        u[k] = fixed_biased((unsigned)__double2hiint(x[k]), (unsigned)__double2loint(x[k]), emax);
-      // this thread's row of the six input digit planes
-#pragma unroll
-      for (int j = 0; j < kDigits; ++j) {
-        const int pos = 10 * (kDigits - 1 - j);
-        uint4 lo4, hi4;
-        lo4.x = digit_pair(u[0], u[1], pos);
-        lo4.y = digit_pair(u[2], u[3], pos);
-        lo4.z = digit_pair(u[4], u[5], pos);
-        lo4.w = digit_pair(u[6], u[7], pos);
-        hi4.x = digit_pair(u[8], u[9], pos);
-        hi4.y = digit_pair(u[10], u[11], pos);
-        hi4.z = digit_pair(u[12], u[13], pos);
-        hi4.w = digit_pair(u[14], u[15], pos);
-        *reinterpret_cast<uint4*>(smem + j * kPlaneA + core_off(t, 0)) = lo4;
-        *reinterpret_cast<uint4*>(smem + j * kPlaneA + core_off(t, 8)) = hi4;
-      }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (t == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-      for (int i = 0; i < kDigits; ++i) {
-        const unsigned long long bdesc = smem_desc(sB + i * kPlaneB);
-#pragma unroll
-        for (int j = 0; i + j < kDigits; ++j) {
-          const unsigned long long adesc = smem_desc(sA + j * kPlaneA);
-          const uint32_t d = tmem + 16u * (uint32_t)(i + j);
-          const uint32_t accumulate = i > 0 ? 1u : 0u;  // pair (0, L) starts level L
-          asm volatile(
-              "{ .reg .pred q; setp.ne.u32 q, %4, 0; "
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q; }" ::"r"(d),
-              "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
-              : "memory");
-        }
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                   : "memory");
+    for (int c = 0; c < 2; ++c) {
+      const unsigned e8[8] = {eh, eh, eh, eh, eh, eh, eh, eh};
+      split8<kPlaneA>(smem + core_off(t, 8 * c), x + 8 * c, e8);
     }
     // the next tile's inputs load while the tensor cores and the
     // recombination work on this one
     const int64_t bc = b;
     const bool livec = live;
-    double xn[16];
-    load_tile(tile + gridDim.x, xn, b, live);
-    if (t == 0) {
-      uint32_t done = 0;
-      for (long long spin = 0; spin < kSpinLimit && !done; ++spin)
-        asm volatile(
-            "{ .reg .pred q; mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }"
-            : "=r"(done)
-            : "r"(bar), "r"(phase)
-            : "memory");
-      *flag = done;
-    }
-    phase ^= 1u;
+    load_tile(tile + gridDim.x, x, b, live);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (*flag == 0u) {  // the same value in every thread
+    if (__syncthreads_or(done ? 0 : 1)) {
       timed_out = true;
       break;
     }
-    // outputs: rows r = 4c .. 4c + 3 = (ra = c, rb = 0 .. 3), six levels each
+    if (t == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned long long bdesc = smem_desc(sB);
+#pragma unroll
+      for (int j = 0; j < kPlanes; ++j) {
+        // input plane j against PTM planes 0 .. 7 - j, whose levels j .. 7 are
+        // adjacent accumulator columns; plane 7 is zero (j = 0 clears level 7)
+        const unsigned long long adesc = smem_desc(sA + j * kPlaneA);
+        const uint32_t idesc = kIdesc0 | ((16u * (uint32_t)(kLevels - j) >> 3) << 17);
+        asm volatile(
+            "{ .reg .pred q; setp.ne.u32 q, %4, 0; "
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, q; }" ::"r"(tmem + 16u * (uint32_t)j),
+            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(j)
+            : "memory");
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+                   : "memory");
+    }
+    // every thread waits for the MMAs itself (bounded); a time-out ends the
+    // block at its next barrier
+    {
+      uint32_t seen = 0;
+      for (long long spin = 0; spin < kSpinLimit && !seen; ++spin)
+        asm volatile(
+            "{ .reg .pred q; mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }"
+            : "=r"(seen)
+            : "r"(bar), "r"(phase)
+            : "memory");
+      done = seen != 0u;
+    }
+    phase ^= 1u;
+    __syncwarp();  // the tensor-memory loads below are warp-wide
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // outputs: rows r = 4c .. 4c + 3 = (ra = c, rb = 0 .. 3), eight levels each
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      uint32_t w[kDigits][4];
+      uint32_t w[kLevels][4];
 #pragma unroll
-      for (int l = 0; l < kDigits; ++l) tmem_ld4(tlane + 16u * l + 4u * c, w[l]);
+      for (int l = 0; l < kLevels; ++l) tmem_ld4(tlane + 16u * l + 4u * c, w[l]);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       double y[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const uint32_t lv[kDigits] = {w[0][q], w[1][q], w[2][q], w[3][q], w[4][q], w[5][q]};
-        y[q] = combine_words(lv, (int)emax - 1022 + (DEVP ? srow[4 * c + q] : p.row_exp[4 * c + q]), bad);
+        int pr[kLevels / 2];
+#pragma unroll
+        for (int l = 0; l < kLevels; l += 2)
+          pr[l / 2] = level_pair(__uint_as_float(w[l][q]), __uint_as_float(w[l + 1][q]));
+        y[q] = scale8(combine8(pr[0], pr[1], pr[2], pr[3]),
+                      eh + ((unsigned)srow[4 * c + q] << 20));
       }
       if (livec) {
         if (p.vec_z1) {
-          *reinterpret_cast<double2*>(p.out + bc + c * p.sao) = make_double2(y[0], y[1]);
-          *reinterpret_cast<double2*>(p.out + bc + c * p.sao + 2) = make_double2(y[2], y[3]);
+          asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p.out + bc + c * p.sao), "d"(y[0]), "d"(y[1]),
+                       "d"(y[2]), "d"(y[3])
+                       : "memory");
         } else {
 #pragma unroll
           for (int q = 0; q < 4; ++q) p.out[bc + c * p.sao + q * p.sbo] = y[q];
@@ -502,17 +497,16 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
         p.out[bc + (r >> 2) * p.sao + (r & 3) * p.sbo] = a;
       }
     }
-#pragma unroll
-    for (int k = 0; k < 16; ++k) x[k] = xn[k];
   }
+  timed_out = __syncthreads_or(timed_out || !done ? 1 : 0) != 0;
   if (timed_out && t == 0) {
     if (p.status) atomicOr(p.status, QSGB_DEV_TIMEOUT);
     // bounded wait for the MMAs still in flight before the memory is freed
-    uint32_t done = 0;
-    for (long long spin = 0; spin < kSpinLimit && !done; ++spin)
+    uint32_t seen = 0;
+    for (long long spin = 0; spin < kSpinLimit && !seen; ++spin)
       asm volatile(
           "{ .reg .pred q; mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }"
-          : "=r"(done)
+          : "=r"(seen)
           : "r"(bar), "r"(phase ^ 1u)
           : "memory");
   }
@@ -597,7 +591,7 @@ int launch_umma(TcParams& p, const void* in, void* out, uint64_t Z, cudaStream_t
   // tcgen05 form: tiles of 128 groups per block, at most 4 blocks per SM
   p.n_tiles = (p.n_groups + kUBlock - 1) / kUBlock;
   const bool contig = Z % kUBlock == 0;
-  p.vec_z1 = Z == 1 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0 ? 1 : 0;
+  p.vec_z1 = Z == 1 && (uintptr_t)in % 32 == 0 && (uintptr_t)out % 32 == 0 ? 1 : 0;
   auto kern = contig ? apply16_umma_kernel<true, DEVP> : apply16_umma_kernel<false, DEVP>;
   QSGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaSmem));
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(p.n_tiles, (uint64_t)sm_count() * 4));
@@ -609,24 +603,16 @@ int launch_umma(TcParams& p, const void* in, void* out, uint64_t Z, cudaStream_t
 
 int launch(const double* op, const void* in, void* out, uint64_t X, uint64_t Y, uint64_t Z, unsigned* status,
            cudaStream_t stream) {
-  TcParams p;
-  std::memset(&p, 0, sizeof p);
-  for (int r = 0; r < 16; ++r) {
-    split_row(op + 16 * r, p.digits, r, p.row_exp);
-    for (int k = 0; k < 16; ++k) p.ptm[r][k] = op[16 * r + k];
-  }
-  // the same digits in the operand layout: element (row r, column k) of plane
-  // i at byte core_off(r, k)
-  for (int i = 0; i < kDigits; ++i)
-    for (int r = 0; r < 16; ++r)
-      for (int k = 0; k < 16; ++k) p.bplanes[i][core_off(r, k) / 2] = p.digits[i][r][k];
-  set_geometry(p, in, out, X, Y, Z, status);
   static const bool mma_sync = [] {
     const char* v = std::getenv("QSGB_TC_KERNEL");
     return v && std::strcmp(v, "mma_sync") == 0;
   }();
   if (mma_sync) {
     // warp-level form: tiles of 8 groups per warp
+    TcWarpParams p{};
+    std::memcpy(p.ptm, op, sizeof p.ptm);
+    set_geometry(p, in, out, X, Y, Z, status);
+    for (int r = 0; r < 16; ++r) split_row(op + 16 * r, p.digits, r, p.row_exp);
     const bool contig = Z % 8 == 0;
     p.pair_store = contig && (uintptr_t)out % 16 == 0 ? 1 : 0;
     const uint64_t blocks = (p.n_tiles + kBlock / 32 - 1) / (kBlock / 32);
@@ -637,13 +623,15 @@ int launch(const double* op, const void* in, void* out, uint64_t X, uint64_t Y, 
       apply16_tc_kernel<false><<<grid, kBlock, 0, stream>>>(p);
     return launch_status();
   }
+  TcParams p{};
+  std::memcpy(p.ptm, op, sizeof p.ptm);
+  set_geometry(p, in, out, X, Y, Z, status);
   return launch_umma<false>(p, in, out, Z, stream);
 }
 
 int launch_device(const double* dptm, int layout, const void* in, void* out, uint64_t X, uint64_t Y, uint64_t Z,
                   unsigned* status, cudaStream_t stream) {
-  TcParams p;
-  std::memset(&p, 0, sizeof p);
+  TcParams p{};
   p.dptm = dptm;
   p.dlayout = layout & 3;
   set_geometry(p, in, out, X, Y, Z, status);

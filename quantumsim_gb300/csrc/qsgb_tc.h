@@ -11,15 +11,125 @@
 namespace qsgb {
 namespace tc {
 
-// digit planes of the split (six balanced base-1024 digits of a 57-bit
-// fixed-point value plus sign)
+// ------------------------------------------------ base-256 digits
+// The split of the tcgen05 kernels and of the PTM gradient: a value against
+// a block exponent as a signed 55-bit fixed-point integer F in seven balanced
+// base-256 digits, each exactly an FP16 number.  Byte digits cost one byte
+// permute and one three-input logic operation per pair of values and digit
+// (base 1024, six digits: two shifts, a permute and a logic operation), their
+// products are at most 2^14, and every level sum of K <= 16 terms stays below
+// 2^21, so that all levels are exact in FP32, leave it by adding 1.5 * 2^23
+// (no F2I, which runs at a quarter rate) and combine pairwise in 32 bits.
+// With digit pairs up to i + j = 7 the error is about half of base 1024's with
+// i + j <= 5 (exact integer model, 16 terms: 6.1e-17 against 1.45e-16
+// relative for inputs of one scale, 2.1e-16 against 3.8e-16 over three
+// decades).
+constexpr int kPlanes = 7;  // digits
+constexpr int kLevels = 8;  // levels i + j = 0 .. 7
+constexpr unsigned long long kBias8 = 0x0080808080808080ull;
+// biased exponents below this are not scaled by: a block whose values are all
+// smaller is recomputed in native FP64 (zeros are exact)
+constexpr unsigned kMinExp = 64;
+
+// |F| + B for x = (hi, lo) against the block exponent, given in place (eh =
+// biased exponent << 20, >= kMinExp << 20): |F| <= 2^55; values with exponent 0
+// (zero, subnormals) and those 2^-54 below the block give 0.  The sign goes
+// onto the digits (Signs).
+__device__ __forceinline__ unsigned long long fixed8(unsigned hi, unsigned lo, unsigned eh) {
+  const unsigned s = (eh - (hi & 0x7ff00000u)) >> 20;
+  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 2;
+  unsigned long long f;
+  asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(m), "r"(s));  // shifts of 64 and more give 0
+  return f + kBias8;
+}
+
+// (+-1, +-1) and -1152 (+-1, +-1) as FP16x2: the signs of two values
+struct Signs {
+  unsigned one, bias;
+};
+__device__ __forceinline__ Signs signs_of(unsigned hi_a, unsigned hi_b) {
+  const unsigned q = __byte_perm(hi_a, hi_b, 0x7632) & 0x80008000u;
+  return {q | 0x3c003c00u, q ^ 0xe480e480u};
+}
+
+// FP16x2 of digit j (0 the most significant) of two values: byte 6 - j, the
+// top digit with its carry bit (16 bits), as 0x6400 | v = 1024 + v, minus
+// 1152, with the value's sign
+template <int J>
+__device__ __forceinline__ unsigned digit8_pair(unsigned long long ua, unsigned long long ub, const Signs& s) {
+  constexpr int byte = 6 - J;
+  unsigned r;
+  if (byte == 6) {
+    r = __byte_perm((unsigned)(ua >> 32), (unsigned)(ub >> 32), 0x7632) | 0x64006400u;
+  } else if (byte >= 4) {
+    r = __byte_perm((unsigned)(ua >> 32), (unsigned)(ub >> 32), byte == 4 ? 0x0400 : 0x0501);
+    r = (r & 0x00ff00ffu) | 0x64006400u;
+  } else {
+    constexpr unsigned sel = (unsigned)(byte | ((byte + 4) << 8));
+    r = __byte_perm((unsigned)ua, (unsigned)ub, sel);
+    r = (r & 0x00ff00ffu) | 0x64006400u;
+  }
+  unsigned out;
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(out) : "r"(r), "r"(s.one), "r"(s.bias));
+  return out;
+}
+
+// Eight values of one row of a digit plane, every plane: 16 bytes at
+// dst + J * STRIDE
+template <int J, int STRIDE>
+__device__ __forceinline__ void store_digits8(unsigned char* dst, const unsigned long long (&u)[8],
+                                              const Signs (&s)[4]) {
+  if constexpr (J < kPlanes) {
+    *reinterpret_cast<uint4*>(dst + J * STRIDE) =
+        make_uint4(digit8_pair<J>(u[0], u[1], s[0]), digit8_pair<J>(u[2], u[3], s[1]),
+                   digit8_pair<J>(u[4], u[5], s[2]), digit8_pair<J>(u[6], u[7], s[3]));
+    store_digits8<J + 1, STRIDE>(dst, u, s);
+  }
+}
+template <int STRIDE>
+__device__ __forceinline__ void split8(unsigned char* dst, const double* x, const unsigned* eh) {
+  unsigned long long u[8];
+  Signs s[4];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) u[k] = fixed8((unsigned)__double2hiint(x[k]), (unsigned)__double2loint(x[k]), eh[k]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    s[k] = signs_of((unsigned)__double2hiint(x[2 * k]), (unsigned)__double2hiint(x[2 * k + 1]));
+  store_digits8<0, STRIDE>(dst, u, s);
+}
+
+// An FP32 level sum, an integer below 2^22, as an integer plus kMagic
+constexpr unsigned kMagic = 0x4b400000u;  // bits of 1.5 * 2^23
+__device__ __forceinline__ unsigned level_bits(float a) { return __float_as_uint(a + 12582912.0f); }
+// Two consecutive levels as one 32-bit integer: 256 a + b
+__device__ __forceinline__ int level_pair(float a, float b) {
+  return (int)((level_bits(a) << 8) + level_bits(b) - ((kMagic << 8) + kMagic));
+}
+// sum_L A_L 2^(56 - 8 L) / 2^14 of eight levels, given as pairs, in 64 bits
+__device__ __forceinline__ long long combine8(int p01, int p23, int p45, int p67) {
+  return (long long)p23 * 262144ll + (long long)(p45 * 4 + (p67 >> 14)) + ((long long)p01 << 34);
+}
+// v 2^sc as a double, sc given as sc << 20.  For v = combine8 of values split
+// against ex and PTM entries against ep (biased exponents),
+// sc = ex + ep - kScale8; scale8_ok(sc) says that every result is zero or a
+// normal double (1 <= |v| < 2^61), so that the results need no test of their
+// own: blocks for which it fails are recomputed in native FP64.
+constexpr int kScale8 = 2100;
+__host__ __device__ constexpr bool scale8_ok(int sc) { return sc >= 1 - 1023 && sc <= 2046 - 1023 - 61; }
+__device__ __forceinline__ double scale8(long long v, unsigned sc20) {
+  const double d = __ll2double_rn(v);
+  unsigned hi = (unsigned)__double2hiint(d);
+  if (hi != 0u) hi += sc20;
+  return __hiloint2double((int)hi, __double2loint(d));
+}
+
+// ------------------------------------------------ base-1024 digits
+// digit planes of the split of the warp-level kernel (six balanced base-1024
+// digits of a 57-bit fixed-point value plus sign)
 constexpr int kDigits = 6;
 constexpr unsigned long long kDigitBias =
     512ull * (1ull + (1ull << 10) + (1ull << 20) + (1ull << 30) + (1ull << 40) + (1ull << 50));
 
-// The digit split shared by the tensor-core kernels (apply and PTM
-// gradient): a fixed-point value relative to a block exponent, its six
-// balanced base-1024 digits as exact FP16 numbers.
 // Biased exponent of x as used for scaling (subnormals and zero count as 1)
 // and its 53-bit significand (implicit bit included for normal numbers).
 __device__ __forceinline__ unsigned exp_eff(unsigned hi) {
@@ -69,20 +179,19 @@ struct TcParams {
   int64_t sxi, syi, sai, sbi;  // strides of (x, a, y, b) in elements; z stride 1
   int64_t sxo, syo, sao, sbo;
   int pair_store;  // groups 2c, 2c+1 are adjacent and 16-byte aligned
-  int vec_z1;      // Z == 1 and both tensors 16-byte aligned: a group's
-                   // runs along the last target move as 16-byte vectors
-  const double* dptm;  // device PTM (launch_device): split by each block
+  int vec_z1;      // Z == 1 and both tensors 32-byte aligned: a group's
+                   // runs along the last target move as 32-byte vectors
+  const double* dptm;  // device PTM (launch_device)
   int dlayout;         // its storage (QSGB_PTM_SWAPPED / QSGB_PTM_TRANSPOSED bits)
-  int row_exp[16];                                // Ep_r - 1022 - 54 per row
-  unsigned short digits[kDigits][16][16];         // FP16 digit planes e_i[r][k]
-  alignas(16) unsigned short bplanes[kDigits][256];  // the same in the shared-memory
-                                                     // operand layout of tcgen05.mma
-                                                     // (copied with 16-byte loads)
-  double ptm[16][16];                             // the op matrix (FP64 fallback)
+  double ptm[16][16];  // the op matrix of a host PTM
+};
+// the warp-level kernel's: the PTM split on the host
+struct TcWarpParams : TcParams {
+  int row_exp[16];                         // Ep_r - 1022 - 54 per row
+  unsigned short digits[kDigits][16][16];  // FP16 digit planes e_i[r][k]
 };
 
-static_assert(offsetof(TcParams, bplanes) % 16 == 0, "16-byte loads of the operand planes");
-static_assert(sizeof(TcParams) <= 32764, "kernel parameter limit");
+static_assert(sizeof(TcWarpParams) <= 32764, "kernel parameter limit");
 
 // The op matrix is 16 x 16 without inf or nan.
 bool eligible(const double* op, int kin, int kout);

@@ -450,6 +450,7 @@ __global__ void __launch_bounds__(kBlock) apply_ptm_kernel(const __grid_constant
   using V = typename Vec<T, PAIR>::type;
   constexpr int NL = PAIR ? 2 : 1;
   extern __shared__ __align__(16) unsigned char smem[];
+  pdl_wait();
   if (!build_terms<T>(p, L, smem)) return;
 
   V* xs = reinterpret_cast<V*>(smem + L.xs_off);
@@ -620,6 +621,7 @@ __global__ void __launch_bounds__(kDenseBlock) apply_dense_kernel(const __grid_c
   __shared__ double wmax[kDenseBlock / 32];
   const int t = threadIdx.x;
   const int ne = p.kin * p.kout;  // <= kDenseBlock
+  pdl_wait();
   double v = 0.0;
   if (t < ne) {
     const int r = t / p.kin, k = t - r * p.kin;
@@ -697,8 +699,7 @@ int launch_apply(ApplyParams& p, cudaStream_t stream) {
   const uint64_t tiles = (p.n_items + 32 * iw - 1) / (32 * iw);
   const uint64_t cap = (uint64_t)sm_count() * occ;
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(tiles, cap));
-  kern<<<grid, kBlock, L.total, stream>>>(p, L);
-  return launch_status();
+  return launch_pdl(kern, grid, kBlock, L.total, stream, p, L);
 }
 
 
@@ -953,11 +954,8 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
       const uint64_t blocks = (p.n_items + kDenseBlock - 1) / kDenseBlock;
       const unsigned grid =
           (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)sm_count() * 8));
-      if (f32)
-        apply_dense_kernel<float, kDenseMaxK><<<grid, kDenseBlock, 0, s>>>(p);
-      else
-        apply_dense_kernel<double, 4><<<grid, kDenseBlock, 0, s>>>(p);
-      return launch_status();
+      if (f32) return launch_pdl(apply_dense_kernel<float, kDenseMaxK>, grid, kDenseBlock, 0, s, p);
+      return launch_pdl(apply_dense_kernel<double, 4>, grid, kDenseBlock, 0, s, p);
     }
   }
   // 2. generic kernel; a host PTM travels inside its launch parameters

@@ -44,6 +44,21 @@ int allow_dynamic_smem(const void* func, int bytes) {
   return QSGB_OK;
 }
 
+int launch_pdl(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void** args, bool overlap) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  QSGB_CUDA_TRY(cudaLaunchKernelExC(&cfg, func, args));
+  return QSGB_OK;
+}
+
 int launch_status() {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? QSGB_OK : QSGB_ERR_CUDA;

@@ -29,6 +29,22 @@ int launch_status();    // cudaGetLastError mapped to a status code
 // kernel ask for less.
 int allow_dynamic_smem(const void* func, int bytes);
 
+// Launch kernel `func` so that it may start while its predecessor on the stream
+// finishes (programmatic dependent launch; also inside graph captures).  The
+// kernel must call pdl_wait() before it touches memory: that returns when the
+// predecessor is complete and its writes are visible, and since every kernel
+// here waits before it works, so is everything before the predecessor.
+int launch_pdl(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void** args,
+               bool overlap = true);
+template <typename... Params, typename... Args>
+int launch_pdl(void (*kern)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+               const Args&... args) {
+  static_assert(sizeof...(Params) == sizeof...(Args), "one argument per parameter");
+  void* ptrs[] = {const_cast<void*>(static_cast<const void*>(&args))...};
+  return launch_pdl(reinterpret_cast<const void*>(kern), dim3(grid), dim3(block), smem, stream, ptrs);
+}
+__device__ __forceinline__ void pdl_wait() { qsgb_pdl_wait(); }
+
 // ---------------------------------------------------------------------------
 // Unsigned 64-bit division by an invariant divisor (Granlund & Montgomery,
 // "Division by invariant integers using multiplication", PLDI 1994, Fig. 4.1,

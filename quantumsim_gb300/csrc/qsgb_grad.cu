@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(kGradBlock) grad_stage1(const __grid_constant_
     }
   }
   if (t == 0) *fb_any = 0;
+  pdl_wait();
   __syncthreads();
 
   // loader role: group gg_ld of the tile, rows r0_ld + j * rstep
@@ -343,6 +344,7 @@ __global__ void __launch_bounds__(kStage2Entries* kStage2Slices)
   const int el = threadIdx.x % kStage2Entries, sl = threadIdx.x / kStage2Entries;
   const int e = blockIdx.x * kStage2Entries + el;
   double acc = 0.0;
+  pdl_wait();
   if (e < E) {
 #pragma unroll 8
     for (int b = sl; b < nblocks; b += kStage2Slices) acc += part[(int64_t)b * E + e];
@@ -423,6 +425,7 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
     const int ra = k / p.db_out, rb = k - ra * p.db_out;
     sm.oout[k] = ra * p.sao + rb * p.sbo;
   }
+  pdl_wait();
   __syncthreads();
   // byte offset of half row c of group g in a plane
   auto half_row = [](int g, int c) { return g * 32 + ((c ^ ((g >> 2) & 1)) << 4); };
@@ -659,8 +662,12 @@ int launch_stage1(const GradParams& p, unsigned nb, double* part, cudaStream_t s
   auto kern = grad_stage1<T, MPT>;
   const int st = allow_dynamic_smem((const void*)kern, p.smem);
   if (st != QSGB_OK) return st;
-  kern<<<nb, kGradBlock, p.smem, s>>>(p, part);
-  return QSGB_OK;
+  return launch_pdl(kern, nb, kGradBlock, (size_t)p.smem, s, p, part);
+}
+
+int launch_stage2(const double* part, int nblocks, int E, double* dptm, cudaStream_t s) {
+  return launch_pdl(grad_stage2, (unsigned)((E + kStage2Entries - 1) / kStage2Entries),
+                    (unsigned)(kStage2Entries * kStage2Slices), 0, s, part, nblocks, E, dptm);
 }
 
 int grad_common(const void* x_in, const void* g_out, double* dptm, int64_t da_out, int64_t db_out, int64_t da_in,
@@ -684,10 +691,8 @@ int grad_common(const void* x_in, const void* g_out, double* dptm, int64_t da_ou
     const int smem_bytes = std::max((int)sizeof(TcgSmem), kTcgWarps * 256 * (int)sizeof(double));
     const int st = allow_dynamic_smem((const void*)grad16_tc_kernel, smem_bytes);
     if (st != QSGB_OK) return st;
-    grad16_tc_kernel<<<nbt, kTcgBlock, smem_bytes, s>>>(p, part);
-    grad_stage2<<<(E + kStage2Entries - 1) / kStage2Entries, kStage2Entries * kStage2Slices, 0, s>>>(part, (int)nbt,
-                                                                                                     E, dptm);
-    return launch_status();
+    const int s1 = launch_pdl(grad16_tc_kernel, nbt, kTcgBlock, (size_t)smem_bytes, s, p, part);
+    return s1 != QSGB_OK ? s1 : launch_stage2(part, (int)nbt, E, dptm, s);
   }
   const bool two = p.nmt > kGradBlock;
   int st;
@@ -696,9 +701,7 @@ int grad_common(const void* x_in, const void* g_out, double* dptm, int64_t da_ou
   else
     st = two ? launch_stage1<float, 2>(p, nb, part, s) : launch_stage1<float, 1>(p, nb, part, s);
   if (st != QSGB_OK) return st;
-  grad_stage2<<<(E + kStage2Entries - 1) / kStage2Entries, kStage2Entries * kStage2Slices, 0, s>>>(part, (int)nb, E,
-                                                                                                   dptm);
-  return launch_status();
+  return launch_stage2(part, (int)nb, E, dptm, s);
 }
 
 }  // namespace

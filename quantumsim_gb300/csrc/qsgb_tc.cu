@@ -339,7 +339,20 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
   int64_t b;
   bool live;
   uint64_t tile = blockIdx.x;
-  load_tile(tile, x, b, live);  // in flight during the set-up below
+  // set-up that reads no memory, while the preceding kernel finishes
+  if (t < kPlaneB / 16) *reinterpret_cast<uint4*>(smem + kSmemB + kPlanes * kPlaneB + 16 * t) = make_uint4(0, 0, 0, 0);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + kSmemTmem),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (t == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  pdl_wait();
+  load_tile(tile, x, b, live);  // in flight during the split of the PTM
   int* srow = reinterpret_cast<int*>(smem + kSmemRowExp);
   int ptm_bad = 0;  // inf or nan entries, or a row too small to scale by (this thread's pair)
   {
@@ -367,17 +380,6 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
     *reinterpret_cast<unsigned*>(dst + 5 * kPlaneB) = digit8_pair<5>(u0, u1, sg);
     *reinterpret_cast<unsigned*>(dst + 6 * kPlaneB) = digit8_pair<6>(u0, u1, sg);
     if ((t & 7) == 0) srow[r] = (int)emax - kScale8;
-  }
-  if (t < kPlaneB / 16) *reinterpret_cast<uint4*>(smem + kSmemB + kPlanes * kPlaneB + 16 * t) = make_uint4(0, 0, 0, 0);
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + kSmemTmem),
-                 "r"(kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (t == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -593,10 +595,10 @@ int launch_umma(TcParams& p, const void* in, void* out, uint64_t Z, cudaStream_t
   const bool contig = Z % kUBlock == 0;
   p.vec_z1 = Z == 1 && (uintptr_t)in % 32 == 0 && (uintptr_t)out % 32 == 0 ? 1 : 0;
   auto kern = contig ? apply16_umma_kernel<true, DEVP> : apply16_umma_kernel<false, DEVP>;
-  QSGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaSmem));
+  const int st = allow_dynamic_smem((const void*)kern, kUmmaSmem);
+  if (st != QSGB_OK) return st;
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(p.n_tiles, (uint64_t)sm_count() * 4));
-  kern<<<grid, kUBlock, kUmmaSmem, stream>>>(p);
-  return launch_status();
+  return launch_pdl(kern, grid, kUBlock, kUmmaSmem, stream, p);
 }
 
 }  // namespace

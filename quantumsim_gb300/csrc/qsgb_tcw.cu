@@ -180,6 +180,7 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
   T* __restrict__ out = static_cast<T*>(p.out);
   const int dbi = p.db_in | 1, dbo = p.db_out | 1;  // odd: staged rows without bank conflicts
 
+  pdl_wait();
   for (int k = t; k < kWMaxK; k += kWBlock) {
     if (k < p.kin) {
       const int ka = k / p.db_in, kb = k - ka * p.db_in;
@@ -502,8 +503,7 @@ int wide_launch(WideParams& p, cudaStream_t stream) {
   const int st = allow_dynamic_smem((const void*)apply_wide_kernel<T, KH>, smem);
   if (st != QSGB_OK) return st;
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(p.n_tiles, (uint64_t)sm_count()));
-  apply_wide_kernel<T, KH><<<grid, kWBlock, smem, stream>>>(p);
-  return launch_status();
+  return launch_pdl(apply_wide_kernel<T, KH>, grid, kWBlock, smem, stream, p);
 }
 
 }  // namespace

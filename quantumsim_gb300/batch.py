@@ -27,9 +27,10 @@ program is built once per circuit structure:
 after which batched 16 x 16 contractions turn the units' gradients into
 dL/dP of every original op.
 
-Each op on a large instance is split into tiles of `tile` groups, so blocks
-share big instances while small ones take one item.  ``autotune()`` times the
-candidate tile sizes and keeps the fastest (cached in a JSON file).
+Each op is split into items, so that blocks share the instances of a stage: by
+default evenly over the device's blocks (`adaptive_chunks`), or in tiles of
+`tile` groups.  ``autotune()`` times candidate tile sizes and keeps the fastest
+(cached in a JSON file).
 
 The reference has no batching; the per-instance comparison is the plain GPU
 path (``plain_gradients``): one instance at a time through the ``ApplyPTM``
@@ -327,8 +328,41 @@ def map_unit_gradients(g_one, g_two, c, a, b, chain_factors,
     return dc, chain_gradients(torch.cat(parts), chain_factors)
 
 
+# Adaptive split of a stage into items, in vector elements (build_program):
+# an item is a multiple of ADAPT_STEP, at most ADAPT_MAX unless a stage is so
+# large that it gives every block ADAPT_ROUNDS items anyway.  ADAPT_STEP is what
+# a block takes between two folds of its FP32 gradient sums into FP64 (1024
+# groups of a two-qubit op, 4096 of a one-qubit op), so these folds hold the
+# same products however a stage is split.
+ADAPT_STEP, ADAPT_MAX, ADAPT_ROUNDS = 16384, 65536, 6
+
+
+def adaptive_chunks(stage, total, width, grid):
+    """Items' lengths (in units of `width` elements) for entries of `total`
+    units each, grouped in stages, on `grid` blocks.
+
+    A stage takes as long as its slowest block.  With few or small instances
+    one fixed length leaves most blocks idle (64 items of 16384 groups of a
+    12-qubit instance on 304 blocks; one item of a whole 8-qubit instance), so
+    a stage is split evenly over the blocks, between those limits.  Measured on
+    GB300, one step of 20 circuits of 4 to 12 qubits: 125 ms at the fixed 8192
+    groups and at most 64 items per op, 106 ms here; 7 circuits of up to 11
+    qubits 14.0 and 4.2 ms; 14 of up to 8 qubits 7.9 and 4.7 ms.  (Items of 256
+    groups would take these last two to 3.5 and 2.8 ms, with other FP32 sums.)
+    """
+    n_stages = int(stage.max()) + 1
+    elems = np.bincount(stage, weights=(total * width).astype(float),
+                        minlength=n_stages)
+    per = np.maximum(np.minimum(elems / grid, ADAPT_MAX),
+                     elems / (ADAPT_ROUNDS * grid))
+    # smaller instances in finer items, which fill the gaps at the end
+    per = np.minimum(per[stage], total * width / 64)
+    per = np.maximum(np.ceil(per / ADAPT_STEP), 1).astype(np.int64)
+    return per * ADAPT_STEP // width
+
+
 def build_program(units, unit_base, sizes, depths, every, tile,
-                  max_items=64):
+                  max_items=64, grid=304):
     """Host part of the device program, in numpy: (items, stage_begin,
     n_slots).
 
@@ -337,11 +371,12 @@ def build_program(units, unit_base, sizes, depths, every, tile,
     max(tile, ceil(total / max_items)) -- large ops are shared by many
     blocks, and no op has more than `max_items` items.  `tile` is a multiple
     of 4: the kernel takes 4 consecutive groups along z per access, and an
-    item boundary must not split them.  Stages per instance: INIT, APPLY of
+    item boundary must not split them.  With tile 0 the chunks are chosen per
+    stage for `grid` blocks (adaptive_chunks).  Stages per instance: INIT, APPLY of
     every unit (SAVE after every `every`-th layer), ZERO_G, LOSS, ADJOINT of
     the units in reverse (RESTORE at the saved layers); a last stage holds
     one GRADSUM item per unit over the dP slots of its ADJOINT items."""
-    if tile < 4 or tile % 4:
+    if tile != 0 and (tile < 4 or tile % 4):
         raise ValueError('tile must be a positive multiple of 4')
     ent = []  # (stage, op, inst, q0, q1, ptm or checkpoint, total)
     for i, (unit_list, size, depth) in enumerate(zip(units, sizes, depths)):
@@ -376,17 +411,31 @@ def build_program(units, unit_base, sizes, depths, every, tile,
     e = np.array(ent, dtype=np.int64)
     stage, op, inst, q0, q1, pp, total = e.T
     is_loss = op == BOP_LOSS
-    chunk = np.where(is_loss, 1, np.maximum(tile, -(-total // max_items)))
+    if tile:
+        chunk = np.maximum(tile, -(-total // max_items))
+    else:
+        width = np.where((op == BOP_APPLY) | (op == BOP_ADJOINT),
+                         np.where(q1 < 0, 4, 16), 1)
+        chunk = adaptive_chunks(stage, total, width, grid)
+    chunk = np.where(is_loss, 1, chunk)
     n_items = -(-total // chunk)
     # one dP partial slot per ADJOINT item
     adj = op == BOP_ADJOINT
     slot_base = np.zeros(len(e), dtype=np.int64)
     slot_base[adj] = np.cumsum(np.concatenate([[0], n_items[adj][:-1]]))
     n_slots = int(n_items[adj].sum())
-    # expand entries into items
-    rep = np.repeat(np.arange(len(e)), n_items)
-    first = np.repeat(np.cumsum(n_items) - n_items, n_items)
-    j = np.arange(len(rep)) - first
+    # last stage: GRADSUM per PTM over the slots of its ADJOINT items
+    gitems = np.zeros(int(adj.sum()), dtype=_ITEM_DTYPE)
+    gitems['op'] = BOP_GRADSUM
+    gitems['ptm'] = pp[adj]
+    gitems['q1'] = -1
+    gitems['beg'] = slot_base[adj]
+    gitems['end'] = slot_base[adj] + n_items[adj]
+    # expand entries into items, stage by stage
+    order = np.argsort(stage, kind='stable')
+    n_items = n_items[order]
+    rep = np.repeat(order, n_items)
+    j = np.arange(len(rep)) - np.repeat(np.cumsum(n_items) - n_items, n_items)
     beg = j * chunk[rep]
     end_ = np.minimum(total[rep], beg + chunk[rep])
     items = np.zeros(len(rep), dtype=_ITEM_DTYPE)
@@ -398,19 +447,8 @@ def build_program(units, unit_base, sizes, depths, every, tile,
     items['slot'] = np.where(adj[rep], slot_base[rep] + j, 0)
     items['beg'] = np.where(is_loss[rep], 0, beg)
     items['end'] = np.where(is_loss[rep], 0, end_)
-    st = stage[rep]
-    n_main = int(st.max()) + 1
-    # last stage: GRADSUM per PTM over the slots of its ADJOINT items
-    gitems = np.zeros(int(adj.sum()), dtype=_ITEM_DTYPE)
-    gitems['op'] = BOP_GRADSUM
-    gitems['ptm'] = pp[adj]
-    gitems['q1'] = -1
-    gitems['beg'] = slot_base[adj]
-    gitems['end'] = slot_base[adj] + n_items[adj]
-    order = np.argsort(st, kind='stable')
-    items = np.concatenate([items[order], gitems])
-    counts = np.concatenate([np.bincount(st, minlength=n_main),
-                             [len(gitems)]])
+    items = np.concatenate([items, gitems])
+    counts = np.concatenate([np.bincount(stage[rep]), [len(gitems)]])
     begin = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
     return items, begin, n_slots
 
@@ -487,7 +525,8 @@ class BatchedSimulator:
         self.max_grid = self.lib.qsgb_batch_max_grid(BLOCK)
         if self.max_grid < 1:
             raise RuntimeError('batched kernel cannot be made resident')
-        self.tile = tile or self._cached_tile() or 8192
+        # 0: items sized per stage for the device (adaptive_chunks)
+        self.tile = tile or self._cached_tile() or 0
         self._build_program(self.tile)
         self.graph = None
 
@@ -497,7 +536,8 @@ class BatchedSimulator:
         host, then uploaded)."""
         items, begin, n_slots = build_program(
             self.units, self.unit_base, self.sizes,
-            [s.depth for s in self.specs], self.every, tile, max_items)
+            [s.depth for s in self.specs], self.every, tile, max_items,
+            self.max_grid)
         n_main = len(begin) - 2
         dev = self.device
         self.n_stages = n_main + 1
@@ -732,7 +772,7 @@ class BatchedSimulator:
 
     def autotune(self, candidates=(2048, 4096, 8192, 16384, 32768), reps=2):
         """Time one step per tile size, keep the fastest; returns
-        {tile: ms}."""
+        {tile: ms}.  (0 stands for the default, items sized per stage.)"""
         times = {}
         for t in candidates:
             self._build_program(t)

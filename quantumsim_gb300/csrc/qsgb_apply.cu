@@ -936,7 +936,7 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
   // kernels take, 12 terms per row at 81 x 81); a device PTM's values are not
   // read on the host, so it counts all its entries, as 16 x 16 ones do above.
   // Measured on GB300, dense 81 x 81 on 7 qutrits (38 MB): 1210 us in the
-  // generic kernel, 141 us here, with 1/20 of its error.
+  // generic kernel, 84 us here, with 1/60 of its error.
   if (!(flags & (QSGB_PTM_HOST | QSGB_PTM_NOJIT)) && p.max_terms > jit::kMaxJitTerms && kin <= tc::kWideMax &&
       kout <= tc::kWideMax && (arith == QSGB_ARITH_AUTO || arith == QSGB_ARITH_F32) && tc_device_auto())
     return tc::launch_wide(ptm, flags & 3, in, out, dtype, (int)da_out, (int)db_out, (int)da_in, (int)db_in,

@@ -4,39 +4,45 @@
 // A dense 81 x 81 PTM costs 81 multiply-adds per output.  The generic kernel
 // interprets term lists (1.21 ms on 7 qutrits, 38 MB in and out); float-float
 // on the FP32 pipes would be bound by ~10 operations per term.  Here the
-// contraction runs in the error-free digit split of qsgb_tc.cu (after Ozaki,
-// Ogita, Oishi and Rump, Numer. Algorithms 59, 2012) with digits fitted to the
-// longer sums:
+// contraction runs in the error-free base-256 digit split of the 16 x 16
+// kernel (qsgb_tc.h; after Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59,
+// 2012):
 //
 //  * Each group's inputs and each PTM row are scaled by their largest binary
-//    exponent and written as signed fixed-point integers in ND balanced
-//    base-512 digits, exact FP16 numbers in [-256, 256]: ND = 6 (54 bits) for
-//    FP64 storage, ND = 4 (36 bits) for FP32.  A product of two digits is at
-//    most 2^16 and a K = 81 sum at most 2^22.4, so that a level (all digit
-//    pairs i + j = L) of up to three pairs (two for K = 96) stays below 2^24,
-//    where FP32 sums of integers are exact for any input; the deeper levels
-//    hold up to six pairs, and only sums that use their whole range could
-//    round there, in the last bit of a level 2^-27 below the first.
-//  * The levels are combined in int64 and rounded to the storage type once.
-//    The dropped levels (i + j >= ND) bound the error by about
-//    5 K 2^-54 max_k |P_rk| max_k |x_k| for FP64 (typically 2^-51 of that
-//    product); for FP32 it is far below one rounding of the result.
-//  * Groups that hold inf or nan, and FP64 results outside the normal range,
-//    are recomputed in plain arithmetic by their own threads.
+//    exponent and written as fixed-point integers in PL balanced byte digits,
+//    exact FP16 numbers: PL = 7 (55 bits) for FP64 storage, PL = 5 (39 bits)
+//    for FP32.  A product of two digits is at most 2^14 and a K = 96 sum at
+//    most 2^20.6, so a level (all digit pairs i + j = L, L < LV = PL + 1; at
+//    most seven pairs) stays below 2^24, where FP32 sums of integers are exact.
+//  * Levels pair up in 32-bit integers, are combined in int64 and rounded to
+//    the storage type once.  Truncation and the dropped levels bound the error
+//    by about 2^-47 max_k |P_rk| max_k |x_k| for FP64 at K = 81 (typically
+//    2^-53 of that product); for FP32 it is far below one rounding.
+//  * Groups that hold inf or nan, or whose scales leave the range where every
+//    result is a normal number, are recomputed in the storage type's plain
+//    arithmetic by their own threads.
 //
-// Work split: one block of 256 threads per SM takes tiles of 128 groups (the M
-// of one MMA); two threads share a group, half of the inputs and half of the
-// outputs each.  All digit planes of the inputs do not fit shared memory
-// beside those of the PTM (147 + 110 KB for 81 x 81), so the input planes, the
-// A operand, live in tensor memory: ND x 48 columns, plus two accumulator
-// buffers of N columns (288 + 192 of the 512).  The levels are computed one
-// after another, L + 1 digit pairs of N = 96 wide MMAs each, alternating the
-// two buffers: while the tensor cores work on level L + 1, the threads read
-// level L and add it to their int64 sums.
+// Work split: one block of 512 threads per SM takes tiles of 128 groups (the M
+// of one MMA); four threads share a group, a quarter of the inputs and of each
+// half of the outputs each.  All digit planes of the inputs do not fit shared
+// memory beside those of the PTM, so the input planes, the A operand, live in
+// tensor memory: PL x 48 columns, plus three accumulator buffers of 48 columns
+// (336 + 144 of the 512).  The outputs are computed in two halves of up to 48
+// rows; a group of three levels at a time is accumulated, one buffer each, with
+// the MMAs of the three interleaved; while the threads add a group to their
+// sums, the tensor cores work on the next.
 //
 // When the less significant target is the last qudit (Z == 1) a thread's group
 // is not adjacent to its neighbour's; the tile then goes through shared memory
 // both ways, copied in runs of consecutive elements.
+//
+// Measured on GB300, dense 81 x 81 on 7 qutrits (461 tiles, 38 MB): 84 us a
+// pass against 1210 us in the generic kernel, with 1/60 of its error.  A first
+// form of this kernel (base-512 digits, six levels of N = 96 one after another,
+// 256 threads) took 140 us; this one with a level per commit 113 us, and 162 us
+// with its MMAs issued by one thread from rolled loops.  What bounds it now:
+// latency, over 408 small MMAs and ~150 instructions per element on one block
+// of 16 warps; issue is a quarter busy.
 #include <algorithm>
 
 #include "qsgb_common.cuh"
@@ -46,8 +52,11 @@ namespace qsgb {
 namespace tc {
 namespace {
 
-constexpr int kWBlock = 256;
+constexpr int kWBlock = 512;
+constexpr int kWWarps = kWBlock / 32;
 constexpr int kWGroups = 128;  // groups per tile
+constexpr int kWParts = kWBlock / kWGroups;
+constexpr int kWBufs = 3;      // accumulator buffers
 constexpr long long kWSpinLimit = 1ll << 26;
 
 struct WideParams {
@@ -57,10 +66,11 @@ struct WideParams {
   unsigned* status;
   int kin, kout;
   int da_in, db_in, da_out, db_out;
-  int layout;        // QSGB_PTM_SWAPPED / QSGB_PTM_TRANSPOSED bits
-  int npad, ksteps;  // N of the MMA (multiple of 16), K steps of 16
-  int staged;        // Z == 1: tiles through shared memory
-  int off_stage;     // shared-memory offset of the staged tile
+  int layout;     // QSGB_PTM_SWAPPED / QSGB_PTM_TRANSPOSED bits
+  int nhalf;      // N of the MMA: 16, 32 or 48 (two halves cover kout)
+  int ksteps;     // K steps of 16
+  int staged;     // Z == 1: tiles through shared memory
+  int off_stage;  // shared-memory offset of the staged tile
   uint64_t n_groups, n_tiles;
   FastDiv div_z, div_y;
   int64_t sxi, syi, sai, sbi;
@@ -69,74 +79,70 @@ struct WideParams {
 
 // shared-memory byte offsets before the PTM planes
 constexpr int kWMaxK = 96;
-constexpr int kWOffBar = 0;                          // two mbarriers
-constexpr int kWOffTmem = 16;                        // tensor-memory base
-constexpr int kWOffRow = 32;                         // int[96]: row exponents
-constexpr int kWOffEmax = kWOffRow + 4 * kWMaxK;     // unsigned[2][128]: half-group exponents
-constexpr int kWOffIn = kWOffEmax + 8 * kWGroups;    // int64[96]: input offsets
-constexpr int kWOffOut = kWOffIn + 8 * kWMaxK;       // int64[96]: output offsets
-constexpr int kWOffSin = kWOffOut + 8 * kWMaxK;      // int[96]: staged input offsets
-constexpr int kWOffSout = kWOffSin + 4 * kWMaxK;     // int[96]: staged output offsets
-constexpr int kWOffGin = kWOffSout + 4 * kWMaxK;     // int64[128]: group bases, in
-constexpr int kWOffGout = kWOffGin + 8 * kWGroups;   // int64[128]: group bases, out
+constexpr int kWOffFull = 0;                             // mbarrier: accumulators ready
+constexpr int kWOffEmpty = 8;                            // mbarrier: accumulators read
+constexpr int kWOffTmem = 16;                            // tensor-memory base
+constexpr int kWOffRow = 64;                             // int[96]: row scales
+constexpr int kWOffEmax = kWOffRow + 4 * kWMaxK;         // unsigned[4][128]: quarter-group exponents
+constexpr int kWOffIn = kWOffEmax + 4 * kWParts * kWGroups;  // int64[96]: input offsets
+constexpr int kWOffOut = kWOffIn + 8 * kWMaxK;           // int64[96]: output offsets
+constexpr int kWOffSin = kWOffOut + 8 * kWMaxK;          // int[96]: staged input offsets
+constexpr int kWOffSout = kWOffSin + 4 * kWMaxK;         // int[96]: staged output offsets
+constexpr int kWOffProw = kWOffSout + 4 * kWMaxK;        // int[96]: PTM offsets of rows
+constexpr int kWOffPcol = kWOffProw + 4 * kWMaxK;        // int[96]: PTM offsets of columns
+constexpr int kWOffGin = kWOffPcol + 4 * kWMaxK;         // int64[128]: group bases, in
+constexpr int kWOffGout = kWOffGin + 8 * kWGroups;       // int64[128]: group bases, out
 constexpr int kWOffB = (kWOffGout + 8 * kWGroups + 127) / 128 * 128;
 
-// biased exponent and significand (implicit bit included) of a value
-struct Parts {
-  unsigned e;
-  unsigned neg;
-  unsigned long long m;
-};
-__device__ __forceinline__ Parts parts(double v) {
-  const unsigned h = (unsigned)__double2hiint(v);
-  Parts r;
-  r.e = (h >> 20) & 0x7ffu;
-  r.neg = h >> 31;
-  r.m = ((unsigned long long)((h & 0xfffffu) | (r.e ? 0x100000u : 0u)) << 32) | (unsigned)__double2loint(v);
-  return r;
-}
-__device__ __forceinline__ Parts parts(float v) {
-  const unsigned b = __float_as_uint(v);
-  Parts r;
-  r.e = (b >> 23) & 0xffu;
-  r.neg = b >> 31;
-  r.m = (b & 0x7fffffu) | (r.e ? 0x800000u : 0u);
-  return r;
-}
 __device__ __forceinline__ unsigned exp_of(double v) { return ((unsigned)__double2hiint(v) >> 20) & 0x7ffu; }
 __device__ __forceinline__ unsigned exp_of(float v) { return (__float_as_uint(v) >> 23) & 0xffu; }
-template <typename T>
-constexpr unsigned kExpAll = sizeof(T) == 8 ? 0x7ffu : 0xffu;
+__device__ __forceinline__ unsigned sign_word(double v) { return (unsigned)__double2hiint(v); }
+__device__ __forceinline__ unsigned sign_word(float v) { return __float_as_uint(v); }
 
-// F + B: the value as a (9 ND)-bit non-negative integer against exponent emax
-// (F = sign * m aligned, |F| < 2^(9 ND - 1); B = 256 in every base-512 digit)
-template <int ND, int MBITS>
-__device__ __forceinline__ unsigned long long fixed9(const Parts& p, unsigned emax) {
-  constexpr int kUp = 9 * ND - 1 - MBITS;  // alignment of an MBITS significand
-  constexpr unsigned long long kBias = 256ull * (((1ull << (9 * ND)) - 1ull) / 511ull);
-  const unsigned s = emax - (p.e ? p.e : 1u) + (kUp < 0 ? (unsigned)-kUp : 0u);
-  const unsigned long long m = kUp > 0 ? p.m << (kUp > 0 ? kUp : 0) : p.m;
-  unsigned long long f = s < 64u ? m >> s : 0ull;
-  if (p.neg) f = 0ull - f;
+// |F| + B against the block exponent e (in place: exponent field): F has
+// 8 PL - 1 bits; exponent-0 values (zero, subnormals) give 0 when the block's
+// exponent is kMinExp or more (FP64) or 40 or more (FP32)
+template <int PL>
+__device__ __forceinline__ unsigned long long fixed_bytes(double v, unsigned e) {
+  constexpr unsigned long long kBias = 0x8080808080808080ull >> (8 * (8 - PL));
+  const unsigned h = (unsigned)__double2hiint(v);
+  const unsigned long long m = (unsigned long long)((h & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(v);
+  constexpr int up = 8 * PL - 1 - 53;
+  const unsigned s = e - ((h >> 20) & 0x7ffu) + (up < 0 ? (unsigned)-up : 0u);
+  unsigned long long f;
+  asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(up > 0 ? m << (up > 0 ? up : 0) : m), "r"(s));
   return f + kBias;
 }
-
-// FP16x2 of one base-512 digit (bit position pos) of two values: 0x6400 | v
-// is 1024 + v; minus 1280
-__device__ __forceinline__ unsigned digit9_pair(unsigned long long ua, unsigned long long ub, int pos, unsigned mask) {
-  const unsigned a = (unsigned)(ua >> pos) & mask;
-  const unsigned b = (unsigned)(ub >> pos) & mask;
-  const unsigned r = a | (b << 16) | 0x64006400u;
+template <int PL>
+__device__ __forceinline__ unsigned long long fixed_bytes(float v, unsigned e) {
+  constexpr unsigned long long kBias = 0x8080808080808080ull >> (8 * (8 - PL));
+  const unsigned b = __float_as_uint(v);
+  const unsigned long long m = (unsigned long long)((b & 0x7fffffu) | 0x800000u) << (8 * PL - 1 - 24);
+  unsigned long long f;
+  asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(m), "r"(e - ((b >> 23) & 0xffu)));
+  return f + kBias;
+}
+// digit J (0 the most significant) of two values as signed FP16x2 (digit8_pair
+// for PL planes)
+template <int PL, int J>
+__device__ __forceinline__ unsigned digit_bytes(unsigned long long ua, unsigned long long ub, const Signs& s) {
+  constexpr int byte = PL - 1 - J, b4 = byte & 3;
+  const unsigned a = (unsigned)(byte >= 4 ? ua >> 32 : ua), b = (unsigned)(byte >= 4 ? ub >> 32 : ub);
+  unsigned r;
+  if (J == 0)  // the top digit with its carry bit: 16 bits
+    r = __byte_perm(a, b, (unsigned)(b4 | ((b4 + 1) << 4) | ((b4 + 4) << 8) | ((b4 + 5) << 12))) | 0x64006400u;
+  else
+    r = (__byte_perm(a, b, (unsigned)(b4 | ((b4 + 4) << 8))) & 0x00ff00ffu) | 0x64006400u;
   unsigned out;
-  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(out) : "r"(r), "r"(0x65006500u));
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(out) : "r"(r), "r"(s.one), "r"(s.bias));
   return out;
 }
 
 // shared-memory matrix descriptor of a K-major plane without swizzling whose
-// 8-column (K) slabs of npad rows x 16 bytes follow one another: leading (K)
-// byte offset 16 npad, stride (8 rows) 128
-__device__ __forceinline__ unsigned long long wide_desc(uint32_t saddr, int npad) {
-  return (unsigned long long)((saddr >> 4) & 0x3fffu) | ((unsigned long long)npad << 16) |
+// 8-column (K) slabs of `rows` rows x 16 bytes follow one another: leading (K)
+// byte offset 16 rows, stride (8 rows) 128
+__device__ __forceinline__ unsigned long long wide_desc(uint32_t saddr, int rows) {
+  return (unsigned long long)((saddr >> 4) & 0x3fffu) | ((unsigned long long)rows << 16) |
          ((unsigned long long)(128 >> 4) << 32) | (1ull << 46);
 }
 
@@ -145,107 +151,92 @@ __device__ __forceinline__ void tmem_st4(uint32_t addr, const unsigned (&r)[4]) 
                "r"(r[2]), "r"(r[3])
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, float (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3])
                : "r"(addr));
 }
 
-// T: storage type; KH: K and N are at most 16 KH, a thread owns 8 KH inputs
-// and 8 KH outputs of its group
-template <typename T, int KH>
+// the digits of 8 inputs: 4 columns of every input plane (stride `plane`)
+template <int PL, int J>
+__device__ __forceinline__ void store_planes(uint32_t addr, uint32_t plane, const unsigned long long (&u)[8],
+                                             const Signs (&s)[4]) {
+  if constexpr (J < PL) {
+    const unsigned w[4] = {digit_bytes<PL, J>(u[0], u[1], s[0]), digit_bytes<PL, J>(u[2], u[3], s[1]),
+                           digit_bytes<PL, J>(u[4], u[5], s[2]), digit_bytes<PL, J>(u[6], u[7], s[3])};
+    tmem_st4(addr, w);
+    store_planes<PL, J + 1>(addr + plane, plane, u, s);
+  }
+}
+template <int PL, int J>
+__device__ __forceinline__ void store_ptm_planes(unsigned char* dst, int plane, const unsigned long long (&u)[8],
+                                                 const Signs (&s)[4]) {
+  if constexpr (J < PL) {
+    *reinterpret_cast<uint4*>(dst) =
+        make_uint4(digit_bytes<PL, J>(u[0], u[1], s[0]), digit_bytes<PL, J>(u[2], u[3], s[1]),
+                   digit_bytes<PL, J>(u[4], u[5], s[2]), digit_bytes<PL, J>(u[6], u[7], s[3]));
+    store_ptm_planes<PL, J + 1>(dst + plane, plane, u, s);
+  }
+}
+
+// T: storage type; a thread owns KQ inputs (K <= 4 KQ) and up to KQ outputs
+template <typename T, int KQ>
 __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_constant__ WideParams p) {
   constexpr bool F64 = sizeof(T) == 8;
-  constexpr int ND = F64 ? 6 : 4;
-  constexpr int MB = F64 ? 53 : 24;
-  constexpr int kHalf = 8 * KH;             // inputs (outputs) of a thread
-  constexpr int kPlaneCols = 8 * KH;        // tensor-memory columns of an input plane
-  constexpr int kDCol = ND * kPlaneCols;    // first accumulator column
-  constexpr unsigned kCols = kDCol + 32 * KH <= 256 ? 256u : 512u;
+  constexpr int PL = F64 ? 7 : 5, LV = PL + 1;
+  constexpr unsigned kExpAll = F64 ? 0x7ffu : 0xffu;
+  constexpr unsigned kMinX = F64 ? kMinExp : 40u;  // least block exponent of the inputs
+  constexpr int kPlaneCols = 2 * KQ;         // tensor-memory columns of an input plane
+  constexpr int kDCol = PL * kPlaneCols;     // first accumulator column
+  static_assert(kDCol + kWBufs * 48 <= 512, "tensor memory");
+  constexpr unsigned kCols = 512u;
+  constexpr int kMaxOut = 12;                // outputs of a thread per half: nhalf / 4
   extern __shared__ __align__(1024) unsigned char smem[];
   const int t = threadIdx.x, warp = t >> 5;
-  const int gl = t & (kWGroups - 1), h = t >> 7;  // group of the tile, half
+  const int gl = t & (kWGroups - 1), h = t >> 7;  // group of the tile, quarter
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-  const uint32_t bar = sbase + kWOffBar;
+  const uint32_t full = sbase + kWOffFull, empty = sbase + kWOffEmpty;
   int* srow = reinterpret_cast<int*>(smem + kWOffRow);
   unsigned* semax = reinterpret_cast<unsigned*>(smem + kWOffEmax);
   int64_t* goff_in = reinterpret_cast<int64_t*>(smem + kWOffIn);
   int64_t* goff_out = reinterpret_cast<int64_t*>(smem + kWOffOut);
   int* soff_in = reinterpret_cast<int*>(smem + kWOffSin);
   int* soff_out = reinterpret_cast<int*>(smem + kWOffSout);
+  int* prow = reinterpret_cast<int*>(smem + kWOffProw);
+  int* pcol = reinterpret_cast<int*>(smem + kWOffPcol);
   int64_t* gin = reinterpret_cast<int64_t*>(smem + kWOffGin);
   int64_t* gout = reinterpret_cast<int64_t*>(smem + kWOffGout);
   T* stage = reinterpret_cast<T*>(smem + p.off_stage);
   const T* __restrict__ in = static_cast<const T*>(p.in);
   T* __restrict__ out = static_cast<T*>(p.out);
   const int dbi = p.db_in | 1, dbo = p.db_out | 1;  // odd: staged rows without bank conflicts
+  const int nhalf = p.nhalf, npad = 2 * nhalf;
 
-  pdl_wait();
-  for (int k = t; k < kWMaxK; k += kWBlock) {
-    if (k < p.kin) {
-      const int ka = k / p.db_in, kb = k - ka * p.db_in;
-      goff_in[k] = ka * p.sai + kb * p.sbi;
-      soff_in[k] = ka * kWGroups * dbi + kb;
+  // ---- set-up that reads no memory, while the preceding kernel finishes
+  if (t < kWMaxK) {
+    // element offsets of inputs, outputs, and of the PTM: a stored offset is a
+    // row part plus a column part in every layout
+    if (t < p.kin) {
+      const int ka = t / p.db_in, kb = t - ka * p.db_in;
+      goff_in[t] = ka * p.sai + kb * p.sbi;
+      soff_in[t] = ka * kWGroups * dbi + kb;
+      switch (p.layout & 3) {
+        case 0: pcol[t] = t; break;
+        case QSGB_PTM_SWAPPED: pcol[t] = kb * p.da_in + ka; break;
+        case QSGB_PTM_TRANSPOSED: pcol[t] = t * p.kout; break;
+        default: pcol[t] = (kb * p.da_in + ka) * p.kout; break;
+      }
     }
-    if (k < p.kout) {
-      const int ra = k / p.db_out, rb = k - ra * p.db_out;
-      goff_out[k] = ra * p.sao + rb * p.sbo;
-      soff_out[k] = ra * kWGroups * dbo + rb;
-    }
-  }
-
-  // ---- the PTM's digit planes (the B operand), once per block.  A stored
-  // offset is a row part plus a column part in every layout.
-  auto row_off = [&](int r) {
-    const int ra = r / p.db_out, rb = r - ra * p.db_out;
-    switch (p.layout & 3) {
-      case 0: return r * p.kin;
-      case QSGB_PTM_SWAPPED: return (rb * p.da_out + ra) * p.kin;
-      case QSGB_PTM_TRANSPOSED: return r;
-      default: return rb * p.da_out + ra;
-    }
-  };
-  auto col_off = [&](int k) {
-    const int ka = k / p.db_in, kb = k - ka * p.db_in;
-    switch (p.layout & 3) {
-      case 0: return k;
-      case QSGB_PTM_SWAPPED: return kb * p.da_in + ka;
-      case QSGB_PTM_TRANSPOSED: return k * p.kout;
-      default: return (kb * p.da_in + ka) * p.kout;
-    }
-  };
-  int ptm_bad = 0;
-  for (int r = warp; r < p.npad; r += kWBlock / 32) {
-    unsigned e = 1u;
-    if (r < p.kout) {
-      const int ro = row_off(r);
-      for (int k = t & 31; k < p.kin; k += 32) e = max(e, exp_of(p.ptm[ro + col_off(k)]));
-    }
-    for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
-    if (e == 0x7ffu) ptm_bad = 1;
-    if ((t & 31) == 0) srow[r] = (int)e;
-  }
-  __syncthreads();
-  const int plane_b = p.ksteps * 2 * p.npad * 16;  // bytes
-  for (int u = t; u < p.npad * p.ksteps * 2; u += kWBlock) {
-    const int kc = u / p.npad, r = u - kc * p.npad;  // 8 columns of row r
-    unsigned long long f[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int k = kc * 8 + q;
-      const double v = (r < p.kout && k < p.kin) ? p.ptm[row_off(r) + col_off(k)] : 0.0;
-      f[q] = fixed9<ND, 53>(parts(v), (unsigned)srow[r]);
-    }
-#pragma unroll
-    for (int j = 0; j < ND; ++j) {
-      uint4 w;
-      const int pos = 9 * (ND - 1 - j);
-      const unsigned mask = j == 0 ? 0x3ffu : 0x1ffu;
-      w.x = digit9_pair(f[0], f[1], pos, mask);
-      w.y = digit9_pair(f[2], f[3], pos, mask);
-      w.z = digit9_pair(f[4], f[5], pos, mask);
-      w.w = digit9_pair(f[6], f[7], pos, mask);
-      *reinterpret_cast<uint4*>(smem + kWOffB + j * plane_b + (kc * p.npad + r) * 16) = w;
+    if (t < p.kout) {
+      const int ra = t / p.db_out, rb = t - ra * p.db_out;
+      goff_out[t] = ra * p.sao + rb * p.sbo;
+      soff_out[t] = ra * kWGroups * dbo + rb;
+      switch (p.layout & 3) {
+        case 0: prow[t] = t * p.kin; break;
+        case QSGB_PTM_SWAPPED: prow[t] = (rb * p.da_out + ra) * p.kin; break;
+        case QSGB_PTM_TRANSPOSED: prow[t] = t; break;
+        default: prow[t] = rb * p.da_out + ra; break;
+      }
     }
   }
   if (warp == 0) {
@@ -255,50 +246,124 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (t == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty), "r"(kWWarps) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  pdl_wait();
+  __syncthreads();
+
+  // ---- the PTM's digit planes (the B operand), once per block
+  int ptm_bad = 0;
+  for (int r = warp; r < npad; r += kWWarps) {
+    unsigned e = 0u, nz = 0u;
+    if (r < p.kout) {
+      const int ro = prow[r];
+      for (int k = t & 31; k < p.kin; k += 32) {
+        const double v = p.ptm[ro + pcol[k]];
+        e = max(e, exp_of(v));
+        nz |= v != 0.0 ? 1u : 0u;
+      }
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    nz = __reduce_or_sync(0xffffffffu, nz);
+    // inf, nan, or a non-zero row below the smallest scale
+    if (e == 0x7ffu || (e < kMinExp && nz)) ptm_bad = 1;
+    if (e < kMinExp) e = 1023u;  // any scale serves a row of zeros
+    if ((t & 31) == 0) srow[r] = (int)e;
+  }
+  __syncthreads();
+  const int plane_b = p.ksteps * 2 * npad * 16;  // bytes
+  for (int u = t; u < npad * p.ksteps * 2; u += kWBlock) {
+    const int kc = u / npad, r = u - kc * npad;  // 8 columns of row r
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int k = kc * 8 + q;
+      v[q] = (r < p.kout && k < p.kin) ? p.ptm[prow[r] + pcol[k]] : 0.0;
+    }
+    unsigned long long f[8];
+    Signs s[4];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) f[q] = fixed_bytes<PL>(v[q], (unsigned)srow[r]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s[q] = signs_of(sign_word(v[2 * q]), sign_word(v[2 * q + 1]));
+    store_ptm_planes<PL, 0>(smem + kWOffB + (kc * npad + r) * 16, plane_b, f, s);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   ptm_bad = __syncthreads_or(ptm_bad);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  int rmin = srow[0], rmax = srow[0];  // row scales, least and greatest
+  for (int r = 1; r < p.kout; ++r) {
+    rmin = min(rmin, srow[r]);
+    rmax = max(rmax, srow[r]);
+  }
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + kWOffTmem);
+  const uint32_t utmem = __shfl_sync(0xffffffffu, tmem, 0);  // warp-uniform
+  const int uwarp = __shfl_sync(0xffffffffu, warp, 0);
   const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
   const uint32_t idesc =
-      (1u << 4) | ((uint32_t)(p.npad >> 3) << 17) | ((128u >> 4) << 24);  // D F32, A and B F16, K-major
+      (1u << 4) | ((uint32_t)(nhalf >> 3) << 17) | ((128u >> 4) << 24);  // D F32, A and B F16, K-major
 
-  // level L: every digit pair i + j = L over all K steps into buffer L & 1
-  auto issue_level = [&](int L) {
-    const uint32_t d = tmem + (uint32_t)(kDCol + (L & 1) * p.npad);
-    for (int i = 0; i <= L; ++i) {  // PTM plane i, input plane L - i
-      const uint32_t a0 = tmem + (uint32_t)((L - i) * kPlaneCols);
-      const uint32_t b0 = sbase + kWOffB + i * plane_b;
-      for (int ks = 0; ks < p.ksteps; ++ks) {
-        const unsigned long long bdesc = wide_desc(b0 + ks * 2 * p.npad * 16, p.npad);
-        const uint32_t accumulate = (i | ks) ? 1u : 0u;
-        asm volatile(
-            "{ .reg .pred q; setp.ne.u32 q, %4, 0; "
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, q; }" ::"r"(d),
-            "r"(a0 + 8u * (uint32_t)ks), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-      }
-    }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar + 8 * (L & 1))
-                 : "memory");
-  };
-  uint32_t phases = 0u;  // bit b: parity of barrier b's next completion
-  auto wait_bar = [&](int b) -> bool {
-    uint32_t done = 0;
+  bool dead = false;  // a wait of this thread ran out
+  auto wait_bar = [&](uint32_t bar, uint32_t parity) {
+    uint32_t done = dead ? 1u : 0u;
     for (long long spin = 0; spin < kWSpinLimit && !done; ++spin)
       asm volatile(
           "{ .reg .pred q; mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }"
           : "=r"(done)
-          : "r"(bar + 8 * b), "r"((phases >> b) & 1u)
+          : "r"(bar), "r"(parity)
           : "memory");
-    phases ^= 1u << b;
-    __syncwarp();  // the tensor-memory loads that follow are warp-wide
-    return done != 0u;
+    dead = dead || !done;
+  };
+  // Group g of the block (kGroups per half of the outputs, tile after tile):
+  // up to three consecutive levels, one accumulator buffer each, their MMAs
+  // interleaved: an MMA that adds to the accumulator of the one before waits
+  // for it (~130 cycles at N = 48).  The whole of warp 0 runs this, so that the
+  // operands stay warp-uniform, and one elected lane issues; loops are unrolled
+  // over the K steps, whose descriptors differ by a constant.
+  auto issue_group = [&](uint32_t g, int half, int L0) {
+    if (g > 0) wait_bar(empty, (g - 1) & 1u);  // the buffers' last contents have been read
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned long long dk = (unsigned long long)(2 * npad);      // per K step, in 16-byte units
+    const unsigned long long dp = (unsigned long long)(plane_b >> 4);  // per plane
+    uint32_t a0[kWBufs];
+    unsigned long long b0[kWBufs];
+    int cnt[kWBufs];
+#pragma unroll
+    for (int l = 0; l < kWBufs; ++l) {  // PTM planes i0 .. i1 with input planes L - i
+      const int L = L0 + l;
+      const int i0 = L > PL - 1 ? L - (PL - 1) : 0, i1 = L < PL - 1 ? L : PL - 1;
+      cnt[l] = L < LV ? i1 - i0 + 1 : 0;
+      a0[l] = utmem + (uint32_t)((L - i0) * kPlaneCols);
+      b0[l] = wide_desc(sbase + kWOffB + i0 * plane_b + half * nhalf * 16, npad);
+    }
+    for (int i = 0; i < PL; ++i) {
+#pragma unroll
+      for (int ks = 0; ks < KQ / 4; ++ks) {
+        if (ks < p.ksteps) {
+#pragma unroll
+          for (int l = 0; l < kWBufs; ++l)
+            if (i < cnt[l])
+              asm volatile(
+                  "{ .reg .pred e, q; elect.sync _|e, 0xffffffff; setp.ne.u32 q, %4, 0; "
+                  "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, q; }" ::"r"(utmem + (uint32_t)(kDCol + 48 * l)),
+                  "r"(a0[l] + 8u * (uint32_t)ks), "l"(b0[l] + dk * (unsigned)ks), "r"(idesc), "r"(i > 0 || ks > 0 ? 1 : 0)
+                  : "memory");
+        }
+      }
+#pragma unroll
+      for (int l = 0; l < kWBufs; ++l) {
+        a0[l] -= (uint32_t)kPlaneCols;
+        b0[l] += dp;
+      }
+    }
+    asm volatile(
+        "{ .reg .pred e; elect.sync _|e, 0xffffffff; "
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0]; }" ::"r"(full)
+        : "memory");
   };
   // copies of a staged tile: element e of the run of ka (all groups of the
   // tile, db consecutive elements each), thread by thread
@@ -325,7 +390,8 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
     }
   };
 
-  bool timed_out = false;
+  constexpr int kGroups = (LV + kWBufs - 1) / kWBufs;  // of levels, per half
+  uint32_t group = 0;  // groups issued so far
   for (uint64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
     const uint64_t gi = tile * kWGroups + gl;
     const bool live = gi < p.n_groups;
@@ -350,133 +416,157 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
       __syncthreads();
     }
     // ---- this thread's inputs, the group's exponent, the digits
-    unsigned emax = 1u;
+    unsigned emax = 0u;
     {
-      T x[kHalf];
+      T x[KQ];
 #pragma unroll
-      for (int j = 0; j < kHalf; ++j) {
-        const int k = h * kHalf + j;
+      for (int j = 0; j < KQ; ++j) {
+        const int k = h * KQ + j;
         x[j] = (T)0;
         if (live && k < p.kin) x[j] = p.staged ? stage[soff_in[k] + gl * dbi] : in[bi + goff_in[k]];
-        emax = max(emax, exp_of(x[j]));
+      }
+#pragma unroll
+      for (int j = 0; j < KQ; ++j) emax = max(emax, exp_of(x[j]));
+      if (emax < kMinX) {  // bit 16: a non-zero value
+#pragma unroll
+        for (int j = 0; j < KQ; ++j) emax |= x[j] != (T)0 ? 0x10000u : 0u;
       }
       semax[h * kWGroups + gl] = emax;
       __syncthreads();
-      emax = max(emax, semax[(h ^ 1) * kWGroups + gl]);
+      unsigned some = 0u;
+      emax = 0u;
 #pragma unroll
-      for (int b = 0; b < KH; ++b) {  // 8 inputs: 4 columns of every plane
-        unsigned long long u[8];
+      for (int q = 0; q < kWParts; ++q) {
+        const unsigned e = semax[q * kWGroups + gl];
+        some |= e;
+        emax = max(emax, e & 0xffffu);
+      }
+      // below the smallest scale: recomputed; all zero: any scale serves
+      if (emax < kMinX) emax = some >= 0x10000u ? kExpAll : (F64 ? 1023u : 127u);
+      if (h * KQ < 16 * p.ksteps) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) u[q] = fixed9<ND, MB>(parts(x[8 * b + q]), emax);
+        for (int b = 0; b < KQ / 8; ++b) {  // 8 inputs: 4 columns of every plane
+          unsigned long long u[8];
+          Signs s[4];
 #pragma unroll
-        for (int j = 0; j < ND; ++j) {
-          const int pos = 9 * (ND - 1 - j);
-          const unsigned mask = j == 0 ? 0x3ffu : 0x1ffu;
-          unsigned w[4];
+          for (int q = 0; q < 8; ++q) u[q] = fixed_bytes<PL>(x[8 * b + q], emax);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) w[q] = digit9_pair(u[2 * q], u[2 * q + 1], pos, mask);
-          tmem_st4(tlane + (uint32_t)(j * kPlaneCols + h * 4 * KH + 4 * b), w);
+          for (int q = 0; q < 4; ++q) s[q] = signs_of(sign_word(x[8 * b + 2 * q]), sign_word(x[8 * b + 2 * q + 1]));
+          store_planes<PL, 0>(tlane + (uint32_t)((h * KQ + 8 * b) / 2), (uint32_t)kPlaneCols, u, s);
         }
       }
     }
-    unsigned bad = (ptm_bad || emax == kExpAll<T>) ? 1u : 0u;
+    // inf, nan, too small a scale, or results that may leave the normal range
+    bool bad = ptm_bad || emax == kExpAll;
+    // (|v| < 2^63 here, 2 bits more than scale8_ok allows for)
+    if (F64) bad = bad || !scale8_ok((int)emax + rmin - kScale8) || !scale8_ok((int)emax + rmax + 2 - kScale8);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (t == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      issue_level(0);
-      issue_level(1);
-    }
-    // ---- levels: V = sum_L A_L 2^(top - 9 L)
-    long long v[kHalf];
-#pragma unroll
-    for (int j = 0; j < kHalf; ++j) v[j] = 0;
+    if (uwarp == 0) issue_group(group, 0, 0);
+    // ---- the outputs, half after half, level group after level group
 #pragma unroll 1
-    for (int L = 0; L < ND; ++L) {
-      const bool done = wait_bar(L & 1);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int sh = (F64 ? 40 : 27) - 9 * L;  // F64: 40, 31, 22, 13, 4, -5
-      const uint32_t col = tlane + (uint32_t)(kDCol + (L & 1) * p.npad + h * kHalf);
+    for (int half = 0; half < 2; ++half) {
+      long long v[kMaxOut];
+      int pr[kMaxOut];
 #pragma unroll
-      for (int b = 0; b < KH; ++b) {
-        if (h * kHalf + 8 * b < p.kout) {
-          uint32_t w[8];
-          tmem_ld8(col + 8 * b, w);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (sh >= 0) {
+      for (int j = 0; j < kMaxOut; ++j) v[j] = 0;
+      const int col = h * (nhalf >> 2);  // this thread's first column of the half
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[8 * b + q] += (long long)__float2int_rn(__uint_as_float(w[q])) << sh;
-          } else {
+      for (int G = 0; G < kGroups; ++G) {
+        wait_bar(full, group & 1u);
+        __syncwarp();  // the tensor-memory loads are warp-wide
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        float w[kWBufs][3][4];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[8 * b + q] += (long long)(__float2int_rn(__uint_as_float(w[q])) >> -sh);
+        for (int l = 0; l < kWBufs; ++l)
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            if (G * kWBufs + l < LV && 16 * c < nhalf)
+              tmem_ld4(tlane + (uint32_t)(kDCol + 48 * l + col + 4 * c), w[l][c]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if ((t & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty) : "memory");
+        ++group;
+        if (uwarp == 0 && (G + 1 < kGroups || half == 0))
+          issue_group(group, G + 1 < kGroups ? half : 1, G + 1 < kGroups ? (G + 1) * kWBufs : 0);
+        // levels 0 and 1 stay below 2^22: the magic number; F2I for the others
+#pragma unroll
+        for (int l = 0; l < kWBufs; ++l) {
+          const int L = G * kWBufs + l;
+          if (L < LV) {
+#pragma unroll
+            for (int j = 0; j < kMaxOut; ++j) {
+              const float a = w[l][j >> 2][j & 3];
+              const int i = L <= 1 ? (int)(level_bits(a) - kMagic) : __float2int_rn(a);
+              if (L == 6)  // seven pairs of K = 96 may fill 32 bits: scaled first
+                pr[j] = i >> 6;
+              else if (L == 7)
+                pr[j] += i >> 14;
+              else
+                pr[j] = (L & 1) ? pr[j] + i : i << 8;
+              // V = sum_L A_L 2^(top - 8 L)
+              if (F64) {
+                if (L == 1) v[j] = (long long)pr[j] << 34;
+                if (L == 3) v[j] += (long long)pr[j] * 262144ll;
+                if (L == 5) v[j] += (long long)pr[j] * 4ll;
+                if (L == 7) v[j] += (long long)pr[j];
+              } else {
+                if (L == 1) v[j] = (long long)pr[j] << 32;
+                if (L == 3) v[j] += (long long)pr[j] * 65536ll;
+                if (L == 5) v[j] += (long long)pr[j];
+              }
+            }
           }
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      if (__syncthreads_or(done ? 0 : 1)) {
-        timed_out = true;
-        phases ^= 1u << (L & 1);  // this level's commit was not seen
-        break;
+      // ---- results of this half
+#pragma unroll
+      for (int j = 0; j < kMaxOut; ++j) {
+        const int r = half * nhalf + col + j;
+        if (j < (nhalf >> 2) && r < p.kout) {
+          T y;
+          if constexpr (F64)
+            y = scale8(v[j], (unsigned)((int)emax + srow[r] - kScale8) << 20);
+          else
+            y = ldexpf(__ll2float_rn(v[j]), (int)emax + srow[r] - 1202);
+          if (p.staged)
+            stage[soff_out[r] + gl * dbo] = y;
+          else if (live)
+            out[bo + goff_out[r]] = y;
+        }
       }
-      if (t == 0 && L + 2 < ND) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        issue_level(L + 2);
+      if (bad && live) {
+        // this thread's outputs again, in the storage type's plain arithmetic
+#pragma unroll 1
+        for (int j = 0; j < (nhalf >> 2); ++j) {
+          const int r = half * nhalf + col + j;
+          if (r >= p.kout) break;
+          T a = (T)0;
+#pragma unroll 1
+          for (int k = 0; k < p.kin; ++k) a = fma((T)p.ptm[prow[r] + pcol[k]], in[bi + goff_in[k]], a);
+          if (p.staged)
+            stage[soff_out[r] + gl * dbo] = a;
+          else
+            out[bo + goff_out[r]] = a;
+        }
       }
     }
-    if (timed_out) {
-      // bounded waits for the MMAs in flight (this level's and the next
-      // one's) before the tensor memory is freed
-      if (t == 0 && p.status) atomicOr(p.status, QSGB_DEV_TIMEOUT);
-      wait_bar(0);
-      wait_bar(1);
+    if (__syncthreads_or(dead ? 1 : 0)) {
+      dead = true;
       break;
     }
-    // ---- results
-    const int sc0 = (int)emax - (F64 ? 2100 : 1191);
-#pragma unroll
-    for (int j = 0; j < kHalf; ++j) {
-      const int r = h * kHalf + j;
-      if (r < p.kout) {
-        T y = (T)0;
-        if (v[j] != 0) {
-          const int sc = sc0 + srow[r];
-          if constexpr (F64) {
-            const double d = __ll2double_rn(v[j]);
-            const int hi = __double2hiint(d);
-            const int e = ((hi >> 20) & 0x7ff) + sc;
-            bad |= (e < 1 || e > 2046) ? 1u : 0u;
-            y = __hiloint2double(hi + (sc << 20), __double2loint(d));
-          } else {
-            y = ldexpf(__ll2float_rn(v[j]), sc);
-          }
-        }
-        if (p.staged)
-          stage[soff_out[r] + gl * dbo] = y;
-        else if (live)
-          out[bo + goff_out[r]] = y;
-      }
-    }
-    if (bad && live) {
-      // inf or nan inputs or results outside the normal range: this thread's
-      // outputs again, in the storage type's plain arithmetic
-#pragma unroll 1
-      for (int r = h * kHalf; r < (h + 1) * kHalf && r < p.kout; ++r) {
-        T a = (T)0;
-        const int ro = row_off(r);
-#pragma unroll 1
-        for (int k = 0; k < p.kin; ++k) a = fma((T)p.ptm[ro + col_off(k)], in[bi + goff_in[k]], a);
-        if (p.staged)
-          stage[soff_out[r] + gl * dbo] = a;
-        else
-          out[bo + goff_out[r]] = a;
-      }
-    }
     if (p.staged) {
-      __syncthreads();
       staged_copy(false, nv);
       __syncthreads();  // the tables and the tile are free
     }
+  }
+  if (dead) {
+    // a wait ran out: bounded waits for the MMAs that may be in flight before
+    // the tensor memory is freed
+    if (t == 0 && p.status) atomicOr(p.status, QSGB_DEV_TIMEOUT);
+    dead = false;
+    wait_bar(full, group & 1u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -486,10 +576,10 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
   }
 }
 
-template <typename T, int KH>
+template <typename T, int KQ>
 int wide_launch(WideParams& p, cudaStream_t stream) {
-  constexpr int ND = sizeof(T) == 8 ? 6 : 4;
-  const int planes = ND * p.ksteps * 2 * p.npad * 16;
+  constexpr int PL = sizeof(T) == 8 ? 7 : 5;
+  const int planes = PL * p.ksteps * 2 * 2 * p.nhalf * 16;
   p.off_stage = kWOffB + planes;
   int smem = p.off_stage;
   if (p.staged) {
@@ -500,10 +590,10 @@ int wide_launch(WideParams& p, cudaStream_t stream) {
     else
       p.staged = 0;
   }
-  const int st = allow_dynamic_smem((const void*)apply_wide_kernel<T, KH>, smem);
+  const int st = allow_dynamic_smem((const void*)apply_wide_kernel<T, KQ>, smem);
   if (st != QSGB_OK) return st;
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(p.n_tiles, (uint64_t)sm_count()));
-  return launch_pdl(apply_wide_kernel<T, KH>, grid, kWBlock, smem, stream, p);
+  return launch_pdl(apply_wide_kernel<T, KQ>, grid, kWBlock, smem, stream, p);
 }
 
 }  // namespace
@@ -522,7 +612,7 @@ int launch_wide(const double* dptm, int layout, const void* in, void* out, int d
   p.da_out = da_out;
   p.db_out = db_out;
   p.layout = layout & 3;
-  p.npad = (p.kout + 15) / 16 * 16;
+  p.nhalf = (p.kout + 31) / 32 * 16;
   p.ksteps = (p.kin + 15) / 16;
   p.staged = Z == 1 ? 1 : 0;
   p.n_groups = X * Y * Z;
@@ -537,9 +627,9 @@ int launch_wide(const double* dptm, int layout, const void* in, void* out, int d
   p.syo = db_out * (int64_t)Z;
   p.sao = (int64_t)(Y * db_out * Z);
   p.sxo = (int64_t)da_out * p.sao;
-  const bool small = p.npad <= 48 && p.ksteps <= 3;
-  if (dtype == QSGB_F64) return small ? wide_launch<double, 3>(p, stream) : wide_launch<double, 6>(p, stream);
-  return small ? wide_launch<float, 3>(p, stream) : wide_launch<float, 6>(p, stream);
+  const bool small = p.ksteps <= 4;
+  if (dtype == QSGB_F64) return small ? wide_launch<double, 16>(p, stream) : wide_launch<double, 24>(p, stream);
+  return small ? wide_launch<float, 16>(p, stream) : wide_launch<float, 24>(p, stream);
 }
 
 }  // namespace tc

@@ -541,6 +541,42 @@ def eager_apply(pv, ptm, plan, arith, out=None):
     return out
 
 
+# a host PTM with more entries may exceed what the specialised kernels take
+# (jit::kMaxJitTerms terms)
+MAX_JIT_TERMS = 1024
+
+
+def eager_apply_dense(pv, ptm, plan, arith, out=None):
+    """eager_apply for a host PTM of more than MAX_JIT_TERMS terms: the
+    library's kernels for such PTMs read it from device memory.  The copy goes
+    through a page-locked block of torch's host allocator, which keeps it until
+    the copy is done, so the call does not wait for the stream.  None when the
+    request needs eager_apply or the general operator path (fewer terms, a
+    capture, whose replays would read that block later)."""
+    if np.count_nonzero(ptm) <= MAX_JIT_TERMS or \
+            torch.cuda.is_current_stream_capturing():
+        return None
+    ptm = np.ascontiguousarray(ptm, dtype=np.float64)
+    terms = nnz_terms(ptm, arith)
+    if terms <= MAX_JIT_TERMS:
+        return None
+    new_shape, two, sizes, flags, code = plan
+    if out is None:
+        out = torch.empty(new_shape, dtype=pv.dtype, device=pv.device)
+    if out.numel() == 0:
+        return out
+    dev = torch.from_numpy(ptm).pin_memory().to(pv.device, non_blocking=True)
+    idx = pv.device.index
+    stream = _RAW_STREAM(idx) if _RAW_STREAM is not None else \
+        torch.cuda.current_stream(pv.device).cuda_stream
+    lib = L.load()
+    fn = lib.qsgb_apply_ptm2 if two else lib.qsgb_apply_ptm1
+    st = fn(pv.data_ptr(), out.data_ptr(), dev.data_ptr(), *sizes,
+            flags & ~L.PTM_HOST, code, arith, terms, status_ptr(idx), stream)
+    L.check(st, 'qsgb_apply_ptm')
+    return out
+
+
 def diag_marginals(pv, plan_arrays, axis):
     """Marginals (axis >= 0) or trace (axis == -1) of the DM diagonal of the
     CUDA tensor `pv` through the gather plan, in one launch and one

@@ -298,7 +298,12 @@ class PauliVectorGB300(_Base):
             work = self._work
             if work is not None and work.shape != plan[0]:
                 self._work = work = None
-            out = ops.eager_apply(data, ptm, plan, self._arith, work)
+            out = None
+            if ptm.size > ops.MAX_JIT_TERMS:
+                out = ops.eager_apply_dense(data, ptm, plan, self._arith,
+                                            work)
+            if out is None:
+                out = ops.eager_apply(data, ptm, plan, self._arith, work)
             if out is not None:
                 self._work = data if self._owned else None
                 self._data = out

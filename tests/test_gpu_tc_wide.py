@@ -3,12 +3,13 @@ one group, a partial last tile and several tiles, strides with the less
 significant target last (tiles through shared memory) and not, odd and even
 dimensions, rectangular PTMs, FP64 and FP32.
 
-Bound, derived from the split, with at most 81 terms: 54-bit fixed point per
-row and group (36 bits for FP32) truncates each factor by 2^-53 (2^-35) of its
-maximum, and the digit pairs beyond the last level add 5 * 2^-54 (3 * 2^-36)
-a term, so FP64 errs by less than 81 * 9 * 2^-54 < 2^-44 of
+Bound, derived from the split, with at most 81 terms: the fixed point of a row
+or group truncates each factor by at most 2^-53 (FP32: 2^-35) of its maximum,
+and the digit pairs beyond the last level add at most 5 * 2^-54 (3 * 2^-36) a
+term, so FP64 errs by less than 81 * 9 * 2^-54 < 2^-44 of
 max_k |P_rk| max_k |x_k| plus the rounding of the result, FP32 by
-81 * 7 * 2^-36 < 2^-26 of it plus 2^-24 of the result."""
+81 * 7 * 2^-36 < 2^-26 of it plus 2^-24 of the result.  (The digits are finer
+than that: 55 and 39 bits.)"""
 import zlib
 
 import numpy as np

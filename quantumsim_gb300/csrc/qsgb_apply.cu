@@ -779,6 +779,15 @@ int try_jit(const double* ptm_host, int64_t da_out, int64_t db_out, int64_t da_i
   const bool contiguous = Z == 1 && (p.div_y.d == 1 || (da_in == 1 && da_out == 1)) &&
                           (uintptr_t)p.in % 16 == 0 && (uintptr_t)p.out % 16 == 0;
   const int vin = vwidth(db_in, p.in), vout = vwidth(db_out, p.out);
+  // vectors too small to fill the device get kernels of their own
+  // (jit::split_rows); the class is the power of two of their groups
+  const uint64_t groups = p.n_items * (pair ? 2 : 1);
+  unsigned char size_class = 0;
+  if (dtype == QSGB_F64 && groups <= (uint64_t)sm_count() * 256) {
+    size_class = 1;
+    while (groups > 1ull << (size_class - 1)) ++size_class;
+  }
+  const bool small = size_class != 0;
   // the cached kernel and term list of this geometry class and term mask
   // (the rule of jit::make_spec: entries above 2^-52 of the largest, 2^-30
   // for FP32, non-zero for native FP64 or a PTM outside [2^-100, 2^100])
@@ -795,7 +804,7 @@ int try_jit(const double* ptm_host, int64_t da_out, int64_t db_out, int64_t da_i
                                    (unsigned char)db_in, (unsigned char)(flags & 3), (unsigned char)dtype,
                                    (unsigned char)eff, (unsigned char)pair, (unsigned char)(Z == 1),
                                    (unsigned char)contiguous, (unsigned char)vin, (unsigned char)vout,
-                                   (unsigned char)(mode == kLaunch), 0, 0, 0};
+                                   (unsigned char)(mode == kLaunch), size_class, 0, 0};
     std::memcpy(key.hdr, hdr, sizeof hdr);
     key.nwords = (ne + 63) / 64;
     for (int w = 0; w < key.nwords; ++w) key.mask[w] = 0;
@@ -844,6 +853,18 @@ int try_jit(const double* ptm_host, int64_t da_out, int64_t db_out, int64_t da_i
     if (!jit::make_spec(ptm_host, (int)da_out, (int)db_out, (int)da_in, (int)db_in, flags & 3, dtype, arith, false,
                         Z == 1, contiguous, vin, vout, spec, coef))
       return QSGB_ERR_UNSUPPORTED;
+  }
+  // a small vector: single groups, and an item's rows over several threads
+  // when that brings more of the device to work
+  if (small) {
+    if (spec.pair &&
+        !jit::make_spec(ptm_host, (int)da_out, (int)db_out, (int)da_in, (int)db_in, flags & 3, dtype, arith, false,
+                        Z == 1, contiguous, vin, vout, spec, coef))
+      return QSGB_ERR_UNSUPPORTED;
+    if (arith == QSGB_ARITH_AUTO)
+      jit::small_in_fp64(spec, coef, ptm_host, (int)da_out, (int)db_out, (int)da_in, (int)db_in, flags & 3,
+                         1ull << (size_class - 1));
+    jit::split_rows(spec, 1ull << (size_class - 1));
   }
   if (mode == kPrepare) return jit::prepare(spec);
   if (mode == kCompileOnly) return jit::compile_only(spec, src_out);

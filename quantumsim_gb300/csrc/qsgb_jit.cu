@@ -130,6 +130,33 @@ std::vector<int> row_order(const Spec& s) {
   return order;
 }
 
+// Order in which rows are emitted.
+std::vector<int> emit_order(const Spec& s) {
+  if (s.lookahead < s.kin) return row_order(s);
+  std::vector<int> order(s.kout);
+  for (int r = 0; r < s.kout; ++r) order[r] = r;
+  return order;
+}
+
+// Part of every row: contiguous shares of the emission order with about equal
+// work (a row's terms and its fixed cost), groups of vout rows kept together.
+std::vector<int> row_parts(const Spec& s) {
+  std::vector<int> part(s.kout, 0);
+  if (s.parts <= 1) return part;
+  const std::vector<int> order = emit_order(s);
+  auto weight = [&](int r) { return s.mode[r] == kModeDF ? 10 * (int)s.cols[r].size() + 40 : 4 * (int)s.cols[r].size() + 4; };
+  long long total = 0, before = 0;
+  for (int r = 0; r < s.kout; ++r) total += weight(r);
+  for (int i = 0; i < s.kout; i += s.vout) {
+    long long w = 0;
+    for (int j = 0; j < s.vout; ++j) w += weight(order[i + j]);
+    const int q = (int)std::min<long long>(s.parts - 1, (2 * before + w) * s.parts / (2 * std::max<long long>(total, 1)));
+    for (int j = 0; j < s.vout; ++j) part[order[i + j]] = q;
+    before += w;
+  }
+  return part;
+}
+
 // A staged kernel writes each component's results over the tile slots of
 // their own row indices; that is safe when no later component reads those
 // slots as inputs.
@@ -172,11 +199,13 @@ std::string gen_source(const Spec& s) {
   if (std::count(s.mode.begin(), s.mode.end(), (int)kModeDF) > 0) {
     std::string tk, te, td;
     int t = 0;
+    const std::vector<int> part = row_parts(s);
     for (int r = 0; r < s.kout; ++r) {
       for (int k : s.cols[r]) tk += std::to_string(k) + ",";
       t += (int)s.cols[r].size();
       te += std::to_string(t) + ",";
-      td += s.mode[r] == kModeDF ? "1," : "0,";
+      // 0: not a float-float row, else 1 + the part that computes it
+      td += std::to_string(s.mode[r] == kModeDF ? 1 + part[r] : 0) + ",";
     }
     if (tk.empty()) tk = "0,";
     src += "__constant__ unsigned short qfb_k[] = {" + tk + "};\n";
@@ -189,7 +218,7 @@ std::string gen_source(const Spec& s) {
                   "#pragma unroll 1\n"
                   "      for (int r = 0; r < %d; ++r) {\n"
                   "        const unsigned te = qfb_end[r];\n"
-                  "        if (!qfb_df[r]) { tq = te; continue; }\n"
+                  "        if (%s) { tq = te; continue; }\n"
                   "        double a0 = 0.0, a1 = 0.0;\n"
                   "#pragma unroll 1\n"
                   "        for (; tq < te; ++tq) {\n"
@@ -201,7 +230,8 @@ std::string gen_source(const Spec& s) {
                   "%s"
                   "      }\n"
                   "    }\n",
-                  staged ? " && lane < nv" : "", s.kout, s.db_in, s.db_in, staged ? "1" : "p.h.sbi",
+                  staged ? " && lane < nv" : "", s.kout, s.parts > 1 ? "qfb_df[r] != blockIdx.y + 1" : "!qfb_df[r]", s.db_in,
+                  s.db_in, staged ? "1" : "p.h.sbi",
                   s.pair ? "          a0 = fma(cf, xv.x, a0); a1 = fma(cf, xv.y, a1);\n"
                          : "          a0 = fma(cf, xv, a0);\n",
                   "");
@@ -377,21 +407,16 @@ std::string gen_source(const Spec& s) {
   // few inputs ahead of its first use, so the live registers of an item are
   // those of a few components rather than all Kin inputs.  Every result is
   // stored as soon as it (or its vector of vout results) is complete.
-  std::vector<int> order(s.kout);
-  if (s.lookahead >= s.kin) {
-    for (int r = 0; r < s.kout; ++r) order[r] = r;
-  } else {
-    order = row_order(s);
-  }
+  const std::vector<int> all_rows = emit_order(s);
   // comp_last[r]: r is the last row (in `order`) of its component; with all
   // inputs loaded first the whole row set counts as one component
   std::vector<char> comp_last(s.kout, 0);
   {
     const std::vector<int> comp = row_components(s);
-    for (size_t i = 0; i < order.size(); ++i) {
-      const bool last = i + 1 == order.size() ||
-                        (s.lookahead < s.kin && comp[order[i + 1]] != comp[order[i]]);
-      comp_last[order[i]] = last ? 1 : 0;
+    for (size_t i = 0; i < all_rows.size(); ++i) {
+      const bool last = i + 1 == all_rows.size() ||
+                        (s.lookahead < s.kin && comp[all_rows[i + 1]] != comp[all_rows[i]]);
+      comp_last[all_rows[i]] = last ? 1 : 0;
     }
   }
   std::vector<int> pending;
@@ -432,7 +457,19 @@ std::string gen_source(const Spec& s) {
       src += buf;
     }
   };
-  for (int r = 0; r < s.kout; ++r) {
+  const std::vector<int> part_of = row_parts(s);
+  for (int part = 0; part < s.parts; ++part) {
+  // with parts, a thread computes the rows of part blockIdx.y
+  std::vector<int> order;
+  for (int r : all_rows)
+    if (part_of[r] == part) order.push_back(r);
+  if (s.parts > 1) {
+    std::snprintf(buf, sizeof buf, "    if (blockIdx.y == %du) {\n", (unsigned)part);
+    src += buf;
+    loaded.assign(s.kin, 0);
+    splitd.assign(s.kin, 0);
+  }
+  for (int r : order) {
     std::snprintf(buf, sizeof buf, "    V y%d;\n", r);
     src += buf;
   }
@@ -454,7 +491,7 @@ std::string gen_source(const Spec& s) {
   };
   load_upto((size_t)s.lookahead);
   if (s.lookahead >= s.kin) {  // small items: everything loaded and split up front
-    for (int r = 0; r < s.kout; ++r)
+    for (int r : order)
       if (s.mode[r] == kModeDF)
         for (int k : s.cols[r]) split_input(k);
   }
@@ -543,6 +580,8 @@ std::string gen_source(const Spec& s) {
       std::snprintf(buf, sizeof buf, "    out[bo + %dLL * p.h.sao + %dLL * p.h.sbo] = y%d;\n", ra, rb, r);
       src += buf;
     }
+  }
+  if (s.parts > 1) src += "    }\n";
   }
   if (s.stage_warps) {
     src += fallback;
@@ -804,6 +843,20 @@ int Spec::n_coef() const {
 // 9 to 11 is a plateau before a cliff at 12.
 int lookahead_for(int kin, bool pair) { return kin * (pair ? 2 : 1) <= 36 ? kin : 10; }
 
+namespace {
+// Offset of op element (r, k) in a PTM stored in `layout`.
+int stored_index(int r, int k, int da_out, int db_out, int da_in, int db_in, int layout) {
+  const int kin = da_in * db_in, kout = da_out * db_out;
+  const int ra = r / db_out, rb = r % db_out, ka = k / db_in, kb = k % db_in;
+  switch (layout & 3) {
+    case 0: return r * kin + k;
+    case QSGB_PTM_SWAPPED: return ((rb * da_out + ra) * db_in + kb) * da_in + ka;
+    case QSGB_PTM_TRANSPOSED: return k * kout + r;
+    default: return ((kb * da_in + ka) * db_out + rb) * da_out + ra;
+  }
+}
+}  // namespace
+
 bool make_spec(const double* ptm_host, int da_out, int db_out, int da_in, int db_in, int layout, int dtype,
                int arith, bool pair, bool z1, bool contiguous, int vin, int vout, Spec& spec,
                std::vector<double>& coef) {
@@ -814,15 +867,7 @@ bool make_spec(const double* ptm_host, int da_out, int db_out, int da_in, int db
   double amax = 0.0;
   for (int r = 0; r < kout; ++r)
     for (int k = 0; k < kin; ++k) {
-      const int ra = r / db_out, rb = r % db_out;
-      const int ka = k / db_in, kb = k % db_in;
-      int idx;
-      switch (layout & 3) {
-        case 0: idx = r * kin + k; break;
-        case QSGB_PTM_SWAPPED: idx = ((rb * da_out + ra) * db_in + kb) * da_in + ka; break;
-        case QSGB_PTM_TRANSPOSED: idx = k * kout + r; break;
-        default: idx = ((kb * da_in + ka) * db_out + rb) * da_out + ra; break;
-      }
+      const int idx = stored_index(r, k, da_out, db_out, da_in, db_in, layout);
       const double v = ptm_host[idx];
       M[(size_t)r * kin + k] = v;
       amax = std::max(amax, std::fabs(v));
@@ -850,6 +895,7 @@ bool make_spec(const double* ptm_host, int da_out, int db_out, int da_in, int db
   // memory, as many warps per block as fit 48 KB of tiles (at most 4)
   spec.stage_warps = 0;
   spec.stage_bulk = false;
+  spec.parts = 1;
   // (measured on GB300: staging instead of 32-byte vector accesses loses 20 %
   // on a 16x16 PTM on the last two qubits, 5453 -> 4324 GB/s)
   if (z1 && !pair && (vin == 1 || vout == 1) && staged_in_place_ok(spec)) {
@@ -878,6 +924,47 @@ bool make_spec(const double* ptm_host, int da_out, int db_out, int da_in, int db
   return true;
 }
 
+// Below a few warps per SM sub-partition a pass takes as long as one thread's
+// chain: load, split, every row of the item.  The rows then go to up to eight
+// threads, which read the inputs they need each (from L2: such vectors are
+// small).  Measured on GB300, us in a graph, one thread an item / split: 7
+// qubits, noisy CZ 2.8 / 1.65, 3.1 terms 2.6 / 2.0, 6.2 terms 3.4 / 2.1; 9
+// qubits 2.9 / 2.0, 2.6 / 2.7, 3.5 / 3.1.  With vector accesses along the last
+// qudit (Z == 1) the parts have 4 rows each and gain up to 8 qubits only.
+bool split_rows(Spec& s, unsigned long long n_items) {
+  if (s.stage_warps > 0 || (s.vout > 1 && s.lookahead < s.kin)) return false;
+  const unsigned long long enough = (unsigned long long)sm_count() * (s.vout > 1 ? 128 : 512);
+  int parts = 1;
+  while (parts < 8 && 2 * parts * s.vout <= s.kout && n_items * (unsigned long long)(2 * parts) <= enough) parts *= 2;
+  if (parts == 1) return false;
+  s.parts = parts;
+  return true;
+}
+
+// Rows of up to 2.5 terms on average and at most 2^19 FP64 multiply-adds (0.9 us
+// of the device's FP64 pipes): a thread's few rows are shorter in native FP64
+// than in float-float (no splits, no rounding), and exact to the last
+// rounding.  Longer rows are not: a warp's FP64 instruction takes 64 cycles of
+// its sub-partition.  Measured on GB300, us in a graph, 7 qubits, float-float /
+// FP64 with the rows split over threads: rotation 1.43 / 1.28, noisy CZ 1.65 /
+// 1.42, 3.1 terms 2.0 / 2.3, 6.2 terms 2.1 / 3.2.
+bool small_in_fp64(Spec& s, std::vector<double>& coef, const double* ptm_host, int da_out, int db_out, int da_in,
+                   int db_in, int layout, unsigned long long n_items) {
+  if (s.f32 || 2 * s.n_coef() > 5 * s.kout || (unsigned long long)s.n_coef() * n_items > (1ull << 19)) return false;
+  bool changed = false;
+  size_t t = 0;
+  for (int r = 0; r < s.kout; ++r) {
+    const bool df = s.mode[r] == kModeDF;
+    if (df) s.mode[r] = kModeDP;
+    changed |= df;
+    for (int k : s.cols[r]) {
+      if (df) coef[t] = ptm_host[stored_index(r, k, da_out, db_out, da_in, db_in, layout)];
+      ++t;
+    }
+  }
+  return changed;
+}
+
 std::string source(const Spec& s) { return gen_source(s); }
 
 bool available() { return nvrtc().ok && !std::getenv("QSGB_NO_JIT"); }
@@ -888,7 +975,7 @@ std::string spec_key(const Spec& s) {
   std::string k;
   k.reserve(8 + 2 * s.kout + s.n_coef());
   for (int v : {s.kin, s.kout, s.db_in, s.db_out, (int)s.pair, (int)s.f32, s.vin, s.vout, s.lookahead,
-                s.stage_warps, (int)s.stage_bulk})
+                s.stage_warps, (int)s.stage_bulk, s.parts})
     k.push_back((char)v);
   for (int r = 0; r < s.kout; ++r) {
     k.push_back((char)s.mode[r]);
@@ -979,10 +1066,13 @@ int launch_blob(cudaKernel_t kern, const Spec& s, const Geometry& g, unsigned ch
   fill_header(h, g);
   std::memcpy(blob, &h, sizeof h);
   void* args[] = {blob};
-  const unsigned block = s.stage_warps ? 32u * (unsigned)s.stage_warps : 128u;
+  unsigned block = s.stage_warps ? 32u * (unsigned)s.stage_warps : 128u;
+  // few items: smaller blocks reach more SMs
+  if (!s.stage_warps)
+    while (block > 32 && g.n_items * (unsigned)s.parts < (uint64_t)block * sm_count()) block /= 2;
   const uint64_t need = (g.n_items + block - 1) / block;
   const uint64_t cap = (uint64_t)sm_count() * 16;
-  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(need, cap));
+  const dim3 grid((unsigned)std::max<uint64_t>(1, std::min(need, cap)), (unsigned)s.parts);
   // Overlapped launches take 0.3 us off each small kernel and 2.6 % off a
   // 13-qubit FP32 layer (1674 -> 1631 us); on large FP64 vectors they gain
   // nothing on sparse PTMs (14-qubit layer 14.43 against 14.41 ms) and lose
@@ -990,7 +1080,7 @@ int launch_blob(cudaKernel_t kern, const Spec& s, const Geometry& g, unsigned ch
   // qubits, 9.63 -> 9.99 ms).
   const uint64_t bytes = (uint64_t)g.n_items * (s.pair ? 2 : 1) * (uint64_t)(s.kin + s.kout) * (s.f32 ? 4 : 8);
   const bool overlap = s.f32 || bytes <= (64ull << 20);
-  return launch_pdl((const void*)kern, dim3(grid), dim3(block), 0, stream, args, overlap);
+  return launch_pdl((const void*)kern, grid, dim3(block), 0, stream, args, overlap);
 }
 
 struct FastKeyHash {
@@ -1030,17 +1120,9 @@ const FastEntry* fast_insert(const FastKey& key, const Spec& spec, int layout, i
   FastEntry e;
   if (kernel_for(spec, &e.kern, nullptr) != QSGB_OK) return nullptr;
   e.spec = spec;
-  const int kin = da_in * db_in, kout = da_out * db_out;
   for (int r = 0; r < spec.kout; ++r)
     for (int k : spec.cols[r]) {
-      const int ra = r / db_out, rb = r % db_out, ka = k / db_in, kb = k % db_in;
-      int idx;
-      switch (layout & 3) {
-        case 0: idx = r * kin + k; break;
-        case QSGB_PTM_SWAPPED: idx = ((rb * da_out + ra) * db_in + kb) * da_in + ka; break;
-        case QSGB_PTM_TRANSPOSED: idx = k * kout + r; break;
-        default: idx = ((kb * da_in + ka) * db_out + rb) * da_out + ra; break;
-      }
+      const int idx = stored_index(r, k, da_out, db_out, da_in, db_in, layout);
       e.src.push_back(idx);
       e.kind.push_back((unsigned char)spec.mode[r]);
     }

@@ -30,6 +30,7 @@ struct Spec {
   int lookahead;        // loads are emitted this many inputs ahead of first use
   int stage_warps;      // > 0: Z == 1 items staged in shared memory, warps per block
   bool stage_bulk;      // staged tiles are contiguous spans moved by bulk copies
+  int parts;            // threads per item, each with a share of the rows (blockIdx.y)
   std::vector<int> mode;               // per output row
   std::vector<std::vector<int>> cols;  // per output row: input indices of its terms
   int n_coef() const;
@@ -57,6 +58,15 @@ bool available();
 bool make_spec(const double* ptm_host, int da_out, int db_out, int da_in, int db_in, int layout, int dtype,
                int arith, bool pair, bool z1, bool contiguous, int vin, int vout, Spec& spec,
                std::vector<double>& coef);
+// Give the rows of an item to several threads when the vector has too few
+// items to fill the device (n_items: the items of the view, pairs counted as
+// one).  Returns true if `s` changed.
+bool split_rows(Spec& s, unsigned long long n_items);
+// Compute the float-float rows of `s` in native FP64 instead when the vector is
+// small enough for the FP64 pipe; `coef` is adjusted (ptm_host and the layout
+// as for make_spec).  Returns true if `s` changed.
+bool small_in_fp64(Spec& s, std::vector<double>& coef, const double* ptm_host, int da_out, int db_out, int da_in,
+                   int db_in, int layout, unsigned long long n_items);
 // CUDA source of the kernel of `s`.
 std::string source(const Spec& s);
 // Compile (or fetch from the cache) the kernel of `s`; optionally return its source.

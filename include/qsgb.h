@@ -173,6 +173,17 @@ int qsgb_gather(const void* in, void* out, int in_dtype, int out_dtype,
                 const int32_t* idx, void* stream);
 
 /*
+ * qsgb_gather to the host, widened to FP64: the n taken values and then the
+ * value of the device status word *dev_status (0 when NULL), n + 1 doubles
+ * written by the kernel straight into host_out, which must be page-locked
+ * (QSGB_ERR_UNSUPPORTED for other memory).  Waits on the stream.
+ */
+int qsgb_gather_host(const void* in, int in_dtype, int ndim,
+                     const int64_t* in_shape, const int32_t* idx_off,
+                     const int32_t* idx, const unsigned* dev_status,
+                     double* host_out, void* stream);
+
+/*
  * Take along one axis: out[o, j, i] = in[o, idx[j], i] for a tensor viewed as
  * (outer, d_in, inner).  The per-qudit basis reduction (`reduce_basis`, e.g.
  * 9 -> 3 with the computational subbasis) and `project` (-> 1 element).
@@ -246,10 +257,11 @@ int qsgb_marginals_noalloc(const double* diag, int ndim, const int64_t* shape,
  * FP32 vectors.  out[n_out] receives the value of the device status word
  * *dev_status (0 when dev_status is NULL) as it stands when the kernel runs,
  * so a single device-to-host copy of n_out + 1 doubles returns the result
- * and every earlier kernel's status bits.  With host_out != NULL the call
- * also makes that copy into host_out (pinned memory for an asynchronous
- * copy) and waits for it on the stream before returning; with NULL it
- * returns at once, the results on the device.  Diagonals of at most 2^22 entries
+ * and every earlier kernel's status bits.  With host_out != NULL the values
+ * are in host_out, too, when the call returns: page-locked memory is written
+ * by the kernel itself and watched by the host (no copy and no stream
+ * synchronisation), other memory gets a copy and a synchronisation.  With
+ * NULL the call returns at once, the results on the device.  Diagonals of at most 2^22 entries
  * and axes of at most 64 indices; larger ones return QSGB_ERR_UNSUPPORTED
  * (use qsgb_gather and qsgb_marginals).  Without scratch (below) one block
  * does the whole reduction.
@@ -283,6 +295,19 @@ int64_t qsgb_diag_marginals_scratch_bytes(void);
 int qsgb_partial_trace(const void* in, void* out, int dtype, int ndim,
                        const int64_t* shape, const int32_t* keep,
                        const double* weights, void* stream);
+
+/*
+ * The full weighted trace (no qudit kept) as a double, whatever the dtype:
+ * out[0] = sum of in[...] * prod_t weights_t[k_t] over all qudits, out[1] =
+ * the value of *dev_status (0 when NULL); host_out as in
+ * qsgb_diag_marginals.  Expectation values of operator products: weights_t[k]
+ * = Re tr(O_t P_k) (quantumsim/states/state.py:43-83).  scratch as in
+ * qsgb_diag_marginals (same buffer and rules): more than one block.
+ */
+int qsgb_expectation(const void* in, int dtype, int ndim,
+                     const int64_t* shape, const double* weights, double* out,
+                     const unsigned* dev_status, double* host_out,
+                     void* scratch, int64_t scratch_bytes, void* stream);
 
 /* x[i] *= alpha for i < n (renormalize: numpy.py:109-117, cuda.py:386-395) */
 int qsgb_scale(void* x, int dtype, int64_t n, double alpha, void* stream);

@@ -58,6 +58,8 @@ SIGNATURES = {
                                    _i64]),
     'qsgb_gather': (_int, [_c_void_p, _c_void_p, _int, _int, _int, _p_i64,
                            _p_i32, _p_i32, _c_void_p]),
+    'qsgb_gather_host': (_int, [_c_void_p, _int, _int, _p_i64, _p_i32,
+                                _p_i32, _c_void_p, _c_void_p, _c_void_p]),
     'qsgb_diag_marginals': (_int, [_c_void_p, _int, _int, _p_i64, _p_i32,
                                    _p_i32, _int, _c_void_p, _c_void_p,
                                    _c_void_p, _c_void_p, _i64, _c_void_p]),
@@ -73,6 +75,10 @@ SIGNATURES = {
     'qsgb_partial_trace': (_int, [_c_void_p, _c_void_p, _int, _int, _p_i64,
                                   _p_i32, ctypes.POINTER(ctypes.c_double),
                                   _c_void_p]),
+    'qsgb_expectation': (_int, [_c_void_p, _int, _int, _p_i64,
+                                ctypes.POINTER(ctypes.c_double), _c_void_p,
+                                _c_void_p, _c_void_p, _c_void_p, _i64,
+                                _c_void_p]),
     'qsgb_scale': (_int, [_c_void_p, _int, _i64, _dbl, _c_void_p]),
     'qsgb_scale_by_inverse': (_int, [_c_void_p, _int, _i64, _c_void_p, _dbl,
                                      _c_void_p]),

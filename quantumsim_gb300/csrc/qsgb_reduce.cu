@@ -4,6 +4,8 @@
 //
 // All reductions are deterministic (fixed trees, no floating-point atomics)
 // and accumulate in FP64 for both storage types.
+#include <time.h>
+
 #include <algorithm>
 #include <mutex>
 
@@ -33,14 +35,23 @@ struct GatherParams {
   int in_dtype, out_dtype;
   int ndim;
   uint64_t n_out;
+  const unsigned* status;     // device status word
+  double* status_out;         // where its value goes (nullptr: nowhere)
   FastDiv div[kMaxDim];       // out_shape per axis
   int64_t in_stride[kMaxDim];
   int idx_off[kMaxDim + 1];
   int idx[kMaxIdx];
 };
 
+// The index lists are copied to shared memory first: lanes look them up at
+// different places, which the constant bank of the parameters serves one lane
+// at a time.
 template <typename TI, typename TO>
 __global__ void gather_kernel(const __grid_constant__ GatherParams p) {
+  __shared__ int sidx[kMaxIdx];
+  for (int i = threadIdx.x; i < p.idx_off[p.ndim]; i += blockDim.x) sidx[i] = p.idx[i];
+  pdl_wait();
+  __syncthreads();
   const TI* __restrict__ in = static_cast<const TI*>(p.in);
   TO* __restrict__ out = static_cast<TO*>(p.out);
   for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < p.n_out;
@@ -52,12 +63,13 @@ __global__ void gather_kernel(const __grid_constant__ GatherParams p) {
       const uint64_t q = fdiv(rem, p.div[a]);
       const int i = (int)(rem - q * p.div[a].d);
       rem = q;
-      const int j = p.idx[p.idx_off[a] + i];
+      const int j = sidx[p.idx_off[a] + i];
       zero |= (j < 0);
       addr += (int64_t)(j < 0 ? 0 : j) * p.in_stride[a];
     }
     out[o] = zero ? (TO)0 : (TO)in[addr];
   }
+  if (p.status_out && blockIdx.x == 0 && threadIdx.x == 0) *p.status_out = p.status ? (double)*p.status : 0.0;
 }
 
 // ---------------------------------------------------------------- take axis
@@ -203,93 +215,138 @@ __global__ void marg_stage2(const double* __restrict__ part, int nchunks, double
 struct DiagRedParams {
   const void* in;
   double* out;
+  double* host;            // host memory the device can write, or nullptr
   const unsigned* status;
   double* part;      // per-block partial sums [grid][n_out] (grid > 1)
   unsigned* ticket;  // blocks finished (grid > 1); zero between calls
   int in_dtype;
   int ndim;
-  int axis;        // -1: trace
+  int split;       // axes [split, ndim) make up the low table
   int n_out;       // 1 for the trace, else the Hilbert dim of `axis`
-  uint64_t per_j;  // diagonal entries per outcome
-  FastDiv div_s;   // entries of the diagonal index after `axis`
-  uint64_t s_axis;
-  FastDiv div[kMaxDim];  // Hilbert dims per axis (diagonal index space)
+  unsigned n_lo, n_hi;  // table sizes: products of the axes' lengths
+  unsigned per_j;       // diagonal entries per outcome (n_out outcomes)
+  unsigned chunk;       // entries per outcome and block
+  unsigned s_axis;      // entries of the diagonal index after `axis`
   int64_t in_stride[kMaxDim];
   int idx_off[kMaxDim + 1];
   int idx[kMaxIdx];
 };
 
-constexpr int kDiagRedBlock = 1024;
+constexpr int kDiagRedBlock = 256;
+constexpr int kDiagRedWarps = kDiagRedBlock / 32;
 
-__global__ void __launch_bounds__(kDiagRedBlock) diag_marginals_kernel(const __grid_constant__ DiagRedParams p) {
-  __shared__ double sh[32];
-  __shared__ int last;
-  const uint64_t d_axis = p.axis < 0 ? 1 : p.div[p.axis].d;
-  constexpr int U = 8;  // independent loads in flight per thread
-  // this block's share of each outcome's entries: the scattered diagonal
-  // loads of one SM are bounded by its outstanding misses, so a large
-  // diagonal is spread over many blocks
-  const uint64_t chunk = (p.per_j + gridDim.x - 1) / gridDim.x;
-  const uint64_t m_beg = (uint64_t)blockIdx.x * chunk;
-  const uint64_t m_end = m_beg + chunk < p.per_j ? m_beg + chunk : p.per_j;
-  for (int j = 0; j < p.n_out; ++j) {
-    double acc = 0.0;
-    for (uint64_t m0 = m_beg + threadIdx.x; m0 < m_end; m0 += (uint64_t)U * kDiagRedBlock) {
-      double v[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        // m-th diagonal entry whose index along `axis` is j
-        const uint64_t m = m0 + (uint64_t)u * kDiagRedBlock;
-        v[u] = 0.0;
-        if (m < m_end) {
-          const uint64_t hi = fdiv(m, p.div_s);
-          const uint64_t lo = m - hi * p.s_axis;
-          uint64_t rem = (hi * d_axis + (uint64_t)j) * p.s_axis + lo;
-          int64_t addr = 0;
-          bool zero = false;
-          for (int a = p.ndim - 1; a >= 0; --a) {
-            const uint64_t q = fdiv(rem, p.div[a]);
-            const int i = (int)(rem - q * p.div[a].d);
-            rem = q;
-            const int k = p.idx[p.idx_off[a] + i];
-            zero |= k < 0;
-            addr += (int64_t)(k < 0 ? 0 : k) * p.in_stride[a];
-          }
-          if (!zero) v[u] = load_f64(p.in, addr, p.in_dtype);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) acc += v[u];  // fixed order
+// Results for the host go straight into page-locked memory, then, after a
+// system-wide fence, the status word as the flag that they are there.  All
+// threads of the block call this; value(j) gives result j.
+template <typename F>
+__device__ __forceinline__ void store_results(double* out, double* host, const unsigned* status, int n_out, F value) {
+  for (int j = threadIdx.x; j < n_out; j += blockDim.x) {
+    const double v = value(j);
+    if (out) out[j] = v;
+    if (host) {
+      *(volatile double*)(host + j) = v;
+      __threadfence_system();
     }
-    const double r = block_sum(acc, sh);
-    if (threadIdx.x == 0) {
-      if (gridDim.x == 1)
-        p.out[j] = r;
-      else
-        p.part[(int64_t)blockIdx.x * p.n_out + j] = r;
-    }
-  }
-  if (gridDim.x == 1) {
-    if (threadIdx.x == 0) p.out[p.n_out] = p.status ? (double)*p.status : 0.0;
-    return;
-  }
-  // the last block to finish adds the partials in block order
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(p.ticket, 1u) == gridDim.x - 1 ? 1 : 0;
   }
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int j = threadIdx.x; j < p.n_out; j += kDiagRedBlock) {
-    double s = 0.0;
-    for (unsigned b = 0; b < gridDim.x; ++b) s += __ldcg(p.part + (int64_t)b * p.n_out + j);
-    p.out[j] = s;
-  }
   if (threadIdx.x == 0) {
-    p.out[p.n_out] = p.status ? (double)*p.status : 0.0;
-    *p.ticket = 0u;  // ready for the next call
+    const double st = status ? (double)*(volatile const unsigned*)status : 0.0;
+    if (out) out[n_out] = st;
+    if (host) *(volatile double*)(host + n_out) = st;
   }
+}
+
+// The diagonal index of an entry is cut in two; each half's address part comes
+// from a table in shared memory that the block builds before its first load
+// (n_lo + n_hi entries, two square roots of the diagonal): per entry two
+// look-ups instead of a 64-bit division and a divergent parameter look-up per
+// axis.  One load per thread (more on diagonals beyond 256 entries per SM):
+// the loads of a diagonal are scattered, and one SM is bounded by its
+// outstanding misses (the 4096 entries of a 12-qubit state: 15.8 us on 4
+// blocks with the divisions, 9.6 us here on 16, nearly all of it the latency
+// of a launch, the tables, one load and the last block).
+__global__ void __launch_bounds__(kDiagRedBlock) diag_marginals_kernel(const __grid_constant__ DiagRedParams p) {
+  extern __shared__ int64_t tables[];  // [n_hi], [n_lo], then the index lists
+  int64_t* thi = tables;
+  int64_t* tlo = tables + p.n_hi;
+  int* sidx = reinterpret_cast<int*>(tlo + p.n_lo);
+  __shared__ double sh[kDiagRedWarps];
+  __shared__ int last;
+  constexpr int64_t kZero = INT64_MIN;
+  for (int i = threadIdx.x; i < p.idx_off[p.ndim]; i += kDiagRedBlock) sidx[i] = p.idx[i];
+  __syncthreads();
+  for (unsigned e = threadIdx.x; e < p.n_hi + p.n_lo; e += kDiagRedBlock) {
+    const bool low = e >= p.n_hi;
+    unsigned rem = low ? e - p.n_hi : e;
+    int64_t addr = 0;
+    bool zero = false;
+    for (int a = (low ? p.ndim : p.split) - 1; a >= (low ? p.split : 0); --a) {
+      const unsigned len = (unsigned)(p.idx_off[a + 1] - p.idx_off[a]);
+      const unsigned q = rem / len;
+      const int k = sidx[p.idx_off[a] + (int)(rem - q * len)];
+      rem = q;
+      zero |= k < 0;
+      addr += (int64_t)(k < 0 ? 0 : k) * p.in_stride[a];
+    }
+    tables[e] = zero ? kZero : addr;
+  }
+  pdl_wait();
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // warps per outcome; with more outcomes than warps a warp takes several
+  const int wpj = p.n_out < kDiagRedWarps ? kDiagRedWarps / p.n_out : 1;
+  const unsigned m_beg = blockIdx.x * p.chunk;  // at most 2^22 entries in all
+  const unsigned m_end = min(m_beg + p.chunk, p.per_j);
+  const bool single = gridDim.x == 1;
+  for (int j0 = 0; j0 < p.n_out; j0 += kDiagRedWarps / wpj) {
+    const int j = j0 + warp / wpj;
+    double acc = 0.0;
+    if (j < p.n_out && warp / wpj < kDiagRedWarps / wpj) {
+#pragma unroll 4
+      for (unsigned m = m_beg + (unsigned)((warp % wpj) * 32 + lane); m < m_end; m += (unsigned)wpj * 32) {
+        // m-th diagonal entry whose index along the axis is j
+        const unsigned hi = m / p.s_axis;
+        const unsigned e = (hi * (unsigned)p.n_out + (unsigned)j) * p.s_axis + (m - hi * p.s_axis);
+        const unsigned eh = e / p.n_lo;
+        const int64_t ah = thi[eh], al = tlo[e - eh * p.n_lo];
+        if (ah != kZero && al != kZero) acc += load_f64(p.in, ah + al, p.in_dtype);
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) sh[warp] = acc;
+    __syncthreads();
+    // the warps of an outcome, in order
+    const int jj = j0 + (int)threadIdx.x;
+    if ((int)threadIdx.x < kDiagRedWarps / wpj && jj < p.n_out) {
+      double r = 0.0;
+      for (int w = 0; w < wpj; ++w) r += sh[(int)threadIdx.x * wpj + w];
+      if (single)
+        p.out[jj] = r;
+      else
+        p.part[(int64_t)blockIdx.x * p.n_out + jj] = r;
+    }
+    __syncthreads();
+  }
+  if (!single) {
+    // the last block to finish adds the partials of each outcome in a fixed
+    // order: a warp per outcome, its lanes' shares by shuffles
+    if (threadIdx.x == 0) {
+      __threadfence();
+      last = atomicAdd(p.ticket, 1u) == gridDim.x - 1 ? 1 : 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int j = warp; j < p.n_out; j += kDiagRedWarps) {
+      double s = 0.0;
+      for (unsigned b = lane; b < gridDim.x; b += 32) s += __ldcg(p.part + (int64_t)b * p.n_out + j);
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) p.out[j] = s;
+    }
+    if (threadIdx.x == 0) *p.ticket = 0u;  // ready for the next call
+    __syncthreads();
+  }
+  store_results(p.out, p.host, p.status, p.n_out, [&](int j) { return *(volatile double*)(p.out + j); });
 }
 
 // ---------------------------------------------------------------- partial trace
@@ -320,40 +377,95 @@ __device__ __forceinline__ int64_t pt_base(const PtParams& p, uint64_t o) {
   return base;
 }
 
-__device__ __forceinline__ double pt_term(const PtParams& p, int64_t base, uint64_t c) {
+// The traced qudits' indices and weights, copied to shared memory: lanes look
+// them up at different places (one lane at a time in the parameters' constant
+// bank).
+struct PtTables {
+  int idx[kMaxPtEntries];
+  double w[kMaxPtEntries];
+};
+__device__ __forceinline__ void pt_tables(const PtParams& p, PtTables& t) {
+  for (int i = threadIdx.x; i < p.toff[p.ntr]; i += blockDim.x) {
+    t.idx[i] = p.tidx[i];
+    t.w[i] = p.tw[i];
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ double pt_term(const PtParams& p, const PtTables& t, int64_t base, uint64_t c) {
   int64_t addr = base;
   double w = 1.0;
   for (int a = p.ntr - 1; a >= 0; --a) {
     const uint64_t q = fdiv(c, p.tdiv[a]);
     const int i = p.toff[a] + (int)(c - q * p.tdiv[a].d);
     c = q;
-    addr += (int64_t)p.tidx[i] * p.tstride[a];
-    w *= p.tw[i];
+    addr += (int64_t)t.idx[i] * p.tstride[a];
+    w *= t.w[i];
   }
   return w * load_f64(p.in, addr, p.dtype);
 }
 
-// few combos: one thread per output element
+// few combos and many outputs: one thread per output element
 __global__ void pt_thread_kernel(const __grid_constant__ PtParams p) {
+  __shared__ PtTables t;
+  pt_tables(p, t);
+  pdl_wait();
   for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < p.n_out;
        o += (uint64_t)gridDim.x * blockDim.x) {
     const int64_t base = pt_base(p, o);
     double acc = 0.0;
-    for (uint64_t c = 0; c < p.n_combos; ++c) acc += pt_term(p, base, c);
+    for (uint64_t c = 0; c < p.n_combos; ++c) acc += pt_term(p, t, base, c);
     store_from_f64(p.out, (int64_t)o, p.dtype, acc);
   }
 }
 
-// many combos: one block per output element
+// otherwise one block per output element
 __global__ void pt_block_kernel(const __grid_constant__ PtParams p) {
+  __shared__ PtTables t;
   __shared__ double sh[32];
+  pt_tables(p, t);
+  pdl_wait();
   for (uint64_t o = blockIdx.x; o < p.n_out; o += gridDim.x) {
     const int64_t base = pt_base(p, o);
     double acc = 0.0;
-    for (uint64_t c = threadIdx.x; c < p.n_combos; c += blockDim.x) acc += pt_term(p, base, c);
+    for (uint64_t c = threadIdx.x; c < p.n_combos; c += blockDim.x) acc += pt_term(p, t, base, c);
     const double r = block_sum(acc, sh);
     if (threadIdx.x == 0) store_from_f64(p.out, (int64_t)o, p.dtype, r);
   }
+}
+
+// no qudit kept: one value, summed by all blocks (the last to finish adds
+// their sums in block order) and stored with the status word
+__global__ void pt_scalar_kernel(const __grid_constant__ PtParams p, double* out, double* host,
+                                 const unsigned* status, double* part, unsigned* ticket) {
+  __shared__ PtTables t;
+  __shared__ double sh[32];
+  __shared__ double sum;
+  __shared__ int last;
+  pt_tables(p, t);
+  pdl_wait();
+  double acc = 0.0;
+  for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < p.n_combos;
+       c += (uint64_t)gridDim.x * blockDim.x)
+    acc += pt_term(p, t, 0, c);
+  double r = block_sum(acc, sh);
+  if (gridDim.x > 1) {
+    if (threadIdx.x == 0) {
+      part[blockIdx.x] = r;
+      __threadfence();
+      last = atomicAdd(ticket, 1u) == gridDim.x - 1 ? 1 : 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    acc = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc += __ldcg(part + b);
+    r = block_sum(acc, sh);
+    if (threadIdx.x == 0) *ticket = 0u;  // ready for the next call
+  }
+  if (threadIdx.x == 0) sum = r;
+  __syncthreads();
+  store_results(out, host, status, 1, [&](int) { return sum; });
 }
 
 // ---------------------------------------------------------------- scaling
@@ -371,6 +483,38 @@ __global__ void scale_kernel(T* __restrict__ x, uint64_t n, double alpha, const 
     x[i] = x[i] * ta;
 }
 
+// Device address of page-locked host memory, or nullptr for other pointers.
+double* mapped_host(double* host) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return a.type == cudaMemoryTypeHost ? static_cast<double*>(a.devicePointer) : nullptr;
+}
+
+// A result is there when its last double, the status, is no longer this
+// pattern (a nan that no conversion of the status word gives).
+constexpr uint64_t kPendingBits = 0xfff8dead0badf00dull;
+void mark_pending(double* flag) {
+  __atomic_store_n(reinterpret_cast<uint64_t*>(flag), kPendingBits, __ATOMIC_RELEASE);
+}
+// Wait for it by reading the flag, for about a millisecond; then by the stream
+// (work queued before, or an error).
+int wait_result(double* flag, cudaStream_t stream) {
+  timespec t0, t1;
+  clock_gettime(CLOCK_MONOTONIC, &t0);
+  for (;;) {
+    for (int i = 0; i < 256; ++i)
+      if (__atomic_load_n(reinterpret_cast<uint64_t*>(flag), __ATOMIC_ACQUIRE) != kPendingBits) return QSGB_OK;
+    clock_gettime(CLOCK_MONOTONIC, &t1);
+    if ((t1.tv_sec - t0.tv_sec) * 1000000000ll + (t1.tv_nsec - t0.tv_nsec) > 1000000ll) break;
+  }
+  QSGB_CUDA_TRY(cudaStreamSynchronize(stream));
+  return __atomic_load_n(reinterpret_cast<uint64_t*>(flag), __ATOMIC_ACQUIRE) != kPendingBits ? QSGB_OK
+                                                                                               : QSGB_ERR_CUDA;
+}
+
 unsigned grid_for(uint64_t n, int block, int per_sm = 8) {
   const uint64_t need = (n + block - 1) / block;
   const uint64_t cap = (uint64_t)sm_count() * per_sm;
@@ -382,8 +526,9 @@ unsigned grid_for(uint64_t n, int block, int per_sm = 8) {
 
 using namespace qsgb;
 
-extern "C" int qsgb_gather(const void* in, void* out, int in_dtype, int out_dtype, int ndim, const int64_t* in_shape,
-                           const int32_t* idx_off, const int32_t* idx, void* stream) {
+static int gather_common(const void* in, void* out, int in_dtype, int out_dtype, int ndim, const int64_t* in_shape,
+                         const int32_t* idx_off, const int32_t* idx, const unsigned* status, double* status_out,
+                         cudaStream_t s) {
   if (!in || !out || !in_shape || !idx_off || (!idx && ndim > 0)) return QSGB_ERR_INVALID;
   if (ndim < 0 || ndim > kMaxDim) return QSGB_ERR_UNSUPPORTED;
   if ((in_dtype != QSGB_F64 && in_dtype != QSGB_F32) || (out_dtype != QSGB_F64 && out_dtype != QSGB_F32))
@@ -395,6 +540,8 @@ extern "C" int qsgb_gather(const void* in, void* out, int in_dtype, int out_dtyp
   p.in_dtype = in_dtype;
   p.out_dtype = out_dtype;
   p.ndim = ndim;
+  p.status = status;
+  p.status_out = status_out;
   uint64_t n_out = 1;
   int64_t stride = 1;
   for (int a = ndim - 1; a >= 0; --a) {
@@ -410,18 +557,37 @@ extern "C" int qsgb_gather(const void* in, void* out, int in_dtype, int out_dtyp
   for (int a = 0; a <= ndim; ++a) p.idx_off[a] = idx_off[a];
   for (int i = 0; i < idx_off[ndim]; ++i) p.idx[i] = idx[i];
   p.n_out = n_out;
-  cudaStream_t s = as_stream(stream);
   const int block = 256;
   const unsigned grid = grid_for(n_out, block);
   if (in_dtype == QSGB_F64 && out_dtype == QSGB_F64)
-    gather_kernel<double, double><<<grid, block, 0, s>>>(p);
-  else if (in_dtype == QSGB_F32 && out_dtype == QSGB_F64)
-    gather_kernel<float, double><<<grid, block, 0, s>>>(p);
-  else if (in_dtype == QSGB_F64 && out_dtype == QSGB_F32)
-    gather_kernel<double, float><<<grid, block, 0, s>>>(p);
-  else
-    gather_kernel<float, float><<<grid, block, 0, s>>>(p);
-  return launch_status();
+    return launch_pdl(gather_kernel<double, double>, grid, block, 0, s, p);
+  if (in_dtype == QSGB_F32 && out_dtype == QSGB_F64)
+    return launch_pdl(gather_kernel<float, double>, grid, block, 0, s, p);
+  if (in_dtype == QSGB_F64 && out_dtype == QSGB_F32)
+    return launch_pdl(gather_kernel<double, float>, grid, block, 0, s, p);
+  return launch_pdl(gather_kernel<float, float>, grid, block, 0, s, p);
+}
+
+extern "C" int qsgb_gather(const void* in, void* out, int in_dtype, int out_dtype, int ndim, const int64_t* in_shape,
+                           const int32_t* idx_off, const int32_t* idx, void* stream) {
+  return gather_common(in, out, in_dtype, out_dtype, ndim, in_shape, idx_off, idx, nullptr, nullptr,
+                       as_stream(stream));
+}
+
+extern "C" int qsgb_gather_host(const void* in, int in_dtype, int ndim, const int64_t* in_shape,
+                                const int32_t* idx_off, const int32_t* idx, const unsigned* dev_status,
+                                double* host_out, void* stream) {
+  if (!host_out || !idx_off) return QSGB_ERR_INVALID;
+  if (ndim < 0 || ndim > kMaxDim) return QSGB_ERR_UNSUPPORTED;
+  double* mapped = mapped_host(host_out);
+  if (!mapped) return QSGB_ERR_UNSUPPORTED;  // not page-locked
+  uint64_t n = 1;
+  for (int a = 0; a < ndim; ++a) n *= (uint64_t)std::max(0, idx_off[a + 1] - idx_off[a]);
+  cudaStream_t s = as_stream(stream);
+  const int st = gather_common(in, mapped, in_dtype, QSGB_F64, ndim, in_shape, idx_off, idx, dev_status, mapped + n, s);
+  if (st != QSGB_OK) return st;
+  QSGB_CUDA_TRY(cudaStreamSynchronize(s));
+  return QSGB_OK;
 }
 
 template <int NIDX>
@@ -479,7 +645,6 @@ extern "C" int qsgb_take_axis(const void* in, void* out, int dtype, int64_t oute
 
 namespace qsgb {
 namespace {
-constexpr int kDiagEntriesPerBlock = 512;  // diagonal entries per block (per outcome)
 constexpr int kDiagMaxOut = 64;
 }  // namespace
 }  // namespace qsgb
@@ -502,7 +667,6 @@ extern "C" int qsgb_diag_marginals(const void* in, int in_dtype, int ndim, const
   p.status = dev_status;
   p.in_dtype = in_dtype;
   p.ndim = ndim;
-  p.axis = axis;
   uint64_t n = 1, s_axis = 1;
   int64_t stride = 1;
   for (int a = ndim - 1; a >= 0; --a) {
@@ -510,25 +674,38 @@ extern "C" int qsgb_diag_marginals(const void* in, int in_dtype, int ndim, const
     if (len < 1 || in_shape[a] < 1) return QSGB_ERR_INVALID;
     for (int i = idx_off[a]; i < idx_off[a + 1]; ++i)
       if (idx[i] >= in_shape[a] || idx[i] < -1) return QSGB_ERR_INVALID;
-    p.div[a] = make_fastdiv((uint64_t)len);
     p.in_stride[a] = stride;
     stride *= in_shape[a];
     if (axis >= 0 && a > axis) s_axis *= (uint64_t)len;
     n *= (uint64_t)len;
   }
-  // one block: diagonals of up to 2^22 entries (prod of Hilbert dims)
+  // diagonals of up to 2^22 entries (prod of Hilbert dims)
   if (n > (1ull << 22)) return QSGB_ERR_UNSUPPORTED;
   const uint64_t d = axis < 0 ? 1 : (uint64_t)(idx_off[axis + 1] - idx_off[axis]);
   if (d > 64) return QSGB_ERR_UNSUPPORTED;
   p.n_out = (int)d;
-  p.per_j = n / d;
-  p.s_axis = axis < 0 ? 1 : s_axis;
-  p.div_s = make_fastdiv(p.s_axis);
+  p.per_j = (unsigned)(n / d);
+  p.s_axis = (unsigned)s_axis;
   for (int a = 0; a <= ndim; ++a) p.idx_off[a] = idx_off[a];
   for (int i = 0; i < idx_off[ndim]; ++i) p.idx[i] = idx[i];
-  // blocks: one per kDiagEntriesPerBlock entries of an outcome, at most one
-  // per SM, and as many as the scratch holds partials for
-  uint64_t grid = (p.per_j + kDiagEntriesPerBlock - 1) / kDiagEntriesPerBlock;
+  // the low table takes axes from the last one while its square stays within
+  // the diagonal
+  p.split = ndim;
+  uint64_t lo = 1;
+  while (p.split > 0) {
+    const uint64_t next = lo * (uint64_t)(idx_off[p.split] - idx_off[p.split - 1]);
+    if (lo > 1 && next * next > 2 * n) break;
+    lo = next;
+    --p.split;
+  }
+  p.n_lo = (unsigned)lo;
+  p.n_hi = (unsigned)(n / lo);
+  const int smem = (int)((p.n_lo + p.n_hi) * sizeof(int64_t) + (size_t)idx_off[ndim] * sizeof(int));
+  const int as = allow_dynamic_smem((const void*)diag_marginals_kernel, smem);
+  if (as != QSGB_OK || smem > 200 * 1024) return QSGB_ERR_UNSUPPORTED;
+  // blocks: one per 256 entries, at most one per SM, and as many as the scratch
+  // holds partials for
+  uint64_t grid = (n + kDiagRedBlock - 1) / kDiagRedBlock;
   grid = std::min<uint64_t>(grid, (uint64_t)sm_count());
   if (!scratch || scratch_bytes < 16 + (int64_t)sizeof(double) * p.n_out) grid = 1;
   if (grid > 1) {
@@ -537,10 +714,17 @@ extern "C" int qsgb_diag_marginals(const void* in, int in_dtype, int ndim, const
     p.ticket = static_cast<unsigned*>(scratch);
     p.part = reinterpret_cast<double*>(static_cast<unsigned char*>(scratch) + 16);
   }
+  grid = std::max<uint64_t>(grid, 1);
+  p.chunk = (unsigned)((p.per_j + grid - 1) / grid);
   cudaStream_t st = as_stream(stream);
-  diag_marginals_kernel<<<(unsigned)std::max<uint64_t>(grid, 1), kDiagRedBlock, 0, st>>>(p);
-  const int ls = launch_status();
+  double* mapped = host_out ? mapped_host(host_out) : nullptr;
+  if (mapped) {
+    p.host = mapped;
+    mark_pending(host_out + d);
+  }
+  const int ls = launch_pdl(diag_marginals_kernel, (unsigned)grid, (unsigned)kDiagRedBlock, (size_t)smem, st, p);
   if (ls != QSGB_OK || !host_out) return ls;
+  if (mapped) return wait_result(host_out + d, st);
   QSGB_CUDA_TRY(cudaMemcpyAsync(host_out, out, (d + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
   QSGB_CUDA_TRY(cudaStreamSynchronize(st));
   return QSGB_OK;
@@ -587,12 +771,9 @@ extern "C" int qsgb_marginals(const double* diag, int ndim, const int64_t* shape
   return launch_status();
 }
 
-extern "C" int qsgb_partial_trace(const void* in, void* out, int dtype, int ndim, const int64_t* shape,
-                                  const int32_t* keep, const double* weights, void* stream) {
-  if (!in || !out || in == out || (ndim > 0 && (!shape || !keep))) return QSGB_ERR_INVALID;
-  if (dtype != QSGB_F64 && dtype != QSGB_F32) return QSGB_ERR_INVALID;
-  if (ndim < 0 || ndim > kMaxDim) return QSGB_ERR_UNSUPPORTED;
-  PtParams p{};
+// The kernel parameters of a weighted trace, from the host arrays.
+static int pt_params(PtParams& p, const void* in, void* out, int dtype, int ndim, const int64_t* shape,
+                     const int32_t* keep, const double* weights) {
   p.in = in;
   p.out = out;
   p.dtype = dtype;
@@ -650,18 +831,62 @@ extern "C" int qsgb_partial_trace(const void* in, void* out, int dtype, int ndim
   p.ntr = ntr;
   p.n_out = n_out;
   p.n_combos = n_combos;
+  return QSGB_OK;
+}
+
+extern "C" int qsgb_partial_trace(const void* in, void* out, int dtype, int ndim, const int64_t* shape,
+                                  const int32_t* keep, const double* weights, void* stream) {
+  if (!in || !out || in == out || (ndim > 0 && (!shape || !keep))) return QSGB_ERR_INVALID;
+  if (dtype != QSGB_F64 && dtype != QSGB_F32) return QSGB_ERR_INVALID;
+  if (ndim < 0 || ndim > kMaxDim) return QSGB_ERR_UNSUPPORTED;
+  PtParams p{};
+  const int st = pt_params(p, in, out, dtype, ndim, shape, keep, weights);
+  if (st != QSGB_OK) return st;
   cudaStream_t s = as_stream(stream);
-  if (n_combos == 0) {
-    QSGB_CUDA_TRY(cudaMemsetAsync(out, 0, n_out * (dtype == QSGB_F64 ? 8 : 4), s));
+  if (p.n_combos == 0) {
+    QSGB_CUDA_TRY(cudaMemsetAsync(out, 0, p.n_out * (dtype == QSGB_F64 ? 8 : 4), s));
     return QSGB_OK;
   }
-  if (n_combos <= 64) {
-    pt_thread_kernel<<<grid_for(n_out, 256), 256, 0, s>>>(p);
-  } else {
-    const int block = n_combos >= 256 ? 256 : 128;
-    pt_block_kernel<<<(unsigned)std::min<uint64_t>(n_out, (uint64_t)sm_count() * 16), block, 0, s>>>(p);
+  // a block per output unless the outputs alone fill the device: one thread's
+  // chain of up to 64 scattered loads takes 1.7 us each (a Pauli string of 64
+  // terms, 12 qubits: 107 us in one thread, 7 us in a block of 128)
+  const uint64_t fill = (uint64_t)sm_count() * 64;
+  if (p.n_combos <= 64 && p.n_out >= fill) return launch_pdl(pt_thread_kernel, grid_for(p.n_out, 256), 256u, 0, s, p);
+  const unsigned block = p.n_combos >= 256 ? 256u : p.n_combos > 64 ? 128u : p.n_combos > 32 ? 64u : 32u;
+  return launch_pdl(pt_block_kernel, (unsigned)std::min<uint64_t>(p.n_out, (uint64_t)sm_count() * 16), block, 0, s, p);
+}
+
+extern "C" int qsgb_expectation(const void* in, int dtype, int ndim, const int64_t* shape, const double* weights,
+                                double* out, const unsigned* dev_status, double* host_out, void* scratch,
+                                int64_t scratch_bytes, void* stream) {
+  if (!in || !out || (ndim > 0 && (!shape || !weights))) return QSGB_ERR_INVALID;
+  if (dtype != QSGB_F64 && dtype != QSGB_F32) return QSGB_ERR_INVALID;
+  if (ndim < 0 || ndim > kMaxDim) return QSGB_ERR_UNSUPPORTED;
+  PtParams p{};
+  const int32_t keep[kMaxDim] = {};
+  const int st = pt_params(p, in, out, dtype, ndim, shape, keep, weights);
+  if (st != QSGB_OK) return st;
+  cudaStream_t s = as_stream(stream);
+  uint64_t grid = std::min<uint64_t>((p.n_combos + 255) / 256, (uint64_t)sm_count());
+  if (!scratch || scratch_bytes < 16 + 2 * (int64_t)sizeof(double)) grid = 1;
+  unsigned* ticket = nullptr;
+  double* part = nullptr;
+  if (grid > 1) {
+    if ((uintptr_t)scratch % 16 != 0) return QSGB_ERR_INVALID;
+    grid = std::min<uint64_t>(grid, (uint64_t)((scratch_bytes - 16) / (int64_t)sizeof(double)));
+    ticket = static_cast<unsigned*>(scratch);
+    part = reinterpret_cast<double*>(static_cast<unsigned char*>(scratch) + 16);
   }
-  return launch_status();
+  double* mapped = host_out ? mapped_host(host_out) : nullptr;
+  if (mapped) mark_pending(host_out + 1);
+  const unsigned block = p.n_combos > 128 ? 256u : p.n_combos > 32 ? 128u : 32u;
+  const int ls = launch_pdl(pt_scalar_kernel, (unsigned)std::max<uint64_t>(grid, 1), block, 0, s, p, out, mapped,
+                            dev_status, part, ticket);
+  if (ls != QSGB_OK || !host_out) return ls;
+  if (mapped) return wait_result(host_out + 1, s);
+  QSGB_CUDA_TRY(cudaMemcpyAsync(host_out, out, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  QSGB_CUDA_TRY(cudaStreamSynchronize(s));
+  return QSGB_OK;
 }
 
 extern "C" int qsgb_scale(void* x, int dtype, int64_t n, double alpha, void* stream) {

@@ -11,6 +11,7 @@ operators raise.
 """
 import ctypes
 import math
+import threading
 from typing import List
 
 import numpy as np
@@ -441,7 +442,7 @@ def scale_by_inverse_(pv: torch.Tensor, denom: torch.Tensor,
 # Python); an eager application with a cached, validated plan costs the
 # output allocation and one ctypes call.
 _STATUS_PTR = {}
-_DIAG_BUF = {}
+_READ_BUF = threading.local()
 
 
 def status_ptr(index):
@@ -577,30 +578,87 @@ def eager_apply_dense(pv, ptm, plan, arith, out=None):
     return out
 
 
-def diag_marginals(pv, plan_arrays, axis):
-    """Marginals (axis >= 0) or trace (axis == -1) of the DM diagonal of the
-    CUDA tensor `pv` through the gather plan, in one launch and one
-    device-to-host copy that also returns the device status word (raises
-    like check_device_status).  None when the fused kernel does not serve
-    the request (the caller takes the gather + reduction path)."""
-    idx_off_c, idx_c, shape_c, n_out = plan_arrays
-    index = pv.device.index
-    bufs = _DIAG_BUF.get(index)
-    if bufs is None:
+def _read_buffers(index, device):
+    """This thread's buffers for results read by the host, one set per CUDA
+    device: device values, the pinned values the kernels write and the block
+    partials (another thread's call may run at the same time)."""
+    bufs = _READ_BUF.__dict__.setdefault('bufs', {})
+    b = bufs.get(index)
+    if b is None:
         nscr = int(L.load().qsgb_diag_marginals_scratch_bytes())
         # the scratch's first 16 bytes (the kernel's block ticket) start at
         # zero and every call leaves them zero
-        bufs = (torch.empty(80, dtype=torch.float64, device=pv.device),
-                torch.empty(80, dtype=torch.float64, pin_memory=True),
-                torch.zeros(nscr, dtype=torch.uint8, device=pv.device))
-        _DIAG_BUF[index] = bufs
-    dev, host, scratch = bufs
-    n = (1 if axis < 0 else n_out[axis]) + 1
-    if n > 65:
+        host = torch.empty(80, dtype=torch.float64, pin_memory=True)
+        b = (torch.empty(80, dtype=torch.float64, device=device), host,
+             torch.zeros(nscr, dtype=torch.uint8, device=device),
+             host.numpy())
+        # zeroed on this stream; later calls may come on others
+        torch.cuda.current_stream(device).synchronize()
+        bufs[index] = b
+    return b
+
+
+def _read_values(pv, host, n):
+    vals = host[:n + 1].copy()
+    if vals[-1]:
+        _raise_status(status_tensor(pv.device), int(vals[-1]))
+    return vals[:-1]
+
+
+def expectation(pv, weights):
+    """Sum of the CUDA tensor `pv` weighted by the per-element `weights` of
+    its axes (concatenated, ascending), FP64 accumulation: a float, read with
+    the device status word (raises like check_device_status)."""
+    pv = pv.contiguous()
+    index = pv.device.index
+    dev, host, scratch, values = _read_buffers(index, pv.device)
+    st = L.load().qsgb_expectation(
+        pv.data_ptr(), _dtype_code(pv), pv.dim(), L.i64_array(pv.shape),
+        L.f64_array(weights), dev.data_ptr(), status_ptr(index),
+        host.data_ptr(), scratch.data_ptr(), scratch.numel(),
+        _stream_handle(pv))
+    L.check(st, 'qsgb_expectation')
+    return float(_read_values(pv, values, 1)[0])
+
+
+# diagonals up to this many entries are read by the gather kernel writing
+# page-locked memory (one launch); larger ones by a copy
+HOST_DIAG_MAX = 1 << 20
+
+
+def diagonal_host(pv, plan_arrays):
+    """The DM diagonal of the CUDA tensor `pv` through the gather plan as a
+    numpy array, read with the device status word (raises like
+    check_device_status).  None when the caller has to take the gather and
+    the copy."""
+    idx_off_c, idx_c, shape_c, n_out = plan_arrays
+    n = math.prod(n_out)
+    if n > HOST_DIAG_MAX or not n_out:
+        return None
+    host = torch.empty(n + 1, dtype=torch.float64, pin_memory=True)
+    st = L.load().qsgb_gather_host(
+        pv.data_ptr(), _dtype_code(pv), pv.dim(), shape_c, idx_off_c, idx_c,
+        status_ptr(pv.device.index), host.data_ptr(), _stream_handle(pv))
+    if st == L.ERR_UNSUPPORTED:
+        return None
+    L.check(st, 'qsgb_gather_host')
+    return _read_values(pv, host.numpy(), n)
+
+
+def diag_marginals(pv, plan_arrays, axis):
+    """Marginals (axis >= 0) or trace (axis == -1) of the DM diagonal of the
+    CUDA tensor `pv` through the gather plan, in one launch that also
+    returns the device status word (raises like check_device_status).  None when the fused kernel does not serve
+    the request (the caller takes the gather + reduction path)."""
+    idx_off_c, idx_c, shape_c, n_out = plan_arrays
+    index = pv.device.index
+    dev, host, scratch, values = _read_buffers(index, pv.device)
+    n = 1 if axis < 0 else n_out[axis]
+    if n > 64:
         return None
     stream = _RAW_STREAM(index) if _RAW_STREAM is not None else \
         torch.cuda.current_stream(pv.device).cuda_stream
-    # the library copies the n values into the pinned buffer and waits
+    # the kernel writes the n values and the status into the pinned buffer
     st = L.load().qsgb_diag_marginals(
         pv.data_ptr(), _dtype_code(pv), pv.dim(), shape_c, idx_off_c, idx_c,
         axis, dev.data_ptr(), status_ptr(index), host.data_ptr(),
@@ -608,10 +666,7 @@ def diag_marginals(pv, plan_arrays, axis):
     if st == L.ERR_UNSUPPORTED:
         return None
     L.check(st, 'qsgb_diag_marginals')
-    vals = host.numpy()[:n].copy()
-    if vals[-1]:
-        _raise_status(status_tensor(pv.device), int(vals[-1]))
-    return vals[:-1]
+    return _read_values(pv, values, n)
 
 
 def prepare_ptm(shape, dtype, ptm, qudits, arith, transpose=False):

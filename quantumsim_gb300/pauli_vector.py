@@ -401,6 +401,14 @@ class PauliVectorGB300(_Base):
         `target_array` is an already allocated CUDA tensor that receives the
         values (ValueError when too small), and `flatten=False` shapes the
         result as dim_hilbert."""
+        if get_data and target_array is None and \
+                not self._data.requires_grad and self._data.is_contiguous():
+            arrays = _diag_arrays(self.bases, self._data.shape)
+            if arrays is not None:
+                out = ops.diagonal_host(self._data, arrays)
+                if out is not None:
+                    return out if flatten else out.reshape(
+                        tuple(self.dim_hilbert))
         diag = self._diagonal_device()
         if target_array is not None:
             n = diag.numel()
@@ -503,6 +511,8 @@ class PauliVectorGB300(_Base):
                                  'of dimension {}'.format(b.dim_hilbert))
             w = np.einsum('ab,kba->k', s, np.asarray(b.vectors))
             weights.extend(float(v) for v in np.real(w))
+        if not self._data.requires_grad:
+            return ops.expectation(self._data, weights)
         out = torch.ops.qsgb.partial_trace(self._data, [0] * n, weights)
         return float(ops.fetch_checked(out)[0])
 

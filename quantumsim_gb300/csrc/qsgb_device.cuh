@@ -44,6 +44,8 @@ __device__ __forceinline__ qsgb_u64 qsgb_fdiv(qsgb_u64 n, qsgb_u64 m, int l) {
 // lo * lo small.  Inputs the float pair cannot carry to that precision set
 // `bad`: a non-zero |x| < 2^-102 and |x| >= 2^127, inf and nan; hi and lo are
 // then meaningless, and callers recompute the affected results in native FP64.
+// E0 and N: the exponents taken, e in [E0, E0 + N).
+template <unsigned E0 = 921u, unsigned N = 229u>
 __device__ __forceinline__ void qsgb_split_f64(double x, float& hi, float& lo, unsigned& bad) {
   const unsigned h = (unsigned)__double2hiint(x);
   const unsigned l = (unsigned)__double2loint(x);
@@ -55,7 +57,7 @@ __device__ __forceinline__ void qsgb_split_f64(double x, float& hi, float& lo, u
   const float scale = __uint_as_float((hb & 0xff800000u) - (24u << 23));
   lo = (__int2float_rn((int)(l << 3)) * 0x1p-31f) * scale;
   // e in [921, 1149] is 2^-102 <= |x| < 2^127; zero is carried exactly
-  const bool out = h + h - (921u << 21) >= (229u << 21);
+  const bool out = h + h - (E0 << 21) >= (N << 21);
   hi = out ? 0.0f : __uint_as_float(hb + ((l >> 28) & 1u));
   if (out) bad |= (h + h) | l;
 }

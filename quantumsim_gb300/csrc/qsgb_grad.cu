@@ -336,6 +336,163 @@ __global__ void __launch_bounds__(kGradBlock) grad_stage1(const __grid_constant_
   }
 }
 
+// ---------------------------------------------------------------------------
+// One qudit of at most four Pauli elements: a group per thread
+// ---------------------------------------------------------------------------
+// At up to 4 x 4 entries a group's whole outer product fits a thread: its (up
+// to) eight values come straight into registers, the next group's while this
+// one is multiplied, and nothing is staged in shared memory or shared between
+// threads until the sums are complete.  The same float-float products and band
+// as in stage 1 above; a block that met a value outside the band does its
+// groups again in native FP64.  The warps' sums are scattered over their lanes
+// by exchanges (16 entries: 16 shuffles of a pair instead of 80) and the block's
+// added in warp order.  Bound by instruction issue (about 400 a group, 160 of
+// them the products) and the latency of one group ahead per thread; a ring of
+// asynchronous copies three groups ahead gave 4 % at 12 qubits and took 5 % at
+// 10.  A gradient with its second stage, against the staged kernel above: 10
+// qubits (2^18 groups) 19.5 -> 10.9 us, 11 qubits 46 -> 21, 12 qubits 147 -> 67
+// (4.0 TB/s); FP32 vectors of 12 qubits 132 -> 51.
+// A thread's walk over its groups: the place in the two tensors, moved by a
+// fixed number of groups at a time without a division.
+struct Grad4Walk {
+  int64_t z, x, o;       // place along the inner bystander, offsets of the group
+  int64_t dz, dx, dxo;   // a step, while z stays below its length
+  __device__ __forceinline__ Grad4Walk(const GradParams& p, uint64_t g, uint64_t stride) {
+    uint64_t y = fdiv(g, p.div_z);
+    z = (int64_t)(g - y * p.div_z.d);
+    x = (int64_t)y * p.syi + z;
+    o = (int64_t)y * p.syo + z;
+    y = fdiv(stride, p.div_z);
+    dz = (int64_t)(stride - y * p.div_z.d);
+    dx = (int64_t)y * p.syi + dz;
+    dxo = (int64_t)y * p.syo + dz;
+  }
+  __device__ __forceinline__ void step(const GradParams& p) {
+    z += dz;
+    x += dx;
+    o += dxo;
+    if (z >= (int64_t)p.div_z.d) {
+      z -= (int64_t)p.div_z.d;
+      x += p.syi - (int64_t)p.div_z.d;
+      o += p.syo - (int64_t)p.div_z.d;
+    }
+  }
+};
+
+// FULL: four input and four output elements
+template <typename T, bool FULL>
+__device__ __forceinline__ void grad4_load(T (&v)[8], const T* __restrict__ X, const T* __restrict__ G,
+                                           const GradParams& p, const Grad4Walk& w) {
+  const T* x = X + w.x;
+  const T* o = G + w.o;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    v[k] = FULL || k < p.kin ? x[k * p.sbi] : (T)0;
+    v[4 + k] = FULL || k < p.kout ? o[k * p.sbo] : (T)0;
+  }
+}
+
+__device__ __forceinline__ void split_band(double v, float& h, float& l, unsigned& bad) {
+  qsgb_split_f64<923u, 141u>(v, h, l, bad);  // 2^-100 <= |v| < 2^41
+}
+__device__ __forceinline__ void split_band(float v, float& h, float& l, unsigned& bad) {
+  bad |= out_of_band(v);
+  h = v;
+  l = 0.0f;
+}
+
+// lanes 2H apart share the sums of entries [0, 2H): each keeps H of them
+template <int H>
+__device__ __forceinline__ void grad4_halve(float (&s)[16], float (&c)[16], int lane) {
+  const bool up = (lane & (2 * H)) != 0;  // keeps the upper ones
+#pragma unroll
+  for (int q = 0; q < H; ++q) {
+    const float ss = up ? s[q] : s[q + H], sc = up ? c[q] : c[q + H];
+    s[q] = up ? s[q + H] : s[q];
+    c[q] = up ? c[q + H] : c[q];
+    df_add(s[q], c[q], __shfl_xor_sync(0xffffffffu, ss, 2 * H), __shfl_xor_sync(0xffffffffu, sc, 2 * H));
+  }
+}
+
+template <typename T, bool FULL>
+__global__ void __launch_bounds__(kGradBlock, 2) grad4_kernel(const __grid_constant__ GradParams p,
+                                                              double* __restrict__ part) {
+  __shared__ double sums[kGradBlock / 32][16];
+  const T* __restrict__ X = static_cast<const T*>(p.x);
+  const T* __restrict__ G = static_cast<const T*>(p.g);
+  const int t = threadIdx.x, lane = t & 31;
+  const uint64_t first = (uint64_t)blockIdx.x * kGradBlock + t, stride = (uint64_t)gridDim.x * kGradBlock;
+  float s[16], c[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) s[q] = c[q] = 0.0f;
+  unsigned bad = 0;
+  pdl_wait();
+  T v[8];
+  Grad4Walk walk(p, first, stride);
+  if (first < p.n_groups) grad4_load<T, FULL>(v, X, G, p, walk);
+  for (uint64_t g = first; g < p.n_groups; g += stride) {
+    float h[8], l[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) split_band(v[k], h[k], l[k], bad);
+    if (g + stride < p.n_groups) {
+      walk.step(p);
+      grad4_load<T, FULL>(v, X, G, p, walk);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int q = 4 * r + k;
+        if constexpr (sizeof(T) == 8) {
+          qsgb_df_fma(s[q], c[q], h[4 + r], l[4 + r], h[k], l[k]);
+        } else {  // the same without the low parts
+          const float s2 = s[q] + __fmul_rn(h[4 + r], h[k]);
+          const float bp = s2 - s[q];
+          c[q] += fmaf(h[4 + r], h[k], -bp) + (s[q] - (s2 - bp));
+          s[q] = s2;
+        }
+      }
+  }
+  double d;  // entry lane / 2 of this warp
+  if (!__syncthreads_or((int)bad)) {
+    grad4_halve<8>(s, c, lane);
+    grad4_halve<4>(s, c, lane);
+    grad4_halve<2>(s, c, lane);
+    grad4_halve<1>(s, c, lane);
+    const float s2 = __shfl_xor_sync(0xffffffffu, s[0], 1), c2 = __shfl_xor_sync(0xffffffffu, c[0], 1);
+    df_add(s[0], c[0], s2, c2);
+    d = qsgb_df_to_double(s[0], c[0]);
+  } else {
+    double f[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) f[q] = 0.0;
+    Grad4Walk again(p, first, stride);
+#pragma unroll 1
+    for (uint64_t g = first; g < p.n_groups; g += stride, again.step(p)) {
+      grad4_load<T, FULL>(v, X, G, p, again);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) f[4 * r + k] = fma((double)v[4 + r], (double)v[k], f[4 * r + k]);
+    }
+    d = 0.0;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) f[q] += __shfl_xor_sync(0xffffffffu, f[q], o);
+      if ((lane >> 1) == q) d = f[q];
+    }
+  }
+  if ((lane & 1) == 0) sums[t >> 5][lane >> 1] = d;
+  __syncthreads();
+  if (t < 16) {
+    const int r = t >> 2, k = t & 3;
+    double r0 = 0.0;
+    for (int w = 0; w < kGradBlock / 32; ++w) r0 += sums[w][t];
+    if (r < p.kout && k < p.kin) part[(int64_t)blockIdx.x * (p.kin * p.kout) + r * p.kin + k] = r0;
+  }
+}
+
 // out[e] = sum over blocks b of part[b][e]: kStage2Entries entries x
 // kStage2Slices block slices per thread block, slices added in order
 __global__ void __launch_bounds__(kStage2Entries* kStage2Slices)
@@ -693,6 +850,15 @@ int grad_common(const void* x_in, const void* g_out, double* dptm, int64_t da_ou
     if (st != QSGB_OK) return st;
     const int s1 = launch_pdl(grad16_tc_kernel, nbt, kTcgBlock, (size_t)smem_bytes, s, p, part);
     return s1 != QSGB_OK ? s1 : launch_stage2(part, (int)nbt, E, dptm, s);
+  }
+  // one qudit (a group's rows lie a stride apart) of at most 4 elements: a
+  // thread's registers hold the outer product
+  if (da_in == 1 && da_out == 1 && X == 1 && kin <= 4 && kout <= 4) {
+    const bool full = kin == 4 && kout == 4;
+    const auto kern = dtype == QSGB_F64 ? (full ? grad4_kernel<double, true> : grad4_kernel<double, false>)
+                                        : (full ? grad4_kernel<float, true> : grad4_kernel<float, false>);
+    const int s1 = launch_pdl(kern, nb, (unsigned)kGradBlock, 0, s, p, part);
+    return s1 != QSGB_OK ? s1 : launch_stage2(part, (int)nb, E, dptm, s);
   }
   const bool two = p.nmt > kGradBlock;
   int st;

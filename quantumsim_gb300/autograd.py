@@ -60,11 +60,22 @@ class ApplyPTM(torch.autograd.Function):
     def backward(ctx, g):
         (x,) = ctx.saved_tensors
         g = g.contiguous()
-        gx = gp = None
-        if ctx.needs_input_grad[0]:
-            gx = torch.ops.qsgb.apply_ptm(g, ctx.ptm_host, list(ctx.qudits),
-                                          ctx.arith, ctx.max_terms, True)
-        if ctx.needs_input_grad[1]:
+        gx = gp = pending = None
+        if ctx.needs_input_grad[1] and ctx.ptm_device.type == 'cpu' and \
+                ops.HostPtmGrad.serves(x, g):
+            # the PTM's gradient goes first and to the host on its own; the
+            # host waits for it while the state's gradient is computed (one
+            # layer on 11 qubits, 16 PTMs: 4.48 -> 4.09 ms)
+            pending = ops.HostPtmGrad(x.contiguous(), g, list(ctx.qudits))
+        try:
+            if ctx.needs_input_grad[0]:
+                gx = torch.ops.qsgb.apply_ptm(
+                    g, ctx.ptm_host, list(ctx.qudits), ctx.arith,
+                    ctx.max_terms, True)
+        finally:
+            if pending is not None:  # its memory is in use until then
+                gp = pending.wait()
+        if ctx.needs_input_grad[1] and pending is None:
             gp = torch.ops.qsgb.ptm_grad(x.contiguous(), g, list(ctx.qudits))
             gp = gp.to(ctx.ptm_device)
         return gx, gp, None, None

@@ -254,6 +254,15 @@ def ptm_grad(x_in: torch.Tensor, g_out: torch.Tensor,
     """dL/dPTM for out = apply_ptm(x_in, PTM, qudits), given dL/dout.
 
     Returned in the PTM's argument-order layout (out..., in...), float64."""
+    res, swap = _ptm_grad_launch(x_in, g_out, qudits)
+    return res.permute(1, 0, 3, 2).contiguous() if swap else res
+
+
+def _ptm_grad_launch(x_in, g_out, qudits, to_host=False):
+    """Enqueue the gradient kernels; returns (result with the qudits in
+    ascending order, exchange the qudits?).  With `to_host` the second stage
+    writes a page-locked host tensor, to be read when the stream is past it.
+    """
     _require_cuda(x_in, g_out)
     if x_in.dtype != g_out.dtype:
         raise TypeError('x_in and g_out must share a dtype')
@@ -276,7 +285,8 @@ def ptm_grad(x_in: torch.Tensor, g_out: torch.Tensor,
         groups = X * Y * Z
         kout, kin = outs[0] * outs[1], ins[0] * ins[1]
     out_sorted = torch.empty(kout * kin, dtype=torch.float64,
-                             device=x_in.device)
+                             pin_memory=True) if to_host else \
+        torch.empty(kout * kin, dtype=torch.float64, device=x_in.device)
     nbytes = lib.qsgb_ptm_grad_scratch_bytes(groups, kout, kin)
     scratch = torch.empty(max(nbytes, 8), dtype=torch.uint8,
                           device=x_in.device)
@@ -285,7 +295,7 @@ def ptm_grad(x_in: torch.Tensor, g_out: torch.Tensor,
             _ptr(x_in), _ptr(g_out), _ptr(out_sorted), outs[0], ins[0], Y, Z,
             _dtype_code(x_in), _ptr(scratch), nbytes, _stream_handle(x_in))
         L.check(status, 'qsgb_ptm_grad1')
-        return out_sorted.view(outs[0], ins[0])
+        return out_sorted.view(outs[0], ins[0]), False
     a, b = sorted(qudits)
     da_o, db_o = g_out.shape[a], g_out.shape[b]
     da_i, db_i = x_in.shape[a], x_in.shape[b]
@@ -293,10 +303,32 @@ def ptm_grad(x_in: torch.Tensor, g_out: torch.Tensor,
         _ptr(x_in), _ptr(g_out), _ptr(out_sorted), da_o, db_o, da_i, db_i, X,
         Y, Z, _dtype_code(x_in), _ptr(scratch), nbytes, _stream_handle(x_in))
     L.check(status, 'qsgb_ptm_grad2')
-    res = out_sorted.view(da_o, db_o, da_i, db_i)
-    if qudits[0] > qudits[1]:
-        res = res.permute(1, 0, 3, 2).contiguous()
-    return res
+    return out_sorted.view(da_o, db_o, da_i, db_i), qudits[0] > qudits[1]
+
+
+class HostPtmGrad:
+    """The gradient of a PTM that lives on the host, on its way: the kernels
+    are enqueued and write page-locked memory; `wait` returns the CPU tensor.
+    Work enqueued in between runs meanwhile."""
+
+    def __init__(self, x_in, g_out, qudits):
+        self._res, self._swap = _ptm_grad_launch(x_in, g_out, qudits, True)
+        self._done = torch.cuda.Event()
+        self._done.record(torch.cuda.current_stream(x_in.device))
+
+    @staticmethod
+    def serves(*tensors):
+        """Whether the kernels may be called outside the dispatcher: plain
+        tensors, no gradient of the gradient, no tracing, no capture."""
+        return (not torch.is_grad_enabled() and
+                all(type(t) is torch.Tensor for t in tensors) and
+                torch._C._len_torch_dispatch_stack() == 0 and
+                not torch.cuda.is_current_stream_capturing())
+
+    def wait(self):
+        self._done.synchronize()
+        res = self._res.permute(1, 0, 3, 2) if self._swap else self._res
+        return res.clone(memory_format=torch.contiguous_format)
 
 
 @_fake('ptm_grad')

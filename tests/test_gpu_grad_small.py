@@ -68,3 +68,37 @@ def test_values_outside_the_band(value):
         fin = np.isfinite(ref)
         np.testing.assert_array_equal(np.isfinite(got), fin)
         assert np.all(np.abs(got[fin] - ref[fin]) <= TOL * mag[fin])
+
+
+@pytest.mark.parametrize('qs,pshape', [((1,), (4, 4)), ((0, 2), (4, 4, 4, 4)),
+                                       ((3, 1), (4, 3, 4, 4)),
+                                       ((2,), (3, 4))])
+def test_host_ptm_gradient_is_the_device_one(qs, pshape):
+    """A PTM on the host gets its gradient through page-locked memory while
+    the state's is computed: the bits of the same PTM on the device, also
+    when it is used twice, and with a graph of the gradient (another path)."""
+    rng = np.random.default_rng(len(pshape))
+    x = torch.from_numpy(rng.normal(size=(4,) * 5)).cuda()
+    p = rng.normal(size=pshape)
+    twice = pshape[:len(qs)] == pshape[len(qs):]
+
+    def grads(ptm, **kw):
+        a = x.clone().requires_grad_(True)
+        y = quantumsim_gb300.apply_ptm_diff(a, ptm, *qs)
+        if twice:
+            y = quantumsim_gb300.apply_ptm_diff(y, ptm, *qs)
+        return torch.autograd.grad((y * y).sum(), [a, ptm], **kw)
+
+    host = torch.from_numpy(p).requires_grad_(True)
+    ga, gp = grads(host)
+    assert not gp.is_cuda and not gp.is_pinned() and gp.shape == host.shape
+    for got, want in zip(grads(host), (ga, gp)):
+        assert torch.equal(got, want)
+    for got, want in zip(grads(host, create_graph=True), (ga, gp)):
+        assert torch.equal(got.detach(), want)
+    dev = torch.ops.qsgb.ptm_grad  # one application, the operator's result
+    a = x.clone().requires_grad_(True)
+    y = quantumsim_gb300.apply_ptm_diff(a, host, *qs)
+    g = torch.randn_like(y)
+    (gp,) = torch.autograd.grad(y, [host], g)
+    assert torch.equal(gp, dev(x, g, list(qs)).cpu())

@@ -254,81 +254,122 @@ def ptm_grad(x_in: torch.Tensor, g_out: torch.Tensor,
     """dL/dPTM for out = apply_ptm(x_in, PTM, qudits), given dL/dout.
 
     Returned in the PTM's argument-order layout (out..., in...), float64."""
-    res, swap = _ptm_grad_launch(x_in, g_out, qudits)
-    return res.permute(1, 0, 3, 2).contiguous() if swap else res
-
-
-def _ptm_grad_launch(x_in, g_out, qudits, to_host=False):
-    """Enqueue the gradient kernels; returns (result with the qudits in
-    ascending order, exchange the qudits?).  With `to_host` the second stage
-    writes a page-locked host tensor, to be read when the stream is past it.
-    """
     _require_cuda(x_in, g_out)
     if x_in.dtype != g_out.dtype:
         raise TypeError('x_in and g_out must share a dtype')
-    n = len(qudits)
-    outs = [g_out.shape[q] for q in qudits]
-    ins = [x_in.shape[q] for q in qudits]
-    x_in = x_in.contiguous()
-    g_out = g_out.contiguous()
-    lib = L.load()
-    shape = list(x_in.shape)
-    if n == 1:
-        (q,) = qudits
-        Y, Z = math.prod(shape[:q]), math.prod(shape[q + 1:])
-        groups, kout, kin = Y * Z, outs[0], ins[0]
+    plan = grad_plan(x_in.shape, g_out.shape, qudits)
+    _, shape, kk, _, swap = plan
+    out = torch.empty(kk, dtype=torch.float64, device=x_in.device)
+    _ptm_grad_launch(plan, x_in.contiguous(), g_out.contiguous(),
+                     out.data_ptr())
+    res = out.view(shape)
+    return res.permute(1, 0, 3, 2).contiguous() if swap else res
+
+
+def grad_plan(x_shape, g_shape, qudits):
+    """Geometry of ptm_grad: (size arguments, shape of the result with the
+    qudits in ascending order, its entries, groups and sizes for the scratch,
+    exchange the qudits?)."""
+    order = sorted(qudits)
+    ins, outs = [x_shape[q] for q in order], [g_shape[q] for q in order]
+    kin, kout = math.prod(ins), math.prod(outs)
+    if len(order) == 1:
+        (q,) = order
+        outer = [math.prod(x_shape[:q]), math.prod(x_shape[q + 1:])]
     else:
-        a, b = sorted(qudits)
-        X = math.prod(shape[:a])
-        Y = math.prod(shape[a + 1:b])
-        Z = math.prod(shape[b + 1:])
-        groups = X * Y * Z
-        kout, kin = outs[0] * outs[1], ins[0] * ins[1]
-    out_sorted = torch.empty(kout * kin, dtype=torch.float64,
-                             pin_memory=True) if to_host else \
-        torch.empty(kout * kin, dtype=torch.float64, device=x_in.device)
-    nbytes = lib.qsgb_ptm_grad_scratch_bytes(groups, kout, kin)
+        a, b = order
+        outer = [math.prod(x_shape[:a]), math.prod(x_shape[a + 1:b]),
+                 math.prod(x_shape[b + 1:])]
+    return (tuple(outs + ins + outer), tuple(outs + ins), kout * kin,
+            (math.prod(outer), kout, kin), list(qudits) != order)
+
+
+def _ptm_grad_launch(plan, x_in, g_out, out_ptr):
+    """Enqueue the gradient kernels on contiguous tensors; the result goes to
+    the address `out_ptr`, on the device or page-locked on the host."""
+    sizes, _, _, parts, _ = plan
+    lib = L.load()
+    nbytes = lib.qsgb_ptm_grad_scratch_bytes(*parts)
     scratch = torch.empty(max(nbytes, 8), dtype=torch.uint8,
                           device=x_in.device)
-    if n == 1:
-        status = lib.qsgb_ptm_grad1(
-            _ptr(x_in), _ptr(g_out), _ptr(out_sorted), outs[0], ins[0], Y, Z,
-            _dtype_code(x_in), _ptr(scratch), nbytes, _stream_handle(x_in))
-        L.check(status, 'qsgb_ptm_grad1')
-        return out_sorted.view(outs[0], ins[0]), False
-    a, b = sorted(qudits)
-    da_o, db_o = g_out.shape[a], g_out.shape[b]
-    da_i, db_i = x_in.shape[a], x_in.shape[b]
-    status = lib.qsgb_ptm_grad2(
-        _ptr(x_in), _ptr(g_out), _ptr(out_sorted), da_o, db_o, da_i, db_i, X,
-        Y, Z, _dtype_code(x_in), _ptr(scratch), nbytes, _stream_handle(x_in))
-    L.check(status, 'qsgb_ptm_grad2')
-    return out_sorted.view(da_o, db_o, da_i, db_i), qudits[0] > qudits[1]
+    fn = lib.qsgb_ptm_grad1 if len(sizes) == 4 else lib.qsgb_ptm_grad2
+    status = fn(x_in.data_ptr(), g_out.data_ptr(), out_ptr, *sizes,
+                _dtype_code(x_in), scratch.data_ptr(), nbytes,
+                _stream_handle(x_in))
+    L.check(status, fn.__name__)
+
+
+_DIRECT_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
+def direct(*tensors):
+    """Whether kernels may be called on these tensors past the dispatcher:
+    plain CUDA tensors of the two storage types, nothing to be recorded for a
+    gradient and no tracing."""
+    if torch.is_grad_enabled() or torch._C._len_torch_dispatch_stack():
+        return False
+    for t in tensors:
+        if type(t) not in _DIRECT_TYPES or not t.is_cuda or \
+                t.dtype not in (torch.float64, torch.float32):
+            return False
+    return True
+
+
+_DIRECT_PLANS = {}  # geometry alone
+
+
+def _direct_plan(make, *key):
+    plan = _DIRECT_PLANS.get((make, key))
+    if plan is None:
+        plan = make(*key)
+        if len(_DIRECT_PLANS) > 4096:
+            _DIRECT_PLANS.clear()
+        _DIRECT_PLANS[make, key] = plan
+    return plan
+
+
+def apply_direct(x, ptm, qudits, arith, transpose):
+    """torch.ops.qsgb.apply_ptm for `direct` tensors and a host PTM: the
+    compiled per-call entry point with a cached plan (~6 us of host time
+    instead of ~28)."""
+    if ptm.dtype == torch.float64 and ptm.is_contiguous():
+        plan = _direct_plan(eager_plan, x.shape, x.dtype, qudits, ptm.shape,
+                            transpose)
+        out = eager_apply(x.contiguous(), ptm.numpy(), plan, arith)
+        if out is not None:
+            return out
+    return torch.ops.qsgb.apply_ptm(x, ptm, list(qudits), arith, 0, transpose)
 
 
 class HostPtmGrad:
     """The gradient of a PTM that lives on the host, on its way: the kernels
     are enqueued and write page-locked memory; `wait` returns the CPU tensor.
-    Work enqueued in between runs meanwhile."""
+    Work enqueued in between runs meanwhile.  One at a time per thread and
+    device: the memory and the event are the thread's."""
 
     def __init__(self, x_in, g_out, qudits):
-        self._res, self._swap = _ptm_grad_launch(x_in, g_out, qudits, True)
-        self._done = torch.cuda.Event()
+        index = x_in.device.index
+        bufs = _READ_BUF.__dict__.setdefault('grads', {})
+        plan = _direct_plan(grad_plan, x_in.shape, g_out.shape, qudits)
+        _, self._shape, self._n, _, self._swap = plan
+        b = bufs.get(index)
+        if b is None or b[0].numel() < self._n:
+            host = torch.empty(max(self._n, 256), dtype=torch.float64,
+                               pin_memory=True)
+            b = (host, host.numpy(), host.data_ptr(), torch.cuda.Event())
+            bufs[index] = b
+        _, self._host, out_ptr, self._done = b
+        if x_in.dtype != g_out.dtype:
+            raise TypeError('x_in and g_out must share a dtype')
+        _ptm_grad_launch(plan, x_in, g_out, out_ptr)
         self._done.record(torch.cuda.current_stream(x_in.device))
-
-    @staticmethod
-    def serves(*tensors):
-        """Whether the kernels may be called outside the dispatcher: plain
-        tensors, no gradient of the gradient, no tracing, no capture."""
-        return (not torch.is_grad_enabled() and
-                all(type(t) is torch.Tensor for t in tensors) and
-                torch._C._len_torch_dispatch_stack() == 0 and
-                not torch.cuda.is_current_stream_capturing())
 
     def wait(self):
         self._done.synchronize()
-        res = self._res.permute(1, 0, 3, 2) if self._swap else self._res
-        return res.clone(memory_format=torch.contiguous_format)
+        res = self._host[:self._n].reshape(self._shape)
+        if self._swap:
+            res = res.transpose(1, 0, 3, 2)
+        return torch.from_numpy(res.copy(order='C'))
 
 
 @_fake('ptm_grad')
@@ -486,14 +527,15 @@ def status_ptr(index):
     return p
 
 
-def eager_plan(shape, dtype, qudits, ptm_shape):
-    """Validated geometry of applying a host PTM of `ptm_shape` to `qudits`
-    of a contiguous vector of `shape` and torch `dtype`: (output shape, two
+def eager_plan(shape, dtype, qudits, ptm_shape, transpose=False):
+    """Validated geometry of applying a host PTM of `ptm_shape` (or its
+    transpose) to `qudits` of a contiguous vector of `shape` and torch `dtype`: (output shape, two
     qudits?, size arguments, layout flags, dtype code).  Raises ValueError
     like apply_geometry."""
     new_shape, (X, Y, Z), (dao, dbo, dai, dbi), swapped = apply_geometry(
-        shape, list(qudits), ptm_shape)
-    flags = L.PTM_HOST | (L.PTM_SWAPPED if swapped else 0)
+        shape, list(qudits), ptm_shape, transpose)
+    flags = L.PTM_HOST | (L.PTM_SWAPPED if swapped else 0) | (
+        L.PTM_TRANSPOSED if transpose else 0)
     code = L.F64 if dtype == torch.float64 else L.F32
     if len(qudits) == 1:
         return tuple(new_shape), False, (dbo, dbi, Y, Z), flags, code

@@ -173,6 +173,15 @@ int qsgb_gather(const void* in, void* out, int in_dtype, int out_dtype,
                 const int32_t* idx, void* stream);
 
 /*
+ * The adjoint of qsgb_gather: out (of out_shape, out_dtype) is zeroed and
+ * the FP64 value in[o] is added where the gather with the same index lists
+ * reads entry o; entries with an index of -1 go nowhere.
+ */
+int qsgb_scatter(const double* in, void* out, int out_dtype, int ndim,
+                 const int64_t* out_shape, const int32_t* idx_off,
+                 const int32_t* idx, void* stream);
+
+/*
  * qsgb_gather to the host, widened to FP64: the n taken values and then the
  * value of the device status word *dev_status (0 when NULL), n + 1 doubles
  * written by the kernel straight into host_out, which must be page-locked

@@ -58,6 +58,8 @@ SIGNATURES = {
                                    _i64]),
     'qsgb_gather': (_int, [_c_void_p, _c_void_p, _int, _int, _int, _p_i64,
                            _p_i32, _p_i32, _c_void_p]),
+    'qsgb_scatter': (_int, [_c_void_p, _c_void_p, _int, _int, _p_i64, _p_i32,
+                            _p_i32, _c_void_p]),
     'qsgb_gather_host': (_int, [_c_void_p, _int, _int, _p_i64, _p_i32,
                                 _p_i32, _c_void_p, _c_void_p, _c_void_p]),
     'qsgb_diag_marginals': (_int, [_c_void_p, _int, _int, _p_i64, _p_i32,

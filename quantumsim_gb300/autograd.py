@@ -117,34 +117,36 @@ def diagonal_indices(bases):
 
 
 class Diagonal(torch.autograd.Function):
-    """Diagonal (FP64) of a Pauli vector: gather forward, scatter back."""
+    """Diagonal (FP64) of a Pauli vector: gather forward, scatter back.  The
+    index lists travel in both launches (computing every entry's flat index
+    and copying them to the device took most of a call); `flat_idx` is not
+    needed and may be None."""
 
     @staticmethod
     def forward(ctx, x, flat_idx, idx_off, idx_list):
         d = torch.ops.qsgb.gather(x.contiguous(), idx_off, idx_list, True)
-        ctx.save_for_backward(flat_idx)
+        ctx.idx = idx_off, idx_list
         ctx.shape = x.shape
         ctx.dtype = x.dtype
         return d
 
     @staticmethod
     def backward(ctx, g):
-        (flat_idx,) = ctx.saved_tensors
-        gx = torch.zeros(math.prod(ctx.shape), dtype=ctx.dtype,
-                         device=g.device)
-        gx.index_copy_(0, flat_idx, g.to(ctx.dtype))
-        return gx.view(ctx.shape), None, None, None
+        gx = torch.ops.qsgb.scatter(g, list(ctx.shape), *ctx.idx,
+                                    ctx.dtype == torch.float64)
+        return gx, None, None, None
 
 
 def diagonal_diff(x, bases):
     """Differentiable diagonal() (length prod(d_hilbert), float64)."""
-    flat = torch.from_numpy(diagonal_indices(bases)).to(x.device)
     idx_off, idx_list = [0], []
     for b in bases:
-        idx_list += [int(b.computational_basis_indices[i])
-                     for i in range(b.dim_hilbert)]
+        idx = [b.computational_basis_indices[i] for i in range(b.dim_hilbert)]
+        if any(i is None for i in idx):
+            raise ValueError('basis without unit computational vectors')
+        idx_list += idx
         idx_off.append(len(idx_list))
-    return Diagonal.apply(x, flat, idx_off, idx_list)
+    return Diagonal.apply(x, None, idx_off, idx_list)
 
 
 def checkpointed(layers, x, every=8):

@@ -72,6 +72,32 @@ __global__ void gather_kernel(const __grid_constant__ GatherParams p) {
   if (p.status_out && blockIdx.x == 0 && threadIdx.x == 0) *p.status_out = p.status ? (double)*p.status : 0.0;
 }
 
+// The adjoint: in[o] is added to the element of out (zeroed before) that the
+// gather reads for o; places with an index of -1 go nowhere.  One value meets
+// one element unless an axis names an index twice.
+template <typename T>
+__global__ void scatter_kernel(const __grid_constant__ GatherParams p) {
+  __shared__ int sidx[kMaxIdx];
+  for (int i = threadIdx.x; i < p.idx_off[p.ndim]; i += blockDim.x) sidx[i] = p.idx[i];
+  __syncthreads();
+  const double* __restrict__ in = static_cast<const double*>(p.in);
+  T* __restrict__ out = static_cast<T*>(p.out);
+  for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < p.n_out;
+       o += (uint64_t)gridDim.x * blockDim.x) {
+    uint64_t rem = o;
+    int64_t addr = 0;
+    bool none = false;
+    for (int a = p.ndim - 1; a >= 0; --a) {
+      const uint64_t q = fdiv(rem, p.div[a]);
+      const int j = sidx[p.idx_off[a] + (int)(rem - q * p.div[a].d)];
+      rem = q;
+      none |= (j < 0);
+      addr += (int64_t)(j < 0 ? 0 : j) * p.in_stride[a];
+    }
+    if (!none) atomicAdd(out + addr, (T)in[o]);
+  }
+}
+
 // ---------------------------------------------------------------- take axis
 // out[o, j, :] = in[o, idx[j], :] for a tensor viewed as (outer, d_in,
 // inner): a copy of rows of `inner` contiguous elements, moved as raw bits
@@ -526,22 +552,20 @@ unsigned grid_for(uint64_t n, int block, int per_sm = 8) {
 
 using namespace qsgb;
 
-static int gather_common(const void* in, void* out, int in_dtype, int out_dtype, int ndim, const int64_t* in_shape,
-                         const int32_t* idx_off, const int32_t* idx, const unsigned* status, double* status_out,
-                         cudaStream_t s) {
+// Checks and parameters of a gather from, or a scatter to, a tensor of `shape`;
+// its number of elements comes back in n_tensor.
+static int gather_params(GatherParams& p, uint64_t& n_tensor, const void* in, void* out, int in_dtype, int out_dtype,
+                         int ndim, const int64_t* in_shape, const int32_t* idx_off, const int32_t* idx) {
   if (!in || !out || !in_shape || !idx_off || (!idx && ndim > 0)) return QSGB_ERR_INVALID;
   if (ndim < 0 || ndim > kMaxDim) return QSGB_ERR_UNSUPPORTED;
   if ((in_dtype != QSGB_F64 && in_dtype != QSGB_F32) || (out_dtype != QSGB_F64 && out_dtype != QSGB_F32))
     return QSGB_ERR_INVALID;
   if (idx_off[0] != 0 || idx_off[ndim] > kMaxIdx) return QSGB_ERR_UNSUPPORTED;
-  GatherParams p{};  // copied into the launch
   p.in = in;
   p.out = out;
   p.in_dtype = in_dtype;
   p.out_dtype = out_dtype;
   p.ndim = ndim;
-  p.status = status;
-  p.status_out = status_out;
   uint64_t n_out = 1;
   int64_t stride = 1;
   for (int a = ndim - 1; a >= 0; --a) {
@@ -557,8 +581,21 @@ static int gather_common(const void* in, void* out, int in_dtype, int out_dtype,
   for (int a = 0; a <= ndim; ++a) p.idx_off[a] = idx_off[a];
   for (int i = 0; i < idx_off[ndim]; ++i) p.idx[i] = idx[i];
   p.n_out = n_out;
+  n_tensor = (uint64_t)stride;
+  return QSGB_OK;
+}
+
+static int gather_common(const void* in, void* out, int in_dtype, int out_dtype, int ndim, const int64_t* in_shape,
+                         const int32_t* idx_off, const int32_t* idx, const unsigned* status, double* status_out,
+                         cudaStream_t s) {
+  GatherParams p{};  // copied into the launch
+  uint64_t n_tensor;
+  const int st = gather_params(p, n_tensor, in, out, in_dtype, out_dtype, ndim, in_shape, idx_off, idx);
+  if (st != QSGB_OK) return st;
+  p.status = status;
+  p.status_out = status_out;
   const int block = 256;
-  const unsigned grid = grid_for(n_out, block);
+  const unsigned grid = grid_for(p.n_out, block);
   if (in_dtype == QSGB_F64 && out_dtype == QSGB_F64)
     return launch_pdl(gather_kernel<double, double>, grid, block, 0, s, p);
   if (in_dtype == QSGB_F32 && out_dtype == QSGB_F64)
@@ -566,6 +603,22 @@ static int gather_common(const void* in, void* out, int in_dtype, int out_dtype,
   if (in_dtype == QSGB_F64 && out_dtype == QSGB_F32)
     return launch_pdl(gather_kernel<double, float>, grid, block, 0, s, p);
   return launch_pdl(gather_kernel<float, float>, grid, block, 0, s, p);
+}
+
+extern "C" int qsgb_scatter(const double* in, void* out, int out_dtype, int ndim, const int64_t* out_shape,
+                            const int32_t* idx_off, const int32_t* idx, void* stream) {
+  GatherParams p{};
+  uint64_t n_tensor;
+  const int st = gather_params(p, n_tensor, in, out, QSGB_F64, out_dtype, ndim, out_shape, idx_off, idx);
+  if (st != QSGB_OK) return st;
+  cudaStream_t s = as_stream(stream);
+  QSGB_CUDA_TRY(cudaMemsetAsync(out, 0, n_tensor * (out_dtype == QSGB_F64 ? 8 : 4), s));
+  const unsigned block = 256, grid = grid_for(p.n_out, (int)block);
+  if (out_dtype == QSGB_F64)
+    scatter_kernel<double><<<grid, block, 0, s>>>(p);
+  else
+    scatter_kernel<float><<<grid, block, 0, s>>>(p);
+  return launch_status();
 }
 
 extern "C" int qsgb_gather(const void* in, void* out, int in_dtype, int out_dtype, int ndim, const int64_t* in_shape,

@@ -407,6 +407,31 @@ def _(pv, idx_off, idx, out_f64):
     return pv.new_empty(n_out, dtype=torch.float64 if out_f64 else pv.dtype)
 
 
+@_op('scatter(Tensor g, int[] shape, int[] idx_off, int[] idx, bool out_f64) '
+     '-> Tensor')
+def scatter(g: torch.Tensor, shape: List[int], idx_off: List[int],
+            idx: List[int], out_f64: bool) -> torch.Tensor:
+    """The adjoint of gather: zeros of `shape` plus the float64 values `g`
+    where the gather with the same indices reads."""
+    _require_cuda(g)
+    if g.dtype != torch.float64:
+        raise TypeError('scatter takes float64 values')
+    g = g.contiguous()
+    out = torch.empty(shape, dtype=torch.float64 if out_f64 else
+                      torch.float32, device=g.device)
+    status = L.load().qsgb_scatter(
+        _ptr(g), _ptr(out), _dtype_code(out), len(shape), L.i64_array(shape),
+        L.i32_array(idx_off), L.i32_array(idx), _stream_handle(g))
+    L.check(status, 'qsgb_scatter')
+    return out
+
+
+@_fake('scatter')
+def _(g, shape, idx_off, idx, out_f64):
+    return g.new_empty(shape, dtype=torch.float64 if out_f64 else
+                       torch.float32)
+
+
 @_op('take_axis(Tensor pv, int axis, int[] idx) -> Tensor')
 def take_axis(pv: torch.Tensor, axis: int, idx: List[int]) -> torch.Tensor:
     """pv.index_select(axis, idx) as a bit-exact copy; -1 selects a zero."""

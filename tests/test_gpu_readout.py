@@ -114,3 +114,24 @@ def test_status_is_read_along():
         with pytest.raises(RuntimeError, match='float-float range'):
             read()
         read()
+
+
+@pytest.mark.parametrize('dtype', [torch.float64, torch.float32])
+@pytest.mark.parametrize('shape,idx', [
+    ((4,), [[0, 3]]), ((4, 3, 4), [[2], [0, 1, 2], [3, 0]]),
+    ((4, 9), [[1, -1], [8, 0, 4]]), ((4,) * 9, [[0, 3]] * 9)], ids=str)
+def test_scatter_is_the_adjoint_of_gather(shape, idx, dtype):
+    """Whole values: exact."""
+    off = np.cumsum([0] + [len(i) for i in idx]).tolist()
+    flat = [int(i) for axis in idx for i in axis]
+    n = int(np.prod([len(i) for i in idx]))
+    g = torch.arange(1, n + 1, dtype=torch.float64, device='cuda')
+    got = torch.ops.qsgb.scatter(g, list(shape), off, flat,
+                                 dtype == torch.float64)
+    assert got.dtype == dtype and got.shape == shape
+    ref = np.zeros(shape)
+    for o, pos in enumerate(np.ndindex(*[len(i) for i in idx])):
+        at = tuple(axis[k] for axis, k in zip(idx, pos))
+        if min(at) >= 0:
+            ref[at] += o + 1
+    np.testing.assert_array_equal(got.cpu().numpy(), ref)

@@ -196,7 +196,7 @@ class NoisyCircuitModel:
                 self.layers(p, lambda s, pt, qs: apply_ptm_diff(s, pt, *qs,
                                                                 **kw),
                             fuse=fuse),
-                x, checkpoint_every)
+                x, checkpoint_every, keep_last=True)
             return diagonal_diff(x, [self.basis] * self.n)
         device = device or torch.device('cpu')
         x = self.initial_state(device, torch.float64)
@@ -309,7 +309,7 @@ class GraphedGradient:
                     x = apply_ptm_diff(x, leaves[kind][i], *qs)
                 return x
             fns.append(layer)
-        x = checkpointed(fns, self.x0.clone(), self.every)
+        x = checkpointed(fns, self.x0.clone(), self.every, keep_last=True)
         prob = self._diag.apply(x, self.flat, self.idx_off, self.idx_list)
         t = self.target
         return torch.sum(t * (torch.log(t) - torch.log(prob)))

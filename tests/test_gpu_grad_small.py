@@ -102,3 +102,28 @@ def test_host_ptm_gradient_is_the_device_one(qs, pshape):
     g = torch.randn_like(y)
     (gp,) = torch.autograd.grad(y, [host], g)
     assert torch.equal(gp, dev(x, g, list(qs)).cpu())
+
+
+@pytest.mark.parametrize('n_layers,every', [(1, 1), (3, 8), (4, 2), (5, 2)])
+def test_last_segment_kept(n_layers, every):
+    """The last segment's states kept or recomputed: the same bits."""
+    rng = np.random.default_rng(n_layers)
+    ptms = [torch.from_numpy(rng.normal(size=(4, 4, 4, 4))).cuda()
+            .requires_grad_(True) for _ in range(n_layers)]
+    x = torch.from_numpy(rng.normal(size=(4,) * 4)).cuda().requires_grad_(True)
+    calls = []
+
+    def layer(s, i):
+        calls.append(i)
+        return quantumsim_gb300.apply_ptm_diff(s, ptms[i], i % 3, 3)
+
+    fns = [lambda s, i=i: layer(s, i) for i in range(n_layers)]
+    out = []
+    for keep in (False, True):
+        calls.clear()
+        y = quantumsim_gb300.checkpointed(fns, x, every, keep_last=keep)
+        out.append([y] + list(torch.autograd.grad((y * y).sum(), [x] + ptms)))
+        last = n_layers - (n_layers - 1) // every * every
+        assert len(calls) == 2 * n_layers - (last if keep else 0)
+    for a, b in zip(*out):
+        assert torch.equal(a, b)

@@ -58,6 +58,7 @@ struct GradParams {
   int64_t sxo, syo, sao, sbo;
   // shared-memory byte offsets
   int off_gb, off_offs, off_fb, off_red2, off_flag, smem;
+  int vec_z1;  // 16 x 16: the second qudit's four elements are one 32-byte word
 };
 
 unsigned grad_blocks(uint64_t n_groups, int tg) {
@@ -521,7 +522,7 @@ __global__ void __launch_bounds__(kStage2Entries* kStage2Slices)
 // The same reduction as a product over groups, dP = G^T X per chunk of 16
 // groups, on mma.sync.m16n8k16 (FP16 operands, FP32 accumulators) with the
 // error-free digit split of the apply kernel (qsgb_tc.h): within a chunk,
-// row r of A = G^T is scaled by its largest exponent over the chunk's 16
+// row r of A = G^T is scaled by its largest exponent over the chunk's
 // groups and column k of B = X by its own, each value written as a 55-bit
 // fixed-point integer in seven balanced base-256 FP16 digits.  For every digit
 // pair (i, j) with i + j <= 7 two MMAs (n = 0..7, 8..15) add into level
@@ -540,21 +541,33 @@ __global__ void __launch_bounds__(kStage2Entries* kStage2Slices)
 // exchanged, so that 8 groups' half rows fall into different banks).  The
 // fragments come back transposed (ldmatrix.trans): lane
 // (gid, tig) = (l / 4, l % 4) ends with entries
-// (r, k) = (gid or gid + 8, nt * 8 + 2 tig + {0, 1}).  Measured on GB300, a
-// gradient with its second stage, against base-1024 digits stored in two bytes
-// each and read by 4-byte loads: 10 qubits (4096 chunks) 21.8 -> 18.1 us, 12
-// qubits 173 -> 140 us.
+// (r, k) = (gid or gid + 8, nt * 8 + 2 tig + {0, 1}).
+//
+// H = 2: a chunk of 32 groups, two such halves with common exponents whose
+// level sums are added as integers (a bit more each).  Exponent search,
+// recombination and the FP64 sums (16 operations of a pipe that takes a warp
+// 16 cycles) are paid once for both, and twice the loads are in flight; the
+// planes of 16 warps fill an SM's shared memory in one block.  With no more
+// chunks of 16 than resident warps, H = 1 spreads the work further.
+//
+// Bound by instruction issue and latency: at 12 qubits 2.0 TB/s.  Measured on
+// GB300, a gradient with its second stage, at 10 and 12 qubits (4096 and 65536
+// chunks of 16): base-1024 digits 21.8 and 173 us, base 256 with H = 1 19.9 and
+// 144, H = 2 17.3 and 131; on the last two qudits, with 32-byte loads instead
+// of 8-byte ones, 25.0 and 174 -> 18.6 and 138.
 constexpr int kTcgBlock = 256;
 constexpr int kTcgWarps = kTcgBlock / 32;
 constexpr int kTcgPlane = 16 * 16 * 2;  // bytes per digit plane
 
+template <int H>
 struct TcgWarpSmem {
-  unsigned char a[tc::kPlanes * kTcgPlane];  // digits of g_out: [g][r]
-  unsigned char b[tc::kPlanes * kTcgPlane];  // digits of x_in: [g][k]
-  int er[16], ek[16];                        // chunk exponents of rows, columns
+  unsigned char a[H][tc::kPlanes * kTcgPlane];  // digits of g_out: [g][r]
+  unsigned char b[H][tc::kPlanes * kTcgPlane];  // digits of x_in: [g][k]
+  int er[16], ek[16];                           // chunk exponents of rows, columns
 };
+template <int H>
 struct TcgSmem {
-  TcgWarpSmem warp[kTcgWarps];
+  TcgWarpSmem<H> warp[kTcgWarps * H];
   int64_t oin[16], oout[16];  // row offsets of x_in and g_out
 };
 
@@ -565,12 +578,17 @@ __device__ __forceinline__ void ldmatrix4_trans(unsigned (&r)[4], uint32_t addr)
                : "memory");
 }
 
-__global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_constant__ GradParams p,
+__device__ __forceinline__ void load4(double* v, const double* src) {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(src));
+}
+
+template <int H>
+__global__ void __launch_bounds__(kTcgBlock* H, 2 / H) grad16_tc_kernel(const __grid_constant__ GradParams p,
                                                               double* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  TcgSmem& sm = *reinterpret_cast<TcgSmem*>(smem);
-  TcgWarpSmem& ws = sm.warp[w];
+  TcgSmem<H>& sm = *reinterpret_cast<TcgSmem<H>*>(smem);
+  TcgWarpSmem<H>& ws = sm.warp[w];
   const double* __restrict__ X = static_cast<const double*>(p.x);
   const double* __restrict__ G = static_cast<const double*>(p.g);
   const int h = lane >> 4, i = lane & 15;
@@ -589,8 +607,8 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
   // ldmatrix source rows: A tiles (g 0-7 | r 0-7), (0-7 | 8-15), (8-15 | 0-7), (8-15 | 8-15);
   // B tiles (g 0-7 | k 0-7), (8-15 | 0-7), (0-7 | 8-15), (8-15 | 8-15)
   const int lr = lane & 7, t1b = (lane >> 3) & 1, t2b = lane >> 4;
-  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(ws.a) + half_row(lr + 8 * t2b, t1b);
-  const uint32_t sb = (uint32_t)__cvta_generic_to_shared(ws.b) + half_row(lr + 8 * t1b, t2b);
+  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(ws.a[0]) + half_row(lr + 8 * t2b, t1b);
+  const uint32_t sb = (uint32_t)__cvta_generic_to_shared(ws.b[0]) + half_row(lr + 8 * t1b, t2b);
   auto bases = [&](uint64_t g, int64_t& bi, int64_t& bo) {
     const uint64_t t1 = fdiv(g, p.div_z);
     const uint64_t z = g - t1 * p.div_z.d;
@@ -605,31 +623,45 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[nt][q] = 0.0;
 
-  const uint64_t n_chunks = (p.n_groups + 15) / 16;
-  const uint64_t wstride = (uint64_t)gridDim.x * kTcgWarps;
-  for (uint64_t c = (uint64_t)blockIdx.x * kTcgWarps + w; c < n_chunks; c += wstride) {
-    const uint64_t g = c * 16 + i;
-    const bool live = g < p.n_groups;
-    double gv[8], xv[8];
-    if (live) {
-      int64_t bi, bo;
-      bases(g, bi, bo);
+  const uint64_t n_chunks = (p.n_groups + 16 * H - 1) / (16 * H);
+  const uint64_t wstride = (uint64_t)gridDim.x * kTcgWarps * H;
+  for (uint64_t c = (uint64_t)blockIdx.x * kTcgWarps * H + w; c < n_chunks; c += wstride) {
+    double gv[H][8], xv[H][8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        gv[j] = G[bo + sm.oout[8 * h + j]];
-        xv[j] = X[bi + sm.oin[8 * h + j]];
+    for (int hf = 0; hf < H; ++hf) {
+      const uint64_t g = c * (16 * H) + 16 * hf + i;
+      if (g < p.n_groups) {
+        int64_t bi, bo;
+        bases(g, bi, bo);
+        if (p.vec_z1) {
+#pragma unroll
+          for (int j = 0; j < 8; j += 4) {
+            load4(gv[hf] + j, G + bo + sm.oout[8 * h + j]);
+            load4(xv[hf] + j, X + bi + sm.oin[8 * h + j]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            gv[hf][j] = G[bo + sm.oout[8 * h + j]];
+            xv[hf][j] = X[bi + sm.oin[8 * h + j]];
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gv[hf][j] = xv[hf][j] = 0.0;
       }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) gv[j] = xv[j] = 0.0;
     }
     // chunk exponents of rows 8h+j (g_out, low half word) and columns 8h+j
     // (x_in, high half word): maxima over the 16 lanes of this half
     unsigned e2[8], nonfinite = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const unsigned hg = (unsigned)__double2hiint(gv[j]), hx = (unsigned)__double2hiint(xv[j]);
-      e2[j] = ((hg >> 20) & 0x7ffu) | ((hx >> 4) & 0x7ff0000u);
+      e2[j] = 0u;
+#pragma unroll
+      for (int hf = 0; hf < H; ++hf) {
+        const unsigned hg = (unsigned)__double2hiint(gv[hf][j]), hx = (unsigned)__double2hiint(xv[hf][j]);
+        e2[j] = __vmaxu2(e2[j], ((hg >> 20) & 0x7ffu) | ((hx >> 4) & 0x7ff0000u));
+      }
     }
 #pragma unroll
     for (int o = 1; o < 16; o <<= 1)
@@ -647,8 +679,11 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
         // a row or column that is all zero (exact) or below the smallest scale
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          if ((e2[j] & 0xffffu) < tc::kMinExp && gv[j] != 0.0) nonfinite = 1u;
-          if ((e2[j] >> 16) < tc::kMinExp && xv[j] != 0.0) nonfinite = 1u;
+#pragma unroll
+          for (int hf = 0; hf < H; ++hf) {
+            if ((e2[j] & 0xffffu) < tc::kMinExp && gv[hf][j] != 0.0) nonfinite = 1u;
+            if ((e2[j] >> 16) < tc::kMinExp && xv[hf][j] != 0.0) nonfinite = 1u;
+          }
           // any scale serves zeros
           if ((e2[j] & 0xffffu) < tc::kMinExp) e2[j] = (e2[j] & 0xffff0000u) | 1023u;
           if ((e2[j] >> 16) < tc::kMinExp) e2[j] = (e2[j] & 0xffffu) | (1023u << 16);
@@ -666,33 +701,41 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
       unsigned eh[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) eh[j] = (e2[j] & 0xffffu) << 20;
-      tc::split8<kTcgPlane>(ws.a + half_row(i, h), gv, eh);
+#pragma unroll
+      for (int hf = 0; hf < H; ++hf) tc::split8<kTcgPlane>(ws.a[hf] + half_row(i, h), gv[hf], eh);
 #pragma unroll
       for (int j = 0; j < 8; ++j) eh[j] = (e2[j] & 0xffff0000u) << 4;
-      tc::split8<kTcgPlane>(ws.b + half_row(i, h), xv, eh);
+#pragma unroll
+      for (int hf = 0; hf < H; ++hf) tc::split8<kTcgPlane>(ws.b[hf] + half_row(i, h), xv[hf], eh);
     }
     const bool chunk_bad = __any_sync(0xffffffffu, nonfinite != 0u);
     __syncwarp();
-    unsigned fa[tc::kPlanes][4], fb[tc::kPlanes][4];
+    int pr[2][4][tc::kLevels / 2];  // two levels each, of all halves
 #pragma unroll
-    for (int d = 0; d < tc::kPlanes; ++d) {
-      ldmatrix4_trans(fa[d], sa + d * kTcgPlane);
-      ldmatrix4_trans(fb[d], sb + d * kTcgPlane);
-    }
-    int pr[2][4][tc::kLevels / 2];  // two levels each
+    for (int hf = 0; hf < H; ++hf) {
+      unsigned fa[tc::kPlanes][4], fb[tc::kPlanes][4];
 #pragma unroll
-    for (int L = 0; L < tc::kLevels; L += 2)
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-        for (int a = 0; a < tc::kPlanes; ++a) {
-          if (L - a >= 0 && L - a < tc::kPlanes) tc::mma16816(d[0], fa[a], fb[L - a] + 2 * nt);
-          if (L + 1 - a >= 0 && L + 1 - a < tc::kPlanes) tc::mma16816(d[1], fa[a], fb[L + 1 - a] + 2 * nt);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) pr[nt][q][L / 2] = tc::level_pair(d[0][q], d[1][q]);
+      for (int d = 0; d < tc::kPlanes; ++d) {
+        ldmatrix4_trans(fa[d], sa + (hf * tc::kPlanes + d) * kTcgPlane);
+        ldmatrix4_trans(fb[d], sb + (hf * tc::kPlanes + d) * kTcgPlane);
       }
+#pragma unroll
+      for (int L = 0; L < tc::kLevels; L += 2)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+          for (int a = 0; a < tc::kPlanes; ++a) {
+            if (L - a >= 0 && L - a < tc::kPlanes) tc::mma16816(d[0], fa[a], fb[L - a] + 2 * nt);
+            if (L + 1 - a >= 0 && L + 1 - a < tc::kPlanes) tc::mma16816(d[1], fa[a], fb[L + 1 - a] + 2 * nt);
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int pair = tc::level_pair(d[0][q], d[1][q]);
+            pr[nt][q][L / 2] = hf == 0 ? pair : pr[nt][q][L / 2] + pair;
+          }
+        }
+    }
     // scale and accumulate (in FP64 from global memory when the chunk or a
     // result is out of range)
     double y[2][4];
@@ -703,8 +746,9 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
       for (int q = 0; q < 4; ++q) {
         const int r = gid + (q >= 2 ? 8 : 0), k = nt * 8 + 2 * tig + (q & 1);
         const int sc = ws.er[r] + ws.ek[k] - tc::kScale8;
-        bad |= tc::scale8_ok(sc) ? 0u : 1u;
-        y[nt][q] = tc::scale8(tc::combine8(pr[nt][q][0], pr[nt][q][1], pr[nt][q][2], pr[nt][q][3]),
+        // twice the groups: a bit more
+        bad |= tc::scale8_ok(sc) && tc::scale8_ok(sc + H - 1) ? 0u : 1u;
+        y[nt][q] = tc::scale8(tc::combine8<H == 1>(pr[nt][q][0], pr[nt][q][1], pr[nt][q][2], pr[nt][q][3]),
                               (unsigned)sc << 20);
       }
     if (chunk_bad || __any_sync(0xffffffffu, bad != 0u)) {
@@ -717,8 +761,8 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
           const int64_t ok = ka * p.sai + kb * p.sbi, orr = ra * p.sao + rb * p.sbo;
           double s2 = 0.0;
 #pragma unroll 1
-          for (int gg = 0; gg < 16; ++gg) {
-            const uint64_t g2 = c * 16 + gg;
+          for (int gg = 0; gg < 16 * H; ++gg) {
+            const uint64_t g2 = c * (16 * H) + gg;
             if (g2 >= p.n_groups) break;
             int64_t bi, bo;
             bases(g2, bi, bo);
@@ -744,10 +788,10 @@ __global__ void __launch_bounds__(kTcgBlock) grad16_tc_kernel(const __grid_const
       red[w * 256 + r * 16 + k] = acc[nt][q];
     }
   __syncthreads();
-  {
-    const int e = threadIdx.x;  // 256 entries, 256 threads
+  if (threadIdx.x < 256) {
+    const int e = threadIdx.x;
     double s2 = 0.0;
-    for (int ww = 0; ww < kTcgWarps; ++ww) s2 += red[ww * 256 + e];
+    for (int ww = 0; ww < kTcgWarps * H; ++ww) s2 += red[ww * 256 + e];
     part[(int64_t)blockIdx.x * 256 + e] = s2;
   }
 }
@@ -756,6 +800,14 @@ unsigned tcg_blocks(uint64_t n_groups) {
   const uint64_t chunks = (n_groups + 15) / 16;
   const uint64_t blocks = (chunks + kTcgWarps - 1) / kTcgWarps;
   return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)sm_count() * 2));
+}
+
+template <int H>
+int launch_grad16(const GradParams& p, unsigned nb, double* part, cudaStream_t s) {
+  const int smem = std::max((int)sizeof(TcgSmem<H>), kTcgWarps * H * 256 * (int)sizeof(double));
+  const int st = allow_dynamic_smem((const void*)grad16_tc_kernel<H>, smem);
+  if (st != QSGB_OK) return st;
+  return launch_pdl(grad16_tc_kernel<H>, nb, (unsigned)(kTcgBlock * H), (size_t)smem, s, p, part);
 }
 
 // 16 x 16 FP64 gradients go to the tensor cores unless QSGB_TC_GRAD=0
@@ -837,18 +889,19 @@ int grad_common(const void* x_in, const void* g_out, double* dptm, int64_t da_ou
   // 4 x 4 micro-tiles: at most 2 per thread
   if (kin > 256 || kout > 256 || ((kin + 3) / 4) * ((kout + 3) / 4) > 2 * kGradBlock)
     return QSGB_ERR_UNSUPPORTED;
-  const GradParams p = make_params(x_in, g_out, da_out, db_out, da_in, db_in, X, Y, Z);
+  GradParams p = make_params(x_in, g_out, da_out, db_out, da_in, db_in, X, Y, Z);
   const unsigned nb = grad_blocks(p.n_groups, p.tg);
   const int E = (int)(kin * kout);
   if (!scratch || scratch_bytes < (int64_t)nb * E * (int64_t)sizeof(double)) return QSGB_ERR_SCRATCH;
   cudaStream_t s = as_stream(stream);
   double* part = static_cast<double*>(scratch);
   if (dtype == QSGB_F64 && kin == 16 && kout == 16 && tc_grad_enabled()) {
-    const unsigned nbt = tcg_blocks(p.n_groups);  // <= nb: the scratch holds its partials
-    const int smem_bytes = std::max((int)sizeof(TcgSmem), kTcgWarps * 256 * (int)sizeof(double));
-    const int st = allow_dynamic_smem((const void*)grad16_tc_kernel, smem_bytes);
-    if (st != QSGB_OK) return st;
-    const int s1 = launch_pdl(grad16_tc_kernel, nbt, kTcgBlock, (size_t)smem_bytes, s, p, part);
+    p.vec_z1 = Z == 1 && db_in == 4 && db_out == 4 && ((uintptr_t)x_in | (uintptr_t)g_out) % 32 == 0;
+    // chunks of 32 groups when those of 16 are more than the resident warps;
+    // the scratch holds the partials of tcg_blocks <= nb blocks either way
+    const bool wide = p.n_groups > (uint64_t)sm_count() * 2 * kTcgWarps * 16;
+    const unsigned nbt = wide ? (unsigned)sm_count() : tcg_blocks(p.n_groups);
+    const int s1 = wide ? launch_grad16<2>(p, nbt, part, s) : launch_grad16<1>(p, nbt, part, s);
     return s1 != QSGB_OK ? s1 : launch_stage2(part, (int)nbt, E, dptm, s);
   }
   // one qudit (a group's rows lie a stride apart) of at most 4 elements: a

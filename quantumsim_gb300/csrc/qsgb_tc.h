@@ -105,9 +105,12 @@ __device__ __forceinline__ unsigned level_bits(float a) { return __float_as_uint
 __device__ __forceinline__ int level_pair(float a, float b) {
   return (int)((level_bits(a) << 8) + level_bits(b) - ((kMagic << 8) + kMagic));
 }
-// sum_L A_L 2^(56 - 8 L) / 2^14 of eight levels, given as pairs, in 64 bits
+// sum_L A_L 2^(56 - 8 L) / 2^14 of eight levels, given as pairs, in 64 bits.
+// NARROW: 4 p45 fits 32 bits (sums over 16 products, not over 32).
+template <bool NARROW = true>
 __device__ __forceinline__ long long combine8(int p01, int p23, int p45, int p67) {
-  return (long long)p23 * 262144ll + (long long)(p45 * 4 + (p67 >> 14)) + ((long long)p01 << 34);
+  const long long low = NARROW ? (long long)(p45 * 4 + (p67 >> 14)) : (long long)p45 * 4 + (p67 >> 14);
+  return (long long)p23 * 262144ll + low + ((long long)p01 << 34);
 }
 // v 2^sc as a double, sc given as sc << 20.  For v = combine8 of values split
 // against ex and PTM entries against ep (biased exponents),

@@ -132,9 +132,23 @@ class Diagonal(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        gx = torch.ops.qsgb.scatter(g, list(ctx.shape), *ctx.idx,
-                                    ctx.dtype == torch.float64)
+        gx = DiagonalAdjoint.apply(g, ctx.shape, ctx.dtype, *ctx.idx)
         return gx, None, None, None
+
+
+class DiagonalAdjoint(torch.autograd.Function):
+    """The scatter of Diagonal's backward pass, with its own derivative for
+    gradients of gradients."""
+
+    @staticmethod
+    def forward(ctx, g, shape, dtype, idx_off, idx_list):
+        ctx.idx = idx_off, idx_list
+        return torch.ops.qsgb.scatter(g, list(shape), idx_off, idx_list,
+                                      dtype == torch.float64)
+
+    @staticmethod
+    def backward(ctx, gg):
+        return (Diagonal.apply(gg, None, *ctx.idx),) + (None,) * 4
 
 
 def diagonal_diff(x, bases):

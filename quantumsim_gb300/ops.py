@@ -304,13 +304,16 @@ _DIRECT_TYPES = (torch.Tensor, torch.nn.Parameter)
 
 def direct(*tensors):
     """Whether kernels may be called on these tensors past the dispatcher:
-    plain CUDA tensors of the two storage types, nothing to be recorded for a
-    gradient and no tracing."""
-    if torch.is_grad_enabled() or torch._C._len_torch_dispatch_stack():
+    plain CUDA tensors of the two storage types without a lazy negation,
+    nothing to be recorded for a gradient, no dispatch mode, tracing or
+    compilation."""
+    if torch.is_grad_enabled() or torch._C._len_torch_dispatch_stack() or \
+            torch._C._get_tracing_state() is not None or \
+            torch.compiler.is_compiling():
         return False
     for t in tensors:
         if type(t) not in _DIRECT_TYPES or not t.is_cuda or \
-                t.dtype not in (torch.float64, torch.float32):
+                t.dtype not in (torch.float64, torch.float32) or t.is_neg():
             return False
     return True
 
@@ -332,7 +335,8 @@ def apply_direct(x, ptm, qudits, arith, transpose):
     """torch.ops.qsgb.apply_ptm for `direct` tensors and a host PTM: the
     compiled per-call entry point with a cached plan (~6 us of host time
     instead of ~28)."""
-    if ptm.dtype == torch.float64 and ptm.is_contiguous():
+    if ptm.dtype == torch.float64 and ptm.is_contiguous() and \
+            not ptm.is_neg():
         plan = _direct_plan(eager_plan, x.shape, x.dtype, qudits, ptm.shape,
                             transpose)
         out = eager_apply(x.contiguous(), ptm.numpy(), plan, arith)

@@ -196,7 +196,7 @@ class NoisyCircuitModel:
                 self.layers(p, lambda s, pt, qs: apply_ptm_diff(s, pt, *qs,
                                                                 **kw),
                             fuse=fuse),
-                x, checkpoint_every, keep_last=True)
+                x, checkpoint_every)
             return diagonal_diff(x, [self.basis] * self.n)
         device = device or torch.device('cpu')
         x = self.initial_state(device, torch.float64)

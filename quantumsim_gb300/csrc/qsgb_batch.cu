@@ -31,26 +31,25 @@ namespace qsgb {
 namespace {
 
 constexpr int kBatchBlock = 256;
-constexpr int kRedRows = kBatchBlock / 16;  // rows of the FP64 dP reduction buffer (>= warps)
-// floats per row of a warp's 16 x 32 adjoint tiles: 32 groups + 8 of
-// padding, so that the fragment loads and 8-byte stores of the two-qubit
-// ADJOINT fall in distinct banks
-constexpr int kAdjStride = 40;
+// floats per row of a warp's 16 x 32 adjoint tiles: 32 groups + 4 of
+// padding, so that the fragment loads and the 16-byte stores of X_in in the
+// two-qubit ADJOINT fall in distinct banks
+constexpr int kAdjStride = 36;
 constexpr int kWarps = kBatchBlock / 32;
 
 struct BatchSmem {
   float P[256];
   float PT[256];  // P transposed (ADJOINT: g_in = P^T g_out)
   float Pi[256];
-  // two-qubit ADJOINT tiles, one pair per warp: x (X_out, then X_in) and g
-  // (G_out, then G_in), 16 rows of kAdjStride floats; reused for the FP64
-  // cross-warp sums of the dP partials
+  // two-qubit ADJOINT tiles, one pair per warp: x (X_in) and g (G_out), 16
+  // rows of kAdjStride floats; reused for the FP64 cross-warp sums of the dP
+  // partials
   union {
     struct {
       float g[kWarps][16 * kAdjStride];
       float x[kWarps][16 * kAdjStride];
     } t;
-    double red[kRedRows][256];
+    double red[kWarps][256];
   } u __attribute__((aligned(16)));
   double acc[kBatchBlock][16];  // per-thread FP64 dP partials (ADJOINT)
   int item;
@@ -349,17 +348,39 @@ __device__ __forceinline__ void mma3(float (&d)[4], const uint32_t (&ah)[4], con
   mma_tf32(d, ah, bh0, bh1);
 }
 
+// 32 bytes (8 floats), 32-byte aligned
+__device__ __forceinline__ void store8(float* dst, const float (&v)[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
 // Two-qubit ADJOINT on the warp-level tensor cores.  A warp takes tiles of 32
-// consecutive groups; lane l loads group t0 + l (coalesced across lanes) and
-// stages its x_out and g_out as column l of two 16 x 32 tiles in its own
-// slice of shared memory ([k][group], rows of kAdjStride floats).  Per tile:
+// consecutive groups:
 //   X_in = P^-1 X_out and G_in = P^T G_out   (M 16, N 32, K 16: 8 mma each)
 //   dP  += G_out X_in^T                      (M 16, N 16, K 32: 8 mma)
-// each mma in 3xTF32 (24 per product).  X_in and G_in go back through the
-// tiles ([r][group]) to the lanes that own the groups and to global memory.
-// The dP fragments are carried in FP32 over 4 tiles, then folded into the
+// each mma in 3xTF32 (24 per product).  Lane l = (gid, tig) = (l / 4, l % 4)
+// holds components 4 j + tig (j = 0..3) of column gid of every n-tile as right
+// operands, and gets components row(gid, 0 / 1) of columns 2 tig and 2 tig + 1.
+// Which group a column stands for, and which component a row, is free, and is
+// chosen for both to be whole runs of memory, so that the first two products
+// need no exchange between lanes:
+//  * Z > 1: column c of n-tile nt is group 4 c + nt.  The lane's four groups
+//    of a component are 16 bytes, its eight results 32.
+//  * Z == 1: group 8 nt + c / 2 + 4 (c % 2), rows 2 gid and 2 gid + 1.  A load
+//    of the warp is 128 consecutive bytes, a lane's results are pairs.
+// G_out and X_in go through the warp's two 16 x 32 tiles in shared memory
+// ([component][group]) for the third product alone, which sums over groups.
+// Its fragments are carried in FP32 over 4 tiles, then folded into the
 // thread's FP64 sums in shared memory; at the end the warps' sums are added
 // in a fixed order and written to dst (256 doubles).
+//
+// Bound by the latency of its loads on 16 warps per SM.  With a group per lane
+// and every product's operands and results staged (96 shared-memory accesses
+// and 64 global ones of 4 bytes per tile, against 56 and 12 here) the step of
+// 512 circuits took 1.198 s, that of 20 circuits 106.4 ms; here 1.087 s and
+// 96.5 ms, with the same bits (G_out read a second time in the third product's
+// order instead of staged: 101.7 ms and other FP32 sums).
 __device__ __noinline__ void adjoint2_warp(float* __restrict__ x, float* __restrict__ gv, const Geo& geo, int64_t beg,
                                            int64_t end, double* __restrict__ dst) {
   constexpr int K = 16;
@@ -368,24 +389,23 @@ __device__ __noinline__ void adjoint2_warp(float* __restrict__ x, float* __restr
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
   const int gid = lane >> 2, tig = lane & 3;
-  float* ta = sm.u.t.x[warp];  // X_out, then X_in
-  float* tb = sm.u.t.g[warp];  // G_out, then G_in
-  const bool vec = geo.lz == 0;
+  float* ta = sm.u.t.x[warp];  // X_in
+  float* tb = sm.u.t.g[warp];  // G_out
+  const int lz = geo.lz, la = geo.lz + geo.ly + 2;  // log2 strides of b and a (component 4 a + b)
+  const bool last = lz == 0;
+  const bool aligned = (((uintptr_t)x | (uintptr_t)gv) & 31) == 0;
+  auto column = [&](int nt, int c) { return last ? 8 * nt + (c >> 1) + 4 * (c & 1) : 4 * c + nt; };
+  const int r0 = last ? 2 * gid : gid, r1 = last ? 2 * gid + 1 : gid + 8;
   // A fragments of P^-1 and P^T (two k-steps each), split into TF32 hi / lo
   uint32_t pih[2][4], pil[2][4], pth[2][4], ptl[2][4];
 #pragma unroll
-  for (int ks = 0; ks < 2; ++ks) {
-    const int c = 8 * ks + tig;
-    const float vi[4] = {sm.Pi[gid * K + c], sm.Pi[(gid + 8) * K + c], sm.Pi[gid * K + c + 4],
-                         sm.Pi[(gid + 8) * K + c + 4]};
-    const float vt[4] = {sm.PT[gid * K + c], sm.PT[(gid + 8) * K + c], sm.PT[gid * K + c + 4],
-                         sm.PT[(gid + 8) * K + c + 4]};
+  for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      split_tf32(vi[i], pih[ks][i], pil[ks][i]);
-      split_tf32(vt[i], pth[ks][i], ptl[ks][i]);
+      const int e = ((i & 1) ? r1 : r0) * K + 8 * ks + 4 * (i >> 1) + tig;
+      split_tf32(sm.Pi[e], pih[ks][i], pil[ks][i]);
+      split_tf32(sm.PT[e], pth[ks][i], ptl[ks][i]);
     }
-  }
   float dp[2][4];  // dP fragments: rows gid, gid + 8; columns 8 nb + 2 tig (+1)
 #pragma unroll
   for (int nb = 0; nb < 2; ++nb)
@@ -395,28 +415,54 @@ __device__ __noinline__ void adjoint2_warp(float* __restrict__ x, float* __restr
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.0;
   int tiles = 0;
+  // offsets inside a group: component tig, the result rows
+  const int in0 = tig << lz, out0 = in_offset<K>(geo, r0), out1 = in_offset<K>(geo, r1);
   for (int64_t t0 = beg + (int64_t)warp * 32; t0 < end; t0 += (int64_t)nwarps * 32) {
-    const int64_t gi = t0 + lane;
-    const bool have = gi < end;
-    const int64_t b = have ? group_base(geo, gi) : 0;
+    // four consecutive groups along z per access, or eight (32 bytes); else
+    // group by group (Z == 1, the end of an item, a start inside a run)
+    const bool full = t0 + 32 <= end;
+    const bool quads = full && lz >= 2 && (t0 & 3) == 0;
+    const bool wide = quads && aligned && lz >= 4 && (t0 & 7) == 0;
+    float xv[4][4], gq[4][4];  // [component 4 j + tig][n-tile]
+    if (quads) {
+      const int64_t b = group_base(geo, t0 + 4 * gid) + in0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 u = *reinterpret_cast<const float4*>(x + b + (j << la));
+        const float4 w = *reinterpret_cast<const float4*>(gv + b + (j << la));
+        xv[j][0] = u.x; xv[j][1] = u.y; xv[j][2] = u.z; xv[j][3] = u.w;
+        gq[j][0] = w.x; gq[j][1] = w.y; gq[j][2] = w.z; gq[j][3] = w.w;
+      }
+    } else {
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const int64_t gi = t0 + column(nt, gid);
+        const bool have = gi < end;
+        const int64_t b = (have ? group_base(geo, gi) : 0) + in0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          xv[j][nt] = have ? x[b + (j << la)] : 0.f;
+          gq[j][nt] = have ? gv[b + (j << la)] : 0.f;
+        }
+      }
+    }
     {
-      // this warp's next tile into L2 while the current one is loaded and
-      // computed (the loads below are bound by their latency): lane l takes
-      // tensor l / 16 and, for Z >= 64, component l % 16 at the tile's first
-      // and last group (one 128-byte run each when the groups are
-      // consecutive along z); for Z == 1, line l % 4 of chunk row
-      // (l / 4) % 4 (the tile's 32 groups are 512 contiguous bytes per
-      // row).  Other strides are not prefetched.  Addresses are those of
-      // groups inside the item.
+      // this warp's next tile into L2 while the current one is computed (the
+      // loads are bound by their latency): lane l takes tensor l / 16 and, for
+      // Z >= 64, component l % 16 at the tile's first and last group (one
+      // 128-byte run each when the groups are consecutive along z); for
+      // Z == 1, line l % 4 of chunk row (l / 4) % 4 (the tile's 32 groups are
+      // 512 contiguous bytes per row).  Other strides are not prefetched.
+      // Addresses are those of groups inside the item.
       const int64_t tn = t0 + (int64_t)nwarps * 32;
       if (tn < end) {
         const float* base = (lane < 16) ? x : gv;
-        if (geo.lz >= 6) {
+        if (lz >= 6) {
           const int off = in_offset<K>(geo, lane & 15);
-          const int64_t last = tn + 31 < end ? tn + 31 : end - 1;
+          const int64_t fin = tn + 31 < end ? tn + 31 : end - 1;
           asm volatile("prefetch.global.L2 [%0];" ::"l"(base + group_base(geo, tn) + off));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(base + group_base(geo, last) + off));
-        } else if (vec && tn + 31 < end) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(base + group_base(geo, fin) + off));
+        } else if (last && tn + 31 < end) {
           const int64_t b0 = group_base(geo, tn), b1 = group_base(geo, tn + 31);
           if (b1 - b0 == 31 * 4) {  // the 32 groups share x: rows are contiguous
             const int q = (lane >> 2) & 3;
@@ -425,33 +471,17 @@ __device__ __noinline__ void adjoint2_warp(float* __restrict__ x, float* __restr
         }
       }
     }
-    {
-      float xo[K], go[K];
-      if (!have) {
+    // G_out into its tile
 #pragma unroll
-        for (int k = 0; k < K; ++k) xo[k] = go[k] = 0.f;
-      } else if (vec) {
+    for (int j = 0; j < 4; ++j) {
+      float* row = tb + (4 * j + tig) * S;
+      if (last) {
 #pragma unroll
-        for (int q = 0; q < K / 4; ++q) {
-          const float4 u = *reinterpret_cast<const float4*>(x + b + in_offset<K>(geo, 4 * q));
-          const float4 w = *reinterpret_cast<const float4*>(gv + b + in_offset<K>(geo, 4 * q));
-          xo[4 * q] = u.x; xo[4 * q + 1] = u.y; xo[4 * q + 2] = u.z; xo[4 * q + 3] = u.w;
-          go[4 * q] = w.x; go[4 * q + 1] = w.y; go[4 * q + 2] = w.z; go[4 * q + 3] = w.w;
-        }
+        for (int nt = 0; nt < 4; ++nt) row[column(nt, gid)] = gq[j][nt];
       } else {
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          xo[k] = x[b + in_offset<K>(geo, k)];
-          go[k] = gv[b + in_offset<K>(geo, k)];
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        ta[k * S + lane] = xo[k];
-        tb[k * S + lane] = go[k];
+        *reinterpret_cast<float4*>(row + 4 * gid) = make_float4(gq[j][0], gq[j][1], gq[j][2], gq[j][3]);
       }
     }
-    __syncwarp();
     // X_in = P^-1 X_out, G_in = P^T G_out: four n-tiles of 8 groups
     float xi[4][4], gn[4][4];
 #pragma unroll
@@ -460,63 +490,80 @@ __device__ __noinline__ void adjoint2_warp(float* __restrict__ x, float* __restr
       for (int i = 0; i < 4; ++i) xi[nt][i] = gn[nt][i] = 0.f;
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks) {
-        const int r0 = (8 * ks + tig) * S + 8 * nt + gid;
-        mma3(xi[nt], pih[ks], pil[ks], ta[r0], ta[r0 + 4 * S]);
-        mma3(gn[nt], pth[ks], ptl[ks], tb[r0], tb[r0 + 4 * S]);
+        mma3(xi[nt], pih[ks], pil[ks], xv[2 * ks][nt], xv[2 * ks + 1][nt]);
+        mma3(gn[nt], pth[ks], ptl[ks], gq[2 * ks][nt], gq[2 * ks + 1][nt]);
       }
     }
-    // dP A fragments: G_out[r][group] for the four k-steps over groups
-    float ga[4][4];
+    // X_in into its tile
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float* row = ta + (h ? r1 : r0) * S;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (last) {
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) row[8 * nt + tig + 4 * c] = xi[nt][2 * h + c];
+        } else {
+          *reinterpret_cast<float4*>(row + 8 * tig + 4 * c) =
+              make_float4(xi[0][2 * h + c], xi[1][2 * h + c], xi[2][2 * h + c], xi[3][2 * h + c]);
+        }
+      }
+    }
+    __syncwarp();  // the tiles are written, and every lane has read what the others overwrite
+    if (wide) {
+      const int64_t b = group_base(geo, t0 + 8 * tig);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v[8], w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          v[i] = xi[i & 3][2 * h + (i >> 2)];
+          w[i] = gn[i & 3][2 * h + (i >> 2)];
+        }
+        store8(x + b + (h ? out1 : out0), v);
+        store8(gv + b + (h ? out1 : out0), w);
+      }
+    } else if (quads) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int64_t b = group_base(geo, t0 + 8 * tig + 4 * c);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = 2 * h + c, o = h ? out1 : out0;
+          *reinterpret_cast<float4*>(x + b + o) = make_float4(xi[0][i], xi[1][i], xi[2][i], xi[3][i]);
+          *reinterpret_cast<float4*>(gv + b + o) = make_float4(gn[0][i], gn[1][i], gn[2][i], gn[3][i]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int64_t gi = t0 + column(nt, 2 * tig + c);
+          if (gi < end) {
+            const int64_t b = group_base(geo, gi);
+            if (last) {
+              *reinterpret_cast<float2*>(x + b + out0) = make_float2(xi[nt][c], xi[nt][2 + c]);
+              *reinterpret_cast<float2*>(gv + b + out0) = make_float2(gn[nt][c], gn[nt][2 + c]);
+            } else {
+              x[b + out0] = xi[nt][c];
+              x[b + out1] = xi[nt][2 + c];
+              gv[b + out0] = gn[nt][c];
+              gv[b + out1] = gn[nt][2 + c];
+            }
+          }
+        }
+    }
+    // dP += G_out X_in^T: A[r][group], B[group][k] = X_in[k][group]
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       const int c = 8 * ks + tig;
-      ga[ks][0] = tb[gid * S + c];
-      ga[ks][1] = tb[(gid + 8) * S + c];
-      ga[ks][2] = tb[gid * S + c + 4];
-      ga[ks][3] = tb[(gid + 8) * S + c + 4];
-    }
-    __syncwarp();
-    // X_in and G_in into the tiles as [r][group]
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int c = 8 * nt + 2 * tig;
-      *reinterpret_cast<float2*>(&ta[gid * S + c]) = make_float2(xi[nt][0], xi[nt][1]);
-      *reinterpret_cast<float2*>(&ta[(gid + 8) * S + c]) = make_float2(xi[nt][2], xi[nt][3]);
-      *reinterpret_cast<float2*>(&tb[gid * S + c]) = make_float2(gn[nt][0], gn[nt][1]);
-      *reinterpret_cast<float2*>(&tb[(gid + 8) * S + c]) = make_float2(gn[nt][2], gn[nt][3]);
-    }
-    __syncwarp();
-    // this lane's group back to global memory
-    if (have) {
-      if (vec) {
-#pragma unroll
-        for (int q = 0; q < K / 4; ++q) {
-          *reinterpret_cast<float4*>(x + b + in_offset<K>(geo, 4 * q)) =
-              make_float4(ta[(4 * q) * S + lane], ta[(4 * q + 1) * S + lane], ta[(4 * q + 2) * S + lane],
-                          ta[(4 * q + 3) * S + lane]);
-          *reinterpret_cast<float4*>(gv + b + in_offset<K>(geo, 4 * q)) =
-              make_float4(tb[(4 * q) * S + lane], tb[(4 * q + 1) * S + lane], tb[(4 * q + 2) * S + lane],
-                          tb[(4 * q + 3) * S + lane]);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < K; ++r) {
-          x[b + in_offset<K>(geo, r)] = ta[r * S + lane];
-          gv[b + in_offset<K>(geo, r)] = tb[r * S + lane];
-        }
-      }
-    }
-    // dP += G_out X_in^T: B[group][k] = X_in[k][group]
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
+      const float ga[4] = {tb[gid * S + c], tb[(gid + 8) * S + c], tb[gid * S + c + 4], tb[(gid + 8) * S + c + 4]};
       uint32_t ah[4], al[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) split_tf32(ga[ks][i], ah[i], al[i]);
+      for (int i = 0; i < 4; ++i) split_tf32(ga[i], ah[i], al[i]);
 #pragma unroll
-      for (int nb = 0; nb < 2; ++nb) {
-        const int r0 = (8 * nb + gid) * S + 8 * ks + tig;
-        mma3(dp[nb], ah, al, ta[r0], ta[r0 + 4]);
-      }
+      for (int nb = 0; nb < 2; ++nb) mma3(dp[nb], ah, al, ta[(8 * nb + gid) * S + c], ta[(8 * nb + gid) * S + c + 4]);
     }
     __syncwarp();
     if ((++tiles & 3) == 0) {

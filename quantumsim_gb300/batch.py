@@ -431,8 +431,11 @@ def build_program(units, unit_base, sizes, depths, every, tile,
     gitems['q1'] = -1
     gitems['beg'] = slot_base[adj]
     gitems['end'] = slot_base[adj] + n_items[adj]
-    # expand entries into items, stage by stage
-    order = np.argsort(stage, kind='stable')
+    # expand entries into items, stage by stage; every second stage in reverse,
+    # so that it begins with the instances whose vectors the stage before left
+    # in L2 (GB300: 20 circuits 94.7 -> 93.5 ms, 512 circuits 1.107 -> 1.088 s)
+    idx = np.arange(len(e))
+    order = np.lexsort((np.where(stage % 2 == 1, -idx, idx), stage))
     n_items = n_items[order]
     rep = np.repeat(order, n_items)
     j = np.arange(len(rep)) - np.repeat(np.cumsum(n_items) - n_items, n_items)

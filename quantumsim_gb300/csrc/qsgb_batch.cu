@@ -204,6 +204,20 @@ __device__ __noinline__ void apply_vec(float* __restrict__ x, const Geo& geo, in
   }
 }
 
+// FP32 sums into FP64 ones (the first ones of an item as they are).  On GB300 a
+// warp's conversion or addition in FP64 takes ~62 cycles of its sub-partition:
+// an item of four tiles per warp is not folded a second time at its end.
+// (Conversions by integer operations on the bit patterns: 58.2 -> 59.0 ms for
+// the step of 64 10-qubit circuits.)
+template <int N>
+__device__ __forceinline__ void fold_fp64(double* acc, float (&v)[N], bool first) {
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    acc[e] = first ? (double)v[e] : acc[e] + (double)v[e];
+    v[e] = 0.f;
+  }
+}
+
 // One-qubit adjoint (pairs of groups when Z >= 4, one contiguous group when
 // Z == 1): x = P^-1 x, g = P^T g, and
 // dP[r][k] = sum g_out[r] x_in[k] accumulated in FP32 registers, folded to
@@ -214,10 +228,7 @@ __device__ __noinline__ void adjoint1_vec(float* __restrict__ x, float* __restri
   float acc[16];
   double* accd = sm.acc[threadIdx.x];  // FP64 running sums live in shared memory
 #pragma unroll
-  for (int e = 0; e < 16; ++e) {
-    acc[e] = 0.f;
-    accd[e] = 0.0;
-  }
+  for (int e = 0; e < 16; ++e) acc[e] = 0.f;
   auto one = [&](const float* xo, const float* go, float* xi, float* gn) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -236,6 +247,7 @@ __device__ __noinline__ void adjoint1_vec(float* __restrict__ x, float* __restri
       for (int k = 0; k < 4; ++k) acc[r * 4 + k] = fmaf(go[r], xi[k], acc[r * 4 + k]);
   };
   int since = 0;
+  bool first = true;
   if (geo.lz >= 2) {  // pairs of groups (z, z+1): 8-byte accesses
     for (int64_t gi = beg + (int64_t)threadIdx.x * 2; gi < end; gi += (int64_t)blockDim.x * 2) {
       const int64_t b = group_base(geo, gi);
@@ -266,11 +278,8 @@ __device__ __noinline__ void adjoint1_vec(float* __restrict__ x, float* __restri
         *reinterpret_cast<float2*>(gv + b + in_offset<4>(geo, r)) = make_float2(gn[r][0], gn[r][1]);
       }
       if (++since == 8) {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          accd[e] += (double)acc[e];
-          acc[e] = 0.f;
-        }
+        fold_fp64(accd, acc, first);
+        first = false;
         since = 0;
       }
     }
@@ -286,23 +295,32 @@ __device__ __noinline__ void adjoint1_vec(float* __restrict__ x, float* __restri
       *reinterpret_cast<float4*>(x + b) = make_float4(xi[0], xi[1], xi[2], xi[3]);
       *reinterpret_cast<float4*>(gv + b) = make_float4(gn[0], gn[1], gn[2], gn[3]);
       if (++since == 16) {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          accd[e] += (double)acc[e];
-          acc[e] = 0.f;
-        }
+        fold_fp64(accd, acc, first);
+        first = false;
         since = 0;
       }
     }
   }
-  // block reduction: warps by shuffle, then across warps in shared memory
-  const int w = threadIdx.x >> 5;
+  if (since || first) fold_fp64(accd, acc, first);
+  // block reduction: over a warp by exchanges that halve the entries a lane
+  // holds (16 FP64 additions a lane; a butterfly per entry, the same sums,
+  // takes 80), then across warps in shared memory.  With the fold above: 64
+  // circuits of 10 qubits 64.4 -> 58.2 ms, 20 circuits of 4 to 12 93.6 -> 90.8.
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v[16];
 #pragma unroll
-  for (int e = 0; e < 16; ++e) {
-    double v = accd[e] + (double)acc[e];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sm.u.red[w][e] = v;
+  for (int e = 0; e < 16; ++e) v[e] = accd[e];
+#pragma unroll
+  for (int h = 8; h > 0; h >>= 1) {
+    const bool up = (lane & (2 * h)) != 0;  // keeps the upper half
+#pragma unroll
+    for (int e = 0; e < h; ++e) {
+      const double send = up ? v[e] : v[e + h], keep = up ? v[e + h] : v[e];
+      v[e] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+    }
   }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  if ((lane & 1) == 0) sm.u.red[w][lane >> 1] = v[0];
   __syncthreads();
   if (threadIdx.x < 16) {
     double s = 0.0;
@@ -330,7 +348,7 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
 
 // d += a * b for one m16n8k8 tile: a = 16 x 8 (row-major fragment a0..a3),
 // b = 8 x 8 (column fragment b0, b1), d = 16 x 8 FP32
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_tf32(float* d, const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
       "{%0, %1, %2, %3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -338,7 +356,7 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
 }
 
 // d += A B with A given as split fragments (ah, al) and B as FP32 values
-__device__ __forceinline__ void mma3(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0,
+__device__ __forceinline__ void mma3(float* d, const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0,
                                      float b1) {
   uint32_t bh0, bl0, bh1, bl1;
   split_tf32(b0, bh0, bl0);
@@ -406,14 +424,10 @@ __device__ __noinline__ void adjoint2_warp(float* __restrict__ x, float* __restr
       split_tf32(sm.Pi[e], pih[ks][i], pil[ks][i]);
       split_tf32(sm.PT[e], pth[ks][i], ptl[ks][i]);
     }
-  float dp[2][4];  // dP fragments: rows gid, gid + 8; columns 8 nb + 2 tig (+1)
+  float dp[8];  // dP fragments: [4 nb + i], rows gid, gid + 8; columns 8 nb + 2 tig (+1)
 #pragma unroll
-  for (int nb = 0; nb < 2; ++nb)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dp[nb][i] = 0.f;
+  for (int i = 0; i < 8; ++i) dp[i] = 0.f;
   double* acc = sm.acc[threadIdx.x];  // FP64 running sums in shared memory
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] = 0.0;
   int tiles = 0;
   // offsets inside a group: component tig, the result rows
   const int in0 = tig << lz, out0 = in_offset<K>(geo, r0), out1 = in_offset<K>(geo, r1);
@@ -570,23 +584,12 @@ __device__ __noinline__ void adjoint2_warp(float* __restrict__ x, float* __restr
 #pragma unroll
       for (int i = 0; i < 4; ++i) split_tf32(ga[i], ah[i], al[i]);
 #pragma unroll
-      for (int nb = 0; nb < 2; ++nb) mma3(dp[nb], ah, al, ta[(8 * nb + gid) * S + c], ta[(8 * nb + gid) * S + c + 4]);
+      for (int nb = 0; nb < 2; ++nb) mma3(dp + 4 * nb, ah, al, ta[(8 * nb + gid) * S + c], ta[(8 * nb + gid) * S + c + 4]);
     }
     __syncwarp();
-    if ((++tiles & 3) == 0) {
-#pragma unroll
-      for (int nb = 0; nb < 2; ++nb)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          acc[nb * 4 + i] += (double)dp[nb][i];
-          dp[nb][i] = 0.f;
-        }
-    }
+    if ((++tiles & 3) == 0) fold_fp64(acc, dp, tiles == 4);
   }
-#pragma unroll
-  for (int nb = 0; nb < 2; ++nb)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[nb * 4 + i] += (double)dp[nb][i];
+  if (tiles < 4 || (tiles & 3)) fold_fp64(acc, dp, tiles < 4);
   __syncthreads();  // every warp is done with the tile: reuse it for the sums
 #pragma unroll
   for (int nb = 0; nb < 2; ++nb)

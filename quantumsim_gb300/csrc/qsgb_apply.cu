@@ -669,6 +669,129 @@ __global__ void __launch_bounds__(kDenseBlock) apply_dense_kernel(const __grid_c
   }
 }
 
+// The same for FP32 vectors whose targets are full qubits (K = 4 or 16, in and
+// out), the usual case: the sizes are known, a row of P is read four entries at
+// a time, and a thread takes V consecutive groups along z (16, 8 or 4 bytes an
+// access) or, with the less significant target last (LAST), the groups' rows as
+// 16 bytes.  The kernel above was bound by one shared-memory load per FMA.
+// V = 1 leaves a vector of 10 qubits the most blocks; V = 4 reads P the least.
+// The products and their order are those above.  Measured on GB300, us in a
+// graph, above / here, one qubit and two, on 8 / 10 / 11 / 12 qubits: 3.8 / 10.1
+// / 23.8 / 82 -> 2.2 / 5.6 / 7.4 / 21 (6.3 TB/s) and 6.1 / 8.1 / 19.6 / 54 -> 3.1
+// / 5.4 / 8.9 / 28; the last two of 12 qubits 104 -> 40.
+constexpr int kQubitBlock = 128;
+
+template <int K, int V, bool LAST>
+__global__ void __launch_bounds__(kQubitBlock) apply_qubits_f32(const __grid_constant__ ApplyParams p) {
+  static_assert(!LAST || V == 1, "a group's rows are the vectors");
+  constexpr int NE = (K * K + kQubitBlock - 1) / kQubitBlock;
+  __shared__ __align__(16) float P[K * K];
+  __shared__ double wmax[kQubitBlock / 32];
+  const int t = threadIdx.x;
+  pdl_wait();
+  double v[NE], m = 0.0;
+#pragma unroll
+  for (int i = 0; i < NE; ++i) {
+    const int e = t + i * kQubitBlock;
+    v[i] = e < K * K ? p.ptm[ptm_index(p, e / K, e % K)] : 0.0;
+    m = fmax(m, fabs(v[i]));
+  }
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((t & 31) == 0) wmax[t >> 5] = m;
+  __syncthreads();
+  double amax = 0.0;
+#pragma unroll
+  for (int w = 0; w < kQubitBlock / 32; ++w) amax = fmax(amax, wmax[w]);
+#pragma unroll
+  for (int i = 0; i < NE; ++i) {
+    const int e = t + i * kQubitBlock;
+    if (e < K * K) P[e] = fabs(v[i]) > amax * 0x1p-30 ? (float)v[i] : 0.0f;
+  }
+  __syncthreads();
+  const float* X = static_cast<const float*>(p.in);
+  float* Y = static_cast<float*>(p.out);
+  for (uint64_t it = (uint64_t)blockIdx.x * kQubitBlock + t; it < p.n_items; it += (uint64_t)gridDim.x * kQubitBlock) {
+    const uint64_t t1 = fdiv(it, p.div_z);
+    const uint64_t z = it - t1 * p.div_z.d;
+    const uint64_t x = fdiv(t1, p.div_y);
+    const uint64_t y = t1 - x * p.div_y.d;
+    const int64_t base = (int64_t)x * p.sxi + (int64_t)y * p.syi + (int64_t)z * V;
+    float in[K][V];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float* src = X + base + (k >> 2) * p.sai + (k & 3) * p.sbi;
+      if constexpr (LAST) {
+        if ((k & 3) == 0) {
+          const float4 u = *reinterpret_cast<const float4*>(src);
+          in[k][0] = u.x; in[k + 1][0] = u.y; in[k + 2][0] = u.z; in[k + 3][0] = u.w;
+        }
+      } else if constexpr (V == 4) {
+        const float4 u = *reinterpret_cast<const float4*>(src);
+        in[k][0] = u.x; in[k][1] = u.y; in[k][2] = u.z; in[k][3] = u.w;
+      } else if constexpr (V == 2) {
+        const float2 u = *reinterpret_cast<const float2*>(src);
+        in[k][0] = u.x; in[k][1] = u.y;
+      } else {
+        in[k][0] = *src;
+      }
+    }
+#pragma unroll 1
+    for (int a = 0; a < K / 4; ++a) {
+      float acc[4][V];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+#pragma unroll
+        for (int l = 0; l < V; ++l) acc[b][l] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < K; k += 4) {
+          const float4 c = *reinterpret_cast<const float4*>(P + (4 * a + b) * K + k);
+#pragma unroll
+          for (int l = 0; l < V; ++l) {
+            acc[b][l] = fmaf(c.x, in[k][l], acc[b][l]);
+            acc[b][l] = fmaf(c.y, in[k + 1][l], acc[b][l]);
+            acc[b][l] = fmaf(c.z, in[k + 2][l], acc[b][l]);
+            acc[b][l] = fmaf(c.w, in[k + 3][l], acc[b][l]);
+          }
+        }
+      }
+      float* dst = Y + base + a * p.sao;
+      if constexpr (LAST) {
+        *reinterpret_cast<float4*>(dst) = make_float4(acc[0][0], acc[1][0], acc[2][0], acc[3][0]);
+      } else {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          if constexpr (V == 4)
+            *reinterpret_cast<float4*>(dst + b * p.sbo) = make_float4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]);
+          else if constexpr (V == 2)
+            *reinterpret_cast<float2*>(dst + b * p.sbo) = make_float2(acc[b][0], acc[b][1]);
+          else
+            dst[b * p.sbo] = acc[b][0];
+        }
+      }
+    }
+  }
+}
+
+template <int K>
+int launch_qubits_f32(ApplyParams& p, uint64_t XY, uint64_t Z, cudaStream_t stream) {
+  const uintptr_t align = (uintptr_t)p.in | (uintptr_t)p.out;
+  const uint64_t groups = XY * Z, full = (uint64_t)sm_count() * 512;
+  int V = 1;
+  if (Z % 4 == 0 && align % 16 == 0 && groups >= 4 * full)
+    V = 4;
+  else if (Z % 2 == 0 && align % 8 == 0 && groups >= 2 * full)
+    V = 2;
+  const bool last = Z == 1 && align % 16 == 0;
+  auto kern = last ? apply_qubits_f32<K, 1, true>
+                   : V == 4 ? apply_qubits_f32<K, 4, false> : V == 2 ? apply_qubits_f32<K, 2, false>
+                                                                     : apply_qubits_f32<K, 1, false>;
+  p.div_z = make_fastdiv(Z / V);
+  p.n_items = groups / V;
+  const uint64_t blocks = (p.n_items + kQubitBlock - 1) / kQubitBlock;
+  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)sm_count() * 16));
+  return launch_pdl(kern, grid, (unsigned)kQubitBlock, 0, stream, p);
+}
+
 // row groups = min(Kout, 4) rounded down to a power of two; the remaining
 // warps of the 8 are item warps (tile = 32 * 8 / row groups items)
 int pick_iw(int kout) {
@@ -983,6 +1106,9 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
     const bool f32 = dtype == QSGB_F32 && kin <= kDenseMaxK && kout <= kDenseMaxK;
     const bool f64 = dtype == QSGB_F64 && (arith == QSGB_ARITH_AUTO || arith == QSGB_ARITH_F64) && kin <= 4 &&
                      kout <= 4 && fmas <= kDenseMaxF64Fma;
+    if (f32 && db_in == 4 && db_out == 4 && da_in == da_out && (da_in == 4 || (da_in == 1 && X == 1)))
+      return da_in == 4 ? launch_qubits_f32<16>(p, (uint64_t)X * Y, (uint64_t)Z, s)
+                        : launch_qubits_f32<4>(p, (uint64_t)Y, (uint64_t)Z, s);
     if (f32 || f64) {
       p.div_z = make_fastdiv((uint64_t)Z);
       p.n_items = (uint64_t)X * Y * Z;

@@ -43,6 +43,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace qsgb {
@@ -669,23 +670,48 @@ __global__ void __launch_bounds__(kDenseBlock) apply_dense_kernel(const __grid_c
   }
 }
 
-// The same for FP32 vectors whose targets are full qubits (K = 4 or 16, in and
-// out), the usual case: the sizes are known, a row of P is read four entries at
-// a time, and a thread takes V consecutive groups along z (16, 8 or 4 bytes an
+// The same for targets that are full qubits (K = 4 or 16, in and out), the usual
+// case: the sizes are known, a row of P is read four entries at
+// a time, and a thread takes V consecutive groups along z (up to 16 bytes an
 // access) or, with the less significant target last (LAST), the groups' rows as
 // 16 bytes.  The kernel above was bound by one shared-memory load per FMA.
 // V = 1 leaves a vector of 10 qubits the most blocks; V = 4 reads P the least.
 // The products and their order are those above.  Measured on GB300, us in a
 // graph, above / here, one qubit and two, on 8 / 10 / 11 / 12 qubits: 3.8 / 10.1
 // / 23.8 / 82 -> 2.2 / 5.6 / 7.4 / 21 (6.3 TB/s) and 6.1 / 8.1 / 19.6 / 54 -> 3.1
-// / 5.4 / 8.9 / 28; the last two of 12 qubits 104 -> 40.
+// / 5.4 / 8.9 / 28; the last two of 12 qubits 104 -> 40.  One qubit in FP64 on 8
+// qubits 3.9 -> 2.9.
 constexpr int kQubitBlock = 128;
 
-template <int K, int V, bool LAST>
-__global__ void __launch_bounds__(kQubitBlock) apply_qubits_f32(const __grid_constant__ ApplyParams p) {
+// B bytes of consecutive values between registers and memory, at most 16 at a
+// time
+template <typename T, int N>
+__device__ __forceinline__ void load_run(T (&v)[N], const T* src) {
+  constexpr int B = N * (int)sizeof(T) >= 16 ? 16 : N * (int)sizeof(T), W = B / (int)sizeof(T);
+  using U = typename std::conditional<B == 16, uint4, typename std::conditional<B == 8, uint2, unsigned>::type>::type;
+#pragma unroll
+  for (int i = 0; i < N; i += W) {
+    const U u = *reinterpret_cast<const U*>(src + i);
+    memcpy(v + i, &u, B);
+  }
+}
+template <typename T, int N>
+__device__ __forceinline__ void store_run(T* dst, const T (&v)[N]) {
+  constexpr int B = N * (int)sizeof(T) >= 16 ? 16 : N * (int)sizeof(T), W = B / (int)sizeof(T);
+  using U = typename std::conditional<B == 16, uint4, typename std::conditional<B == 8, uint2, unsigned>::type>::type;
+#pragma unroll
+  for (int i = 0; i < N; i += W) {
+    U u;
+    memcpy(&u, v + i, B);
+    *reinterpret_cast<U*>(dst + i) = u;
+  }
+}
+
+template <typename T, int K, int V, bool LAST>
+__global__ void __launch_bounds__(kQubitBlock) apply_qubits(const __grid_constant__ ApplyParams p) {
   static_assert(!LAST || V == 1, "a group's rows are the vectors");
   constexpr int NE = (K * K + kQubitBlock - 1) / kQubitBlock;
-  __shared__ __align__(16) float P[K * K];
+  __shared__ __align__(16) T P[K * K];
   __shared__ double wmax[kQubitBlock / 32];
   const int t = threadIdx.x;
   pdl_wait();
@@ -702,89 +728,77 @@ __global__ void __launch_bounds__(kQubitBlock) apply_qubits_f32(const __grid_con
   double amax = 0.0;
 #pragma unroll
   for (int w = 0; w < kQubitBlock / 32; ++w) amax = fmax(amax, wmax[w]);
+  const double thr = sizeof(T) == 4 ? amax * 0x1p-30 : (p.arith == QSGB_ARITH_F64 ? 0.0 : amax * 0x1p-52);
 #pragma unroll
   for (int i = 0; i < NE; ++i) {
     const int e = t + i * kQubitBlock;
-    if (e < K * K) P[e] = fabs(v[i]) > amax * 0x1p-30 ? (float)v[i] : 0.0f;
+    if (e < K * K) P[e] = fabs(v[i]) > thr ? (T)v[i] : (T)0;
   }
   __syncthreads();
-  const float* X = static_cast<const float*>(p.in);
-  float* Y = static_cast<float*>(p.out);
+  const T* X = static_cast<const T*>(p.in);
+  T* Y = static_cast<T*>(p.out);
   for (uint64_t it = (uint64_t)blockIdx.x * kQubitBlock + t; it < p.n_items; it += (uint64_t)gridDim.x * kQubitBlock) {
     const uint64_t t1 = fdiv(it, p.div_z);
     const uint64_t z = it - t1 * p.div_z.d;
     const uint64_t x = fdiv(t1, p.div_y);
     const uint64_t y = t1 - x * p.div_y.d;
     const int64_t base = (int64_t)x * p.sxi + (int64_t)y * p.syi + (int64_t)z * V;
-    float in[K][V];
+    T in[K][V];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const float* src = X + base + (k >> 2) * p.sai + (k & 3) * p.sbi;
-      if constexpr (LAST) {
-        if ((k & 3) == 0) {
-          const float4 u = *reinterpret_cast<const float4*>(src);
-          in[k][0] = u.x; in[k + 1][0] = u.y; in[k + 2][0] = u.z; in[k + 3][0] = u.w;
-        }
-      } else if constexpr (V == 4) {
-        const float4 u = *reinterpret_cast<const float4*>(src);
-        in[k][0] = u.x; in[k][1] = u.y; in[k][2] = u.z; in[k][3] = u.w;
-      } else if constexpr (V == 2) {
-        const float2 u = *reinterpret_cast<const float2*>(src);
-        in[k][0] = u.x; in[k][1] = u.y;
-      } else {
-        in[k][0] = *src;
+      const T* src = X + base + (k >> 2) * p.sai + (k & 3) * p.sbi;
+      if constexpr (!LAST) {
+        load_run(in[k], src);
+      } else if ((k & 3) == 0) {
+        T u[4];
+        load_run(u, src);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) in[k + b][0] = u[b];
       }
     }
 #pragma unroll 1
     for (int a = 0; a < K / 4; ++a) {
-      float acc[4][V];
+      T acc[4][V];
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
 #pragma unroll
-        for (int l = 0; l < V; ++l) acc[b][l] = 0.0f;
+        for (int l = 0; l < V; ++l) acc[b][l] = (T)0;
 #pragma unroll
         for (int k = 0; k < K; k += 4) {
-          const float4 c = *reinterpret_cast<const float4*>(P + (4 * a + b) * K + k);
+          T c[4];
+          load_run(c, P + (4 * a + b) * K + k);
 #pragma unroll
-          for (int l = 0; l < V; ++l) {
-            acc[b][l] = fmaf(c.x, in[k][l], acc[b][l]);
-            acc[b][l] = fmaf(c.y, in[k + 1][l], acc[b][l]);
-            acc[b][l] = fmaf(c.z, in[k + 2][l], acc[b][l]);
-            acc[b][l] = fmaf(c.w, in[k + 3][l], acc[b][l]);
-          }
+          for (int l = 0; l < V; ++l)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[b][l] = fma(c[q], in[k + q][l], acc[b][l]);
         }
       }
-      float* dst = Y + base + a * p.sao;
+      T* dst = Y + base + a * p.sao;
       if constexpr (LAST) {
-        *reinterpret_cast<float4*>(dst) = make_float4(acc[0][0], acc[1][0], acc[2][0], acc[3][0]);
+        const T u[4] = {acc[0][0], acc[1][0], acc[2][0], acc[3][0]};
+        store_run(dst, u);
       } else {
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          if constexpr (V == 4)
-            *reinterpret_cast<float4*>(dst + b * p.sbo) = make_float4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]);
-          else if constexpr (V == 2)
-            *reinterpret_cast<float2*>(dst + b * p.sbo) = make_float2(acc[b][0], acc[b][1]);
-          else
-            dst[b * p.sbo] = acc[b][0];
-        }
+        for (int b = 0; b < 4; ++b) store_run(dst + b * p.sbo, acc[b]);
       }
     }
   }
 }
 
-template <int K>
-int launch_qubits_f32(ApplyParams& p, uint64_t XY, uint64_t Z, cudaStream_t stream) {
+template <typename T, int K>
+int launch_qubits(ApplyParams& p, uint64_t XY, uint64_t Z, cudaStream_t stream) {
+  constexpr int kWidest = 16 / (int)sizeof(T);
   const uintptr_t align = (uintptr_t)p.in | (uintptr_t)p.out;
   const uint64_t groups = XY * Z, full = (uint64_t)sm_count() * 512;
   int V = 1;
-  if (Z % 4 == 0 && align % 16 == 0 && groups >= 4 * full)
+  if (kWidest >= 4 && Z % 4 == 0 && align % 16 == 0 && groups >= 4 * full)
     V = 4;
-  else if (Z % 2 == 0 && align % 8 == 0 && groups >= 2 * full)
+  else if (Z % 2 == 0 && align % (2 * sizeof(T)) == 0 && groups >= 2 * full)
     V = 2;
   const bool last = Z == 1 && align % 16 == 0;
-  auto kern = last ? apply_qubits_f32<K, 1, true>
-                   : V == 4 ? apply_qubits_f32<K, 4, false> : V == 2 ? apply_qubits_f32<K, 2, false>
-                                                                     : apply_qubits_f32<K, 1, false>;
+  auto kern = last ? apply_qubits<T, K, 1, true>
+                   : V == 4 ? apply_qubits<T, K, kWidest, false>
+                            : V == 2 ? apply_qubits<T, K, 2, false> : apply_qubits<T, K, 1, false>;
   p.div_z = make_fastdiv(Z / V);
   p.n_items = groups / V;
   const uint64_t blocks = (p.n_items + kQubitBlock - 1) / kQubitBlock;
@@ -1087,7 +1101,8 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
     return tc::launch_wide(ptm, flags & 3, in, out, dtype, (int)da_out, (int)db_out, (int)da_in, (int)db_in,
                            (uint64_t)X, (uint64_t)Y, (uint64_t)Z, status, s);
   // 1c. one-qubit device PTMs, no term limit: the tensor cores too, from 9
-  // qubits on (on 8 the dense kernel of 2a takes 3.9 us, this 4.2).  FP64 FMAs
+  // qubits on (there the dense kernel of 2a takes as long, on 8 2.9 us against
+  // 4.2 here).  FP64 FMAs
   // alone take 7 us on 10 qubits there, and larger vectors went to the generic
   // kernel.  Measured on GB300, us on 9 / 10 / 11 / 12 qubits: 5.5 / 13.7 / 42
   // / 143 without, 4.9 / 8.2 / 23.7 / 79 here, on the last qubit 5.7 / 13.8 /
@@ -1106,9 +1121,11 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
     const bool f32 = dtype == QSGB_F32 && kin <= kDenseMaxK && kout <= kDenseMaxK;
     const bool f64 = dtype == QSGB_F64 && (arith == QSGB_ARITH_AUTO || arith == QSGB_ARITH_F64) && kin <= 4 &&
                      kout <= 4 && fmas <= kDenseMaxF64Fma;
-    if (f32 && db_in == 4 && db_out == 4 && da_in == da_out && (da_in == 4 || (da_in == 1 && X == 1)))
-      return da_in == 4 ? launch_qubits_f32<16>(p, (uint64_t)X * Y, (uint64_t)Z, s)
-                        : launch_qubits_f32<4>(p, (uint64_t)Y, (uint64_t)Z, s);
+    if (db_in == 4 && db_out == 4 && da_in == da_out && (da_in == 4 || (da_in == 1 && X == 1)) && (f32 || f64)) {
+      if (f64) return launch_qubits<double, 4>(p, (uint64_t)Y, (uint64_t)Z, s);
+      return da_in == 4 ? launch_qubits<float, 16>(p, (uint64_t)X * Y, (uint64_t)Z, s)
+                        : launch_qubits<float, 4>(p, (uint64_t)Y, (uint64_t)Z, s);
+    }
     if (f32 || f64) {
       p.div_z = make_fastdiv((uint64_t)Z);
       p.n_items = (uint64_t)X * Y * Z;

@@ -1,4 +1,4 @@
-"""Device PTMs of full qubits on FP32 vectors: every width of access (vectors
+"""Device PTMs of full qubits on FP32 and small FP64 vectors: every width of access (vectors
 large enough for 4, 2 and 1 groups a thread, the last target, odd inner
 lengths) and tensors that start between two vectors."""
 import numpy as np
@@ -38,3 +38,24 @@ def test_full_qubits(shape, qs, offset):
     tol = apply(p.abs(), x.double().abs()) * (2 * 4 ** k * 2.0 ** -24)
     assert got.dtype == torch.float32
     assert bool(((got.double() - ref).abs() <= tol).all())
+
+
+@pytest.mark.parametrize('shape,q,arith', [
+    ((4,), 0, L.ARITH_AUTO), ((4, 4), 1, L.ARITH_AUTO),
+    ((4,) * 7, 3, L.ARITH_AUTO), ((4,) * 8, 7, L.ARITH_AUTO),
+    ((3, 4, 5), 1, L.ARITH_AUTO), ((4,) * 10, 0, L.ARITH_F64),
+    ((4,) * 10, 9, L.ARITH_F64), ((7, 4, 4096, 3), 1, L.ARITH_F64)])
+@pytest.mark.parametrize('offset', (0, 1))
+def test_one_qubit_fp64(shape, q, arith, offset):
+    rng = np.random.default_rng([len(shape), q, offset])
+    size = int(np.prod(shape))
+    buf = torch.from_numpy(rng.standard_normal(size + offset)).cuda()
+    x = buf[offset:].view(shape)
+    p = torch.from_numpy(rng.standard_normal((4, 4))).cuda()
+    got = torch.ops.qsgb.apply_ptm(x, p, [q], arith, 0, False)
+
+    def apply(a, b):
+        return torch.movedim(torch.tensordot(a, b, dims=([1], [q])), 0, q)
+    # four roundings on either side
+    tol = apply(p.abs(), x.abs()) * (8 * 2.0 ** -53)
+    assert bool(((got - apply(p, x)).abs() <= tol).all())

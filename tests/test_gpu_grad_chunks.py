@@ -70,3 +70,29 @@ def test_values_without_digits(value):
     x[n // 2:n // 2 + 40, 1, 2] = value
     g[:, 3, 3] = 0.0
     check(x, g, (1, 2))
+
+
+@pytest.mark.parametrize('n', [1, 15, 300, 'limit', 'above'])
+@pytest.mark.parametrize('place', ['first', 'last'])
+@pytest.mark.parametrize('value', [1.0, 0.0, 1e-40, 3e38, np.inf, np.nan])
+def test_fp32_vectors(n, place, value):
+    """FP32 values are split as they are; subnormals go to FP64."""
+    n = {'limit': limit(), 'above': limit() + 21}.get(n, n)
+    torch.manual_seed(n)
+    shape, qs = {'first': ((4, 4, n), (0, 1)),
+                 'last': ((n, 4, 4), (1, 2))}[place]
+    x, g = (torch.randn(shape, dtype=torch.float64, device='cuda').float()
+            for _ in range(2))
+    x[n // 2 if place == 'last' else 1] *= float(np.float32(value))
+    got = torch.ops.qsgb.ptm_grad(x, g, list(qs)).cpu()
+    check(x.double(), g.double(), qs)  # the FP64 kernel on the same values
+    xs, gs = (np.moveaxis(t.double().cpu().numpy(), qs, (0, 1))
+              .reshape(16, -1) for t in (x, g))
+    with np.errstate(invalid='ignore', over='ignore'):
+        ref = np.stack([(gs[r] * xs).sum(-1) for r in range(16)])
+    fin = np.isfinite(ref)
+    got = got.reshape(16, 16).numpy()
+    np.testing.assert_array_equal(np.isfinite(got), fin)
+    fx, fg = (np.where(np.isfinite(v), np.abs(v), 0) for v in (xs, gs))
+    tol = -(-n // 16) * (2.0 ** -49 + 1024 * 2.0 ** -53) * fx.max() * fg.max()
+    assert np.all(np.abs(got[fin] - ref[fin]) <= tol)

@@ -345,8 +345,9 @@ def adaptive_chunks(stage, total, width, grid):
     one fixed length leaves most blocks idle (64 items of 16384 groups of a
     12-qubit instance on 304 blocks; one item of a whole 8-qubit instance), so
     a stage is split evenly over the blocks, between those limits.  Measured on
-    GB300, one step of 20 circuits of 4 to 12 qubits: 125 ms at the fixed 8192
-    groups and at most 64 items per op, 106 ms here; 7 circuits of up to 11
+    GB300 (with an earlier two-qubit adjoint), one step of 20 circuits of 4 to
+    12 qubits: 125 ms at the fixed 8192 groups and at most 64 items per op, 106
+    ms here (90.6 with the present one); 7 circuits of up to 11
     qubits 14.0 and 4.2 ms; 14 of up to 8 qubits 7.9 and 4.7 ms.  (Items of 256
     groups would take these last two to 3.5 and 2.8 ms, with other FP32 sums.)
     """

@@ -610,8 +610,7 @@ __global__ void __launch_bounds__(kBlock) apply_ptm_kernel(const __grid_constant
 // FP64 storage (entries at or below 2^-52 of the largest skipped under
 // 'auto', exact zeros under 'f64'; exact IEEE products and sums, so no
 // range fallback is needed).  FP64 takes this path only for one-qubit PTMs
-// on vectors small enough for the FP64 pipe (at most 2^23 FMAs, ~14 us) that
-// the tensor cores do not take (apply_common 1c: up to 8 qubits, arith='f64').
+// on vectors small enough for the FP64 pipe (at most 2^23 FMAs, ~14 us).
 constexpr int kDenseMaxK = 16;
 constexpr int kDenseBlock = 256;
 constexpr double kDenseMaxF64Fma = 8388608.0;  // 2^23
@@ -1100,20 +1099,6 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
       kout <= tc::kWideMax && (arith == QSGB_ARITH_AUTO || arith == QSGB_ARITH_F32) && tc_device_auto())
     return tc::launch_wide(ptm, flags & 3, in, out, dtype, (int)da_out, (int)db_out, (int)da_in, (int)db_in,
                            (uint64_t)X, (uint64_t)Y, (uint64_t)Z, status, s);
-  // 1c. one-qubit device PTMs, no term limit: the tensor cores too, from 9
-  // qubits on (there the dense kernel of 2a takes as long, on 8 2.9 us against
-  // 4.2 here).  FP64 FMAs
-  // alone take 7 us on 10 qubits there, and larger vectors went to the generic
-  // kernel.  Measured on GB300, us on 9 / 10 / 11 / 12 qubits: 5.5 / 13.7 / 42
-  // / 143 without, 4.9 / 8.2 / 23.7 / 79 here, on the last qubit 5.7 / 13.8 /
-  // 53 / 183 and 4.6 / 9.4 / 26 / 83; a graphed gradient step on 10 qubits
-  // (112 such applications) 10.78 -> 10.10 ms, error against 64 bits as before.
-  if (!(flags & QSGB_PTM_HOST) && dtype == QSGB_F64 && arith == QSGB_ARITH_AUTO && kin == 4 && kout == 4 &&
-      da_in == 1 && da_out == 1 && X == 1 && p.max_terms == 16 && Y * Z >= (1 << 16) && tc_device_auto() &&
-      mode == kLaunch) {
-    const int st = tc::launch_one(ptm, flags & 3, in, out, (uint64_t)Y, (uint64_t)Z, status, s);
-    if (st != QSGB_ERR_UNSUPPORTED) return st;
-  }
   // 2a. small device PTMs, no term limit: the dense kernel (FP32 storage up
   // to 16 x 16; FP64 storage for one-qubit PTMs on small vectors)
   if (!(flags & QSGB_PTM_HOST) && p.max_terms == kin * kout) {

@@ -283,22 +283,12 @@ __device__ __forceinline__ int dev_index(int layout, int r, int k) {
   }
 }
 
-// Offset of the entry of a 4 x 4 one-qudit PTM for rows r % 4, columns k % 4.
-__device__ __forceinline__ int one_index(int layout, int r, int k) {
-  return (layout & QSGB_PTM_TRANSPOSED) ? (k & 3) * 4 + (r & 3) : (r & 3) * 4 + (k & 3);
-}
-
-// ONEQ: a 4 x 4 device PTM, applied as its product with the identity on four
-// neighbouring groups (a = ka = ra, launch_one): four blocks of the 16 inputs
-// that share nothing, each with its own scale, so a group's digits are those
-// of its own four inputs.
-//
 // DEVP: the PTM is in device memory (p.dptm), else in the parameters (p.ptm).
 // Every block splits it into the B operand planes and the row scales, in
 // shared memory: that costs less than carrying the planes in the parameters
 // (3.5 KB more a launch, read back with divergent constant loads: 11.9 against
 // 10.2 us on 10 qubits) and leaves the host nothing to split.
-template <bool CONTIG, bool DEVP, bool ONEQ>
+template <bool CONTIG, bool DEVP>
 __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_constant__ TcParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int t = threadIdx.x, warp = t >> 5;
@@ -368,14 +358,8 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
   {
     // 8 threads per row (lanes 8r' .. 8r'+7 of a warp), two entries each
     const int r = t >> 3, k = 2 * (t & 7);
-    double v0 = 0.0, v1 = 0.0;
-    if (!ONEQ) {
-      v0 = DEVP ? p.dptm[dev_index(p.dlayout, r, k)] : p.ptm[r][k];
-      v1 = DEVP ? p.dptm[dev_index(p.dlayout, r, k + 1)] : p.ptm[r][k + 1];
-    } else if (r >> 2 == k >> 2) {
-      v0 = p.dptm[one_index(p.dlayout, r, k)];
-      v1 = p.dptm[one_index(p.dlayout, r, k + 1)];
-    }
+    const double v0 = DEVP ? p.dptm[dev_index(p.dlayout, r, k)] : p.ptm[r][k];
+    const double v1 = DEVP ? p.dptm[dev_index(p.dlayout, r, k + 1)] : p.ptm[r][k + 1];
     const unsigned h0 = (unsigned)__double2hiint(v0), h1 = (unsigned)__double2hiint(v1);
     unsigned emax = max((h0 >> 20) & 0x7ffu, (h1 >> 20) & 0x7ffu);
     emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 1));
@@ -411,30 +395,22 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
   }
   bool done = true;  // this thread saw the last tile's MMAs complete
   for (; tile < p.n_tiles; tile += gridDim.x) {
-    // exponents of the inputs that share a scale (in place), and whether the
-    // group needs native FP64
-    constexpr int kScales = ONEQ ? 4 : 1, kEach = 16 / kScales;
-    unsigned eh[kScales], bad = ptm_bad ? 1u : 0u;
+    unsigned eh = 0u;
 #pragma unroll
-    for (int c = 0; c < kScales; ++c) {
-      eh[c] = 0u;
+    for (int k = 0; k < 16; ++k) eh = max(eh, (unsigned)__double2hiint(x[k]) & 0x7ff00000u);
+    unsigned emax = eh >> 20;
+    unsigned bad = (ptm_bad || emax == 0x7ffu) ? 1u : 0u;  // inf, nan
+    if (emax < kMinExp) {  // all zero, or all below the smallest scale
 #pragma unroll
-      for (int k = 0; k < kEach; ++k) eh[c] = max(eh[c], (unsigned)__double2hiint(x[kEach * c + k]) & 0x7ff00000u);
-      unsigned emax = eh[c] >> 20;
-      bad |= emax == 0x7ffu ? 1u : 0u;  // inf, nan
-      if (emax < kMinExp) {  // all zero, or all below the smallest scale
-#pragma unroll
-        for (int k = 0; k < kEach; ++k) bad |= x[kEach * c + k] != 0.0 ? 1u : 0u;
-        emax = 1023u;  // any scale serves zeros
-      }
-      bad |= (scale8_ok((int)emax + rmin) && scale8_ok((int)emax + rmax)) ? 0u : 1u;
-      eh[c] = emax << 20;
+      for (int k = 0; k < 16; ++k) bad |= x[k] != 0.0 ? 1u : 0u;
+      emax = 1023u;  // any scale serves zeros
     }
+    bad |= (scale8_ok((int)emax + rmin) && scale8_ok((int)emax + rmax)) ? 0u : 1u;
+    eh = emax << 20;
     // this thread's row of the seven input digit planes, 8 inputs at a time
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      const unsigned ea = eh[ONEQ ? 2 * c : 0], eb = eh[ONEQ ? 2 * c + 1 : 0];
-      const unsigned e8[8] = {ea, ea, ea, ea, eb, eb, eb, eb};
+      const unsigned e8[8] = {eh, eh, eh, eh, eh, eh, eh, eh};
       split8<kPlaneA>(smem + core_off(t, 8 * c), x + 8 * c, e8);
     }
     // the next tile's inputs load while the tensor cores and the
@@ -496,7 +472,7 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
         for (int l = 0; l < kLevels; l += 2)
           pr[l / 2] = level_pair(__uint_as_float(w[l][q]), __uint_as_float(w[l + 1][q]));
         y[q] = scale8(combine8(pr[0], pr[1], pr[2], pr[3]),
-                      eh[ONEQ ? c : 0] + ((unsigned)srow[4 * c + q] << 20));
+                      eh + ((unsigned)srow[4 * c + q] << 20));
       }
       if (livec) {
         if (p.vec_z1) {
@@ -516,9 +492,8 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
       for (int r = 0; r < 16; ++r) {
         double a = 0.0;
 #pragma unroll 1
-        for (int k = ONEQ ? r & 12 : 0; k < (ONEQ ? (r & 12) + 4 : 16); ++k) {
-          const double pk = ONEQ ? p.dptm[one_index(p.dlayout, r, k)]
-                                 : DEVP ? p.dptm[dev_index(p.dlayout, r, k)] : p.ptm[r][k];
+        for (int k = 0; k < 16; ++k) {
+          const double pk = DEVP ? p.dptm[dev_index(p.dlayout, r, k)] : p.ptm[r][k];
           a = fma(pk, p.in[bc + (k >> 2) * sai + (k & 3) * sbi], a);
         }
         p.out[bc + (r >> 2) * p.sao + (r & 3) * p.sbo] = a;
@@ -613,13 +588,13 @@ void set_geometry(TcParams& p, const void* in, void* out, uint64_t X, uint64_t Y
   p.sxo = p.sxi;
 }
 
-template <bool DEVP, bool ONEQ = false>
+template <bool DEVP>
 int launch_umma(TcParams& p, const void* in, void* out, uint64_t Z, cudaStream_t stream) {
   // tcgen05 form: tiles of 128 groups per block, at most 4 blocks per SM
   p.n_tiles = (p.n_groups + kUBlock - 1) / kUBlock;
   const bool contig = Z % kUBlock == 0;
-  p.vec_z1 = Z == 1 && p.sbi == 1 && (uintptr_t)in % 32 == 0 && (uintptr_t)out % 32 == 0 ? 1 : 0;
-  auto kern = contig ? apply16_umma_kernel<true, DEVP, ONEQ> : apply16_umma_kernel<false, DEVP, ONEQ>;
+  p.vec_z1 = Z == 1 && (uintptr_t)in % 32 == 0 && (uintptr_t)out % 32 == 0 ? 1 : 0;
+  auto kern = contig ? apply16_umma_kernel<true, DEVP> : apply16_umma_kernel<false, DEVP>;
   const int st = allow_dynamic_smem((const void*)kern, kUmmaSmem);
   if (st != QSGB_OK) return st;
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(p.n_tiles, (uint64_t)sm_count() * 4));
@@ -663,21 +638,6 @@ int launch_device(const double* dptm, int layout, const void* in, void* out, uin
   p.dlayout = layout & 3;
   set_geometry(p, in, out, X, Y, Z, status);
   return launch_umma<true>(p, in, out, Z, stream);
-}
-
-int launch_one(const double* dptm, int layout, const void* in, void* out, uint64_t Y, uint64_t Z, unsigned* status,
-               cudaStream_t stream) {
-  TcParams p{};
-  p.dptm = dptm;
-  p.dlayout = layout & 3;
-  const bool outer = Y % 4 == 0;  // four neighbours along y, else four quarters of z
-  if (!outer && Z % 4 != 0) return QSGB_ERR_UNSUPPORTED;
-  set_geometry(p, in, out, outer ? Y / 4 : 1, outer ? 1 : Y, outer ? Z : Z / 4, status);
-  p.sai = p.sao = (int64_t)(outer ? 4 * Z : Z / 4);
-  p.sbi = p.sbo = (int64_t)Z;
-  p.syi = p.syo = 4 * (int64_t)Z;
-  p.sxi = p.sxo = 16 * (int64_t)Z;
-  return launch_umma<true, true>(p, in, out, outer ? Z : Z / 4, stream);
 }
 
 }  // namespace tc

@@ -210,11 +210,6 @@ int launch(const double* op, const void* in, void* out, uint64_t X, uint64_t Y, 
 int launch_device(const double* dptm, int layout, const void* in, void* out, uint64_t X, uint64_t Y, uint64_t Z,
                   unsigned* status, cudaStream_t stream);
 
-// A 4 x 4 one-qudit PTM in device memory on an FP64 tensor viewed as (Y, 4, Z),
-// Y or Z a multiple of 4 (else QSGB_ERR_UNSUPPORTED).
-int launch_one(const double* dptm, int layout, const void* in, void* out, uint64_t Y, uint64_t Z, unsigned* status,
-               cudaStream_t stream);
-
 // Larger dense PTMs (Kin, Kout <= kWideMax) in device memory, FP64 or FP32
 // vectors (qsgb_tcw.cu); dimensions and strides as for launch_device.
 constexpr int kWideMax = 96;

@@ -1,0 +1,54 @@
+"""Components far below the largest of their group keep their own precision
+where no digit split is used: one-qubit device PTMs.
+
+Bounds are per component, against sums of magnitudes: native FP64 rows of four
+terms err by less than 2^-45 of sum |P| |x|, float-float ones by less than the
+repository's bound for FP64 rows."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import RTOL_F64
+from quantumsim_gb300 import _lib as L
+from oracle import pauli_vector_np as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _bounded(got, x, p, qs, eps):
+    """|got - P x| <= eps |P| |x|, every component (the reference's own
+    roundings, 2^-53 a term, are a small part of eps)."""
+    ref = O.apply_ptm(x, p, *qs)
+    mag = O.apply_ptm(np.abs(x), np.abs(p), *qs)
+    excess = float(np.max(np.abs(got - ref) - eps * mag))
+    assert excess <= 0
+
+
+@pytest.mark.parametrize('size', [1e-8, 1e-12, 1e-17, 1e-40])
+@pytest.mark.parametrize('n,q', [(8, 3), (9, 0), (9, 8), (10, 4), (11, 2),
+                                 (11, 10)])
+def test_one_qubit_device_ptm(n, q, size):
+    """A rotation about z with dephasing: coherences beside populations; and
+    a row whose large entry meets a zero."""
+    eps = 2.0 ** -45 if n <= 10 else RTOL_F64
+    rng = np.random.default_rng([n, q])
+    x = rng.uniform(0.2, 0.8, (4,) * n)
+    at = [slice(None)] * n
+    for k in (2, 3):
+        at[q] = k
+        x[tuple(at)] *= size
+    c, s = np.cos(0.7) * 0.99, np.sin(0.7) * 0.99
+    rot = np.array([[1, 0, 0, 0], [0, 1, 0, 0], [0, 0, c, -s], [0, 0, s, c]])
+    xt = torch.from_numpy(x).cuda()
+    for p in (rot, rot.T):
+        got = torch.ops.qsgb.apply_ptm(xt, torch.from_numpy(p.copy()).cuda(),
+                                       [q], L.ARITH_AUTO, 0, False)
+        _bounded(got.cpu().numpy(), x, p, (q,), eps)
+    at[q] = 0
+    x[tuple(at)] = 0.0
+    p = np.full((4, 4), 1e-10) * rng.uniform(0.5, 1, (4, 4))
+    p[:, 0] = 1.0
+    got = torch.ops.qsgb.apply_ptm(torch.from_numpy(x).cuda(),
+                                   torch.from_numpy(p).cuda(), [q],
+                                   L.ARITH_AUTO, 0, False)
+    _bounded(got.cpu().numpy(), x, p, (q,), eps)

@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(kStage2Entries* kStage2Slices)
 }
 
 // ---------------------------------------------------------------------------
-// 16 x 16 gradients: the tensor cores
+// 16 x 16 gradients on FP64 vectors: the tensor cores
 // ---------------------------------------------------------------------------
 // The same reduction as a product over groups, dP = G^T X per chunk of 16
 // groups, on mma.sync.m16n8k16 (FP16 operands, FP32 accumulators) with the
@@ -555,9 +555,6 @@ __global__ void __launch_bounds__(kStage2Entries* kStage2Slices)
 // chunks of 16): base-1024 digits 21.8 and 173 us, base 256 with H = 1 19.9 and
 // 144, H = 2 17.3 and 131; on the last two qudits, with 32-byte loads instead
 // of 8-byte ones, 25.0 and 174 -> 18.6 and 138.
-// FP32 vectors are widened exactly and take the same path: against the staged
-// float-float kernel 8 / 9 / 10 / 12 qubits 8.2 / 12.4 / 20.7 / 197 -> 7.9 / 9.1 /
-// 18.8 / 160 us.
 constexpr int kTcgBlock = 256;
 constexpr int kTcgWarps = kTcgBlock / 32;
 constexpr int kTcgPlane = 16 * 16 * 2;  // bytes per digit plane
@@ -585,32 +582,15 @@ __device__ __forceinline__ void load4(double* v, const double* src) {
   asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(src));
 }
 
-// four FP32 values as doubles, by integer operations (the conversions would
-// keep the FP64 pipe as busy as the products of the float-float kernel);
-// subnormals, inf and nan are not: their chunk is computed in native FP64
-__device__ __forceinline__ double widen(float f, unsigned& bad) {
-  const unsigned u = __float_as_uint(f), t = u & 0x7fffffffu;
-  bad |= (t - 1u < 0x7fffffu || t >= 0x7f800000u) ? 1u : 0u;
-  return __hiloint2double((int)((t ? (t >> 3) + 0x38000000u : 0u) | (u & 0x80000000u)), (int)(u << 29));
-}
-__device__ __forceinline__ double widen(double v, unsigned&) { return v; }
-__device__ __forceinline__ void load4(float* v, const float* src) {
-  const float4 u = *reinterpret_cast<const float4*>(src);
-  v[0] = u.x;
-  v[1] = u.y;
-  v[2] = u.z;
-  v[3] = u.w;
-}
-
-template <int H, typename T>
+template <int H>
 __global__ void __launch_bounds__(kTcgBlock* H, 2 / H) grad16_tc_kernel(const __grid_constant__ GradParams p,
                                                               double* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   TcgSmem<H>& sm = *reinterpret_cast<TcgSmem<H>*>(smem);
   TcgWarpSmem<H>& ws = sm.warp[w];
-  const T* __restrict__ X = static_cast<const T*>(p.x);
-  const T* __restrict__ G = static_cast<const T*>(p.g);
+  const double* __restrict__ X = static_cast<const double*>(p.x);
+  const double* __restrict__ G = static_cast<const double*>(p.g);
   const int h = lane >> 4, i = lane & 15;
   const int gid = lane >> 2, tig = lane & 3;
   if (threadIdx.x < 16) {
@@ -646,7 +626,7 @@ __global__ void __launch_bounds__(kTcgBlock* H, 2 / H) grad16_tc_kernel(const __
   const uint64_t n_chunks = (p.n_groups + 16 * H - 1) / (16 * H);
   const uint64_t wstride = (uint64_t)gridDim.x * kTcgWarps * H;
   for (uint64_t c = (uint64_t)blockIdx.x * kTcgWarps * H + w; c < n_chunks; c += wstride) {
-    T gt[H][8], xt[H][8];
+    double gv[H][8], xv[H][8];
 #pragma unroll
     for (int hf = 0; hf < H; ++hf) {
       const uint64_t g = c * (16 * H) + 16 * hf + i;
@@ -656,32 +636,30 @@ __global__ void __launch_bounds__(kTcgBlock* H, 2 / H) grad16_tc_kernel(const __
         if (p.vec_z1) {
 #pragma unroll
           for (int j = 0; j < 8; j += 4) {
-            load4(gt[hf] + j, G + bo + sm.oout[8 * h + j]);
-            load4(xt[hf] + j, X + bi + sm.oin[8 * h + j]);
+            load4(gv[hf] + j, G + bo + sm.oout[8 * h + j]);
+            load4(xv[hf] + j, X + bi + sm.oin[8 * h + j]);
           }
         } else {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            gt[hf][j] = G[bo + sm.oout[8 * h + j]];
-            xt[hf][j] = X[bi + sm.oin[8 * h + j]];
+            gv[hf][j] = G[bo + sm.oout[8 * h + j]];
+            xv[hf][j] = X[bi + sm.oin[8 * h + j]];
           }
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) gt[hf][j] = xt[hf][j] = (T)0;
+        for (int j = 0; j < 8; ++j) gv[hf][j] = xv[hf][j] = 0.0;
       }
     }
-    unsigned nonfinite = 0;
     // chunk exponents of rows 8h+j (g_out, low half word) and columns 8h+j
     // (x_in, high half word): maxima over the 16 lanes of this half
-    unsigned e2[8];
+    unsigned e2[8], nonfinite = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       e2[j] = 0u;
 #pragma unroll
       for (int hf = 0; hf < H; ++hf) {
-        const unsigned hg = (unsigned)__double2hiint(widen(gt[hf][j], nonfinite)),
-                       hx = (unsigned)__double2hiint(widen(xt[hf][j], nonfinite));
+        const unsigned hg = (unsigned)__double2hiint(gv[hf][j]), hx = (unsigned)__double2hiint(xv[hf][j]);
         e2[j] = __vmaxu2(e2[j], ((hg >> 20) & 0x7ffu) | ((hx >> 4) & 0x7ff0000u));
       }
     }
@@ -696,15 +674,15 @@ __global__ void __launch_bounds__(kTcgBlock* H, 2 / H) grad16_tc_kernel(const __
         top = __vmaxu2(top, e2[j]);
         low = __vminu2(low, e2[j]);
       }
-      nonfinite |= ((top & 0xffffu) == 0x7ffu || (top >> 16) == 0x7ffu) ? 1u : 0u;
+      nonfinite = ((top & 0xffffu) == 0x7ffu || (top >> 16) == 0x7ffu) ? 1u : 0u;
       if ((low & 0xffffu) < tc::kMinExp || (low >> 16) < tc::kMinExp) {
         // a row or column that is all zero (exact) or below the smallest scale
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
 #pragma unroll
           for (int hf = 0; hf < H; ++hf) {
-            if ((e2[j] & 0xffffu) < tc::kMinExp && gt[hf][j] != (T)0) nonfinite = 1u;
-            if ((e2[j] >> 16) < tc::kMinExp && xt[hf][j] != (T)0) nonfinite = 1u;
+            if ((e2[j] & 0xffffu) < tc::kMinExp && gv[hf][j] != 0.0) nonfinite = 1u;
+            if ((e2[j] >> 16) < tc::kMinExp && xv[hf][j] != 0.0) nonfinite = 1u;
           }
           // any scale serves zeros
           if ((e2[j] & 0xffffu) < tc::kMinExp) e2[j] = (e2[j] & 0xffff0000u) | 1023u;
@@ -724,21 +702,11 @@ __global__ void __launch_bounds__(kTcgBlock* H, 2 / H) grad16_tc_kernel(const __
 #pragma unroll
       for (int j = 0; j < 8; ++j) eh[j] = (e2[j] & 0xffffu) << 20;
 #pragma unroll
-      for (int hf = 0; hf < H; ++hf) {
-        double v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = widen(gt[hf][j], nonfinite);
-        tc::split8<kTcgPlane>(ws.a[hf] + half_row(i, h), v, eh);
-      }
+      for (int hf = 0; hf < H; ++hf) tc::split8<kTcgPlane>(ws.a[hf] + half_row(i, h), gv[hf], eh);
 #pragma unroll
       for (int j = 0; j < 8; ++j) eh[j] = (e2[j] & 0xffff0000u) << 4;
 #pragma unroll
-      for (int hf = 0; hf < H; ++hf) {
-        double v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = widen(xt[hf][j], nonfinite);
-        tc::split8<kTcgPlane>(ws.b[hf] + half_row(i, h), v, eh);
-      }
+      for (int hf = 0; hf < H; ++hf) tc::split8<kTcgPlane>(ws.b[hf] + half_row(i, h), xv[hf], eh);
     }
     const bool chunk_bad = __any_sync(0xffffffffu, nonfinite != 0u);
     __syncwarp();
@@ -798,7 +766,7 @@ __global__ void __launch_bounds__(kTcgBlock* H, 2 / H) grad16_tc_kernel(const __
             if (g2 >= p.n_groups) break;
             int64_t bi, bo;
             bases(g2, bi, bo);
-            s2 = fma((double)G[bo + orr], (double)X[bi + ok], s2);
+            s2 = fma(G[bo + orr], X[bi + ok], s2);
           }
           y[nt][q] = s2;
         }
@@ -834,15 +802,15 @@ unsigned tcg_blocks(uint64_t n_groups) {
   return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)sm_count() * 2));
 }
 
-template <int H, typename T>
+template <int H>
 int launch_grad16(const GradParams& p, unsigned nb, double* part, cudaStream_t s) {
   const int smem = std::max((int)sizeof(TcgSmem<H>), kTcgWarps * H * 256 * (int)sizeof(double));
-  const int st = allow_dynamic_smem((const void*)grad16_tc_kernel<H, T>, smem);
+  const int st = allow_dynamic_smem((const void*)grad16_tc_kernel<H>, smem);
   if (st != QSGB_OK) return st;
-  return launch_pdl(grad16_tc_kernel<H, T>, nb, (unsigned)(kTcgBlock * H), (size_t)smem, s, p, part);
+  return launch_pdl(grad16_tc_kernel<H>, nb, (unsigned)(kTcgBlock * H), (size_t)smem, s, p, part);
 }
 
-// 16 x 16 gradients go to the tensor cores unless QSGB_TC_GRAD=0
+// 16 x 16 FP64 gradients go to the tensor cores unless QSGB_TC_GRAD=0
 bool tc_grad_enabled() {
   static const bool on = [] {
     const char* v = std::getenv("QSGB_TC_GRAD");
@@ -927,15 +895,13 @@ int grad_common(const void* x_in, const void* g_out, double* dptm, int64_t da_ou
   if (!scratch || scratch_bytes < (int64_t)nb * E * (int64_t)sizeof(double)) return QSGB_ERR_SCRATCH;
   cudaStream_t s = as_stream(stream);
   double* part = static_cast<double*>(scratch);
-  if (kin == 16 && kout == 16 && tc_grad_enabled()) {
-    const bool f64 = dtype == QSGB_F64;
-    p.vec_z1 = Z == 1 && db_in == 4 && db_out == 4 && ((uintptr_t)x_in | (uintptr_t)g_out) % (f64 ? 32 : 16) == 0;
+  if (dtype == QSGB_F64 && kin == 16 && kout == 16 && tc_grad_enabled()) {
+    p.vec_z1 = Z == 1 && db_in == 4 && db_out == 4 && ((uintptr_t)x_in | (uintptr_t)g_out) % 32 == 0;
     // chunks of 32 groups when those of 16 are more than the resident warps;
     // the scratch holds the partials of tcg_blocks <= nb blocks either way
     const bool wide = p.n_groups > (uint64_t)sm_count() * 2 * kTcgWarps * 16;
     const unsigned nbt = wide ? (unsigned)sm_count() : tcg_blocks(p.n_groups);
-    const int s1 = f64 ? (wide ? launch_grad16<2, double>(p, nbt, part, s) : launch_grad16<1, double>(p, nbt, part, s))
-                       : (wide ? launch_grad16<2, float>(p, nbt, part, s) : launch_grad16<1, float>(p, nbt, part, s));
+    const int s1 = wide ? launch_grad16<2>(p, nbt, part, s) : launch_grad16<1>(p, nbt, part, s);
     return s1 != QSGB_OK ? s1 : launch_stage2(part, (int)nbt, E, dptm, s);
   }
   // one qudit (a group's rows lie a stride apart) of at most 4 elements: a

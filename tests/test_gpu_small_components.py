@@ -1,9 +1,10 @@
 """Components far below the largest of their group keep their own precision
-where no digit split is used: one-qubit device PTMs.
+where no digit split is used: one-qubit device PTMs, gradients of FP32 vectors.
 
 Bounds are per component, against sums of magnitudes: native FP64 rows of four
 terms err by less than 2^-45 of sum |P| |x|, float-float ones by less than the
-repository's bound for FP64 rows."""
+repository's bound for FP64 rows; a float-float gradient of up to 2^11 groups by
+2^-40 of sum |g| |x|, plus 2^-149 a product below the float range."""
 import numpy as np
 import pytest
 import torch
@@ -52,3 +53,27 @@ def test_one_qubit_device_ptm(n, q, size):
                                    torch.from_numpy(p).cuda(), [q],
                                    L.ARITH_AUTO, 0, False)
     _bounded(got.cpu().numpy(), x, p, (q,), eps)
+
+
+@pytest.mark.parametrize('n', [1, 17, 300, 2048])
+@pytest.mark.parametrize('place', ['first', 'last', 'around'])
+@pytest.mark.parametrize('gap', [2.0 ** -40, 2.0 ** -60])
+def test_gradient_of_fp32_vectors(n, place, gap):
+    """Groups where the state is large and the gradient small, and the other
+    way round."""
+    torch.manual_seed(n)
+    x, g = (torch.rand(16, n, dtype=torch.float64) + 0.5 for _ in range(2))
+    x[:, 0::2] *= gap
+    g[:, 1::2] *= gap
+    x, g = x.float(), g.float()
+    xs, gs = x.double().numpy(), g.double().numpy()
+    ref, mag = gs @ xs.T, np.abs(gs) @ np.abs(xs).T
+    shape, qs, perm = {
+        'first': ((4, 4, n), (0, 1), (0, 1, 2)),
+        'last': ((4, 4, n), (1, 2), (2, 0, 1)),
+        'around': ((4, 4, n), (0, 2), (0, 2, 1))}[place]
+    x, g = (t.reshape(shape).permute(perm).contiguous().cuda()
+            for t in (x, g))
+    got = torch.ops.qsgb.ptm_grad(x, g, list(qs)).cpu().numpy().reshape(16, 16)
+    excess = float(np.max(np.abs(got - ref) - 2.0 ** -40 * mag))
+    assert excess <= n * 2.0 ** -149

@@ -78,6 +78,7 @@ struct ApplyParams {
   int arith;
   int max_terms;
   int iw;             // item warps per tile (tile = 32*iw items)
+  int only_marked;    // nothing to do unless `out` holds the mark of a PTM with holes (tc::mark_holes)
   uint64_t n_items;   // groups, or group pairs
   FastDiv div_z, div_y;  // Z (or Z/2 for pairs), Y
   int64_t sxi, syi, sai, sbi;  // input strides (z stride 1)
@@ -452,6 +453,14 @@ __global__ void __launch_bounds__(kBlock) apply_ptm_kernel(const __grid_constant
   constexpr int NL = PAIR ? 2 : 1;
   extern __shared__ __align__(16) unsigned char smem[];
   pdl_wait();
+  if (p.only_marked) {
+    // the first row of this block's first group, which no other block writes
+    const uint64_t it = (uint64_t)blockIdx.x * 32 * p.iw;
+    const uint64_t t1 = fdiv(it, p.div_z);
+    const uint64_t x = fdiv(t1, p.div_y);
+    const int64_t bo = (int64_t)x * p.sxo + (int64_t)(t1 - x * p.div_y.d) * p.syo + (int64_t)(it - t1 * p.div_z.d) * NL;
+    if (!tc::holes_marked(static_cast<const T*>(p.out) + bo)) return;
+  }
   if (!build_terms<T>(p, L, smem)) return;
 
   V* xs = reinterpret_cast<V*>(smem + L.xs_off);
@@ -1060,6 +1069,7 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
   p.sao = Y * db_out * Z;
   p.sxo = da_out * Y * db_out * Z;
   p.status = status;
+  p.only_marked = 0;
   const size_t esz = dtype == QSGB_F64 ? 8 : 4;
   const bool pair = (Z % 2 == 0) && ((uintptr_t)in % (2 * esz) == 0) && ((uintptr_t)out % (2 * esz) == 0);
   p.div_y = make_fastdiv((uint64_t)Y);
@@ -1089,16 +1099,36 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
   // 1. kernel specialised to the PTM's sparsity pattern (host PTMs)
   const int js = try_jit(ptm, da_out, db_out, da_in, db_in, Z, flags, dtype, arith, pair, p, s, mode, src_out);
   if (js != QSGB_ERR_UNSUPPORTED || mode != kLaunch) return js;
+  auto generic = [&]() {
+    if (pair) {
+      const int st = dtype == QSGB_F32 ? launch_apply<float, true>(p, s) : launch_apply<double, true>(p, s);
+      if (st != QSGB_ERR_UNSUPPORTED) return st;
+      // pairs do not fit in shared memory: single groups
+      p.iw = pick_iw((int)kout);
+      p.div_z = make_fastdiv((uint64_t)Z);
+      p.n_items = (uint64_t)X * Y * Z;
+    }
+    return dtype == QSGB_F32 ? launch_apply<float, false>(p, s) : launch_apply<double, false>(p, s);
+  };
   // 1b. dense PTMs larger than 16 x 16: the tensor cores.  Host PTMs come
   // here as a device copy with their term count (more than the specialised
-  // kernels take, 12 terms per row at 81 x 81); a device PTM's values are not
-  // read on the host, so it counts all its entries, as 16 x 16 ones do above.
+  // kernels take, 12 terms per row at 81 x 81); one with zeros stays with the
+  // generic kernel.  A device PTM's values are not read on the host, so it
+  // counts all its entries, as 16 x 16 ones do above; the generic kernel is
+  // launched behind and works if the PTM has holes (qsgb_tcw.cu says why and
+  // what they are; 2 to 3 us where it does not).  It holds the terms of every
+  // size up to kWideMax.
   // Measured on GB300, dense 81 x 81 on 7 qutrits (38 MB): 1210 us in the
   // generic kernel, 84 us here, with 1/60 of its error.
-  if (!(flags & (QSGB_PTM_HOST | QSGB_PTM_NOJIT)) && p.max_terms > jit::kMaxJitTerms && kin <= tc::kWideMax &&
-      kout <= tc::kWideMax && (arith == QSGB_ARITH_AUTO || arith == QSGB_ARITH_F32) && tc_device_auto())
-    return tc::launch_wide(ptm, flags & 3, in, out, dtype, (int)da_out, (int)db_out, (int)da_in, (int)db_in,
-                           (uint64_t)X, (uint64_t)Y, (uint64_t)Z, status, s);
+  if (!(flags & (QSGB_PTM_HOST | QSGB_PTM_NOJIT)) && kin * kout > jit::kMaxJitTerms && p.max_terms == kin * kout &&
+      kin <= tc::kWideMax && kout <= tc::kWideMax && (arith == QSGB_ARITH_AUTO || arith == QSGB_ARITH_F32) &&
+      tc_device_auto()) {
+    const int st = tc::launch_wide(ptm, flags & 3, in, out, dtype, (int)da_out, (int)db_out, (int)da_in, (int)db_in,
+                                   (uint64_t)X, (uint64_t)Y, (uint64_t)Z, status, s);
+    if (st != QSGB_OK) return st;
+    p.only_marked = 1;
+    return generic();
+  }
   // 2a. small device PTMs, no term limit: the dense kernel (FP32 storage up
   // to 16 x 16; FP64 storage for one-qubit PTMs on small vectors)
   if (!(flags & QSGB_PTM_HOST) && p.max_terms == kin * kout) {
@@ -1137,15 +1167,7 @@ int apply_common(const void* in, void* out, const double* ptm, int64_t da_out, i
     p.max_terms = std::max(1, n);
     p.ptm = nullptr;
   }
-  if (pair) {
-    const int st = dtype == QSGB_F32 ? launch_apply<float, true>(p, s) : launch_apply<double, true>(p, s);
-    if (st != QSGB_ERR_UNSUPPORTED) return st;
-    // pairs do not fit in shared memory: single groups
-    p.iw = pick_iw((int)kout);
-    p.div_z = make_fastdiv((uint64_t)Z);
-    p.n_items = (uint64_t)X * Y * Z;
-  }
-  return dtype == QSGB_F32 ? launch_apply<float, false>(p, s) : launch_apply<double, false>(p, s);
+  return generic();
 }
 
 }  // namespace

@@ -211,10 +211,25 @@ int launch_device(const double* dptm, int layout, const void* in, void* out, uin
                   unsigned* status, cudaStream_t stream);
 
 // Larger dense PTMs (Kin, Kout <= kWideMax) in device memory, FP64 or FP32
-// vectors (qsgb_tcw.cu); dimensions and strides as for launch_device.
+// vectors (qsgb_tcw.cu); dimensions and strides as for launch_device.  A PTM
+// with holes is not applied: `out` is marked for the generic kernel, which has
+// to be launched behind (ApplyParams::only_marked).
 constexpr int kWideMax = 96;
 int launch_wide(const double* dptm, int layout, const void* in, void* out, int dtype, int da_out, int db_out,
                 int da_in, int db_in, uint64_t X, uint64_t Y, uint64_t Z, unsigned* status, cudaStream_t stream);
+
+// The mark is a nan that no arithmetic gives, in the first row of every group.
+// (A state that holds this very nan would at worst be computed twice.)
+__device__ __forceinline__ void mark_holes(double* o) {
+  *reinterpret_cast<unsigned long long*>(o) = 0xfff8dead0badf00dull;
+}
+__device__ __forceinline__ void mark_holes(float* o) { *reinterpret_cast<unsigned*>(o) = 0xffc0deadu; }
+__device__ __forceinline__ bool holes_marked(const double* o) {
+  return *reinterpret_cast<const volatile unsigned long long*>(o) == 0xfff8dead0badf00dull;
+}
+__device__ __forceinline__ bool holes_marked(const float* o) {
+  return *reinterpret_cast<const volatile unsigned*>(o) == 0xffc0deadu;
+}
 
 }  // namespace tc
 }  // namespace qsgb

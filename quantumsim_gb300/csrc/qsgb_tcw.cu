@@ -9,24 +9,31 @@
 // 2012):
 //
 //  * Each group's inputs and each PTM row are scaled by their largest binary
-//    exponent and written as fixed-point integers in PL balanced byte digits,
-//    exact FP16 numbers: PL = 7 (55 bits) for FP64 storage, PL = 5 (39 bits)
-//    for FP32.  A product of two digits is at most 2^14 and a K = 96 sum at
-//    most 2^20.6, so a level (all digit pairs i + j = L, L < LV = PL + 1; at
-//    most seven pairs) stays below 2^24, where FP32 sums of integers are exact.
+//    exponent and written as 55-bit fixed-point integers in seven balanced
+//    byte digits, exact FP16 numbers.  A product of two digits is at most 2^14
+//    and a K = 96 sum at most 2^20.6, so a level (all digit pairs i + j = L < 8;
+//    at most seven pairs) stays below 2^24, where FP32 sums of integers are
+//    exact.
 //  * Levels pair up in 32-bit integers, are combined in int64 and rounded to
 //    the storage type once.  Truncation and the dropped levels bound the error
-//    by about 2^-47 max_k |P_rk| max_k |x_k| for FP64 at K = 81 (typically
-//    2^-53 of that product); for FP32 it is far below one rounding.
+//    by about 2^-47 max_k |P_rk| max_k |x_k| at K = 81 (typically 2^-53 of that
+//    product; for FP32 vectors far below one rounding).
+//  * That bound says little about a row that leaves out the group's largest
+//    components.  So a PTM with holes (a zero, or an entry below 2^-24 of its
+//    row's largest, in a row that is not all zero) is left to the generic
+//    kernel, whose rows keep every term's precision: this one, which has the
+//    PTM's exponents at hand, then only marks the output, and the generic
+//    kernel, always launched behind it, works if it finds the mark.  Without
+//    holes every row has a share of its group's largest product.
 //  * Groups that hold inf or nan, or whose scales leave the range where every
-//    result is a normal number, are recomputed in the storage type's plain
-//    arithmetic by their own threads.
+//    result is a normal number, are recomputed, too: in the storage type's
+//    plain arithmetic by their own threads.
 //
 // Work split: one block of 512 threads per SM takes tiles of 128 groups (the M
 // of one MMA); four threads share a group, a quarter of the inputs and of each
 // half of the outputs each.  All digit planes of the inputs do not fit shared
 // memory beside those of the PTM, so the input planes, the A operand, live in
-// tensor memory: PL x 48 columns, plus three accumulator buffers of 48 columns
+// tensor memory: 7 x 48 columns, plus three accumulator buffers of 48 columns
 // (336 + 144 of the 512).  The outputs are computed in two halves of up to 48
 // rows; a group of three levels at a time is accumulated, one buffer each, with
 // the MMAs of the three interleaved; while the threads add a group to their
@@ -36,8 +43,12 @@
 // is not adjacent to its neighbour's; the tile then goes through shared memory
 // both ways, copied in runs of consecutive elements.
 //
-// Measured on GB300, dense 81 x 81 on 7 qutrits (461 tiles, 38 MB): 84 us a
-// pass against 1210 us in the generic kernel, with 1/60 of its error.  A first
+// Measured on GB300, dense 81 x 81 on 7 qutrits (461 tiles, 38 MB), in a graph:
+// 76 us a pass (2.5 of them the generic kernel that finds no mark), 106 on the
+// last two qutrits, against 1200 us in the generic kernel, with 1/60 of its
+// error; FP32 vectors 74 us against 227 (with five planes, 39 bits, it was 56:
+// but FP32 inputs below 2^-15 of the largest kept fewer bits than they have).
+// With zeros in the PTM 977 us, as much as the generic kernel alone.  A first
 // form of this kernel (base-512 digits, six levels of N = 96 one after another,
 // 256 threads) took 140 us; this one with a level per commit 113 us, and 162 us
 // with its MMAs issued by one thread from rolled loops.  What bounds it now:
@@ -96,48 +107,25 @@ constexpr int kWOffB = (kWOffGout + 8 * kWGroups + 127) / 128 * 128;
 
 __device__ __forceinline__ unsigned exp_of(double v) { return ((unsigned)__double2hiint(v) >> 20) & 0x7ffu; }
 __device__ __forceinline__ unsigned exp_of(float v) { return (__float_as_uint(v) >> 23) & 0xffu; }
+// a row whose largest entry has biased exponent e has one of exponent `least`
+// (zeros and subnormals count 0) that is a hole; inf and nan beside others
+// make holes of those
+__device__ __forceinline__ bool hole(unsigned least, unsigned e) { return least + 24u < e; }
 __device__ __forceinline__ unsigned sign_word(double v) { return (unsigned)__double2hiint(v); }
 __device__ __forceinline__ unsigned sign_word(float v) { return __float_as_uint(v); }
 
-// |F| + B against the block exponent e (in place: exponent field): F has
-// 8 PL - 1 bits; exponent-0 values (zero, subnormals) give 0 when the block's
-// exponent is kMinExp or more (FP64) or 40 or more (FP32)
-template <int PL>
+// |F| + B against the block exponent e: F has 55 bits; exponent-0 values (zero,
+// subnormals) give 0 when the block's exponent is kMinX or more
 __device__ __forceinline__ unsigned long long fixed_bytes(double v, unsigned e) {
-  constexpr unsigned long long kBias = 0x8080808080808080ull >> (8 * (8 - PL));
-  const unsigned h = (unsigned)__double2hiint(v);
-  const unsigned long long m = (unsigned long long)((h & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(v);
-  constexpr int up = 8 * PL - 1 - 53;
-  const unsigned s = e - ((h >> 20) & 0x7ffu) + (up < 0 ? (unsigned)-up : 0u);
-  unsigned long long f;
-  asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(up > 0 ? m << (up > 0 ? up : 0) : m), "r"(s));
-  return f + kBias;
+  return fixed8((unsigned)__double2hiint(v), (unsigned)__double2loint(v), e << 20);
 }
-template <int PL>
 __device__ __forceinline__ unsigned long long fixed_bytes(float v, unsigned e) {
-  constexpr unsigned long long kBias = 0x8080808080808080ull >> (8 * (8 - PL));
   const unsigned b = __float_as_uint(v);
-  const unsigned long long m = (unsigned long long)((b & 0x7fffffu) | 0x800000u) << (8 * PL - 1 - 24);
+  const unsigned long long m = (unsigned long long)((b & 0x7fffffu) | 0x800000u) << (55 - 24);
   unsigned long long f;
   asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(m), "r"(e - ((b >> 23) & 0xffu)));
-  return f + kBias;
+  return f + kBias8;
 }
-// digit J (0 the most significant) of two values as signed FP16x2 (digit8_pair
-// for PL planes)
-template <int PL, int J>
-__device__ __forceinline__ unsigned digit_bytes(unsigned long long ua, unsigned long long ub, const Signs& s) {
-  constexpr int byte = PL - 1 - J, b4 = byte & 3;
-  const unsigned a = (unsigned)(byte >= 4 ? ua >> 32 : ua), b = (unsigned)(byte >= 4 ? ub >> 32 : ub);
-  unsigned r;
-  if (J == 0)  // the top digit with its carry bit: 16 bits
-    r = __byte_perm(a, b, (unsigned)(b4 | ((b4 + 1) << 4) | ((b4 + 4) << 8) | ((b4 + 5) << 12))) | 0x64006400u;
-  else
-    r = (__byte_perm(a, b, (unsigned)(b4 | ((b4 + 4) << 8))) & 0x00ff00ffu) | 0x64006400u;
-  unsigned out;
-  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(out) : "r"(r), "r"(s.one), "r"(s.bias));
-  return out;
-}
-
 // shared-memory matrix descriptor of a K-major plane without swizzling whose
 // 8-column (K) slabs of `rows` rows x 16 bytes follow one another: leading (K)
 // byte offset 16 rows, stride (8 rows) 128
@@ -158,24 +146,35 @@ __device__ __forceinline__ void tmem_ld4(uint32_t addr, float (&r)[4]) {
 }
 
 // the digits of 8 inputs: 4 columns of every input plane (stride `plane`)
-template <int PL, int J>
+template <int J = 0>
 __device__ __forceinline__ void store_planes(uint32_t addr, uint32_t plane, const unsigned long long (&u)[8],
                                              const Signs (&s)[4]) {
-  if constexpr (J < PL) {
-    const unsigned w[4] = {digit_bytes<PL, J>(u[0], u[1], s[0]), digit_bytes<PL, J>(u[2], u[3], s[1]),
-                           digit_bytes<PL, J>(u[4], u[5], s[2]), digit_bytes<PL, J>(u[6], u[7], s[3])};
+  if constexpr (J < kPlanes) {
+    const unsigned w[4] = {digit8_pair<J>(u[0], u[1], s[0]), digit8_pair<J>(u[2], u[3], s[1]),
+                           digit8_pair<J>(u[4], u[5], s[2]), digit8_pair<J>(u[6], u[7], s[3])};
     tmem_st4(addr, w);
-    store_planes<PL, J + 1>(addr + plane, plane, u, s);
+    store_planes<J + 1>(addr + plane, plane, u, s);
   }
 }
-template <int PL, int J>
+template <int J = 0>
 __device__ __forceinline__ void store_ptm_planes(unsigned char* dst, int plane, const unsigned long long (&u)[8],
                                                  const Signs (&s)[4]) {
-  if constexpr (J < PL) {
+  if constexpr (J < kPlanes) {
     *reinterpret_cast<uint4*>(dst) =
-        make_uint4(digit_bytes<PL, J>(u[0], u[1], s[0]), digit_bytes<PL, J>(u[2], u[3], s[1]),
-                   digit_bytes<PL, J>(u[4], u[5], s[2]), digit_bytes<PL, J>(u[6], u[7], s[3]));
-    store_ptm_planes<PL, J + 1>(dst + plane, plane, u, s);
+        make_uint4(digit8_pair<J>(u[0], u[1], s[0]), digit8_pair<J>(u[2], u[3], s[1]),
+                   digit8_pair<J>(u[4], u[5], s[2]), digit8_pair<J>(u[6], u[7], s[3]));
+    store_ptm_planes<J + 1>(dst + plane, plane, u, s);
+  }
+}
+
+// The mark of a PTM with holes
+template <typename T>
+__device__ void mark_all(const WideParams& p) {
+  for (uint64_t g = (uint64_t)blockIdx.x * kWBlock + threadIdx.x; g < p.n_groups; g += (uint64_t)gridDim.x * kWBlock) {
+    const uint64_t t1 = fdiv(g, p.div_z);
+    const uint64_t x = fdiv(t1, p.div_y);
+    mark_holes(static_cast<T*>(p.out) + (int64_t)x * p.sxo + (int64_t)(t1 - x * p.div_y.d) * p.syo +
+               (int64_t)(g - t1 * p.div_z.d));
   }
 }
 
@@ -183,9 +182,9 @@ __device__ __forceinline__ void store_ptm_planes(unsigned char* dst, int plane, 
 template <typename T, int KQ>
 __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_constant__ WideParams p) {
   constexpr bool F64 = sizeof(T) == 8;
-  constexpr int PL = F64 ? 7 : 5, LV = PL + 1;
+  constexpr int PL = kPlanes, LV = kLevels;
   constexpr unsigned kExpAll = F64 ? 0x7ffu : 0xffu;
-  constexpr unsigned kMinX = F64 ? kMinExp : 40u;  // least block exponent of the inputs
+  constexpr unsigned kMinX = F64 ? kMinExp : 56u;  // least block exponent of the inputs
   constexpr int kPlaneCols = 2 * KQ;         // tensor-memory columns of an input plane
   constexpr int kDCol = PL * kPlaneCols;     // first accumulator column
   static_assert(kDCol + kWBufs * 48 <= 512, "tensor memory");
@@ -255,20 +254,25 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
 
   // ---- the PTM's digit planes (the B operand), once per block
   int ptm_bad = 0;
+  int holes = 0;
   for (int r = warp; r < npad; r += kWWarps) {
-    unsigned e = 0u, nz = 0u;
+    unsigned e = 0u, nz = 0u, least = 0x7ffu;
     if (r < p.kout) {
       const int ro = prow[r];
       for (int k = t & 31; k < p.kin; k += 32) {
         const double v = p.ptm[ro + pcol[k]];
-        e = max(e, exp_of(v));
+        const unsigned ev = exp_of(v);
+        e = max(e, ev);
+        least = min(least, ev);
         nz |= v != 0.0 ? 1u : 0u;
       }
     }
     e = __reduce_max_sync(0xffffffffu, e);
     nz = __reduce_or_sync(0xffffffffu, nz);
+    least = __reduce_min_sync(0xffffffffu, least);
     // inf, nan, or a non-zero row below the smallest scale
     if (e == 0x7ffu || (e < kMinExp && nz)) ptm_bad = 1;
+    if (nz && hole(least, e)) holes = 1;
     if (e < kMinExp) e = 1023u;  // any scale serves a row of zeros
     if ((t & 31) == 0) srow[r] = (int)e;
   }
@@ -285,14 +289,15 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
     unsigned long long f[8];
     Signs s[4];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) f[q] = fixed_bytes<PL>(v[q], (unsigned)srow[r]);
+    for (int q = 0; q < 8; ++q) f[q] = fixed_bytes(v[q], (unsigned)srow[r]);
 #pragma unroll
     for (int q = 0; q < 4; ++q) s[q] = signs_of(sign_word(v[2 * q]), sign_word(v[2 * q + 1]));
-    store_ptm_planes<PL, 0>(smem + kWOffB + (kc * npad + r) * 16, plane_b, f, s);
+    store_ptm_planes(smem + kWOffB + (kc * npad + r) * 16, plane_b, f, s);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   ptm_bad = __syncthreads_or(ptm_bad);
+  holes = __syncthreads_or(holes);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   int rmin = srow[0], rmax = srow[0];  // row scales, least and greatest
   for (int r = 1; r < p.kout; ++r) {
@@ -392,7 +397,11 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
 
   constexpr int kGroups = (LV + kWBufs - 1) / kWBufs;  // of levels, per half
   uint32_t group = 0;  // groups issued so far
-  for (uint64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
+  // (the shuffle tells the compiler that the answer is the warp's: without it the
+  // MMAs' operands are not warp-uniform to it, 75 -> 97 us on 7 qutrits)
+  const bool leave = __shfl_sync(0xffffffffu, holes, 0) != 0;
+  if (leave) mark_all<T>(p);
+  for (uint64_t tile = leave ? p.n_tiles : blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
     const uint64_t gi = tile * kWGroups + gl;
     const bool live = gi < p.n_groups;
     int64_t bi = 0, bo = 0;
@@ -449,10 +458,10 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
           unsigned long long u[8];
           Signs s[4];
 #pragma unroll
-          for (int q = 0; q < 8; ++q) u[q] = fixed_bytes<PL>(x[8 * b + q], emax);
+          for (int q = 0; q < 8; ++q) u[q] = fixed_bytes(x[8 * b + q], emax);
 #pragma unroll
           for (int q = 0; q < 4; ++q) s[q] = signs_of(sign_word(x[8 * b + 2 * q]), sign_word(x[8 * b + 2 * q + 1]));
-          store_planes<PL, 0>(tlane + (uint32_t)((h * KQ + 8 * b) / 2), (uint32_t)kPlaneCols, u, s);
+          store_planes(tlane + (uint32_t)((h * KQ + 8 * b) / 2), (uint32_t)kPlaneCols, u, s);
         }
       }
     }
@@ -506,16 +515,10 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
               else
                 pr[j] = (L & 1) ? pr[j] + i : i << 8;
               // V = sum_L A_L 2^(top - 8 L)
-              if (F64) {
-                if (L == 1) v[j] = (long long)pr[j] << 34;
-                if (L == 3) v[j] += (long long)pr[j] * 262144ll;
-                if (L == 5) v[j] += (long long)pr[j] * 4ll;
-                if (L == 7) v[j] += (long long)pr[j];
-              } else {
-                if (L == 1) v[j] = (long long)pr[j] << 32;
-                if (L == 3) v[j] += (long long)pr[j] * 65536ll;
-                if (L == 5) v[j] += (long long)pr[j];
-              }
+              if (L == 1) v[j] = (long long)pr[j] << 34;
+              if (L == 3) v[j] += (long long)pr[j] * 262144ll;
+              if (L == 5) v[j] += (long long)pr[j] * 4ll;
+              if (L == 7) v[j] += (long long)pr[j];
             }
           }
         }
@@ -529,7 +532,7 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
           if constexpr (F64)
             y = scale8(v[j], (unsigned)((int)emax + srow[r] - kScale8) << 20);
           else
-            y = ldexpf(__ll2float_rn(v[j]), (int)emax + srow[r] - 1202);
+            y = ldexpf(__ll2float_rn(v[j]), (int)emax + srow[r] - (kScale8 - 1023 + 127));
           if (p.staged)
             stage[soff_out[r] + gl * dbo] = y;
           else if (live)
@@ -578,8 +581,7 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
 
 template <typename T, int KQ>
 int wide_launch(WideParams& p, cudaStream_t stream) {
-  constexpr int PL = sizeof(T) == 8 ? 7 : 5;
-  const int planes = PL * p.ksteps * 2 * 2 * p.nhalf * 16;
+  const int planes = kPlanes * p.ksteps * 2 * 2 * p.nhalf * 16;
   p.off_stage = kWOffB + planes;
   int smem = p.off_stage;
   if (p.staged) {

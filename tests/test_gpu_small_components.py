@@ -1,9 +1,11 @@
 """Components far below the largest of their group keep their own precision
-where no digit split is used: one-qubit device PTMs, gradients of FP32 vectors.
+where no digit split is used (one-qubit device PTMs, gradients of FP32 vectors)
+and where a PTM larger than 16 x 16 has zeros.
 
 Bounds are per component, against sums of magnitudes: native FP64 rows of four
 terms err by less than 2^-45 of sum |P| |x|, float-float ones by less than the
-repository's bound for FP64 rows; a float-float gradient of up to 2^11 groups by
+repository's bound for FP64 rows; FP32 rows of K terms by (K + 2) 2^-24 of it
+(entry and product roundings, K sums); a float-float gradient of up to 2^11 groups by
 2^-40 of sum |g| |x|, plus 2^-149 a product below the float range."""
 import numpy as np
 import pytest
@@ -77,3 +79,49 @@ def test_gradient_of_fp32_vectors(n, place, gap):
     got = torch.ops.qsgb.ptm_grad(x, g, list(qs)).cpu().numpy().reshape(16, 16)
     excess = float(np.max(np.abs(got - ref) - 2.0 ** -40 * mag))
     assert excess <= n * 2.0 ** -149
+
+
+SHAPES = [((9, 9), (0, 1)), ((9, 9, 9), (1, 2)), ((9, 9, 9, 4), (2, 0)),
+          ((9, 4, 9, 9, 4), (0, 3)), ((4, 9, 9), (0, 2))]
+
+
+def _with_one_large(shape, qs, small, rng):
+    """Values of size `small`; the first component of every group is 1."""
+    x = rng.uniform(0.5, 1.0, shape) * small
+    at = [slice(None)] * len(shape)
+    for q in qs:
+        at[q] = 0
+    x[tuple(at)] = 1.0
+    return x
+
+
+@pytest.mark.parametrize('shape,qs', SHAPES, ids=str)
+@pytest.mark.parametrize('small', [2.0 ** -18, 2.0 ** -30, 2.0 ** -60])
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float64])
+@pytest.mark.parametrize('where', ['host', 'device'])
+@pytest.mark.parametrize('hole', ['zero', 'small', None])
+def test_wide_ptm(shape, qs, small, dtype, where, hole):
+    """The large component enters one row alone, and the others see the small
+    ones; or it enters every row, which then has a share of it."""
+    rng = np.random.default_rng(len(shape))
+    x = _with_one_large(shape, qs, small, rng)
+    d = tuple(shape[q] for q in qs)
+    k = int(np.prod(d))
+    m = rng.uniform(0.5, 1.0, (k, k))
+    if hole is not None:  # FP32 rows leave out entries below 2^-30
+        m[1:, 0] = 0.0 if hole == 'zero' else \
+            2.0 ** -40 if dtype == torch.float64 else 2.0 ** -28
+    p = m.reshape(d + d)
+    xt = torch.from_numpy(x).cuda().to(dtype)
+    x = xt.cpu().numpy().astype(np.float64)
+    pt = torch.from_numpy(p)
+    arith = L.ARITH_AUTO if dtype == torch.float64 else L.ARITH_F32
+    got = torch.ops.qsgb.apply_ptm(xt, pt if where == 'host' else pt.cuda(),
+                                   list(qs), arith, 0, False)
+    if dtype == torch.float32:
+        eps = (k + 2) * 2.0 ** -24
+    elif hole is None:  # 81 terms of 9 * 2^-54 of the largest product, half of
+        eps = 2.0 ** -42  # which at least is in every sum
+    else:
+        eps = RTOL_F64
+    _bounded(got.cpu().numpy().astype(np.float64), x, p, qs, eps)

@@ -351,6 +351,7 @@ __global__ void __launch_bounds__(kUBlock) apply16_umma_kernel(const __grid_cons
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncthreads();  // this block has its tensor memory before a dependent's may ask for any
   pdl_wait();
   load_tile(tile, x, b, live);  // in flight during the split of the PTM
   int* srow = reinterpret_cast<int*>(smem + kSmemRowExp);

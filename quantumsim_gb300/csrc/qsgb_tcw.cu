@@ -249,8 +249,8 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty), "r"(kWWarps) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncthreads();  // this block has its tensor memory before a dependent's may ask for any
   pdl_wait();
-  __syncthreads();
 
   // ---- the PTM's digit planes (the B operand), once per block
   int ptm_bad = 0;

@@ -248,7 +248,7 @@ __device__ bool build_terms(const ApplyParams& p, const SmemLayout& L, unsigned 
   int* flag = reinterpret_cast<int*>(red + 33);
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int ne = p.kin * p.kout;
-  const double* __restrict__ src = p.ptm ? p.ptm : p.ptm_inline;
+  const double* src = p.ptm ? p.ptm : p.ptm_inline;
 
   double amax = 0.0;
   for (int i = tid; i < ne; i += nthr) {
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(kBlock) apply_ptm_kernel(const __grid_constant
   const int tile = 32 * p.iw;
   const int buf_len = p.kin * tile;  // V elements per buffer
   const uint64_t n_tiles = (p.n_items + tile - 1) / tile;
-  const V* __restrict__ in = static_cast<const V*>(p.in);
+  const V* in = static_cast<const V*>(p.in);
   V* __restrict__ out = static_cast<V*>(p.out);
 
   // loader role: thread -> (item of the tile, first input row)
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(kDenseBlock) apply_dense_kernel(const __grid_c
   const double thr = sizeof(T) == 4 ? amax * 0x1p-30 : (p.arith == QSGB_ARITH_F64 ? 0.0 : amax * 0x1p-52);
   if (t < ne) P[t] = fabs(v) > thr ? (T)v : (T)0;
   __syncthreads();
-  const T* __restrict__ X = static_cast<const T*>(p.in);
+  const T* X = static_cast<const T*>(p.in);
   T* __restrict__ Y = static_cast<T*>(p.out);
   for (uint64_t g = (uint64_t)blockIdx.x * kDenseBlock + t; g < p.n_items; g += (uint64_t)gridDim.x * kDenseBlock) {
     const uint64_t t1 = fdiv(g, p.div_z);

@@ -33,7 +33,12 @@ int allow_dynamic_smem(const void* func, int bytes);
 // finishes (programmatic dependent launch; also inside graph captures).  The
 // kernel must call pdl_wait() before it touches memory: that returns when the
 // predecessor is complete and its writes are visible, and since every kernel
-// here waits before it works, so is everything before the predecessor.
+// here waits before it works, so is everything before the predecessor.  What it
+// reads is written while it is already running: no pointer to const memory is
+// __restrict__ there, which would allow loads through the non-coherent path and
+// ahead of the wait (the run-time specialised kernels pass theirs through an
+// asm behind the wait).  Tensor memory is allocated, and the block has met at a
+// barrier, before pdl_wait() lets the next kernel start.
 int launch_pdl(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void** args,
                bool overlap = true);
 template <typename... Params, typename... Args>

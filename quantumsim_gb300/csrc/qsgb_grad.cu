@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(kGradBlock) grad_stage1(const __grid_constant_
   int64_t* offs = reinterpret_cast<int64_t*>(smem + p.off_offs);  // [kin + kout] row offsets
   double* fb = reinterpret_cast<double*>(smem + p.off_fb);        // [kGradBlock][MPT][16] FP64 tiles
   int* fb_any = reinterpret_cast<int*>(smem + p.off_flag);
-  const T* __restrict__ X = static_cast<const T*>(p.x);
-  const T* __restrict__ G = static_cast<const T*>(p.g);
+  const T* X = static_cast<const T*>(p.x);
+  const T* G = static_cast<const T*>(p.g);
   const int t = threadIdx.x;
   const int R = p.kin + p.kout;
 
@@ -382,8 +382,7 @@ struct Grad4Walk {
 
 // FULL: four input and four output elements
 template <typename T, bool FULL>
-__device__ __forceinline__ void grad4_load(T (&v)[8], const T* __restrict__ X, const T* __restrict__ G,
-                                           const GradParams& p, const Grad4Walk& w) {
+__device__ __forceinline__ void grad4_load(T (&v)[8], const T* X, const T* G, const GradParams& p, const Grad4Walk& w) {
   const T* x = X + w.x;
   const T* o = G + w.o;
 #pragma unroll
@@ -419,8 +418,8 @@ template <typename T, bool FULL>
 __global__ void __launch_bounds__(kGradBlock, 2) grad4_kernel(const __grid_constant__ GradParams p,
                                                               double* __restrict__ part) {
   __shared__ double sums[kGradBlock / 32][16];
-  const T* __restrict__ X = static_cast<const T*>(p.x);
-  const T* __restrict__ G = static_cast<const T*>(p.g);
+  const T* X = static_cast<const T*>(p.x);
+  const T* G = static_cast<const T*>(p.g);
   const int t = threadIdx.x, lane = t & 31;
   const uint64_t first = (uint64_t)blockIdx.x * kGradBlock + t, stride = (uint64_t)gridDim.x * kGradBlock;
   float s[16], c[16];
@@ -497,7 +496,7 @@ __global__ void __launch_bounds__(kGradBlock, 2) grad4_kernel(const __grid_const
 // out[e] = sum over blocks b of part[b][e]: kStage2Entries entries x
 // kStage2Slices block slices per thread block, slices added in order
 __global__ void __launch_bounds__(kStage2Entries* kStage2Slices)
-    grad_stage2(const double* __restrict__ part, int nblocks, int E, double* __restrict__ out) {
+    grad_stage2(const double* part, int nblocks, int E, double* __restrict__ out) {
   __shared__ double red[kStage2Slices][kStage2Entries + 1];
   const int el = threadIdx.x % kStage2Entries, sl = threadIdx.x / kStage2Entries;
   const int e = blockIdx.x * kStage2Entries + el;
@@ -589,8 +588,8 @@ __global__ void __launch_bounds__(kTcgBlock* H, 2 / H) grad16_tc_kernel(const __
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   TcgSmem<H>& sm = *reinterpret_cast<TcgSmem<H>*>(smem);
   TcgWarpSmem<H>& ws = sm.warp[w];
-  const double* __restrict__ X = static_cast<const double*>(p.x);
-  const double* __restrict__ G = static_cast<const double*>(p.g);
+  const double* X = static_cast<const double*>(p.x);
+  const double* G = static_cast<const double*>(p.g);
   const int h = lane >> 4, i = lane & 15;
   const int gid = lane >> 2, tig = lane & 3;
   if (threadIdx.x < 16) {

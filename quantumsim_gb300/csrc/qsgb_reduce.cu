@@ -52,7 +52,7 @@ __global__ void gather_kernel(const __grid_constant__ GatherParams p) {
   for (int i = threadIdx.x; i < p.idx_off[p.ndim]; i += blockDim.x) sidx[i] = p.idx[i];
   pdl_wait();
   __syncthreads();
-  const TI* __restrict__ in = static_cast<const TI*>(p.in);
+  const TI* in = static_cast<const TI*>(p.in);
   TO* __restrict__ out = static_cast<TO*>(p.out);
   for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < p.n_out;
        o += (uint64_t)gridDim.x * blockDim.x) {

@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
   int64_t* gin = reinterpret_cast<int64_t*>(smem + kWOffGin);
   int64_t* gout = reinterpret_cast<int64_t*>(smem + kWOffGout);
   T* stage = reinterpret_cast<T*>(smem + p.off_stage);
-  const T* __restrict__ in = static_cast<const T*>(p.in);
+  const T* in = static_cast<const T*>(p.in);
   T* __restrict__ out = static_cast<T*>(p.out);
   const int dbi = p.db_in | 1, dbo = p.db_out | 1;  // odd: staged rows without bank conflicts
   const int nhalf = p.nhalf, npad = 2 * nhalf;

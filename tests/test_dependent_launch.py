@@ -3,7 +3,9 @@
 
 * tensor memory is allocated, and the block has met at a barrier since, before
   the kernel lets its dependents start: else a dependent's block on the same SM
-  may take the columns that a block it waits for still needs."""
+  may take the columns that a block it waits for still needs;
+* what a kernel reads is not read-only while it runs (its predecessor may still
+  be writing it), so no pointer to const memory is __restrict__."""
 import glob
 import os
 import re
@@ -20,6 +22,8 @@ def kernels():
     for path in sorted(glob.glob(os.path.join(CSRC, '*.cu'))):
         with open(path) as f:
             text = re.sub(r'//[^\n]*', '', f.read())
+        if path.endswith('qsgb_jit.cu'):
+            continue  # text of generated kernels: below
         for m in re.finditer(r'__global__\s+void\b', text):
             b = text.index('{', m.end())
             depth, e = 1, b + 1
@@ -51,3 +55,33 @@ def test_tensor_memory_before_dependents(k):
         return
     alloc = before.rindex('tcgen05.alloc')  # before the wait
     assert '__syncthreads()' in before[alloc:]
+
+
+READ_ONLY = re.compile(r'const\s+[\w:]+\s*\*\s*(?:const\s+)?__restrict__')
+
+
+@pytest.mark.parametrize('k', DEPENDENT, ids=lambda k: k[1])
+def test_nothing_read_is_declared_read_only(k):
+    assert not READ_ONLY.search(k[2] + k[3])
+
+
+@pytest.mark.parametrize('path', sorted(glob.glob(os.path.join(CSRC, '*.cu'))),
+                         ids=os.path.basename)
+def test_nor_in_the_functions_they_call(path):
+    here = [k for k in kernels() if k[0] == os.path.basename(path)]
+    if not here or any(k not in DEPENDENT for k in here):
+        return  # files whose kernels are all launched so
+    with open(path) as f:
+        assert not READ_ONLY.search(re.sub(r'//[^\n]*', '', f.read()))
+
+
+def test_generated_kernels_pass_their_pointer_through_the_wait():
+    """They keep __restrict__ (loads move above stores) on a pointer that comes
+    out of an asm behind the wait."""
+    with open(os.path.join(CSRC, 'qsgb_jit.cu')) as f:
+        text = f.read()
+    waits = [m.end() for m in re.finditer(r'qsgb_pdl_wait\(\);', text)]
+    assert len(waits) == text.count('"extern \\"C\\" __global__') + 1 == 3
+    for w in waits:
+        assert text[w:].startswith(
+            '\\n  asm volatile(\\"\\" : \\"+l\\"(in));')

@@ -9,10 +9,14 @@
 #include "../../include/qsgb.h"
 #include "qsgb_device.cuh"
 
-#define QSGB_CUDA_TRY(expr)                               \
-  do {                                                    \
-    cudaError_t qsgb_e_ = (expr);                         \
-    if (qsgb_e_ != cudaSuccess) return QSGB_ERR_CUDA;     \
+// A failed call is reported here, once: its error is taken out of the runtime, or
+// the next launch_status() would report it again for a launch that was fine.
+#define QSGB_CUDA_TRY(expr)            \
+  do {                                 \
+    if ((expr) != cudaSuccess) {       \
+      cudaGetLastError();              \
+      return QSGB_ERR_CUDA;            \
+    }                                  \
   } while (0)
 
 namespace qsgb {

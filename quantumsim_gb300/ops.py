@@ -300,20 +300,24 @@ def _ptm_grad_launch(plan, x_in, g_out, out_ptr):
 
 
 _DIRECT_TYPES = (torch.Tensor, torch.nn.Parameter)
+_wrapped = torch._C._functorch.is_functorch_wrapped_tensor
 
 
 def direct(*tensors):
     """Whether kernels may be called on these tensors past the dispatcher:
     plain CUDA tensors of the two storage types without a lazy negation,
-    nothing to be recorded for a gradient, no dispatch mode, tracing or
-    compilation."""
+    nothing to be recorded for a gradient, no dispatch or function mode,
+    tracing or compilation, and no batch of them (a backward pass of batched
+    gradients: its tensors look plain but have no storage of their own)."""
     if torch.is_grad_enabled() or torch._C._len_torch_dispatch_stack() or \
+            torch._C._len_torch_function_stack() or \
             torch._C._get_tracing_state() is not None or \
             torch.compiler.is_compiling():
         return False
     for t in tensors:
         if type(t) not in _DIRECT_TYPES or not t.is_cuda or \
-                t.dtype not in (torch.float64, torch.float32) or t.is_neg():
+                t.dtype not in (torch.float64, torch.float32) or \
+                t.is_neg() or _wrapped(t) or not torch._C._has_storage(t):
             return False
     return True
 

@@ -18,6 +18,23 @@ def _ptm(k, seed):
         size=(4,) * (2 * k)))
 
 
+@pytest.mark.parametrize('qs', [(1,), (0, 2), (2, 0)])
+@pytest.mark.parametrize('where', ['cpu', 'cuda'])
+def test_batched_gradients(qs, where):
+    """is_grads_batched: the backward pass runs on a batch of gradients."""
+    x = torch.randn(4, 4, 4, dtype=torch.float64, device='cuda',
+                    requires_grad=True)
+    p = _ptm(len(qs), 1).to(where).requires_grad_(True)
+    y = qg.apply_ptm_diff(x, p, *qs)
+    gs = torch.randn(3, *y.shape, dtype=torch.float64, device='cuda')
+    got = torch.autograd.grad(y, (x, p), gs, is_grads_batched=True,
+                              retain_graph=True)
+    for i in range(3):
+        want = torch.autograd.grad(y, (x, p), gs[i], retain_graph=True)
+        for a, b in zip(got, want):
+            assert torch.equal(a[i], b)
+
+
 REFUSED = """
 import torch
 import quantumsim_gb300

@@ -362,8 +362,7 @@ class HostPtmGrad:
         _, self._shape, self._n, _, self._swap = plan
         b = bufs.get(index)
         if b is None or b[0].numel() < self._n:
-            host = torch.empty(max(self._n, 256), dtype=torch.float64,
-                               pin_memory=True)
+            host = pinned(max(self._n, 256))
             b = (host, host.numpy(), host.data_ptr(), torch.cuda.Event())
             bufs[index] = b
         _, self._host, out_ptr, self._done = b
@@ -551,6 +550,11 @@ _STATUS_PTR = {}
 _READ_BUF = threading.local()
 
 
+def pinned(n):
+    """n doubles of page-locked host memory (whatever the default device)."""
+    return torch.empty(n, dtype=torch.float64, device='cpu', pin_memory=True)
+
+
 def status_ptr(index):
     """Address of the device status word of CUDA device `index`."""
     p = _STATUS_PTR.get(index)
@@ -695,7 +699,7 @@ def _read_buffers(index, device):
         nscr = int(L.load().qsgb_diag_marginals_scratch_bytes())
         # the scratch's first 16 bytes (the kernel's block ticket) start at
         # zero and every call leaves them zero
-        host = torch.empty(80, dtype=torch.float64, pin_memory=True)
+        host = pinned(80)
         b = (torch.empty(80, dtype=torch.float64, device=device), host,
              torch.zeros(nscr, dtype=torch.uint8, device=device),
              host.numpy())
@@ -742,7 +746,7 @@ def diagonal_host(pv, plan_arrays):
     n = math.prod(n_out)
     if n > HOST_DIAG_MAX or not n_out:
         return None
-    host = torch.empty(n + 1, dtype=torch.float64, pin_memory=True)
+    host = pinned(n + 1)
     st = L.load().qsgb_gather_host(
         pv.data_ptr(), _dtype_code(pv), pv.dim(), shape_c, idx_off_c, idx_c,
         status_ptr(pv.device.index), host.data_ptr(), _stream_handle(pv))

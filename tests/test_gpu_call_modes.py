@@ -35,6 +35,34 @@ def test_batched_gradients(qs, where):
             assert torch.equal(a[i], b)
 
 
+def test_under_a_default_device():
+    """Page-locked buffers are made on the host whatever the default device."""
+    import threading
+    fails = []
+
+    def work():  # a new thread: its buffers are made here
+        try:
+            with torch.device('cuda'):
+                pv = qg.PauliVectorGB300([B.general(2)] * 3)
+                assert pv.diagonal()[0] == 1.0 and pv.trace() == 1.0
+                assert pv.exp_value('ZIZ') == 1.0
+                pv.apply_ptm(np.random.default_rng(0).normal(
+                    size=(4,) * 4), 0, 1)
+                x = pv.data.clone().requires_grad_(True)
+                p = _ptm(2, 2).cpu().requires_grad_(True)
+                y = qg.apply_ptm_diff(x, p, 0, 2)
+                gx, gp = torch.autograd.grad((y * y).sum(), (x, p))
+                assert not gp.is_cuda and gx.is_cuda
+        except Exception as e:  # handed to the test's thread
+            fails.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    if fails:
+        raise fails[0]
+
+
 REFUSED = """
 import torch
 import quantumsim_gb300

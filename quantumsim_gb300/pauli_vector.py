@@ -230,7 +230,9 @@ class PauliVectorGB300(_Base):
             if pv.dtype not in (torch.float16, torch.float32, torch.float64):
                 raise ValueError('`pv` must have floating point data type, '
                                  'got {}'.format(pv.dtype))
-            data = pv.to(device=self._device, dtype=tdtype).contiguous()
+            # (the kernels read its memory: no lazily negated view)
+            data = pv.to(device=self._device,
+                         dtype=tdtype).contiguous().resolve_neg()
         else:
             raise ValueError('`pv` should be a numpy array, a torch tensor or '
                              'None, got type `{}`'.format(type(pv)))

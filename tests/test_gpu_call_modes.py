@@ -63,6 +63,20 @@ def test_under_a_default_device():
         raise fails[0]
 
 
+def test_negated_vector():
+    """A vector given as a lazily negated view has the values of the view."""
+    t = torch.randn(4, 4, 4, dtype=torch.float64, device='cuda')
+    bases = [B.general(2)] * 3
+    a, b = (qg.PauliVectorGB300(bases, v) for v in (torch._neg_view(t), -t))
+    for _ in range(2):
+        np.testing.assert_array_equal(a.diagonal(), b.diagonal())
+        np.testing.assert_array_equal(a.to_pv(), b.to_pv())
+        assert a.exp_value('XZI') == b.exp_value('XZI')
+        assert a.trace() == b.trace()
+        for v in (a, b):
+            v.apply_ptm(_ptm(2, 3).numpy(), 0, 2)
+
+
 REFUSED = """
 import torch
 import quantumsim_gb300

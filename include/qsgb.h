@@ -173,9 +173,11 @@ int qsgb_gather(const void* in, void* out, int in_dtype, int out_dtype,
                 const int32_t* idx, void* stream);
 
 /*
- * The adjoint of qsgb_gather: out (of out_shape, out_dtype) is zeroed and
- * the FP64 value in[o] is added where the gather with the same index lists
- * reads entry o; entries with an index of -1 go nowhere.
+ * The adjoint of qsgb_gather: every element of out (of out_shape, out_dtype)
+ * gets the sum of the FP64 values in[o] whose entries o the gather with the
+ * same index lists reads from it (0 where it reads none; entries with an index
+ * of -1 go nowhere).  Where an axis names an index more than once the sums are
+ * formed in FP64, in ascending order of o, and rounded once.
  */
 int qsgb_scatter(const double* in, void* out, int out_dtype, int ndim,
                  const int64_t* out_shape, const int32_t* idx_off,

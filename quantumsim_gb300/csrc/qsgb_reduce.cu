@@ -72,9 +72,9 @@ __global__ void gather_kernel(const __grid_constant__ GatherParams p) {
   if (p.status_out && blockIdx.x == 0 && threadIdx.x == 0) *p.status_out = p.status ? (double)*p.status : 0.0;
 }
 
-// The adjoint: in[o] is added to the element of out (zeroed before) that the
-// gather reads for o; places with an index of -1 go nowhere.  One value meets
-// one element unless an axis names an index twice.
+// The adjoint where no axis names an index twice, as in every diagonal: in[o]
+// goes to the element of out (zeroed before) that the gather reads for o; places
+// with an index of -1 go nowhere.
 template <typename T>
 __global__ void scatter_kernel(const __grid_constant__ GatherParams p) {
   __shared__ int sidx[kMaxIdx];
@@ -94,7 +94,50 @@ __global__ void scatter_kernel(const __grid_constant__ GatherParams p) {
       none |= (j < 0);
       addr += (int64_t)(j < 0 ? 0 : j) * p.in_stride[a];
     }
-    if (!none) atomicAdd(out + addr, (T)in[o]);
+    if (!none) out[addr] = (T)in[o];
+  }
+}
+
+// The adjoint with repeated indices: every element of out collects the values
+// whose places name it, in ascending order, in FP64.  No speed is sought here: a
+// thread walks the index lists of its element.
+struct ScatterParams : GatherParams {
+  uint64_t n_tensor;
+  int64_t shape[kMaxDim];
+};
+
+template <typename T>
+__global__ void scatter_repeats_kernel(const __grid_constant__ ScatterParams p) {
+  const double* __restrict__ in = static_cast<const double*>(p.in);
+  T* __restrict__ out = static_cast<T*>(p.out);
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < p.n_tensor;
+       e += (uint64_t)gridDim.x * blockDim.x) {
+    int place[kMaxDim];  // of the present value, along every axis
+    // the first place from `from` on that names this element's index along a
+    auto next = [&](int a, int from) {
+      const int64_t k = (int64_t)(e / (uint64_t)p.in_stride[a]) % p.shape[a];
+      int i = p.idx_off[a] + from;
+      while (i < p.idx_off[a + 1] && p.idx[i] != k) ++i;
+      return i < p.idx_off[a + 1] ? i - p.idx_off[a] : -1;
+    };
+    bool some = true;
+    for (int a = 0; a < p.ndim && some; ++a) {
+      place[a] = next(a, 0);
+      some = place[a] >= 0;
+    }
+    double acc = 0.0;
+    while (some) {
+      uint64_t o = 0;
+      for (int a = 0; a < p.ndim; ++a) o = o * p.div[a].d + (uint64_t)place[a];
+      acc += in[o];
+      some = false;
+      for (int a = p.ndim - 1; a >= 0 && !some; --a) {
+        const int n = next(a, place[a] + 1);
+        some = n >= 0;
+        place[a] = some ? n : next(a, 0);
+      }
+    }
+    out[e] = (T)acc;
   }
 }
 
@@ -612,8 +655,25 @@ extern "C" int qsgb_scatter(const double* in, void* out, int out_dtype, int ndim
   const int st = gather_params(p, n_tensor, in, out, QSGB_F64, out_dtype, ndim, out_shape, idx_off, idx);
   if (st != QSGB_OK) return st;
   cudaStream_t s = as_stream(stream);
+  const unsigned block = 256;
+  bool repeats = false;
+  for (int a = 0; a < ndim; ++a)
+    for (int i = idx_off[a]; i < idx_off[a + 1]; ++i)
+      for (int j = idx_off[a]; j < i; ++j) repeats |= idx[i] >= 0 && idx[i] == idx[j];
+  if (repeats) {
+    ScatterParams r{};
+    static_cast<GatherParams&>(r) = p;
+    r.n_tensor = n_tensor;
+    for (int a = 0; a < ndim; ++a) r.shape[a] = out_shape[a];
+    const unsigned grid = grid_for(n_tensor, (int)block);
+    if (out_dtype == QSGB_F64)
+      scatter_repeats_kernel<double><<<grid, block, 0, s>>>(r);
+    else
+      scatter_repeats_kernel<float><<<grid, block, 0, s>>>(r);
+    return launch_status();
+  }
   QSGB_CUDA_TRY(cudaMemsetAsync(out, 0, n_tensor * (out_dtype == QSGB_F64 ? 8 : 4), s));
-  const unsigned block = 256, grid = grid_for(p.n_out, (int)block);
+  const unsigned grid = grid_for(p.n_out, (int)block);
   if (out_dtype == QSGB_F64)
     scatter_kernel<double><<<grid, block, 0, s>>>(p);
   else

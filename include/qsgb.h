@@ -271,9 +271,10 @@ int qsgb_marginals_noalloc(const double* diag, int ndim, const int64_t* shape,
  * and every earlier kernel's status bits.  With host_out != NULL the values
  * are in host_out, too, when the call returns: page-locked memory is written
  * by the kernel itself and watched by the host (no copy and no stream
- * synchronisation), other memory gets a copy and a synchronisation.  With
- * NULL the call returns at once, the results on the device.  Diagonals of at most 2^22 entries
- * and axes of at most 64 indices; larger ones return QSGB_ERR_UNSUPPORTED
+ * synchronisation: by then `out` and the scratch are complete for work on any
+ * stream, but the kernel may not have left this one yet), other memory gets a
+ * copy and a synchronisation.  With NULL the call returns at once, the results
+ * on the device.  Diagonals of at most 2^22 entries and axes of at most 64 indices; larger ones return QSGB_ERR_UNSUPPORTED
  * (use qsgb_gather and qsgb_marginals).  Without scratch (below) one block
  * does the whole reduction.
  * Replaces: cuda.py:347-384 (trace and meas_prob: multitake, then a host

@@ -309,6 +309,11 @@ constexpr int kDiagRedWarps = kDiagRedBlock / 32;
 // threads of the block call this; value(j) gives result j.
 template <typename F>
 __device__ __forceinline__ void store_results(double* out, double* host, const unsigned* status, int n_out, F value) {
+  double st = 0.0;
+  if (threadIdx.x == 0) {  // on the device before the flag, like all else (n_out >= 1: a fence follows)
+    if (status) st = (double)*(volatile const unsigned*)status;
+    if (out) out[n_out] = st;
+  }
   for (int j = threadIdx.x; j < n_out; j += blockDim.x) {
     const double v = value(j);
     if (out) out[j] = v;
@@ -318,11 +323,7 @@ __device__ __forceinline__ void store_results(double* out, double* host, const u
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const double st = status ? (double)*(volatile const unsigned*)status : 0.0;
-    if (out) out[n_out] = st;
-    if (host) *(volatile double*)(host + n_out) = st;
-  }
+  if (threadIdx.x == 0 && host) *(volatile double*)(host + n_out) = st;
 }
 
 // The diagonal index of an entry is cut in two; each half's address part comes

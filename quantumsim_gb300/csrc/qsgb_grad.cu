@@ -344,15 +344,17 @@ __global__ void __launch_bounds__(kGradBlock) grad_stage1(const __grid_constant_
 // to) eight values come straight into registers, the next group's while this
 // one is multiplied, and nothing is staged in shared memory or shared between
 // threads until the sums are complete.  The same float-float products and band
-// as in stage 1 above; a block that met a value outside the band does its
-// groups again in native FP64.  The warps' sums are scattered over their lanes
+// as in stage 1 above; a group with a value outside the band is multiplied in
+// native FP64, into sums of its thread in shared memory (12 qubits, us: none 69,
+// one value in 10^5 74, one in 1000 86, all 148; with the whole block's groups
+// done again 68, 191, 191, 192; the staged kernel 150, 167, 434, 523).  The warps' sums are scattered over their lanes
 // by exchanges (16 entries: 16 shuffles of a pair instead of 80) and the block's
 // added in warp order.  Bound by instruction issue (about 400 a group, 160 of
 // them the products) and the latency of one group ahead per thread; a ring of
 // asynchronous copies three groups ahead gave 4 % at 12 qubits and took 5 % at
 // 10.  A gradient with its second stage, against the staged kernel above: 10
-// qubits (2^18 groups) 19.5 -> 10.9 us, 11 qubits 46 -> 21, 12 qubits 147 -> 67
-// (4.0 TB/s); FP32 vectors of 12 qubits 132 -> 51.
+// qubits (2^18 groups) 19.8 -> 11.3 us, 11 qubits 47 -> 22, 12 qubits 150 -> 69
+// (3.9 TB/s); FP32 vectors of 12 qubits 132 -> 48.
 // A thread's walk over its groups: the place in the two tensors, moved by a
 // fixed number of groups at a time without a division.
 struct Grad4Walk {
@@ -418,6 +420,7 @@ template <typename T, bool FULL>
 __global__ void __launch_bounds__(kGradBlock, 2) grad4_kernel(const __grid_constant__ GradParams p,
                                                               double* __restrict__ part) {
   __shared__ double sums[kGradBlock / 32][16];
+  __shared__ double f64[16][kGradBlock];  // products of groups outside the band, a thread's own
   const T* X = static_cast<const T*>(p.x);
   const T* G = static_cast<const T*>(p.g);
   const int t = threadIdx.x, lane = t & 31;
@@ -425,15 +428,28 @@ __global__ void __launch_bounds__(kGradBlock, 2) grad4_kernel(const __grid_const
   float s[16], c[16];
 #pragma unroll
   for (int q = 0; q < 16; ++q) s[q] = c[q] = 0.0f;
-  unsigned bad = 0;
+  bool met = false;  // this thread has had such a group
   pdl_wait();
   T v[8];
   Grad4Walk walk(p, first, stride);
   if (first < p.n_groups) grad4_load<T, FULL>(v, X, G, p, walk);
   for (uint64_t g = first; g < p.n_groups; g += stride) {
     float h[8], l[8];
+    unsigned bad = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) split_band(v[k], h[k], l[k], bad);
+    if (bad) {  // this group in native FP64
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          double* f = &f64[4 * r + k][t];
+          *f = fma((double)v[4 + r], (double)v[k], met ? *f : 0.0);
+        }
+      met = true;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) h[k] = l[k] = 0.0f;
+    }
     if (g + stride < p.n_groups) {
       walk.step(p);
       grad4_load<T, FULL>(v, X, G, p, walk);
@@ -453,34 +469,20 @@ __global__ void __launch_bounds__(kGradBlock, 2) grad4_kernel(const __grid_const
         }
       }
   }
-  double d;  // entry lane / 2 of this warp
-  if (!__syncthreads_or((int)bad)) {
-    grad4_halve<8>(s, c, lane);
-    grad4_halve<4>(s, c, lane);
-    grad4_halve<2>(s, c, lane);
-    grad4_halve<1>(s, c, lane);
-    const float s2 = __shfl_xor_sync(0xffffffffu, s[0], 1), c2 = __shfl_xor_sync(0xffffffffu, c[0], 1);
-    df_add(s[0], c[0], s2, c2);
-    d = qsgb_df_to_double(s[0], c[0]);
-  } else {
-    double f[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) f[q] = 0.0;
-    Grad4Walk again(p, first, stride);
+  grad4_halve<8>(s, c, lane);
+  grad4_halve<4>(s, c, lane);
+  grad4_halve<2>(s, c, lane);
+  grad4_halve<1>(s, c, lane);
+  const float s2 = __shfl_xor_sync(0xffffffffu, s[0], 1), c2 = __shfl_xor_sync(0xffffffffu, c[0], 1);
+  df_add(s[0], c[0], s2, c2);
+  double d = qsgb_df_to_double(s[0], c[0]);  // entry lane / 2 of this warp
+  if (__any_sync(0xffffffffu, met)) {
 #pragma unroll 1
-    for (uint64_t g = first; g < p.n_groups; g += stride, again.step(p)) {
-      grad4_load<T, FULL>(v, X, G, p, again);
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) f[4 * r + k] = fma((double)v[4 + r], (double)v[k], f[4 * r + k]);
-    }
-    d = 0.0;
-#pragma unroll
     for (int q = 0; q < 16; ++q) {
+      double f = met ? f64[q][t] : 0.0;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) f[q] += __shfl_xor_sync(0xffffffffu, f[q], o);
-      if ((lane >> 1) == q) d = f[q];
+      for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+      if ((lane >> 1) == q) d += f;
     }
   }
   if ((lane & 1) == 0) sums[t >> 5][lane >> 1] = d;

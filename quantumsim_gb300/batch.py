@@ -330,11 +330,13 @@ def map_unit_gradients(g_one, g_two, c, a, b, chain_factors,
 
 # Adaptive split of a stage into items, in vector elements (build_program):
 # an item is a multiple of ADAPT_STEP, at most ADAPT_MAX unless a stage is so
-# large that it gives every block ADAPT_ROUNDS items anyway.  ADAPT_STEP is what
+# large that it gives every block ADAPT_ROUNDS items anyway, and a stage has no
+# more than ADAPT_ITEMS items per block beside the last of each entry.
+# ADAPT_STEP is what
 # a block takes between two folds of its FP32 gradient sums into FP64 (1024
 # groups of a two-qubit op, 4096 of a one-qubit op), so these folds hold the
 # same products however a stage is split.
-ADAPT_STEP, ADAPT_MAX, ADAPT_ROUNDS = 16384, 65536, 6
+ADAPT_STEP, ADAPT_MAX, ADAPT_ROUNDS, ADAPT_ITEMS = 16384, 65536, 6, 12
 
 
 def adaptive_chunks(stage, total, width, grid):
@@ -350,6 +352,11 @@ def adaptive_chunks(stage, total, width, grid):
     ms here (90.6 with the present one); 7 circuits of up to 11
     qubits 14.0 and 4.2 ms; 14 of up to 8 qubits 7.9 and 4.7 ms.  (Items of 256
     groups would take these last two to 3.5 and 2.8 ms, with other FP32 sums.)
+
+    Every ADJOINT item keeps a 2 KB dP partial until the end of the step, so the
+    items of a stage are bounded by the device's blocks however many instances
+    there are: 30 layers of 512 circuits of 10 qubits keep 1.15 GB of partials
+    (1.20 at the fixed 8192 groups, 9.2 with each op cut in 64).
     """
     n_stages = int(stage.max()) + 1
     elems = np.bincount(stage, weights=(total * width).astype(float),
@@ -358,6 +365,7 @@ def adaptive_chunks(stage, total, width, grid):
                      elems / (ADAPT_ROUNDS * grid))
     # smaller instances in finer items, which fill the gaps at the end
     per = np.minimum(per[stage], total * width / 64)
+    per = np.maximum(per, (elems / (ADAPT_ITEMS * grid))[stage])
     per = np.maximum(np.ceil(per / ADAPT_STEP), 1).astype(np.int64)
     return per * ADAPT_STEP // width
 
@@ -577,8 +585,9 @@ class BatchedSimulator:
         APPLY of a unit reads and writes the state (8 N), ADJOINT reads x_out
         and g_out and writes x_in and g_in (16 N), SAVE and RESTORE copy it
         (8 N each), INIT and ZERO_G write it (4 N each), LOSS reads the 2^n
-        diagonal entries.  PTMs, dP partials and their sums are
-        negligible."""
+        diagonal entries.  PTMs, dP partials and their sums (written and read
+        once, at most 12 partials of 2 KB per block and ADJOINT stage) are
+        below 1 % of it for vectors larger than L2."""
         total = 0
         for i, s in enumerate(self.specs):
             n_units = len(self.units[i])

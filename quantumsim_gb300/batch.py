@@ -356,7 +356,10 @@ def adaptive_chunks(stage, total, width, grid):
     Every ADJOINT item keeps a 2 KB dP partial until the end of the step, so the
     items of a stage are bounded by the device's blocks however many instances
     there are: 30 layers of 512 circuits of 10 qubits keep 1.15 GB of partials
-    (1.20 at the fixed 8192 groups, 9.2 with each op cut in 64).
+    (1.20 at the fixed 8192 groups, 9.2 with each op cut in 64).  A step of 64 /
+    256 of them takes 52.9 / 188 ms (fixed 54.1 / 191, cut in 64 58.4 / 225), of
+    512 circuits of 4 to 12 qubits 1.086 s (1.068, 1.080), of 20 91.1 ms (125,
+    90.6).
     """
     n_stages = int(stage.max()) + 1
     elems = np.bincount(stage, weights=(total * width).astype(float),

@@ -541,7 +541,9 @@ class BatchedSimulator:
         if self.max_grid < 1:
             raise RuntimeError('batched kernel cannot be made resident')
         # 0: items sized per stage for the device (adaptive_chunks)
-        self.tile = tile or self._cached_tile() or 0
+        if tile is None:
+            tile = self._cached_tile()
+        self.tile = 0 if tile is None else tile
         self._build_program(self.tile)
         self.graph = None
 
@@ -769,9 +771,10 @@ class BatchedSimulator:
 
     # ------------------------------------------------------------ autotune
     def _cache_key(self):
+        # (v2: measured against the default split as well)
         sig = sorted(s.n for s in self.specs)
-        return '{}:{}:{}:{}'.format(len(sig), sum(4 ** n for n in sig),
-                                    self.max_grid, self.n_ptm)
+        return 'v2:{}:{}:{}:{}'.format(len(sig), sum(4 ** n for n in sig),
+                                       self.max_grid, self.n_ptm)
 
     @staticmethod
     def _cache_path():
@@ -786,9 +789,10 @@ class BatchedSimulator:
         except Exception:
             return None
 
-    def autotune(self, candidates=(2048, 4096, 8192, 16384, 32768), reps=2):
+    def autotune(self, candidates=(0, 2048, 4096, 8192, 16384, 32768),
+                 reps=2):
         """Time one step per tile size, keep the fastest; returns
-        {tile: ms}.  (0 stands for the default, items sized per stage.)"""
+        {tile: ms}.  0 stands for the default, items sized per stage."""
         times = {}
         for t in candidates:
             self._build_program(t)
@@ -884,7 +888,7 @@ def benchmark(n_instances=512, depth=30, q_min=4, q_max=12, seed=0,
     sim.target.copy_(sim.prob)
     targets = [t.clone() for t in sim.results()[0]]
     sim.set_ptms(ptms)
-    tuned = sim.autotune(candidates=(2048, 8192, 32768), reps=1) \
+    tuned = sim.autotune(candidates=(0, 2048, 8192, 32768), reps=1) \
         if autotune else None
     say('batched: {} stages, {} items, tile {}'.format(
         sim.n_stages, sim.n_items, sim.tile))

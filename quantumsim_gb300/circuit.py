@@ -51,6 +51,8 @@ import os
 import numpy as np
 import torch
 
+from . import ops
+
 # Measured application rates of the specialised FP64 kernels on GB300
 # (TB/s of the vector streamed in and out) against non-zero terms per PTM
 # row, per PTM size K (product of the qudits' Pauli dims); 14 qubits or 8
@@ -85,10 +87,10 @@ def terms_per_row(m):
     return float((a > amax * 2.0 ** -52).sum()) / max(1, m.shape[0])
 
 
-# PTMs with more non-zero terms than this are not specialised at run time
-# (the library's limit) and run on the slower generic kernel: never merge
-# into one.
-MAX_SPECIALISED_TERMS = 1024
+# PTMs with more non-zero terms than this are not specialised at run time (the
+# library's limit).  They run on the tensor cores when they have no zeros and on
+# the slower generic kernel else: never merge into one.
+MAX_SPECIALISED_TERMS = ops.MAX_JIT_TERMS
 
 
 # Two-qubit (16 x 16) PTMs with more than TC_MIN_TERMS non-zero terms per
@@ -663,7 +665,6 @@ class FusedCircuit:
         this only moves the work of the first application forward and
         spreads it over the cores."""
         from concurrent.futures import ThreadPoolExecutor
-        from . import ops
         jobs, shape = [], tuple(shape)
         for ptm, qudits in self.fused:
             jobs.append((shape, ptm, qudits))
@@ -706,7 +707,6 @@ class CircuitGraph:
     (eager) pass compiles every specialised kernel before capture."""
 
     def __init__(self, circuit, pv):
-        from . import ops
         self.circuit = circuit
         for ptm, qudits in circuit.fused:
             if ptm.shape[:len(qudits)] != ptm.shape[len(qudits):]:

@@ -237,7 +237,7 @@ class GraphedGradient:
 
     def __init__(self, model, target, dtype=torch.float64, checkpoint_every=8,
                  fuse=True, device=None):
-        from .autograd import Diagonal, diagonal_indices
+        from .autograd import Diagonal
         self.model = model
         self.dev = torch.device(device) if device is not None else \
             torch.device('cuda', torch.cuda.current_device())
@@ -247,8 +247,6 @@ class GraphedGradient:
         n = model.n
         self.target = target.to(self.dev, torch.float64)
         self.x0 = model.initial_state(self.dev, dtype)
-        self.flat = torch.from_numpy(
-            diagonal_indices([model.basis] * n)).to(self.dev)
         self.idx_off, self.idx_list = [0], []
         for _ in range(n):
             self.idx_list += [int(model.basis.computational_basis_indices[i])
@@ -310,7 +308,7 @@ class GraphedGradient:
                 return x
             fns.append(layer)
         x = checkpointed(fns, self.x0.clone(), self.every, keep_last=True)
-        prob = self._diag.apply(x, self.flat, self.idx_off, self.idx_list)
+        prob = self._diag.apply(x, None, self.idx_off, self.idx_list)
         t = self.target
         return torch.sum(t * (torch.log(t) - torch.log(prob)))
 

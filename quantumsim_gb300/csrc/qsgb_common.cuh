@@ -43,6 +43,8 @@ int allow_dynamic_smem(const void* func, int bytes);
 // ahead of the wait (the run-time specialised kernels pass theirs through an
 // asm behind the wait).  Tensor memory is allocated, and the block has met at a
 // barrier, before pdl_wait() lets the next kernel start.
+// Without `overlap`, and for grids that it would place badly (placed_well), the
+// launch is an ordinary one.
 int launch_pdl(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void** args,
                bool overlap = true);
 template <typename... Params, typename... Args>

@@ -1077,7 +1077,9 @@ int launch_blob(cudaKernel_t kern, const Spec& s, const Geometry& g, unsigned ch
   // 13-qubit FP32 layer (1674 -> 1631 us); on large FP64 vectors they gain
   // nothing on sparse PTMs (14-qubit layer 14.43 against 14.41 ms) and lose
   // 3.7 % on a circuit of float-float passes bound by instruction issue (13
-  // qubits, 9.63 -> 9.99 ms).
+  // qubits, 9.63 -> 9.99 ms).  Two layers in a graph, overlapped / not, us: 8
+  // qubits 45 / 49, 9 61 / 67, 11 323 / 335 (fused 155 / 160), 12 1574 / 1583
+  // (fused 698 / 692), 13 6540 / 6504; the line lies between 11 and 12.
   const uint64_t bytes = (uint64_t)g.n_items * (s.pair ? 2 : 1) * (uint64_t)(s.kin + s.kout) * (s.f32 ? 4 : 8);
   const bool overlap = s.f32 || bytes <= (64ull << 20);
   return launch_pdl((const void*)kern, grid, dim3(block), 0, stream, args, overlap);

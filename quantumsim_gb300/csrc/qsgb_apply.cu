@@ -839,8 +839,7 @@ int launch_apply(ApplyParams& p, cudaStream_t stream) {
     const int st = allow_dynamic_smem((const void*)kern, (int)L.total);
     if (st != QSGB_OK) return st;
   }
-  int occ = 0;
-  QSGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBlock, L.total));
+  const int occ = resident_blocks((const void*)kern, kBlock, L.total);
   if (occ < 1) return QSGB_ERR_UNSUPPORTED;
   const uint64_t tiles = (p.n_items + 32 * iw - 1) / (32 * iw);
   const uint64_t cap = (uint64_t)sm_count() * occ;

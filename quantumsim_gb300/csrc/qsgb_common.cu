@@ -46,8 +46,7 @@ int allow_dynamic_smem(const void* func, int bytes) {
   return QSGB_OK;
 }
 
-// Blocks of a kernel that an SM holds (0: unknown).
-static int resident_blocks(const void* func, int threads, size_t smem) {
+int resident_blocks(const void* func, int threads, size_t smem) {
   static std::mutex mu;
   static std::map<std::tuple<const void*, int, int, size_t>, int> known;
   int dev = 0, n = 0;

@@ -33,6 +33,10 @@ int launch_status();    // cudaGetLastError mapped to a status code
 // kernel ask for less.
 int allow_dynamic_smem(const void* func, int bytes);
 
+// Blocks of a kernel that an SM holds (0: unknown); asked once per kernel, block
+// and shared-memory size.
+int resident_blocks(const void* func, int threads, size_t smem);
+
 // Launch kernel `func` so that it may start while its predecessor on the stream
 // finishes (programmatic dependent launch; also inside graph captures).  The
 // kernel must call pdl_wait() before it touches memory: that returns when the

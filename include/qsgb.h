@@ -47,7 +47,25 @@ extern "C" {
 #define QSGB_F32 1
 
 /* ---- arithmetic of apply_ptm ---- */
-#define QSGB_ARITH_AUTO 0  /* F64 storage -> DF64; F32 storage -> F32 */
+#define QSGB_ARITH_AUTO 0  /* F32 storage -> F32, F64 storage -> rows in DF64
+                              or F64, whichever keeps up with memory: every
+                              term of a row keeps at least 47 bits of its own.
+                              Dense PTMs go to the tensor cores instead, where
+                              inputs and entries are cut to 55 bits below the
+                              largest of their group (the inputs of one
+                              output) and row; a result errs by less than
+                              2^-47 (16 x 16: 2^-49) of row maximum x group
+                              maximum, typically 2^-53, and components far
+                              below their group's largest keep fewer bits of
+                              their own than under DF64 or F64.  These are, on
+                              F64 vectors, 16 x 16 PTMs (on the host with more
+                              than 8 non-zero terms per row, on the device
+                              all), and on F64 and F32 vectors PTMs of more
+                              than 1024 entries, at most 96 x 96, without
+                              holes: no entry is zero or below 2^-24 of its
+                              row's largest, so that every row has a share of
+                              the largest product.  Where every component's
+                              own precision counts, choose DF64 or F64 */
 #define QSGB_ARITH_DF64 1  /* float-float (48-bit significand) on the FP32
                               pipes; single-term rows use one FP64 multiply */
 #define QSGB_ARITH_F64 2   /* native FP64 FMA (exact IEEE, slow on GB300) */
@@ -55,9 +73,7 @@ extern "C" {
 #define QSGB_ARITH_TC 4    /* F64 storage: every dense-shaped 16 x 16 host
                               PTM (two full-basis qubits) on the tensor
                               cores (FP64 values split into FP16 digit
-                              planes, exact FP32 sums); other PTMs as AUTO.
-                              AUTO itself sends 16 x 16 host PTMs with more
-                              than 8 non-zero terms per row there */
+                              planes, exact FP32 sums); other PTMs as AUTO */
 
 /* ---- PTM layout flags ---- */
 #define QSGB_PTM_SWAPPED 1    /* 2-qudit PTM given in order (less significant,

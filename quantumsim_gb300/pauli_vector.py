@@ -23,11 +23,14 @@ Numerical semantics follow ``PauliVectorNumpy`` (the reference oracle):
 FP64 storage: by default (``arith='auto'``) the kernel computes each PTM
 row either with native FP64 FMAs or in float-float arithmetic (48-bit
 significand) on the FP32 pipes, whichever keeps the launch closest to the
-HBM bound, and sends dense 16 x 16 PTMs (more than 8 non-zero terms per
-row) to the tensor cores, where FP64 values split into FP16 digit planes
-are multiplied with exact FP32 sums; ``arith='f64'`` forces native FP64
+HBM bound, and sends dense PTMs (16 x 16 with more than 8 non-zero terms per
+row; larger ones without zeros) to the tensor cores, where FP64 values split
+into FP16 digit planes are multiplied with exact FP32 sums.  The digits are cut
+at 55 bits below the largest input of a group, so components far below it keep
+fewer bits of their own there.  ``arith='f64'`` forces native FP64
 everywhere, ``arith='df64'`` float-float for every row with more than one
-term, and ``arith='tc'`` the tensor cores for every 16 x 16 PTM.
+term (both keep every component's own precision), and ``arith='tc'`` the
+tensor cores for every 16 x 16 PTM.
 ``dtype=np.float32`` stores the vector in FP32 while every trace, marginal
 and partial-trace sum still accumulates in FP64.
 """
@@ -173,8 +176,8 @@ class PauliVectorGB300(_Base):
         CUDA device (default: the current one).
     arith : 'auto' | 'df64' | 'f64' | 'f32' | 'tc'
         Arithmetic of apply_ptm ('auto': per PTM, the specialised
-        float-float / FP64 kernels, or the tensor cores for 16 x 16 PTMs
-        with more than 8 terms per row; 'tc': every 16 x 16 PTM on the
+        float-float / FP64 kernels, or the tensor cores for dense PTMs, see
+        above; 'tc': every 16 x 16 PTM on the
         tensor cores; f32 for FP32 storage).
     """
 

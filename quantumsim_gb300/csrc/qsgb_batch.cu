@@ -463,11 +463,10 @@ __device__ __noinline__ void adjoint2_warp(float* __restrict__ x, float* __restr
     {
       // this warp's next tile into L2 while the current one is computed (the
       // loads are bound by their latency): lane l takes tensor l / 16 and, for
-      // Z >= 64, component l % 16 at the tile's first and last group (one
-      // 128-byte run each when the groups are consecutive along z); for
-      // Z == 1, line l % 4 of chunk row (l / 4) % 4 (the tile's 32 groups are
-      // 512 contiguous bytes per row).  Other strides are not prefetched.
-      // Addresses are those of groups inside the item.
+      // Z >= 16, component l % 16 at the tile's first and last group (one
+      // 128-byte run each when the groups are consecutive along z); for Z == 1
+      // and Z == 4, where a row of the tile's 32 groups is 512 contiguous bytes
+      // unless they change x, line l % 4 of chunk row (l / 4) % 4.  Addresses are those of groups inside the item.
       const int64_t tn = t0 + (int64_t)nwarps * 32;
       if (tn < end) {
         const float* base = (lane < 16) ? x : gv;

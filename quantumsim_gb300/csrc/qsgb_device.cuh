@@ -111,7 +111,10 @@ __device__ __forceinline__ void qsgb_df_mul(float& s, float& c, float ph, float 
 // one float->int conversion: as qsgb_df_to_double below without its range
 // selects.  The sign of r goes into the scale, so that the correction T is in
 // the magnitude's direction.  Where r is below 2^-76 and unflagged, s is 0
-// and the two-sum is exact (u = 0): the wrapped scale is finite and T is 0.
+// and the two-sum is exact (u = 0): T is 0 also where the scale wraps to an
+// infinity (an exponent field of 51 in r), for 0 * inf is a nan and a nan
+// converts to the integer 0.  A subnormal r (rows whose leading floats cancel
+// at 2^-102) comes out within 2^-126 of its value.
 __device__ __forceinline__ double qsgb_df_round(float s, float t) {
   const float r = s + t;  // two-sum: no ordering assumption on |s|, |t|
   const float bt = r - s;

@@ -927,7 +927,11 @@ bool make_spec(const double* ptm_host, int da_out, int db_out, int da_in, int db
 // Below a few warps per SM sub-partition a pass takes as long as one thread's
 // chain: load, split, every row of the item.  The rows then go to up to eight
 // threads, which read the inputs they need each (from L2: such vectors are
-// small).  Measured on GB300, us in a graph, one thread an item / split: 7
+// small).  A pattern used on vectors of several sizes is compiled once per
+// number of parts (and per arithmetic of small_in_fp64): a noisy CZ applied to 3 to
+// 13 qubits in turn three times, 254 ms in all, against 173 ms with one kernel; on
+// one size, and with the disk cache, there is no difference.  Measured on GB300,
+// us in a graph, one thread an item / split: 7
 // qubits, noisy CZ 2.8 / 1.65, 3.1 terms 2.6 / 2.0, 6.2 terms 3.4 / 2.1; 9
 // qubits 2.9 / 2.0, 2.6 / 2.7, 3.5 / 3.1.  With vector accesses along the last
 // qudit (Z == 1) the parts have 4 rows each and gain up to 8 qubits only.

@@ -122,7 +122,7 @@ def _raise_status(st, val):
         reasons = []
         if val & L.DEV_RANGE:
             reasons.append('a Pauli-vector entry or PTM result left the '
-                           'float-float range (|x| >= 2^128, inf or nan)')
+                           'float-float range (|x| >= 2^127, inf or nan)')
         if val & L.DEV_TIMEOUT:
             reasons.append('a bounded device-side wait timed out')
         if val & L.DEV_BADITEM:

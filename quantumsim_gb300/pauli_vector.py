@@ -434,8 +434,8 @@ class PauliVectorGB300(_Base):
         return torch.ops.qsgb.marginals(diag, [diag.numel()], -1)
 
     def _diag_reduce(self, axis):
-        """Trace (axis -1) or marginals of one qudit in one launch and one
-        device-to-host copy (ops.diag_marginals); None when the bases have no
+        """Trace (axis -1) or marginals of one qudit in one launch, which
+        writes them to the host (ops.diag_marginals); None when the bases have no
         gather plan or the diagonal is too large for the fused kernel."""
         arrays = _diag_arrays(self.bases, self._data.shape)
         if arrays is None:

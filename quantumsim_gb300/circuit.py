@@ -97,7 +97,8 @@ MAX_SPECIALISED_TERMS = ops.MAX_JIT_TERMS
 # row run on the tensor cores (the library's QSGB_TC_MIN_TERMS rule) at a
 # rate that does not depend on the density: the fused passes of the
 # 14-qubit circuit above 8 terms per row ran at 3.13 TB/s (75 passes, 3.07
-# to 3.22).
+# to 3.22; the kernel of today runs at 3.5 to 3.7, and the float-float rows
+# above are faster, too: the plans were measured with this table).
 TC_MIN_TERMS = 8.0
 TC_RATE = 3.13
 

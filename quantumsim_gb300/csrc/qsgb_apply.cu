@@ -877,7 +877,8 @@ void op_matrix(const double* ptm, int da_out, int db_out, int da_in, int db_in, 
 // tensor-core kernel streams 3.35-3.46 TB/s whatever the density (2.77 when
 // the less significant target is the last qubit); the specialised
 // float-float kernels 4.0 TB/s at 6.12 terms per row, 2.46 at 11.25 and
-// 1.39-1.65 when dense, which crosses 3.3 TB/s near 8 terms per row.
+// 1.39-1.65 when dense, which crosses 3.3 TB/s near 8 terms per row.  (Both have
+// become faster since: 3.5-3.7 and, dense, 1.9 TB/s.)
 bool tc_wanted(const double* op) {
   static const double min_terms = [] {
     const char* v = std::getenv("QSGB_TC_MIN_TERMS");

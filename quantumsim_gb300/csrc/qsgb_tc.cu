@@ -225,8 +225,8 @@ __global__ void __launch_bounds__(kBlock) apply16_tc_kernel(const __grid_constan
 //
 // What bounds it: the serial chain of a tile (load, split, barrier, MMAs,
 // recombination, ~85 instructions per element) over the 4 blocks of an SM that
-// tensor memory allows; issue is about half busy, the FP64 pipe a third (one
-// conversion per output).  Measured on GB300, dense PTMs, us (start of this
+// tensor memory allows; issue is half busy, the FP64 pipe 73 % with one
+// conversion per output (ncu, 12 qubits).  Measured on GB300, dense PTMs, us (start of this
 // design: base-1024 digits, 21 MMAs, two barriers a tile): 13 qubits 349 ->
 // 263 (3.07 -> 4.08 TB/s), 12 qubits 92.7 -> 71.4, 10 qubits 14.3 -> 10.2,
 // last two of 12 qubits 103.8 -> 75.1.  Of the 21 us at 12 qubits, byte digits

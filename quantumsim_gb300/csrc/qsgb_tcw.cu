@@ -52,8 +52,9 @@
 // form of this kernel (base-512 digits, six levels of N = 96 one after another,
 // 256 threads) took 140 us; this one with a level per commit 113 us, and 162 us
 // with its MMAs issued by one thread from rolled loops.  What bounds it now:
-// latency, over 408 small MMAs and ~150 instructions per element on one block
-// of 16 warps; issue is a quarter busy.
+// latency, over 408 small MMAs and ~175 instructions per output on one block
+// of 16 warps; issue is a third busy
+// (ncu, 7 qutrits).
 #include <algorithm>
 
 #include "qsgb_common.cuh"

@@ -256,16 +256,23 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
   // ---- the PTM's digit planes (the B operand), once per block
   int ptm_bad = 0;
   int holes = 0;
+#pragma unroll 3
   for (int r = warp; r < npad; r += kWWarps) {
     unsigned e = 0u, nz = 0u, least = 0x7ffu;
     if (r < p.kout) {
       const int ro = prow[r];
-      for (int k = t & 31; k < p.kin; k += 32) {
-        const double v = p.ptm[ro + pcol[k]];
-        const unsigned ev = exp_of(v);
+      double v[kWMaxK / 32];
+#pragma unroll
+      for (int i = 0; i < kWMaxK / 32; ++i) {  // past the last column: the first one again
+        const int k = (t & 31) + 32 * i;
+        v[i] = p.ptm[ro + pcol[k < p.kin ? k : 0]];
+      }
+#pragma unroll
+      for (int i = 0; i < kWMaxK / 32; ++i) {
+        const unsigned ev = exp_of(v[i]);
         e = max(e, ev);
         least = min(least, ev);
-        nz |= v != 0.0 ? 1u : 0u;
+        nz |= v[i] != 0.0 ? 1u : 0u;
       }
     }
     e = __reduce_max_sync(0xffffffffu, e);
@@ -277,9 +284,12 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
     if (e < kMinExp) e = 1023u;  // any scale serves a row of zeros
     if ((t & 31) == 0) srow[r] = (int)e;
   }
-  __syncthreads();
+  // (the shuffle tells the compiler that the answer is the warp's: without it the
+  // MMAs' operands are not warp-uniform to it, 75 -> 97 us on 7 qutrits)
+  const bool leave = __shfl_sync(0xffffffffu, __syncthreads_or(holes), 0) != 0;
+  if (leave) mark_all<T>(p);
   const int plane_b = p.ksteps * 2 * npad * 16;  // bytes
-  for (int u = t; u < npad * p.ksteps * 2; u += kWBlock) {
+  for (int u = leave ? npad * p.ksteps * 2 : t; u < npad * p.ksteps * 2; u += kWBlock) {
     const int kc = u / npad, r = u - kc * npad;  // 8 columns of row r
     double v[8];
 #pragma unroll
@@ -298,7 +308,6 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   ptm_bad = __syncthreads_or(ptm_bad);
-  holes = __syncthreads_or(holes);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   int rmin = srow[0], rmax = srow[0];  // row scales, least and greatest
   for (int r = 1; r < p.kout; ++r) {
@@ -398,10 +407,6 @@ __global__ void __launch_bounds__(kWBlock, 1) apply_wide_kernel(const __grid_con
 
   constexpr int kGroups = (LV + kWBufs - 1) / kWBufs;  // of levels, per half
   uint32_t group = 0;  // groups issued so far
-  // (the shuffle tells the compiler that the answer is the warp's: without it the
-  // MMAs' operands are not warp-uniform to it, 75 -> 97 us on 7 qutrits)
-  const bool leave = __shfl_sync(0xffffffffu, holes, 0) != 0;
-  if (leave) mark_all<T>(p);
   for (uint64_t tile = leave ? p.n_tiles : blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
     const uint64_t gi = tile * kWGroups + gl;
     const bool live = gi < p.n_groups;

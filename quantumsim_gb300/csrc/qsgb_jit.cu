@@ -251,15 +251,18 @@ std::string gen_source(const Spec& s) {
     fallback.insert(at, store);
   }
   src += "#define QH(v) __int_as_float(__double2hiint(v))\n#define QL(v) __int_as_float(__double2loint(v))\n";
-  // vector loads / stores along the less significant target when Z == 1
+  // vector loads / stores along the less significant target when Z == 1; the
+  // loads are volatile, which keeps them behind the wait for the preceding kernel
+  // (with their addresses from a pointer passed through an asm behind it, an FP32
+  // pass of a fused PTM on the last two of 13 qubits took 105 us instead of 92)
   {
     const char* ty = f32 ? "f32" : "f64";
     const char* cs = f32 ? "f" : "d";
     std::snprintf(buf, sizeof buf,
                   "__device__ __forceinline__ void qld2(const %s* q, %s& a, %s& b) {\n"
-                  "  asm(\"ld.global.v2.%s {%%0,%%1}, [%%2];\" : \"=%s\"(a), \"=%s\"(b) : \"l\"(q)); }\n"
+                  "  asm volatile(\"ld.global.v2.%s {%%0,%%1}, [%%2];\" : \"=%s\"(a), \"=%s\"(b) : \"l\"(q)); }\n"
                   "__device__ __forceinline__ void qld4(const %s* q, %s& a, %s& b, %s& c, %s& d) {\n"
-                  "  asm(\"ld.global.v4.%s {%%0,%%1,%%2,%%3}, [%%4];\" : \"=%s\"(a), \"=%s\"(b), \"=%s\"(c), "
+                  "  asm volatile(\"ld.global.v4.%s {%%0,%%1,%%2,%%3}, [%%4];\" : \"=%s\"(a), \"=%s\"(b), \"=%s\"(c), "
                   "\"=%s\"(d) : \"l\"(q)); }\n"
                   "__device__ __forceinline__ void qst2(%s* q, %s a, %s b) {\n"
                   "  asm volatile(\"st.global.v2.%s [%%0], {%%1,%%2};\" :: \"l\"(q), \"%s\"(a), \"%s\"(b) : \"memory\"); }\n"
@@ -434,7 +437,7 @@ std::string gen_source(const Spec& s) {
         src += buf;
         vars += ", x" + std::to_string(k0 + j);
       }
-      std::snprintf(buf, sizeof buf, "    qld%d(in + bi + %dLL * p.h.sai + %d%s);\n", s.vin,
+      std::snprintf(buf, sizeof buf, "    qld%d((const V*)p.h.in + bi + %dLL * p.h.sai + %d%s);\n", s.vin,
                     k0 / s.db_in, k0 % s.db_in, vars.c_str());
       src += buf;
     } else {
@@ -1085,7 +1088,11 @@ int launch_blob(cudaKernel_t kern, const Spec& s, const Geometry& g, unsigned ch
   // qubits 45 / 49, 9 61 / 67, 11 323 / 335 (fused 155 / 160), 12 1574 / 1583
   // (fused 698 / 692), 13 6540 / 6504; the line lies between 11 and 12.
   const uint64_t bytes = (uint64_t)g.n_items * (s.pair ? 2 : 1) * (uint64_t)(s.kin + s.kout) * (s.f32 ? 4 : 8);
-  const bool overlap = s.f32 || bytes <= (64ull << 20);
+  // Nor does it suit a grid cut to exactly the resident blocks (16 per SM), whose
+  // threads take one or two items: one-qubit FP32 passes on 11 qubits 5.0 / 4.75,
+  // on the last one 5.6 / 5.15.
+  const bool cut = need > cap && resident_blocks((const void*)kern, (int)block, 0) == 16;
+  const bool overlap = (s.f32 || bytes <= (64ull << 20)) && !cut;
   return launch_pdl((const void*)kern, grid, dim3(block), 0, stream, args, overlap);
 }
 

@@ -82,6 +82,9 @@ def test_generated_kernels_pass_their_pointer_through_the_wait():
         text = f.read()
     waits = [m.end() for m in re.finditer(r'qsgb_pdl_wait\(\);', text)]
     assert len(waits) == text.count('"extern \\"C\\" __global__') + 1 == 3
+    # the vector loads of a group stay behind the wait as volatile asm
+    loads = re.findall(r'asm(?: volatile)?\(\\"ld\.global', text)
+    assert len(loads) == 2 and all('volatile' in x for x in loads)
     for w in waits:
         assert text[w:].startswith(
             '\\n  asm volatile(\\"\\" : \\"+l\\"(in));')

@@ -73,7 +73,7 @@ int resident_blocks(const void* func, int threads, size_t smem) {
 // layers of 10 qubits 147 / 126.
 static bool placed_well(const void* func, dim3 grid, dim3 block, size_t smem) {
   const uint64_t blocks = (uint64_t)grid.x * grid.y * grid.z, sms = (uint64_t)sm_count();
-  if (2 * blocks <= sms || blocks >= 32 * sms) return true;
+  if (blocks <= sms || blocks >= 32 * sms) return true;  // no look-up for the smallest calls
   const uint64_t full = sms * (uint64_t)resident_blocks(func, (int)(block.x * block.y * block.z), smem);
   return 2 * blocks <= full || blocks >= full;
 }

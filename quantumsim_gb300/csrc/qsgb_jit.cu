@@ -1090,9 +1090,11 @@ int launch_blob(cudaKernel_t kern, const Spec& s, const Geometry& g, unsigned ch
   const uint64_t bytes = (uint64_t)g.n_items * (s.pair ? 2 : 1) * (uint64_t)(s.kin + s.kout) * (s.f32 ? 4 : 8);
   // Nor does it suit a grid cut to exactly the resident blocks (16 per SM), whose
   // threads take one or two items: one-qubit FP32 passes on 11 qubits 5.0 / 4.75,
-  // on the last one 5.6 / 5.15.
-  const bool cut = need > cap && resident_blocks((const void*)kern, (int)block, 0) == 16;
-  const bool overlap = (s.f32 || bytes <= (64ull << 20)) && !cut;
+  // on the last one 5.6 / 5.15.  On larger vectors they take many (12 qubits 23.1 /
+  // 23.2 alone, the 13-qubit layer 1630 / 1672 with them).
+  const bool small = bytes <= (64ull << 20);
+  const bool cut = small && need > cap && resident_blocks((const void*)kern, (int)block, 0) == 16;
+  const bool overlap = (s.f32 || small) && !cut;
   return launch_pdl((const void*)kern, grid, dim3(block), 0, stream, args, overlap);
 }
 

@@ -840,7 +840,7 @@ int launch_apply(ApplyParams& p, cudaStream_t stream) {
     if (st != QSGB_OK) return st;
   }
   const int occ = resident_blocks((const void*)kern, kBlock, L.total);
-  if (occ < 1) return QSGB_ERR_UNSUPPORTED;
+  if (occ < 1) return QSGB_ERR_CUDA;  // the layout fits: the query failed
   const uint64_t tiles = (p.n_items + 32 * iw - 1) / (32 * iw);
   const uint64_t cap = (uint64_t)sm_count() * occ;
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(tiles, cap));

@@ -57,7 +57,7 @@ int resident_blocks(const void* func, int threads, size_t smem) {
   if (it != known.end()) return it->second;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, func, threads, smem) != cudaSuccess) {
     cudaGetLastError();
-    n = 0;
+    return 0;  // asked again next time
   }
   known.emplace(key, n);  // as many as there are kernels
   return n;

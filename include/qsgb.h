@@ -49,7 +49,8 @@ extern "C" {
 /* ---- arithmetic of apply_ptm ---- */
 #define QSGB_ARITH_AUTO 0  /* F32 storage -> F32, F64 storage -> rows in DF64
                               or F64, whichever keeps up with memory: every
-                              term of a row keeps at least 47 bits of its own.
+                              term of a row is good to some 45 bits of its own
+                              at least.
                               Dense PTMs go to the tensor cores instead, where
                               inputs and entries are cut to 55 bits below the
                               largest of their group (the inputs of one
